@@ -39,15 +39,30 @@ __device__ __forceinline__ bool keep_entry(double m, double threshold) {
 // truncation tile).  Every atomic deposit also ORs its sector's bit into the
 // `dirty` bitmap; the fold visits only dirty sectors, clears their bits and
 // records them in the `touched` bitmap (every sector any batch ever scored).
-// The sums are never cleared in bulk: a sector's first fold writes all four of
-// its entries (d or +0.0), and finalize / truncation read touched sectors
-// only.  0.0 + d == d, so a first write equals the reference's s += d.
+// The sums of a Dij are never cleared in bulk: a sector's first fold writes all
+// four of its entries (d or +0.0), and finalize / truncation read touched
+// sectors only.  0.0 + d == d, so a first write equals the reference's s += d.
 constexpr int kSectorEntries = 4;
 constexpr int kWordEntries = 128;
 static_assert(kTileVoxels == 32 * kWordEntries, "one bitmap word per lane of a tile's warp");
 
 __device__ __forceinline__ void mark_dirty(unsigned int* dirty, long long flat) {
     atomicOr(dirty + (flat >> 7), 1u << ((unsigned)(flat >> 2) & 31u));
+}
+
+// Position of set bit number n (from 0) of w; some position for n >= popc(w).
+// Five popcounts: the library's __fns is a loop over the bits.
+__device__ __forceinline__ int nth_set_bit(unsigned int w, int n) {
+    int pos = 0;
+#pragma unroll
+    for (int step = 16; step >= 1; step >>= 1) {
+        const int below = __popc((w >> pos) & ((1u << step) - 1u));
+        if (below <= n) {
+            n -= below;
+            pos += step;
+        }
+    }
+    return pos & 31;
 }
 
 // One warp holds the 32 bitmap words of a tile (word j in lane j); lane order
@@ -64,7 +79,7 @@ __device__ __forceinline__ int nth_set_sector(unsigned int w, int incl, int k, i
     }
     const unsigned int wj = __shfl_sync(0xffffffffu, w, j);
     const int before = __shfl_sync(0xffffffffu, incl, j) - __popc(wj);
-    bit = (int)__fns(wj, 0u, k - before + 1);
+    bit = nth_set_bit(wj, k - before);
     return j;
 }
 
@@ -78,31 +93,90 @@ __device__ __forceinline__ int warp_inclusive_scan(int v) {
     return v;
 }
 
-// Fold one batch's quanta into the running sums and consume them (reset the
-// folded entries): d = q * 1e-9 / (mass * n), s1 += d, s2 += d^2
-// (kernels.py:804-852).  One warp per (column, tile), dirty sectors only.
+// The four entries of one sector as two 16-byte halves (sectors are 32-byte
+// aligned: the column stride is a multiple of kTileVoxels).
+struct SectorD {
+    double v[kSectorEntries];
+    __device__ __forceinline__ void load(const double* p) {
+        const double2 lo = reinterpret_cast<const double2*>(p)[0], hi = reinterpret_cast<const double2*>(p)[1];
+        v[0] = lo.x; v[1] = lo.y; v[2] = hi.x; v[3] = hi.y;
+    }
+    __device__ __forceinline__ void store(double* p) const {
+        reinterpret_cast<double2*>(p)[0] = make_double2(v[0], v[1]);
+        reinterpret_cast<double2*>(p)[1] = make_double2(v[2], v[3]);
+    }
+};
+
+// mean = S1/n, sigma = sqrt(max(0, S2/n - mean^2) * n / (n - 1) / n) of one entry, in place.
+__device__ __forceinline__ void finalize_entry(double& x, double& y, double n, int n_batches) {
+    if (x == 0.0 && y == 0.0) return;  // mean and sigma are already +0.0
+    const double mean = __ddiv_rn(x, n);
+    double sigma = 0.0;
+    if (n_batches > 1) {
+        double var = __dsub_rn(__ddiv_rn(y, n), __dmul_rn(mean, mean));
+        var = var > 0.0 ? var : 0.0;
+        var = __ddiv_rn(__dmul_rn(var, n), n - 1.0);
+        sigma = __dsqrt_rn(__ddiv_rn(var, n));
+    }
+    x = mean;
+    y = sigma;
+}
+
+__device__ __forceinline__ void column_max(unsigned long long best, unsigned long long* col_max_bits) {
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) {
+        const unsigned long long o = __shfl_xor_sync(0xffffffffu, best, off);
+        best = o > best ? o : best;
+    }
+    if ((threadIdx.x & 31) == 0 && best) atomicMax(col_max_bits, best);
+}
+
+// The part of the sector bitmaps one warp walks: `words` consecutive words (1 to
+// 32, dividing a tile's 32) of one column, one per lane.
+struct FoldShape {
+    long long n_vox, stride;  // voxels and entries of a column
+    int words;                // bitmap words per warp
+    int parts_per_col;        // warps per column
+    long long n_parts;        // warps in all
+    int n_maps;               // quanta maps of the wave, in batch order
+    long long map_entries;    // entries of one map
+};
+
+// Fold a wave's quanta maps, batch by batch, into the running sums and consume
+// them (reset the folded entries): d = q * 1e-9 / (mass * n), s1 += d, s2 += d^2
+// (kernels.py:804-852).  A lane owns one dirty sector: its mass, sums and quanta
+// are read with 16-byte loads and every batch of the wave is added in registers,
+// so the sums cross memory once per wave instead of once per batch.  kFinal: the
+// wave holds every batch of the run, so every touched sector is dirty here and
+// the mean, sigma and column maximum are written at once (finalize_sparse_kernel
+// otherwise).  What bounds it: the latency of the scattered 32-byte sectors.  A
+// warp walks as few bitmap words as leaves the GPU enough warps (fold_words): on
+// a 16^3 map one warp walking the whole map took 88 us a batch, all latency.
+template <bool kFinal>
 __global__ void __launch_bounds__(kReduceThreads)
 fold_sparse_kernel(unsigned long long* __restrict__ edep, const double* __restrict__ mass,
-                   const double* __restrict__ col_nhist, long long n_vox, long long stride,
-                   int tiles_per_col, long long n_tiles, double* __restrict__ s1,
+                   const double* __restrict__ col_nhist, FoldShape f, double* __restrict__ s1,
                    double* __restrict__ s2, unsigned int* __restrict__ dirty,
-                   unsigned int* __restrict__ touched, unsigned long long* __restrict__ total_q) {
+                   unsigned int* __restrict__ touched, int n_batches,
+                   unsigned long long* __restrict__ col_max_bits, unsigned long long* __restrict__ total_q) {
     const int lane = threadIdx.x & 31;
     const long long t = (long long)blockIdx.x * (kReduceThreads / 32) + (threadIdx.x >> 5);
-    if (t >= n_tiles) return;  // warp-uniform
-    const long long widx = t * 32 + lane;
-    const unsigned int w = dirty[widx];
+    if (t >= f.n_parts) return;  // warp-uniform
+    const long long col = t / f.parts_per_col;
+    const long long word0 = (t - col * f.parts_per_col) * f.words;  // in the column
+    const long long widx = col * (f.stride / kWordEntries) + word0 + lane;
+    const long long map_words = f.map_entries / kWordEntries;
+    const bool mine = lane < f.words;
+    unsigned int w = 0u;
+    for (int m = 0; m < f.n_maps; ++m)
+        if (mine) w |= dirty[m * map_words + widx];
     if (__ballot_sync(0xffffffffu, w != 0u) == 0u) return;
-    const unsigned int tw = touched[widx];
+    const unsigned int tw = mine ? touched[widx] : 0u;
     const int incl = warp_inclusive_scan(__popc(w));
     const int total = __shfl_sync(0xffffffffu, incl, 31);
-    const long long col = t / tiles_per_col;
-    const long long tile_v0 = (t - col * tiles_per_col) * (long long)kTileVoxels;
     const double nh = col_nhist[col];
-    unsigned long long* q_col = edep + col * stride;
-    double* a = s1 + col * stride;
-    double* b = s2 + col * stride;
-    unsigned long long local = 0;
+    const double n = (double)n_batches;
+    unsigned long long local = 0, best = 0;
     for (int k0 = 0; k0 < total; k0 += 32) {
         const int k = k0 + lane;
         int bit;
@@ -110,61 +184,73 @@ fold_sparse_kernel(unsigned long long* __restrict__ edep, const double* __restri
         const unsigned int twj = __shfl_sync(0xffffffffu, tw, j);
         if (k >= total) continue;
         const bool first = ((twj >> bit) & 1u) == 0u;
-        const long long v0 = tile_v0 + (long long)j * kWordEntries + bit * kSectorEntries;
+        const long long v0 = (word0 + j) * kWordEntries + bit * kSectorEntries;
+        const long long at = col * f.stride + v0;
+        SectorD a, b;
+        double m_nh[kSectorEntries];
 #pragma unroll
         for (int e = 0; e < kSectorEntries; ++e) {
-            const long long v = v0 + e;
-            if (v >= n_vox) break;
-            const unsigned long long q = q_col[v];
-            if (q != 0ull) {
-                q_col[v] = 0ull;
-                const double m = mass[v];
+            const double m = v0 + e < f.n_vox ? mass[v0 + e] : 0.0;
+            m_nh[e] = m > 0.0 ? __dmul_rn(m, nh) : 0.0;
+            a.v[e] = b.v[e] = 0.0;
+        }
+        if (!first) {
+            a.load(s1 + at);
+            b.load(s2 + at);
+        }
+#pragma unroll 4
+        for (int m = 0; m < f.n_maps; ++m) {
+            ulonglong2* q = reinterpret_cast<ulonglong2*>(edep + m * f.map_entries + at);
+            const ulonglong2 lo = q[0], hi = q[1];
+            const unsigned long long qe[kSectorEntries] = {lo.x, lo.y, hi.x, hi.y};
+            if ((lo.x | lo.y | hi.x | hi.y) == 0ull) continue;
+            q[0] = q[1] = make_ulonglong2(0ull, 0ull);
+#pragma unroll
+            for (int e = 0; e < kSectorEntries; ++e) {
+                if (qe[e] == 0ull) continue;
                 double d = 0.0;
-                if (m > 0.0) {
-                    const double energy = __dmul_rn((double)(long long)q, kQuantum);
-                    d = __ddiv_rn(energy, __dmul_rn(m, nh));
-                }
-                if (first) {
-                    a[v] = d;
-                    b[v] = __dmul_rn(d, d);
-                } else {
-                    a[v] = __dadd_rn(a[v], d);
-                    b[v] = __dadd_rn(b[v], __dmul_rn(d, d));
-                }
-                local += q;
-            } else if (first) {
-                a[v] = 0.0;
-                b[v] = 0.0;
+                if (m_nh[e] > 0.0) d = __ddiv_rn(__dmul_rn((double)(long long)qe[e], kQuantum), m_nh[e]);
+                a.v[e] = __dadd_rn(a.v[e], d);
+                b.v[e] = __dadd_rn(b.v[e], __dmul_rn(d, d));
+                local += qe[e];
             }
         }
+        if constexpr (kFinal) {
+#pragma unroll
+            for (int e = 0; e < kSectorEntries; ++e) {
+                finalize_entry(a.v[e], b.v[e], n, n_batches);
+                const unsigned long long bits = (unsigned long long)__double_as_longlong(a.v[e]);
+                best = bits > best ? bits : best;  // mean >= 0: bit order is value order
+            }
+        }
+        a.store(s1 + at);
+        b.store(s2 + at);
     }
     if (w != 0u) {
-        dirty[widx] = 0u;
+        for (int m = 0; m < f.n_maps; ++m) dirty[m * map_words + widx] = 0u;
         touched[widx] = tw | w;
     }
+    if constexpr (kFinal) column_max(best, col_max_bits + col);
     local = warp_sum_u64(local);
     if (lane == 0 && local) atomicAdd(total_q, local);
 }
 
-// mean = S1/n, sigma = sqrt(max(0, S2/n - mean^2) * n / (n - 1) / n), written in
-// place over the touched sectors; the column maximum of the mean rides along
-// (one atomic per warp).  One warp per (column, tile).
+// Mean and sigma of the touched sectors, in place, with the column maximum of
+// the mean (one atomic per warp).
 __global__ void __launch_bounds__(kReduceThreads)
-finalize_sparse_kernel(double* __restrict__ s1, double* __restrict__ s2, long long n_vox,
-                       long long stride, int tiles_per_col, long long n_tiles, int n_batches,
+finalize_sparse_kernel(double* __restrict__ s1, double* __restrict__ s2, FoldShape f, int n_batches,
                        const unsigned int* __restrict__ touched,
                        unsigned long long* __restrict__ col_max_bits) {
     const int lane = threadIdx.x & 31;
     const long long t = (long long)blockIdx.x * (kReduceThreads / 32) + (threadIdx.x >> 5);
-    if (t >= n_tiles) return;
-    const unsigned int w = touched[t * 32 + lane];
+    if (t >= f.n_parts) return;
+    const long long col = t / f.parts_per_col;
+    const long long word0 = (t - col * f.parts_per_col) * f.words;
+    const unsigned int w =
+        lane < f.words ? touched[col * (f.stride / kWordEntries) + word0 + lane] : 0u;
     if (__ballot_sync(0xffffffffu, w != 0u) == 0u) return;
     const int incl = warp_inclusive_scan(__popc(w));
     const int total = __shfl_sync(0xffffffffu, incl, 31);
-    const long long col = t / tiles_per_col;
-    const long long tile_v0 = (t - col * tiles_per_col) * (long long)kTileVoxels;
-    double* a = s1 + col * stride;
-    double* b = s2 + col * stride;
     const double n = (double)n_batches;
     unsigned long long best = 0ull;
     for (int k0 = 0; k0 < total; k0 += 32) {
@@ -172,34 +258,20 @@ finalize_sparse_kernel(double* __restrict__ s1, double* __restrict__ s2, long lo
         int bit;
         const int j = nth_set_sector(w, incl, k, bit);
         if (k >= total) continue;
-        const long long v0 = tile_v0 + (long long)j * kWordEntries + bit * kSectorEntries;
+        const long long at = col * f.stride + (word0 + j) * kWordEntries + bit * kSectorEntries;
+        SectorD a, b;
+        a.load(s1 + at);
+        b.load(s2 + at);
 #pragma unroll
         for (int e = 0; e < kSectorEntries; ++e) {
-            const long long v = v0 + e;
-            if (v >= n_vox) break;
-            const double x = a[v];
-            const double y = b[v];
-            if (x == 0.0 && y == 0.0) continue;  // mean and sigma are already +0.0
-            const double mean = __ddiv_rn(x, n);
-            double sigma = 0.0;
-            if (n_batches > 1) {
-                double var = __dsub_rn(__ddiv_rn(y, n), __dmul_rn(mean, mean));
-                var = var > 0.0 ? var : 0.0;
-                var = __ddiv_rn(__dmul_rn(var, n), n - 1.0);
-                sigma = __dsqrt_rn(__ddiv_rn(var, n));
-            }
-            a[v] = mean;
-            b[v] = sigma;
-            const unsigned long long bits = (unsigned long long)__double_as_longlong(mean);
-            best = bits > best ? bits : best;  // mean >= 0: bit order is value order
+            finalize_entry(a.v[e], b.v[e], n, n_batches);
+            const unsigned long long bits = (unsigned long long)__double_as_longlong(a.v[e]);
+            best = bits > best ? bits : best;
         }
+        a.store(s1 + at);
+        b.store(s2 + at);
     }
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) {
-        const unsigned long long o = __shfl_xor_sync(0xffffffffu, best, off);
-        best = o > best ? o : best;
-    }
-    if (lane == 0 && best) atomicMax(col_max_bits + col, best);
+    column_max(best, col_max_bits + col);
 }
 
 // Kept entries of the touched sectors of one (column, tile); one warp each.

@@ -85,7 +85,7 @@ struct pmc_engine {
     size_t gs_cap = 0;
 
     // transport buffers
-    DevBuf q[4];
+    DevBuf queues;                // P0, P1, E0, E1, q_capacity slots each
     unsigned int q_capacity = 0;
     DevBuf edep, s1, s2;          // [columns][col_stride] quanta and float64 sums
     DevBuf dirty, touched;        // sector bitmaps of edep / of the sums (pmc_reduce.cuh)
@@ -115,7 +115,7 @@ struct pmc_engine {
 
     pmc_counters counters{};
     cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};
-    std::vector<cudaEvent_t> batch_ev;  // three per batch of a group, read once per group
+    std::vector<cudaEvent_t> batch_ev;  // three per wave of a group, read once per group
     unsigned long long h2d_bytes = 0;  // cumulative over the engine's life
     unsigned long long d2h_bytes = 0;
     pmc_progress_fn progress = nullptr;
@@ -404,13 +404,35 @@ int check_flags(pmc_engine* e, const Sched& s) {
 struct RunPlan {
     LaunchShape shape;
     unsigned long long budget = 0;
+    int wave = 1;  // batches transported together, each into its own quanta map
     long long max_steps = 0;
     int tail_steps = 0;
 };
 
-// max_block: the most primaries one batch block of this call holds; admission
-// never needs more than that per round.
-int prepare_transport(pmc_engine* e, const pmc_run_params* p, unsigned long long max_block,
+long long stride_for(long long n_vox) {
+    return (n_vox + kTileVoxels - 1) / kTileVoxels * kTileVoxels;
+}
+
+// Quanta maps of a wave: at most this many bytes beyond the one map every run
+// needs (a twentieth of the GPU's memory; 4 further maps of a 128^3 Dij of 100
+// columns).
+constexpr double kWaveBytes = 8.0 * 1024 * 1024 * 1024;
+
+// block: the primaries of one batch; cols: the most columns of a group;
+// waves: whether batches may share a wave.
+//
+// A batch is transported in a few rounds, and a round lasts at least as long as
+// its longest electron (some 100 substeps one after another, ~0.1 ms) however few
+// particles it holds.  Batches are independent until they are folded, so a wave
+// of them shares the rounds, each scoring into a quanta map of its own, and the
+// fold adds the maps in batch order: the same numbers with the rounds of one
+// batch.  A wave holds up to four admission windows (16 primaries per resident
+// thread each); past that the last rounds no longer show.  Measured, ten batches:
+// a 16^3 run of 80,000 histories 6.25 -> 1.01 ms, a 64^3 field of 1e6 10.8 ->
+// 3.2 ms, a 35-column Dij of 1.4e6 9.5 -> 4.2 ms, the 100-column 128^3 Dij of
+// 1.9e7 (two waves) 39.4 -> 35.6 ms; admission windows of 8 and 4 primaries per
+// thread are slower there (37.6 and 41.8 ms).
+int prepare_transport(pmc_engine* e, const pmc_run_params* p, unsigned long long block, int cols, bool waves,
                       RunPlan* plan) {
     if (!e->has_grid) return fail(e, PMC_ERR_STATE, "no transport grid uploaded");
     if (!e->has_tables) return fail(e, PMC_ERR_STATE, "no cross-section tables uploaded");
@@ -424,18 +446,26 @@ int prepare_transport(pmc_engine* e, const pmc_run_params* p, unsigned long long
     if (rc) return rc;
     const unsigned long long resident =
         (unsigned long long)std::max(plan->shape.grid_ph, plan->shape.grid_el) * plan->shape.block;
+    if (waves) {
+        const double map_bytes = sizeof(double) * (double)stride_for(e->si.n_voxels) * std::max(cols, 1);
+        const double by_memory = std::floor(kWaveBytes / map_bytes) + 1.0;
+        const unsigned long long by_work = std::max(1ull, 64ull * resident / std::max(1ull, block));
+        const int most = (int)std::min((double)std::min<unsigned long long>(by_work, p->n_batches), by_memory);
+        const int n_waves = (p->n_batches + most - 1) / most;
+        plan->wave = (p->n_batches + n_waves - 1) / n_waves;  // waves of about the same size
+    }
+    // admission never needs more than a wave's primaries per round
     plan->budget = p->chunk_size > 0 ? (unsigned long long)p->chunk_size : 16ull * resident;
-    plan->budget = std::max(1ull, std::min(plan->budget, max_block));
+    plan->budget = std::max(1ull, std::min(plan->budget, block * (unsigned long long)plan->wave));
     const int qf = p->queue_factor > 0 ? p->queue_factor : 16;
     const unsigned long long cap64 = plan->budget * (unsigned long long)qf;
     if (cap64 > 0x7fffffffull)
         return fail(e, PMC_ERR_INVALID, "chunk_size * queue_factor exceeds the queue index range");
     const unsigned int cap = (unsigned int)cap64;
     if (cap > e->q_capacity) {
-        for (int i = 0; i < 4; ++i) {
-            rc = ensure(e, e->q[i], (size_t)cap * sizeof(Slot));
-            if (rc) return rc;
-        }
+        e->q_capacity = 0;  // (a failed call leaves no queue behind)
+        rc = ensure(e, e->queues, 4 * (size_t)cap * sizeof(Slot));
+        if (rc) return rc;
         e->q_capacity = cap;
     }
     plan->max_steps = p->max_steps > 0 ? p->max_steps : kDefaultMaxSteps;
@@ -452,7 +482,7 @@ TransportParams make_params(pmc_engine* e, const pmc_run_params* p, const RunPla
     P.cyl = e->cyl;
     P.vox = e->d_vox;
     P.tab = e->tab;
-    for (int i = 0; i < 4; ++i) P.q[i] = (Slot*)e->q[i].p;
+    for (int i = 0; i < 4; ++i) P.q[i] = (Slot*)e->queues.p + (size_t)i * e->q_capacity;
     P.capacity = e->q_capacity;
     P.sched = e->d_sched;
     P.gen = e->d_gen;
@@ -475,9 +505,10 @@ TransportParams make_params(pmc_engine* e, const pmc_run_params* p, const RunPla
     return P;
 }
 
-// Transport one statistical batch of the current group into e->edep.
-int run_batch(pmc_engine* e, const pmc_run_params* p, const RunPlan& plan, TransportParams& P,
-              int batch, unsigned long long block) {
+// Transport a wave of statistical batches (`batch` the first, `block` primaries
+// in all) of the current group into e->edep.
+int run_wave(pmc_engine* e, const pmc_run_params* p, const RunPlan& plan, TransportParams& P,
+             int batch, unsigned long long block) {
     if (block == 0) return PMC_OK;
     const bool graph = p->use_graph != 0;
     if (graph) {
@@ -521,44 +552,60 @@ int run_batch(pmc_engine* e, const pmc_run_params* p, const RunPlan& plan, Trans
     return PMC_OK;
 }
 
-long long stride_for(long long n_vox) {
-    return (n_vox + kTileVoxels - 1) / kTileVoxels * kTileVoxels;
+int reduce_blocks(long long n_warps) {
+    return (int)((n_warps + kReduceThreads / 32 - 1) / (kReduceThreads / 32));
 }
 
-int reduce_blocks(long long n_tiles) {
-    return (int)((n_tiles + kReduceThreads / 32 - 1) / (kReduceThreads / 32));
+// Bitmap words per warp of the fold and finalize: a whole tile's 32 while that
+// still leaves 32 warps per SM, fewer (down to one) on smaller maps, where the
+// longest warp's chain of sectors is the kernel's time.
+FoldShape fold_shape(const pmc_engine* e, long long n_vox, int group, int n_maps) {
+    FoldShape f{};
+    f.n_vox = n_vox;
+    f.stride = e->col_stride;
+    f.n_maps = n_maps;
+    f.map_entries = e->col_stride * group;
+    const long long words = f.map_entries / kWordEntries;
+    f.words = 32;
+    while (f.words > 1 && words / f.words < 32ll * e->sm_count) f.words /= 2;
+    f.parts_per_col = (int)(e->col_stride / kWordEntries / f.words);
+    f.n_parts = (long long)f.parts_per_col * group;
+    return f;
 }
 
-int launch_fold(pmc_engine* e, long long n_vox, int group, const double* d_col_nhist) {
-    const int tpc = (int)(e->col_stride / kTileVoxels);
-    const long long n_tiles = (long long)tpc * group;
-    fold_sparse_kernel<<<reduce_blocks(n_tiles), kReduceThreads, 0, e->stream>>>(
-        (unsigned long long*)e->edep.p, e->d_mass, d_col_nhist, n_vox, e->col_stride, tpc, n_tiles,
-        (double*)e->s1.p, (double*)e->s2.p, (unsigned int*)e->dirty.p,
-        (unsigned int*)e->touched.p, e->d_total_q);
+// Fold the n_maps quanta maps of a wave; `last`: they hold every batch of the
+// run, so the statistics are finalized in the same pass (launch_finalize not
+// called; d_colmax cleared by the caller).
+int launch_fold(pmc_engine* e, long long n_vox, int group, const double* d_col_nhist, int n_maps,
+                int n_batches, bool last) {
+    const FoldShape f = fold_shape(e, n_vox, group, n_maps);
+    auto kernel = last ? fold_sparse_kernel<true> : fold_sparse_kernel<false>;
+    kernel<<<reduce_blocks(f.n_parts), kReduceThreads, 0, e->stream>>>(
+        (unsigned long long*)e->edep.p, e->d_mass, d_col_nhist, f, (double*)e->s1.p, (double*)e->s2.p,
+        (unsigned int*)e->dirty.p, (unsigned int*)e->touched.p, n_batches, e->d_colmax, e->d_total_q);
     PMC_CUDA(e, cudaGetLastError());
     e->counters.reduce_launches += 1;
     return PMC_OK;
 }
 
-int ensure_colmax(pmc_engine* e, int group) {
+int clear_colmax(pmc_engine* e, int group) {
     if (group > e->colmax_len) {
         if (e->d_colmax) cudaFree(e->d_colmax);
+        e->d_colmax = nullptr;
+        e->colmax_len = 0;
         PMC_CUDA(e, cudaMalloc(&e->d_colmax, sizeof(unsigned long long) * group));
         e->colmax_len = group;
     }
+    PMC_CUDA(e, cudaMemsetAsync(e->d_colmax, 0, sizeof(unsigned long long) * group, e->stream));
     return PMC_OK;
 }
 
 int launch_finalize(pmc_engine* e, long long n_vox, int group, int n_batches) {
-    int rc = ensure_colmax(e, group);
+    int rc = clear_colmax(e, group);
     if (rc) return rc;
-    PMC_CUDA(e, cudaMemsetAsync(e->d_colmax, 0, sizeof(unsigned long long) * group, e->stream));
-    const int tpc = (int)(e->col_stride / kTileVoxels);
-    const long long n_tiles = (long long)tpc * group;
-    finalize_sparse_kernel<<<reduce_blocks(n_tiles), kReduceThreads, 0, e->stream>>>(
-        (double*)e->s1.p, (double*)e->s2.p, n_vox, e->col_stride, tpc, n_tiles, n_batches,
-        (const unsigned int*)e->touched.p, e->d_colmax);
+    const FoldShape f = fold_shape(e, n_vox, group, 1);
+    finalize_sparse_kernel<<<reduce_blocks(f.n_parts), kReduceThreads, 0, e->stream>>>(
+        (double*)e->s1.p, (double*)e->s2.p, f, n_batches, (const unsigned int*)e->touched.p, e->d_colmax);
     PMC_CUDA(e, cudaGetLastError());
     e->counters.reduce_launches += 1;
     return PMC_OK;
@@ -633,29 +680,41 @@ int truncate_compact(pmc_engine* e, long long n_vox, int group, double truncatio
 }
 
 // The [group][stride] maps and their bitmaps, sized for `group` columns of
-// `n_vox` entries.  A freshly allocated quanta map is not yet zero.
-int ensure_maps(pmc_engine* e, int group, long long n_vox) {
+// `n_vox` voxels and `wave` quanta maps (and the dirty bitmaps that go with them).
+int ensure_maps(pmc_engine* e, int group, long long n_vox, int wave = 1) {
     e->col_stride = stride_for(n_vox);
     const long long n = e->col_stride * group;
-    if (e->edep.bytes < sizeof(double) * (size_t)n) e->edep_clean = false;
-    int rc = ensure(e, e->edep, sizeof(double) * (size_t)n);
+    if (e->edep.bytes < sizeof(double) * (size_t)n * wave) e->edep_clean = false;
+    int rc = ensure(e, e->edep, sizeof(double) * (size_t)n * wave);
     if (!rc) rc = ensure(e, e->s1, sizeof(double) * (size_t)n);
     if (!rc) rc = ensure(e, e->s2, sizeof(double) * (size_t)n);
-    if (!rc) rc = ensure(e, e->dirty, sizeof(unsigned int) * (size_t)(n / kWordEntries));
+    if (!rc) rc = ensure(e, e->dirty, sizeof(unsigned int) * (size_t)(n / kWordEntries) * wave);
     if (!rc) rc = ensure(e, e->touched, sizeof(unsigned int) * (size_t)(n / kWordEntries));
     return rc;
 }
 
+// As ensure_maps for the planned wave, one batch at a time where the device has
+// no room for the wave's maps.
+int ensure_wave_maps(pmc_engine* e, int group, long long n_vox, RunPlan* plan) {
+    int rc = ensure_maps(e, group, n_vox, plan->wave);
+    if (rc == PMC_ERR_OOM && plan->wave > 1) {
+        cudaGetLastError();
+        plan->wave = 1;
+        rc = ensure_maps(e, group, n_vox);
+    }
+    return rc;
+}
+
 // Start scoring `group` columns: quanta all zero (cleared in bulk only after a
-// run that did not complete), both bitmaps empty.  The float64 sums are not
+// run that did not complete), all bitmaps empty.  The float64 sums are not
 // cleared: a sector's first fold writes it whole.
-int begin_maps(pmc_engine* e, int group) {
+int begin_maps(pmc_engine* e, int group, int wave = 1) {
     if (!e->edep_clean) {
         PMC_CUDA(e, cudaMemsetAsync(e->edep.p, 0, e->edep.bytes, e->stream));
         e->edep_clean = true;
     }
     const size_t words = sizeof(unsigned int) * (size_t)(e->col_stride * group / kWordEntries);
-    PMC_CUDA(e, cudaMemsetAsync(e->dirty.p, 0, words, e->stream));
+    PMC_CUDA(e, cudaMemsetAsync(e->dirty.p, 0, words * wave, e->stream));
     PMC_CUDA(e, cudaMemsetAsync(e->touched.p, 0, words, e->stream));
     e->edep_clean = false;  // until every batch of the call has been folded
     return PMC_OK;
@@ -879,7 +938,7 @@ void pmc_destroy(pmc_engine* e) {
     if (e->d_mass) cudaFree(e->d_mass);
     if (e->d_cyl_z) cudaFree(e->d_cyl_z);
     if (e->d_cyl_r2) cudaFree(e->d_cyl_r2);
-    for (DevBuf* b : {&e->q[0], &e->q[1], &e->q[2], &e->q[3], &e->edep, &e->s1, &e->s2,
+    for (DevBuf* b : {&e->queues, &e->edep, &e->s1, &e->s2,
                       &e->tile_counts, &e->tile_offsets, &e->col_counts, &e->out_idx,
                       &e->out_dose, &e->out_sigma, &e->col_nhist, &e->dirty, &e->touched,
                       &e->stage})
@@ -1245,10 +1304,10 @@ int pmc_run_forward(pmc_engine* e, const pmc_source_desc* src, const pmc_run_par
     if (p->n_batches < 1 || p->n_histories % p->n_batches != 0)
         return fail(e, PMC_ERR_INVALID, "n_histories=%lld not divisible by n_batches=%d", (long long)p->n_histories, p->n_batches);
     RunPlan plan;
-    int rc = prepare_transport(e, p, (unsigned long long)(p->n_histories / p->n_batches), &plan);
+    int rc = prepare_transport(e, p, (unsigned long long)(p->n_histories / p->n_batches), 1, true, &plan);
     if (rc) return rc;
     const long long n_vox = e->si.n_voxels;
-    rc = ensure_maps(e, 1, n_vox);
+    rc = ensure_wave_maps(e, 1, n_vox, &plan);
     if (rc) return rc;
     rc = ensure(e, e->col_nhist, sizeof(double));
     if (rc) return rc;
@@ -1260,6 +1319,7 @@ int pmc_run_forward(pmc_engine* e, const pmc_source_desc* src, const pmc_run_par
     G.group = 1;
     G.kind = src->kind;
     G.per_batch_fwd = per_batch;
+    G.wave_block = plan.wave > 1 ? (unsigned long long)per_batch : 0ull;
     G.energy = (float)src->energy;
     std::vector<float> z1(1, 0.0f);
     switch (src->type) {
@@ -1368,23 +1428,25 @@ int pmc_run_forward(pmc_engine* e, const pmc_source_desc* src, const pmc_run_par
 
     rc = reset_counters(e);
     if (rc) return rc;
-    // The whole dense map goes back to the caller: zero sums, every sector
-    // marked touched (the fold then adds into them, finalize visits them all).
-    rc = begin_maps(e, 1);
+    // The whole dense map goes back to the caller: a sector that no batch
+    // scores keeps the zero mean and sigma it starts with.
+    rc = begin_maps(e, 1, plan.wave);
     if (rc) return rc;
     PMC_CUDA(e, cudaMemsetAsync(e->s1.p, 0, sizeof(double) * n_vox, e->stream));
     PMC_CUDA(e, cudaMemsetAsync(e->s2.p, 0, sizeof(double) * n_vox, e->stream));
-    rc = fill_bitmap(e, e->touched, 1, 0xffffffffu);
+    const bool one_wave = plan.wave >= p->n_batches;
+    if (one_wave) rc = clear_colmax(e, 1);
     if (rc) return rc;
     PMC_CUDA(e, cudaMemsetAsync(e->d_total_q, 0, sizeof(unsigned long long), e->stream));
     TransportParams P = make_params(e, p, plan);
     float t_tr = 0.0f, t_red = 0.0f;
-    for (int b = 0; b < p->n_batches; ++b) {
+    for (int b = 0; b < p->n_batches; b += plan.wave) {
+        const int in_wave = std::min(plan.wave, p->n_batches - b);
         PMC_CUDA(e, cudaEventRecord(e->ev[0], e->stream));
-        rc = run_batch(e, p, plan, P, b, (unsigned long long)per_batch);
+        rc = run_wave(e, p, plan, P, b, (unsigned long long)per_batch * in_wave);
         if (rc) return rc;
         PMC_CUDA(e, cudaEventRecord(e->ev[1], e->stream));
-        rc = launch_fold(e, n_vox, 1, (const double*)e->col_nhist.p);
+        rc = launch_fold(e, n_vox, 1, (const double*)e->col_nhist.p, in_wave, p->n_batches, one_wave);
         if (rc) return rc;
         PMC_CUDA(e, cudaEventRecord(e->ev[2], e->stream));
         PMC_CUDA(e, cudaEventSynchronize(e->ev[2]));
@@ -1398,10 +1460,10 @@ int pmc_run_forward(pmc_engine* e, const pmc_source_desc* src, const pmc_run_par
         if (rc) return rc;
         rc = check_flags(e, s);
         if (rc) return rc;
-        if (e->progress) e->progress(e->progress_user, per_batch);
+        for (int k = 0; k < in_wave && e->progress; ++k) e->progress(e->progress_user, per_batch);
     }
     PMC_CUDA(e, cudaEventRecord(e->ev[0], e->stream));
-    rc = launch_finalize(e, n_vox, 1, p->n_batches);
+    if (!one_wave) rc = launch_finalize(e, n_vox, 1, p->n_batches);
     if (rc) return rc;
     PMC_CUDA(e, cudaEventRecord(e->ev[1], e->stream));
     PMC_CUDA(e, cudaMemcpyAsync(dose, e->s1.p, sizeof(double) * n_vox, cudaMemcpyDeviceToHost, e->stream));
@@ -1440,11 +1502,13 @@ int pmc_run_dij(pmc_engine* e, const pmc_beamlet_desc* src, const int64_t* count
     unsigned long long all_block = 0;
     for (int j = 0; j < n_beam; ++j) all_block += (unsigned long long)(counts[j] / p->n_batches);
     RunPlan plan;
-    int rc = prepare_transport(e, p, all_block, &plan);
+    const int all_cols = std::min(n_beam, 4096);
+    const int most_cols = p->beamlet_group_size > 0 ? std::min(n_beam, p->beamlet_group_size) : all_cols;
+    // (host-sampled primaries are uploaded batch by batch: no waves)
+    int rc = prepare_transport(e, p, all_block, most_cols, src->type != PMC_BEAMLET_UPLOAD, &plan);
     if (rc) return rc;
     const long long n_vox = e->si.n_voxels;
     int group = p->beamlet_group_size > 0 ? p->beamlet_group_size : 0;
-    const int all_cols = std::min(n_beam, 4096);
     const size_t all_n = (size_t)stride_for(n_vox) * (size_t)all_cols;
     if (group == 0 && e->edep.bytes >= sizeof(double) * all_n && e->s1.bytes >= sizeof(double) * all_n &&
         e->s2.bytes >= sizeof(double) * all_n && e->dirty.bytes >= sizeof(unsigned int) * (all_n / kWordEntries) &&
@@ -1465,7 +1529,7 @@ int pmc_run_dij(pmc_engine* e, const pmc_beamlet_desc* src, const int64_t* count
         group = std::min(group, std::min(n_beam, 4096));
     }
     group = std::min(group, n_beam);
-    rc = ensure_maps(e, group, n_vox);
+    rc = ensure_wave_maps(e, group, n_vox, &plan);
     if (!rc) rc = ensure(e, e->col_nhist, sizeof(double) * group);
     if (rc) return rc;
     // Every in-kernel beamlet source becomes per-beamlet records; the upload
@@ -1506,6 +1570,7 @@ int pmc_run_dij(pmc_engine* e, const pmc_beamlet_desc* src, const int64_t* count
             off[k] = offset[g0 + k];
             nh[k] = (double)pb[k];
         }
+        G.wave_block = plan.wave > 1 ? (unsigned long long)pre[gs] : 0ull;
         rc = upload_vec(e, pb, &G.per_batch);
         if (!rc) rc = upload_vec(e, pre, &G.pb_prefix);
         if (!rc) rc = upload_vec(e, off, &G.hist_offset);
@@ -1542,14 +1607,18 @@ int pmc_run_dij(pmc_engine* e, const pmc_beamlet_desc* src, const int64_t* count
         PMC_CUDA(e, cudaMemcpyAsync(e->col_nhist.p, nh.data(), sizeof(double) * gs, cudaMemcpyHostToDevice,
                                     e->stream));
     e->h2d_bytes += (unsigned long long)(sizeof(double) * gs);
-        rc = begin_maps(e, gs);
-        if (!rc) rc = ensure_batch_events(e, 3 * (size_t)p->n_batches);
+        const bool one_wave = plan.wave >= p->n_batches;
+        const int n_waves = (p->n_batches + plan.wave - 1) / plan.wave;
+        rc = begin_maps(e, gs, plan.wave);
+        if (!rc && one_wave) rc = clear_colmax(e, gs);
+        if (!rc) rc = ensure_batch_events(e, 3 * (size_t)n_waves);
         if (rc) return rc;
         TransportParams P = make_params(e, p, plan);
-        // every batch is enqueued back to back; its timing events are read
-        // once the group's last batch is done (no host round trip per batch)
-        for (int b = 0; b < p->n_batches; ++b) {
-            cudaEvent_t* bev = e->batch_ev.data() + 3 * b;
+        // every wave is enqueued back to back; its timing events are read
+        // once the group's last wave is done (no host round trip per wave)
+        for (int v = 0; v < n_waves; ++v) {
+            const int b = v * plan.wave, in_wave = std::min(plan.wave, p->n_batches - b);
+            cudaEvent_t* bev = e->batch_ev.data() + 3 * v;
             if (G.type == 3) {  // this batch's primaries, sampled on the host
                 for (int k = 0; k < gs; ++k) {
                     const long long r0 = (long long)b * pb[k];
@@ -1568,16 +1637,16 @@ int pmc_run_dij(pmc_engine* e, const pmc_beamlet_desc* src, const int64_t* count
                 e->h2d_bytes += 32ull * n;
             }
             PMC_CUDA(e, cudaEventRecord(bev[0], e->stream));
-            rc = run_batch(e, p, plan, P, b, (unsigned long long)pre[gs]);
+            rc = run_wave(e, p, plan, P, b, (unsigned long long)pre[gs] * in_wave);
             if (rc) return rc;
             PMC_CUDA(e, cudaEventRecord(bev[1], e->stream));
-            rc = launch_fold(e, n_vox, gs, (const double*)e->col_nhist.p);
+            rc = launch_fold(e, n_vox, gs, (const double*)e->col_nhist.p, in_wave, p->n_batches, one_wave);
             if (rc) return rc;
             PMC_CUDA(e, cudaEventRecord(bev[2], e->stream));
         }
-        PMC_CUDA(e, cudaEventSynchronize(e->batch_ev[3 * (size_t)p->n_batches - 1]));
-        for (int b = 0; b < p->n_batches; ++b) {
-            const cudaEvent_t* bev = e->batch_ev.data() + 3 * b;
+        PMC_CUDA(e, cudaEventSynchronize(e->batch_ev[3 * (size_t)n_waves - 1]));
+        for (int v = 0; v < n_waves; ++v) {
+            const cudaEvent_t* bev = e->batch_ev.data() + 3 * v;
             float a = 0, c = 0;
             cudaEventElapsedTime(&a, bev[0], bev[1]);
             cudaEventElapsedTime(&c, bev[1], bev[2]);
@@ -1595,7 +1664,7 @@ int pmc_run_dij(pmc_engine* e, const pmc_beamlet_desc* src, const int64_t* count
         unsigned long long g_nnz = 0;
         std::vector<long long> g_counts;
         PMC_CUDA(e, cudaEventRecord(e->ev[0], e->stream));
-        rc = launch_finalize(e, n_vox, gs, p->n_batches);
+        if (!one_wave) rc = launch_finalize(e, n_vox, gs, p->n_batches);
         if (rc) return rc;
         PMC_CUDA(e, cudaEventRecord(e->ev[1], e->stream));
         rc = truncate_count(e, n_vox, gs, p->truncation, &g_nnz, &g_counts);
@@ -1718,7 +1787,7 @@ int pmc_reduce_dense(pmc_engine* e, const int64_t* quanta, int32_t n_batches, in
         PMC_CUDA(e, cudaMemcpy2DAsync(e->edep.p, pitch, quanta + (size_t)b * n_cols * n_vox, row, row,
                                       (size_t)n_cols, cudaMemcpyHostToDevice, e->stream));
         rc = fill_bitmap(e, e->dirty, n_cols, 0xffffffffu);
-        if (!rc) rc = launch_fold(e, n_vox, n_cols, (const double*)e->col_nhist.p);
+        if (!rc) rc = launch_fold(e, n_vox, n_cols, (const double*)e->col_nhist.p, 1, n_batches, false);
     }
     if (!rc) rc = launch_finalize(e, n_vox, n_cols, n_batches);
     unsigned long long tq = 0;
@@ -1750,9 +1819,8 @@ int pmc_truncate_dense(pmc_engine* e, const double* mean, const double* sigma, i
     e->h2d_bytes += (unsigned long long)(2 * row * n_cols);
     rc = fill_bitmap(e, e->touched, n_cols, 0xffffffffu);  // a dense map: every sector counts
     if (rc) return rc;
-    rc = ensure_colmax(e, n_cols);
+    rc = clear_colmax(e, n_cols);
     if (rc) return rc;
-    PMC_CUDA(e, cudaMemsetAsync(e->d_colmax, 0, sizeof(unsigned long long) * n_cols, e->stream));
     {
         const int n_tiles = (int)(e->col_stride / kTileVoxels);
         colmax_kernel<<<dim3(n_tiles, n_cols), kReduceThreads, 0, e->stream>>>(

@@ -33,21 +33,21 @@ constexpr int kFlagOverflow = 1;
 constexpr int kFlagStepCap = 2;
 constexpr int kFlagRoundCap = 4;
 
-// Device-resident scheduling state of one drain (one statistical batch).
+// Device-resident scheduling state of one drain (a wave of statistical batches).
 struct Sched {
     int p_in, e_in;                 // input photon / electron queue (0/1)
     unsigned int count[4];          // push counters: P0, P1, E0, E1
     unsigned int head[4];           // fetch heads
-    unsigned long long cursor;      // next primary of the batch block
+    unsigned long long cursor;      // next primary of the wave
     unsigned long long limit;       // admission limit of the current round
-    unsigned long long block_end;   // primaries in the batch block
+    unsigned long long block_end;   // primaries in the wave
     unsigned long long budget;      // primaries admitted per round
     unsigned int blocks_done;
     int flags;
     int remaining;                  // 1 while work is left
-    int batch;
-    long long rounds;               // rounds of the current batch
-    long long total_rounds;         // rounds of the whole call (not reset per batch)
+    int batch;                      // first batch of the wave
+    long long rounds;               // rounds of the current wave
+    long long total_rounds;         // rounds of the whole call (not reset per wave)
     long long max_rounds;
     unsigned long long cond_handle; // CUDA graph conditional handle (0: host loop)
 };
@@ -81,6 +81,7 @@ struct GenDesc {
     float uax, uay, uaz, vax, vay, vaz;  // aperture axes
     float width_u, width_v;
     long long per_batch_fwd;             // forward: histories per batch
+    unsigned long long wave_block;       // primaries of one batch when a wave holds several, else 0
     const long long* pb_prefix;          // [group+1] exclusive prefix of per-batch counts
     const long long* per_batch;          // [group]
     const long long* hist_offset;        // [group] first global history of each beamlet
@@ -142,7 +143,7 @@ struct TransportParams {
     unsigned int capacity;
     Sched* sched;
     const GenDesc* gen;
-    unsigned long long* edep;  // [group][col_stride] int64 quanta
+    unsigned long long* edep;  // [batch of the wave][group][col_stride] int64 quanta
     unsigned int* dirty;       // sector bitmap of edep (pmc_reduce.cuh)
     long long col_stride;      // entries per column: scoring voxels rounded up to a tile
     Counters* counters;
@@ -463,14 +464,21 @@ __device__ inline float stack_transmission(const GenDesc& G, const Particle& p) 
 }
 
 // ---- primary generation (kernels.py:1888-2401) -------------------------------------
-// Maps primary t of the current batch block to its beamlet and history, seeds
-// the history's stream, and samples the primary exactly as the host sources do
+// Maps primary t of the current wave (batches `batch` and up, one block each) to
+// its batch, beamlet and history, seeds the history's stream, and samples the
+// primary exactly as the host sources do
 // (same uniforms, same order).  Returns the particle kind, or -1 when the
 // source emits nothing for this history (a masked fan's zero transmission).
 __device__ inline int generate_primary(const TransportParams& P, const GenDesc& G, int batch,
                                        unsigned long long t, Particle& p, BlockBooks& B) {
     // G is the device-resident descriptor, read field by field as needed.
     int local = 0;
+    int map = 0;  // the wave's quanta map this primary's batch scores into
+    if (G.wave_block) {
+        map = (int)(t / G.wave_block);
+        t -= (unsigned long long)map * G.wave_block;
+        batch += map;
+    }
     long long key;
     long long record;
     if (G.forward) {
@@ -496,7 +504,7 @@ __device__ inline int generate_primary(const TransportParams& P, const GenDesc& 
     p.rng.id_hi = (uint32_t)((unsigned long long)key >> 32);
     p.rng.tag = 0u;
     p.rng.ctr = 0u;
-    p.beamlet = local;
+    p.beamlet = map * G.group + local;
     p.primary = 1;
     p.steps = 0;
     p.w = 1.0f;
