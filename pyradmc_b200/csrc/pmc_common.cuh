@@ -109,6 +109,7 @@ struct Rng {
         ++ctr;
         return r;
     }
+    __device__ inline void reserve(int) {}
     // U[0, 1) with 24-bit resolution: cannot return 1.0 (rng/interface.py:55-61).
     __device__ inline float uniform() { return (float)(next_u32() >> 8) * (1.0f / 16777216.0f); }
     // Child stream for a queued secondary: three parent draws name it, so it is a
@@ -123,6 +124,85 @@ struct Rng {
         return c;
     }
     __device__ inline StreamId state() const { return StreamId{id_lo, id_hi, tag, ctr}; }
+};
+
+// The same stream for a lane of the transport kernels, its next words kept in
+// shared memory: two Philox blocks, word w at ring[(w & 7) * kStride].
+//
+// Lanes of a warp stand at different positions of their streams.  With the
+// block held in registers and refilled by the draw that runs out of it (Rng),
+// nearly every draw of a warp met some lane that had to refill, so the ten
+// rounds ran at a quarter of the lanes, once per draw and inlined at each of
+// some 25 draws.  Here a refill stands only where a branch of the kernel begins
+// (reserve: at most four draws announced at once) and every lane with room
+// joins it; a draw is one shared-memory load.  kStride: the largest block of the
+// kernel (a lane's words lie kStride apart, so a warp's draws never share a bank).
+constexpr int kRingWords = 8;
+
+template <int kStride>
+struct RingRng {
+    uint32_t k0, k1;   // run seed
+    uint32_t id_lo, id_hi, tag;
+    uint32_t ctr;      // uniforms consumed
+    uint32_t end;      // words [ctr, end) are in the ring (end a multiple of 4, end - ctr <= 8)
+    uint32_t* ring;    // this lane's column
+
+    __device__ __forceinline__ void load(const StreamId& s) {
+        id_lo = s.id_lo;
+        id_hi = s.id_hi;
+        tag = s.tag;
+        ctr = s.ctr;
+        end = ctr & ~3u;  // (nothing of the current block is held yet)
+    }
+    // Block `block` of the stream into its half of the ring.
+    __device__ __forceinline__ void fill(uint32_t block) {
+        uint32_t c[4] = {block, id_lo, id_hi, tag};
+        philox4x32_10(c, k0, k1);
+        uint32_t* r = ring + (block & 1u) * (4 * kStride);
+        r[0] = c[0];
+        r[kStride] = c[1];
+        r[2 * kStride] = c[2];
+        r[3 * kStride] = c[3];
+    }
+    // Signed: a stream loaded inside a block starts with end < ctr.
+    __device__ __forceinline__ int held() const { return (int)(end - ctr); }
+    // One more block wherever there is room for it: three words at least are then held.
+    __device__ __forceinline__ void top_up() {
+        if (held() <= 4) {
+            do {
+                fill(end >> 2);
+                end += 4u;
+            } while (held() < 3);
+        }
+    }
+    // Both halves, whatever they held: five words at least are then held.
+    __device__ __forceinline__ void fill_both() {
+        fill(ctr >> 2);
+        fill((ctr >> 2) + 1u);
+        end = (ctr & ~3u) + 8u;
+    }
+    // The next n <= 4 draws are held.
+    __device__ __forceinline__ void reserve(int n) {
+        while (held() < n) {
+            fill(end >> 2);
+            end += 4u;
+        }
+    }
+    __device__ __forceinline__ uint32_t next_u32() {
+        const uint32_t r = ring[(ctr & 7u) * kStride];
+        ++ctr;
+        return r;
+    }
+    __device__ __forceinline__ float uniform() { return (float)(next_u32() >> 8) * (1.0f / 16777216.0f); }
+    __device__ __forceinline__ StreamId spawn() {  // three reserved draws
+        StreamId c;
+        c.id_lo = next_u32();
+        c.id_hi = next_u32();
+        c.tag = next_u32() | 1u;
+        c.ctr = 0u;
+        return c;
+    }
+    __device__ __forceinline__ StreamId state() const { return StreamId{id_lo, id_hi, tag, ctr}; }
 };
 
 // ---- queue slot: one particle, 64 bytes (four 16-byte vectors) --------------

@@ -1,6 +1,8 @@
 // pmc_physics.cuh — scalar physics samplers, float32, one per reference
 // function in pyradmc/physics/*.py.  Each consumes exactly the uniforms its
-// reference counterpart consumes, in the same order.
+// reference counterpart consumes, in the same order, from a stream R: Rng, or
+// RingRng, which wants its draws announced (reserve) before they are taken; a
+// sampler whose number of draws is fixed leaves that to its caller.
 #pragma once
 
 #include "pmc_common.cuh"
@@ -8,7 +10,8 @@
 namespace pmc {
 
 // physics/path.py:15 — s = -ln(1 - u) / mu.  1 - u is exact for a 24-bit u.
-__device__ __forceinline__ float sample_path_length(float mu, Rng& rng) {
+template <class R>
+__device__ __forceinline__ float sample_path_length(float mu, R& rng) {
     return -logf(1.0f - rng.uniform()) / mu;
 }
 
@@ -37,7 +40,8 @@ __device__ __forceinline__ void rotate_direction(float& ux, float& uy, float& uz
 }
 
 // physics/direction.py:23 — isotropic direction, two uniforms.
-__device__ __forceinline__ void sample_isotropic_direction(Rng& rng, float& ax, float& ay,
+template <class R>
+__device__ __forceinline__ void sample_isotropic_direction(R& rng, float& ax, float& ay,
                                                            float& az) {
     const float c = 1.0f - 2.0f * rng.uniform();
     const float s = sqrtf(fmaxf(0.0f, 1.0f - c * c));
@@ -50,11 +54,13 @@ __device__ __forceinline__ void sample_isotropic_direction(Rng& rng, float& ax, 
 }
 
 // physics/compton.py:19 — Kahn's rejection for r = E'/E; three uniforms per round.
-__device__ inline float sample_compton_energy_ratio(float energy, Rng& rng) {
+template <class R>
+__device__ inline float sample_compton_energy_ratio(float energy, R& rng) {
     const float alpha = energy / kElectronMass;
     const float two_alpha = 2.0f * alpha;
     const float branch = (1.0f + two_alpha) / (9.0f + two_alpha);
     for (int round = 0; round < (1 << 20); ++round) {
+        rng.reserve(3);
         const float u1 = rng.uniform();
         const float u2 = rng.uniform();
         const float u3 = rng.uniform();
@@ -87,8 +93,9 @@ __device__ __forceinline__ float compton_electron_cos_theta(float energy, float 
 }
 
 // physics/channel.py:17 — channel by cumulative inversion on one uniform.
+template <class R>
 __device__ __forceinline__ int select_photon_process(float c, float p, float pair, float r,
-                                                     Rng& rng) {
+                                                     R& rng) {
     const float threshold = rng.uniform() * (c + p + pair + r);
     if (threshold < c) return 0;
     if (threshold < c + p) return 1;
@@ -97,7 +104,8 @@ __device__ __forceinline__ int select_photon_process(float c, float p, float pai
 }
 
 // physics/roulette.py:25 — one fair game; one uniform.
-__device__ __forceinline__ float roulette_weight(float w, float survival, Rng& rng) {
+template <class R>
+__device__ __forceinline__ float roulette_weight(float w, float survival, R& rng) {
     float survivor = 0.0f;
     if (rng.uniform() < survival) survivor = w / survival;
     return survivor;
@@ -119,12 +127,14 @@ __device__ __forceinline__ void brems_step_parameters(float e, float s_rad, floa
 }
 
 // physics/brems.py:69 — k = PCUT (E/PCUT)^u; one uniform.
-__device__ __forceinline__ float sample_brems_energy(float e, float pcut, Rng& rng) {
+template <class R>
+__device__ __forceinline__ float sample_brems_energy(float e, float pcut, R& rng) {
     return pcut * expf(rng.uniform() * logf(e / pcut));
 }
 
 // physics/moller.py:18 — restricted Moller DCS by rejection; two uniforms per round.
-__device__ inline float sample_moller_delta_energy(float e, float cut, Rng& rng) {
+template <class R>
+__device__ inline float sample_moller_delta_energy(float e, float cut, R& rng) {
     const float tau = e / kElectronMass;
     const float tr = tau / (tau + 1.0f);
     const float tr2 = tr * tr;
@@ -132,6 +142,7 @@ __device__ inline float sample_moller_delta_energy(float e, float cut, Rng& rng)
     const float w_min = cut / e;
     const float bound = 2.0f + 0.25f * tr2;
     for (int round = 0; round < (1 << 20); ++round) {
+        rng.reserve(2);
         const float u = rng.uniform();
         const float x = w_min / (1.0f - u * (1.0f - 2.0f * w_min));
         const float ratio = x / (1.0f - x);
@@ -152,7 +163,8 @@ __device__ __forceinline__ void moller_direction_cosines(float e, float w, float
 }
 
 // physics/msc.py:37 — Gaussian hinge; one uniform.
-__device__ __forceinline__ float sample_hinge_cos_theta(float ms, Rng& rng) {
+template <class R>
+__device__ __forceinline__ float sample_hinge_cos_theta(float ms, R& rng) {
     const float theta = sqrtf(-ms * logf(1.0f - rng.uniform()));
     return cosf(fminf(theta, kPi));
 }
@@ -163,8 +175,9 @@ __device__ __forceinline__ float gs_one_minus_cos(float ms) { return -expm1f(-0.
 
 // physics/gs.py:102 + :39 — bilinear blend of the four bracketing tables at
 // one equal-probability bin; one uniform (none when <theta^2> <= 0).
+template <class R>
 __device__ inline float sample_gs_cos_theta(const Tables& t, float fx, float fy, float ms,
-                                            Rng& rng) {
+                                            R& rng) {
     int ix = (int)floorf(fx) - t.gs_ix0;
     int iy = (int)floorf(fy) - t.gs_iy0;
     ix = min(max(ix, 0), t.gs_n_eta - 2);
@@ -199,11 +212,13 @@ __device__ inline float interp_increasing(float q, const float* xs, const float*
 }
 
 // physics/rayleigh.py:43 — coherent cosine from the form-factor cumulative.
-__device__ inline float sample_coherent_cos_theta(const Tables& t, int mat, float e, Rng& rng) {
+template <class R>
+__device__ inline float sample_coherent_cos_theta(const Tables& t, int mat, float e, R& rng) {
     const float* cum = t.coh_cum + (long long)mat * t.n_coherent;
     const float x_max = kRayleighPerMeV * e;
     const float a_max = interp_increasing(x_max, t.coh_x, cum, t.n_coherent);
     for (int round = 0; round < (1 << 20); ++round) {
+        rng.reserve(2);
         const float target = rng.uniform() * a_max;
         const float x = interp_increasing(target, cum, t.coh_x, t.n_coherent);
         const float ratio = x / x_max;

@@ -40,10 +40,12 @@ struct DevBuf {
 
 // Launch shape of the primary generator and the two transport kernels.
 struct LaunchShape {
-    int grid_ph = 0, grid_el = 0, block = 0;
+    int grid_ph = 0, grid_el = 0;
+    int block_ph = 0, block_el = 0;
     int grid_gen = 0;                 // primary generator, blocks of 256
     bool smem = false;                // table rows staged in shared memory
     int occ = 0;                      // register-budget variant (0, 3 or 4)
+    bool plain = false;               // plain_scoring
     size_t smem_ph = 0, smem_el = 0;  // dynamic shared memory of each kernel
 };
 
@@ -271,20 +273,41 @@ GridInfo make_grid(int nx, int ny, int nz, const double o[3], const double s[3])
 
 constexpr int kDefaultTailSteps = 96;  // steps after a round runs dry before a particle is parked
 
-// Kernel variants: tables in shared memory or not, and the register budget
-// (resident blocks of 256 per SM: 0 = each kernel's default, else 3 or 4).
-void* photon_fn(bool smem, int occ) {
-    if (occ == 4) return smem ? (void*)photon_kernel<true, 4> : (void*)photon_kernel<false, 4>;
-    return smem ? (void*)photon_kernel<true, 3> : (void*)photon_kernel<false, 3>;
+// Kernel variants: tables in shared memory or not, the register budget
+// (resident blocks of 256 per SM: 0 = each kernel's default, else 3 or 4), and
+// plain scoring.
+template <bool kPlain>
+void* photon_variant(bool smem, int occ) {
+    if (occ == 4) return smem ? (void*)photon_kernel<true, 4, kPlain> : (void*)photon_kernel<false, 4, kPlain>;
+    return smem ? (void*)photon_kernel<true, 3, kPlain> : (void*)photon_kernel<false, 3, kPlain>;
 }
-void* electron_fn(bool smem, int occ) {
-    if (occ == 3) return smem ? (void*)electron_kernel<true, 3> : (void*)electron_kernel<false, 3>;
-    return smem ? (void*)electron_kernel<true, 4> : (void*)electron_kernel<false, 4>;
+template <bool kPlain>
+void* electron_variant(bool smem, int occ) {
+    if (occ == 3) return smem ? (void*)electron_kernel<true, 3, kPlain> : (void*)electron_kernel<false, 3, kPlain>;
+    return smem ? (void*)electron_kernel<true, 4, kPlain> : (void*)electron_kernel<false, 4, kPlain>;
+}
+void* photon_fn(const LaunchShape& L) {
+    return L.plain ? photon_variant<true>(L.smem, L.occ) : photon_variant<false>(L.smem, L.occ);
+}
+void* electron_fn(const LaunchShape& L) {
+    return L.plain ? electron_variant<true>(L.smem, L.occ) : electron_variant<false>(L.smem, L.occ);
+}
+
+// The kPlain kernels' terms: the usual run, scoring dose to medium on the
+// transport grid itself; every other option takes the general kernels.
+bool plain_scoring(const pmc_engine* e, const pmc_run_params* p) {
+    return e->score_mode == 0 && std::memcmp(&e->si, &e->gi, sizeof e->gi) == 0 &&
+           e->gi.n_voxels < (1ll << 31) && !p->dose_to_water && !(p->deposit_resolution > 0.0) &&
+           p->photon_split_n <= 1;
 }
 
 int transport_launch_shape(pmc_engine* e, const pmc_run_params* p, LaunchShape* L) {
-    int bs = p->block_size > 0 ? p->block_size : 256;
-    if (bs % 32 != 0 || bs > 256) return fail(e, PMC_ERR_INVALID, "block_size must be a multiple of 32 and <= 256");
+    L->occ = (p->blocks_per_sm == 3 || p->blocks_per_sm == 4) ? p->blocks_per_sm : 0;
+    L->plain = plain_scoring(e, p);
+    // default: blocks of 256, and 512 for the 64-register electron kernel
+    L->block_ph = p->block_size > 0 ? p->block_size : kPhotonThreads;
+    L->block_el = p->block_size > 0 ? p->block_size : L->occ == 3 ? 256 : kElectronThreads;
+    if (L->block_ph % 32 != 0 || L->block_ph > 256) return fail(e, PMC_ERR_INVALID, "block_size must be a multiple of 32 and <= 256");
     const size_t rows = (size_t)e->tab.n_materials * (size_t)e->tab.n_points;
     L->smem_ph = rows * sizeof(float4) + (size_t)e->tab.n_points * sizeof(float);
     L->smem_el = rows * (sizeof(float4) + sizeof(float2));
@@ -294,15 +317,21 @@ int transport_launch_shape(pmc_engine* e, const pmc_run_params* p, LaunchShape* 
     if (!L->smem) L->smem_ph = L->smem_el = 0;
     int max_smem = 0;
     PMC_CUDA(e, cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, e->device));
-    L->occ = (p->blocks_per_sm == 3 || p->blocks_per_sm == 4) ? p->blocks_per_sm : 0;
     if (L->smem && (L->smem_ph + 1024 > (size_t)max_smem || L->smem_el + 1024 > (size_t)max_smem))
         return fail(e, PMC_ERR_INVALID, "tables of %d materials do not fit shared memory; use smem_tables=-1",
                     e->tab.n_materials);
-    PMC_CUDA(e, cudaFuncSetAttribute(photon_fn(L->smem, L->occ), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L->smem_ph));
-    PMC_CUDA(e, cudaFuncSetAttribute(electron_fn(L->smem, L->occ), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L->smem_el));
+    // (tables that fill the block's shared memory but for the random-number ring go through L1)
+    constexpr size_t kRing = kRingWords * sizeof(uint32_t);
+    if (L->smem && (L->smem_ph + 1024 + kRing * kPhotonThreads > (size_t)max_smem ||
+                    L->smem_el + 1024 + kRing * kElectronThreads > (size_t)max_smem)) {
+        L->smem = false;
+        L->smem_ph = L->smem_el = 0;
+    }
+    PMC_CUDA(e, cudaFuncSetAttribute(photon_fn(*L), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L->smem_ph));
+    PMC_CUDA(e, cudaFuncSetAttribute(electron_fn(*L), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L->smem_el));
     int per_sm_ph = 0, per_sm_el = 0;
-    PMC_CUDA(e, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_ph, photon_fn(L->smem, L->occ), bs, L->smem_ph));
-    PMC_CUDA(e, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_el, electron_fn(L->smem, L->occ), bs, L->smem_el));
+    PMC_CUDA(e, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_ph, photon_fn(*L), L->block_ph, L->smem_ph));
+    PMC_CUDA(e, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_el, electron_fn(*L), L->block_el, L->smem_el));
     if (p->blocks_per_sm > 0) {
         per_sm_ph = std::min(per_sm_ph, p->blocks_per_sm);
         per_sm_el = std::min(per_sm_el, p->blocks_per_sm);
@@ -314,7 +343,6 @@ int transport_launch_shape(pmc_engine* e, const pmc_run_params* p, LaunchShape* 
     L->grid_gen = std::max(1, std::min(per_sm_gen, 4)) * e->sm_count;
     L->grid_ph = per_sm_ph * e->sm_count;
     L->grid_el = per_sm_el * e->sm_count;
-    L->block = bs;
     return PMC_OK;
 }
 
@@ -342,13 +370,14 @@ int build_graph(pmc_engine* e, const TransportParams& P, const LaunchShape& L) {
     kp.kernelParams = args;
     cudaGraphNode_t n_gen, n_ph, n_el;
     PMC_CUDA(e, cudaGraphAddKernelNode(&n_gen, body, nullptr, 0, &kp));
-    kp.func = photon_fn(L.smem, L.occ);
+    kp.func = photon_fn(L);
     kp.gridDim = dim3(L.grid_ph);
-    kp.blockDim = dim3(L.block);
+    kp.blockDim = dim3(L.block_ph);
     kp.sharedMemBytes = (unsigned int)L.smem_ph;
     PMC_CUDA(e, cudaGraphAddKernelNode(&n_ph, body, &n_gen, 1, &kp));
-    kp.func = electron_fn(L.smem, L.occ);
+    kp.func = electron_fn(L);
     kp.gridDim = dim3(L.grid_el);
+    kp.blockDim = dim3(L.block_el);
     kp.sharedMemBytes = (unsigned int)L.smem_el;
     PMC_CUDA(e, cudaGraphAddKernelNode(&n_el, body, &n_ph, 1, &kp));
     PMC_CUDA(e, cudaGraphInstantiate(&e->graph_exec, e->graph, 0));
@@ -445,7 +474,8 @@ int prepare_transport(pmc_engine* e, const pmc_run_params* p, unsigned long long
     int rc = transport_launch_shape(e, p, &plan->shape);
     if (rc) return rc;
     const unsigned long long resident =
-        (unsigned long long)std::max(plan->shape.grid_ph, plan->shape.grid_el) * plan->shape.block;
+        std::max((unsigned long long)plan->shape.grid_ph * plan->shape.block_ph,
+                 (unsigned long long)plan->shape.grid_el * plan->shape.block_el);
     if (waves) {
         const double map_bytes = sizeof(double) * (double)stride_for(e->si.n_voxels) * std::max(cols, 1);
         const double by_memory = std::floor(kWaveBytes / map_bytes) + 1.0;
@@ -516,7 +546,8 @@ int run_wave(pmc_engine* e, const pmc_run_params* p, const RunPlan& plan, Transp
         const LaunchShape& L = plan.shape;
         const bool same = e->graph_exec && g.grid_ph == L.grid_ph && g.grid_el == L.grid_el &&
                           g.grid_gen == L.grid_gen &&
-                          g.block == L.block && g.smem == L.smem && g.occ == L.occ &&
+                          g.block_ph == L.block_ph && g.block_el == L.block_el && g.smem == L.smem &&
+                          g.occ == L.occ && g.plain == L.plain &&
                           g.smem_ph == L.smem_ph &&
                           g.smem_el == L.smem_el &&
                           std::memcmp(&e->graph_params, &P, sizeof P) == 0;
@@ -538,9 +569,9 @@ int run_wave(pmc_engine* e, const pmc_run_params* p, const RunPlan& plan, Transp
         const LaunchShape& L = plan.shape;
         generate_kernel<<<L.grid_gen, 256, 0, e->stream>>>(P);
         void* args[] = {&P};
-        PMC_CUDA(e, cudaLaunchKernel(photon_fn(L.smem, L.occ), dim3(L.grid_ph), dim3(L.block), args,
+        PMC_CUDA(e, cudaLaunchKernel(photon_fn(L), dim3(L.grid_ph), dim3(L.block_ph), args,
                                      L.smem_ph, e->stream));
-        PMC_CUDA(e, cudaLaunchKernel(electron_fn(L.smem, L.occ), dim3(L.grid_el), dim3(L.block),
+        PMC_CUDA(e, cudaLaunchKernel(electron_fn(L), dim3(L.grid_el), dim3(L.block_el),
                                      args, L.smem_el, e->stream));
         PMC_CUDA(e, cudaGetLastError());
         e->counters.transport_launches += 3;

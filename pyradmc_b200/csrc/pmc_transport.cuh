@@ -8,8 +8,7 @@
 //     lane whose particle ends takes the next one at once, from the input
 //     queue first and then from the batch's primary cursor, so no lane idles
 //     behind the longest particle of its warp;
-//   * photon primaries are generated inside the photon kernel and never touch
-//     a queue;
+//   * primaries are generated at full warp width and queued (generate_kernel);
 //   * queue rotation, the primary admission window and the "work left" flag
 //     are advanced on the device by the last block of each kernel, so a whole
 //     batch drains without one host round trip (and inside one CUDA graph);
@@ -18,6 +17,8 @@
 #pragma once
 
 #include <cooperative_groups.h>
+
+#include <type_traits>
 
 #include "pmc_common.cuh"
 #include "pmc_physics.cuh"
@@ -189,38 +190,43 @@ __device__ __forceinline__ float spr_factor(const TransportParams& P, float e, i
 // half-substep deposits and its next substep's usually do — so a run of
 // deposits into one voxel costs one atomic.  Integer sums: merging is exact.
 // Every atomic also marks its entry's sector in the dirty bitmap, the only
-// sectors the batch fold visits.
+// sectors the batch fold visits.  Entries are named by their bin in the
+// particle's column; the column's offset is recomputed at each atomic instead of
+// being held in two registers for the particle's whole life.
 struct DirectSink {
     unsigned int n = 0;  // atomics issued
-    __device__ __forceinline__ void add(const TransportParams& P, long long flat,
-                                        unsigned long long q) {
+    template <typename Bin>
+    __device__ __forceinline__ void add(const TransportParams& P, int beamlet, Bin bin, unsigned long long q) {
+        const long long flat = (long long)beamlet * P.col_stride + bin;
         atomicAdd(P.edep + flat, q);
         mark_dirty(P.dirty, flat);
         ++n;
     }
 };
 
+template <typename Bin>
 struct HeldSink {
-    long long idx = -1;
+    Bin bin = -1;
     unsigned long long q = 0;
     unsigned int n = 0;
-    __device__ __forceinline__ void add(const TransportParams& P, long long flat,
-                                        unsigned long long quanta) {
-        if (flat == idx) {
+    __device__ __forceinline__ void add(const TransportParams& P, int beamlet, Bin at, unsigned long long quanta) {
+        if (at == bin) {
             q += quanta;
             return;
         }
-        release(P);
-        idx = flat;
+        release(P, beamlet);
+        bin = at;
         q = quanta;
     }
-    __device__ __forceinline__ void release(const TransportParams& P) {
+    // The pending deposit reaches the map: before the lane changes its beamlet.
+    __device__ __forceinline__ void release(const TransportParams& P, int beamlet) {
         if (q != 0ull) {
-            atomicAdd(P.edep + idx, q);
-            mark_dirty(P.dirty, idx);
+            const long long flat = (long long)beamlet * P.col_stride + bin;
+            atomicAdd(P.edep + flat, q);
+            mark_dirty(P.dirty, flat);
             ++n;
         }
-        idx = -1;
+        bin = -1;
         q = 0ull;
     }
 };
@@ -252,22 +258,33 @@ __device__ __forceinline__ long long scoring_index(const TransportParams& P, flo
     return (long long)depth * c.n_shells + shell;
 }
 
+// Bins of a column: 32-bit in the kPlain kernels (fewer than 2^31 voxels).
+template <bool kPlain>
+using BinOf = std::conditional_t<kPlain, int, long long>;
+
+__device__ __forceinline__ long long quantize(float amount) {
+    return (long long)((double)amount * kInvQuantum + 0.5);
+}
+
 // kernels.py:536 _deposit: quantize once, route by position into the scoring
-// grid of this particle's column, or into the unscored book.
-template <class Sink>
-__device__ __forceinline__ void deposit(const TransportParams& P, BlockBooks& B, long long base,
-                                       float x, float y, float z, float amount, float factor,
-                                       Sink& sink) {
-    const long long idx = scoring_index(P, x, y, z);
-    if (idx >= 0) {
-        const long long q =
-            (long long)((double)amount * (double)factor * kInvQuantum + 0.5);
-        if (q != 0) sink.add(P, base + idx, (unsigned long long)q);
-        if (P.dose_to_water) {
-            book_add(&B.deposited, (long long)((double)amount * kInvQuantum + 0.5));
-        }
+// grid of this particle's column, or into the unscored book.  kPlain: the caller
+// has the position's bin already, and the factor is exactly 1.
+template <bool kPlain, class Sink>
+__device__ __forceinline__ void deposit(const TransportParams& P, BlockBooks& B, int beamlet, float x,
+                                       float y, float z, int voxel, float amount, float factor, Sink& sink) {
+    if constexpr (kPlain) {
+        const long long q = quantize(amount);
+        if (q != 0) sink.add(P, beamlet, voxel, (unsigned long long)q);
     } else {
-        book_add(&B.unscored, (long long)((double)amount * kInvQuantum + 0.5));
+        const long long idx = scoring_index(P, x, y, z);
+        if (idx >= 0) {
+            const long long q =
+                (long long)((double)amount * (double)factor * kInvQuantum + 0.5);
+            if (q != 0) sink.add(P, beamlet, idx, (unsigned long long)q);
+            if (P.dose_to_water) book_add(&B.deposited, quantize(amount));
+        } else {
+            book_add(&B.unscored, quantize(amount));
+        }
     }
 }
 
@@ -275,27 +292,41 @@ __device__ __forceinline__ void escape(BlockBooks& B, float amount) {
     book_add(&B.escaped, quantize_signed(amount));
 }
 
+// flat_index of a grid of fewer than 2^31 voxels.
+__device__ __forceinline__ int flat_index32(float x, float y, float z, const GridInfo& g) {
+    const int ix = axis_index(x, g.x_lo, g.sx, g.nx);
+    const int iy = axis_index(y, g.y_lo, g.sy, g.ny);
+    const int iz = axis_index(z, g.z_lo, g.sz, g.nz);
+    return (ix * g.ny + iy) * g.nz + iz;
+}
+template <bool kPlain>
+__device__ __forceinline__ BinOf<kPlain> voxel_of(float x, float y, float z, const GridInfo& g) {
+    if constexpr (kPlain) return flat_index32(x, y, z, g);
+    else return flat_index(x, y, z, g);
+}
+
 // kernels.py:600 _deposit_or_escape: escape is decided on the transport grid.
-template <class Sink>
-__device__ __forceinline__ void deposit_or_escape(const TransportParams& P, BlockBooks& B,
-                                                  long long base, float x, float y, float z,
-                                                  float amount, float factor, Sink& sink) {
+template <bool kPlain, class Sink>
+__device__ __forceinline__ void deposit_or_escape(const TransportParams& P, BlockBooks& B, int beamlet,
+                                                  float x, float y, float z, float amount, float factor,
+                                                  Sink& sink) {
     if (amount <= 0.0f) return;
-    if (point_inside(x, y, z, P.gi)) deposit(P, B, base, x, y, z, amount, factor, sink);
+    if (point_inside(x, y, z, P.gi))
+        deposit<kPlain>(P, B, beamlet, x, y, z, kPlain ? flat_index32(x, y, z, P.gi) : 0, amount, factor, sink);
     else escape(B, amount);
 }
 
-// kernels.py:631 _deposit_spread: equal pieces at piece midpoints.
-template <class Sink>
-__device__ inline void deposit_spread(const TransportParams& P, BlockBooks& B, long long base,
-                                      float x, float y, float z, float ux, float uy, float uz,
-                                      float length, float amount, float factor, Sink& sink) {
-    const int n = substep_pieces(length, P.deposit_resolution);
-    const float share = amount / (float)n;
-    const float piece = length / (float)n;
+// kernels.py:631 _deposit_spread: equal pieces at piece midpoints (kPlain: one).
+template <bool kPlain, class Sink>
+__device__ __forceinline__ void deposit_spread(const TransportParams& P, BlockBooks& B, int beamlet, float x,
+                                               float y, float z, float ux, float uy, float uz, float length,
+                                               float amount, float factor, Sink& sink) {
+    const int n = kPlain ? 1 : substep_pieces(length, P.deposit_resolution);
+    const float share = kPlain ? amount : amount / (float)n;
+    const float piece = kPlain ? length : length / (float)n;
     for (int k = 0; k < n; ++k) {
         const float t = ((float)k + 0.5f) * piece;
-        deposit_or_escape(P, B, base, x + ux * t, y + uy * t, z + uz * t, share, factor, sink);
+        deposit_or_escape<kPlain>(P, B, beamlet, x + ux * t, y + uy * t, z + uz * t, share, factor, sink);
     }
 }
 
@@ -324,8 +355,10 @@ __device__ __forceinline__ void queue_push(const TransportParams& P, int qi, int
 // Park an unfinished particle in queue qi for the next round: its whole state
 // (phase space, kind, primary flag, beamlet, stream position, steps taken)
 // goes into the slot, so the next round continues it exactly where it stopped.
-struct Particle;
-__device__ __forceinline__ void queue_suspend(const TransportParams& P, int qi, const Particle& p,
+template <class R>
+struct ParticleOf;
+template <class R>
+__device__ __forceinline__ void queue_suspend(const TransportParams& P, int qi, const ParticleOf<R>& p,
                                               unsigned int& n_push);
 
 __device__ __forceinline__ unsigned long long fetch_one(unsigned long long* ctr) {
@@ -344,28 +377,32 @@ __device__ __forceinline__ unsigned int fetch_one(unsigned int* ctr) {
 }
 
 // ---- particle state ----------------------------------------------------------------
-struct Particle {
+template <class R>
+struct ParticleOf {
     float e, w, x, y, z, ux, uy, uz;
-    int kind, primary, beamlet;
-    int steps;  // the host caps max_steps below 2^31
-    Rng rng;
+    uint32_t meta;  // as in a slot: kind, primary, beamlet in one register
+    int steps;      // the host caps max_steps below 2^31
+    R rng;
+    __device__ __forceinline__ int kind() const { return (int)(meta & 3u); }
+    __device__ __forceinline__ bool primary() const { return (meta & 4u) != 0u; }
+    __device__ __forceinline__ int beamlet() const { return (int)(meta >> 3); }
 };
+using Particle = ParticleOf<Rng>;  // of the generator
 
-__device__ __forceinline__ void load_slot(const TransportParams& P, const Slot* q, unsigned int i,
-                                          Particle& p) {
+template <class R>
+__device__ __forceinline__ void load_slot(const Slot* q, unsigned int i, ParticleOf<R>& p) {
     const Slot* s = q + i;
     const float4 a = s->a, b = s->b;
     const uint4 c = s->c, d = s->d;
     p.e = a.x; p.w = a.y; p.x = a.z; p.y = a.w;
     p.z = b.x; p.ux = b.y; p.uy = b.z; p.uz = b.w;
-    p.kind = (int)(d.x & 3u);
-    p.primary = (int)((d.x >> 2) & 1u);
-    p.beamlet = (int)(d.x >> 3);
+    p.meta = d.x;
     p.steps = (int)d.y;
-    p.rng.load(P.seed_lo, P.seed_hi, StreamId{c.x, c.y, c.z, c.w});
+    p.rng.load(StreamId{c.x, c.y, c.z, c.w});
 }
 
-__device__ __forceinline__ void queue_suspend(const TransportParams& P, int qi, const Particle& p,
+template <class R>
+__device__ __forceinline__ void queue_suspend(const TransportParams& P, int qi, const ParticleOf<R>& p,
                                               unsigned int& n_push) {
     cg::coalesced_group g = cg::coalesced_threads();
     unsigned int base = 0;
@@ -382,7 +419,7 @@ __device__ __forceinline__ void queue_suspend(const TransportParams& P, int qi, 
     s->a = make_float4(p.e, p.w, p.x, p.y);
     s->b = make_float4(p.z, p.ux, p.uy, p.uz);
     s->c = make_uint4(sid.id_lo, sid.id_hi, sid.tag, sid.ctr);
-    s->d = make_uint4(pack_meta(p.kind, p.primary, p.beamlet), (uint32_t)p.steps, 0u, 0u);
+    s->d = make_uint4(p.meta, (uint32_t)p.steps, 0u, 0u);
 }
 
 // Copy `n` table entries into the block's shared memory (strided over the block).
@@ -393,7 +430,8 @@ __device__ __forceinline__ void stage(T* dst, const T* src, int n) {
 
 // Vacuum flight to the grid for a particle born outside (photon.py:137-148);
 // returns false (energy escaped) when the flight misses the grid.
-__device__ __forceinline__ bool enter_grid(const TransportParams& P, BlockBooks& B, Particle& p,
+template <class R>
+__device__ __forceinline__ bool enter_grid(const TransportParams& P, BlockBooks& B, ParticleOf<R>& p,
                                            float latent) {
     if (point_inside(p.x, p.y, p.z, P.gi)) return true;
     float t = slab_entry_distance(p.x, p.y, p.z, p.ux, p.uy, p.uz, P.gi);
@@ -504,11 +542,9 @@ __device__ inline int generate_primary(const TransportParams& P, const GenDesc& 
     p.rng.id_hi = (uint32_t)((unsigned long long)key >> 32);
     p.rng.tag = 0u;
     p.rng.ctr = 0u;
-    p.beamlet = map * G.group + local;
-    p.primary = 1;
+    int kind = G.kind;
     p.steps = 0;
     p.w = 1.0f;
-    p.kind = G.kind;
     if (G.type == 0) {  // pencil: no draws
         p.e = G.energy;
         p.x = G.px; p.y = G.py; p.z = G.pz;
@@ -554,7 +590,7 @@ __device__ inline int generate_primary(const TransportParams& P, const GenDesc& 
         const float4 a = __ldg(&r->a), b = __ldg(&r->b);
         const float4 d = __ldg(&r->d);
         const int bits = __float_as_int(d.w);
-        p.kind = kPhoton;
+        kind = kPhoton;
         if ((bits & 1) == 0) {  // lattice rectangle: two uniforms
             p.e = b.y;
             p.x = a.x + a.y * p.rng.uniform();
@@ -593,7 +629,7 @@ __device__ inline int generate_primary(const TransportParams& P, const GenDesc& 
                 ((unsigned long long)p.rng.next_u32() << 32) | (unsigned long long)p.rng.next_u32();
             ri = (long long)__umul64hi(r, (unsigned long long)G.n_records);
         }
-        p.kind = G.up_kind ? __ldg(G.up_kind + ri) : kPhoton;
+        kind = G.up_kind ? __ldg(G.up_kind + ri) : kPhoton;
         p.e = __ldg(G.up_energy + ri);
         p.w = __ldg(G.up_weight + ri);
         p.x = __ldg(G.up_pos + 3 * ri);
@@ -603,6 +639,7 @@ __device__ inline int generate_primary(const TransportParams& P, const GenDesc& 
         p.uy = __ldg(G.up_dir + 3 * ri + 1);
         p.uz = __ldg(G.up_dir + 3 * ri + 2);
     }
+    p.meta = pack_meta(kind, 1, map * G.group + local);
     if (G.type != 3 && G.type != 5) {  // host records carry their own weights
         // a zero weight emits nothing; the history still counts in the batch mean
         if (G.masked) p.w *= mask_transmission(G, p);
@@ -610,29 +647,33 @@ __device__ inline int generate_primary(const TransportParams& P, const GenDesc& 
         if (p.w == 0.0f) return -1;
     }
     if (G.book_emitted) {
-        const float latent = p.kind == kPositron ? 2.0f * kElectronMass : 0.0f;
+        const float latent = kind == kPositron ? 2.0f * kElectronMass : 0.0f;
         book_add(&B.emitted, quantize_signed(p.w * (p.e + latent)));
     }
-    return p.kind;
+    return kind;
 }
 
 // ---- annihilation at rest (transport/particles.py:75, kernels.py:675) ------------
-template <class Sink>
-__device__ inline void annihilate_at_rest(const TransportParams& P, BlockBooks& B, Particle& p,
-                                          long long base, int q_photon, float factor, Sink& sink,
-                                          unsigned int& n_push) {
+template <bool kPlain, class R, class Sink>
+__device__ __forceinline__ void annihilate_at_rest(const TransportParams& P, BlockBooks& B, ParticleOf<R>& p,
+                                                   int voxel, int q_photon, float factor, Sink& sink,
+                                                   unsigned int& n_push) {
     if (P.pcut >= kElectronMass) {
-        deposit(P, B, base, p.x, p.y, p.z, p.w * 2.0f * kElectronMass, factor, sink);
+        deposit<kPlain>(P, B, p.beamlet(), p.x, p.y, p.z, voxel, p.w * 2.0f * kElectronMass, factor, sink);
         return;
     }
     float ax, ay, az;
+    p.rng.reserve(2);
     sample_isotropic_direction(p.rng, ax, ay, az);
-    const StreamId s1 = p.rng.spawn();
-    queue_push(P, q_photon, kPhoton, p.beamlet, kElectronMass, p.w, p.x, p.y, p.z, ax, ay, az, s1,
-               n_push);
-    const StreamId s2 = p.rng.spawn();
-    queue_push(P, q_photon, kPhoton, p.beamlet, kElectronMass, p.w, p.x, p.y, p.z, -ax, -ay, -az,
-               s2, n_push);
+#pragma unroll 1
+    for (int k = 0; k < 2; ++k) {  // two photons back to back
+        p.rng.reserve(3);
+        const StreamId sid = p.rng.spawn();
+        queue_push(P, q_photon, kPhoton, p.beamlet(), kElectronMass, p.w, p.x, p.y, p.z, ax, ay, az, sid, n_push);
+        ax = -ax;
+        ay = -ay;
+        az = -az;
+    }
 }
 
 // ---- last-block scheduler steps ------------------------------------------------------
@@ -681,16 +722,21 @@ __device__ __forceinline__ void block_sum_add(unsigned long long* dst, unsigned 
 }
 
 // ---- the photon kernel ---------------------------------------------------------------
+constexpr int kPhotonThreads = 256;  // the largest block of the photon kernel
+
 // One lane transports one photon to termination (Woodcock tracking), then takes
-// the next: queued photons first, then fresh primaries of the batch block.
+// the round's next queued photon.
 // kSmem: the channel rows of every material and the majorant row are staged in
 // the block's shared memory (dynamic, n_materials * n_points * 16 + n_points * 4
 // bytes) instead of being read through L1.
-// kMinBlocks: resident blocks of 256 per SM the register allocation targets
-// (3: 80 registers, no spill; 4: 64 registers, a few bytes spilled).
-template <bool kSmem, int kMinBlocks = 3>
-__global__ void __launch_bounds__(256, kMinBlocks) photon_kernel(TransportParams P) {
+// kMinBlocks: resident blocks of 256 per SM the register allocation targets.
+// kPlain: dose to medium on the transport grid itself, whole-substep deposits, no
+// Compton splitting, fewer than 2^31 voxels (plain_scoring): a deposit's bin is the
+// voxel already at hand.
+template <bool kSmem, int kMinBlocks, bool kPlain>
+__global__ void __launch_bounds__(kPhotonThreads, kMinBlocks) photon_kernel(TransportParams P) {
     __shared__ BlockBooks B;
+    __shared__ uint32_t ring[kRingWords * kPhotonThreads];
     extern __shared__ __align__(16) unsigned char pmc_smem[];
     const float4* tab_ch = P.tab.ch;
     const float* tab_maj = P.tab.maj;
@@ -713,14 +759,16 @@ __global__ void __launch_bounds__(256, kMinBlocks) photon_kernel(TransportParams
 
     unsigned int n_flight = 0, n_inter = 0, n_push = 0;  // per lane and launch
     DirectSink dep;
-    Particle p;
+    ParticleOf<RingRng<kPhotonThreads>> p;
+    p.rng.k0 = P.seed_lo;
+    p.rng.k1 = P.seed_hi;
+    p.rng.ring = ring + threadIdx.x;
     bool active = false, exhausted = false, dry = false;
     int tail = 0;  // steps of the current photon since its warp found the round dry
     float e_tab = -1.0f, maj = 0.0f;
     LogIdx li{0, 0.0f};
     int mat_tab = -1;
     float4 ch = make_float4(0.f, 0.f, 0.f, 0.f);
-    long long base = 0;
 
     for (unsigned int it = 0;; ++it) {
         if ((it & 255u) == 0u) {
@@ -730,9 +778,8 @@ __global__ void __launch_bounds__(256, kMinBlocks) photon_kernel(TransportParams
         if (!active && !exhausted) {  // the round's photons: secondaries, parked, then primaries
             const unsigned int i = fetch_one(&S->head[q_in]);
             if (i < n_in) {
-                load_slot(P, P.q[q_in], i, p);
+                load_slot(P.q[q_in], i, p);
                 active = enter_grid(P, B, p, 0.0f);
-                base = (long long)p.beamlet * P.col_stride;
                 e_tab = -1.0f;
                 tail = 0;
             } else {
@@ -758,6 +805,7 @@ __global__ void __launch_bounds__(256, kMinBlocks) photon_kernel(TransportParams
             active = false;
             continue;
         }
+        p.rng.top_up();  // path, acceptance, channel
         if (p.e != e_tab) {
             li = log_index(p.e, T.p_log_min, T.p_inv_dlog, T.n_points);
             maj = lerp1<kSmem>(tab_maj, li);
@@ -774,7 +822,9 @@ __global__ void __launch_bounds__(256, kMinBlocks) photon_kernel(TransportParams
             active = false;
             continue;
         }
-        const float2 vx = __ldg(P.vox + flat_index(p.x, p.y, p.z, P.gi));
+        const BinOf<kPlain> flat = voxel_of<kPlain>(p.x, p.y, p.z, P.gi);
+        const float2 vx = __ldg(P.vox + flat);
+        const int voxel = kPlain ? (int)flat : 0;
         const float rho = vx.x;
         const int mat = __float_as_int(vx.y);
         if (mat != mat_tab) {
@@ -792,76 +842,101 @@ __global__ void __launch_bounds__(256, kMinBlocks) photon_kernel(TransportParams
         if (p.rng.uniform() * maj >= mu_real) continue;  // delta scattering
         ++n_inter;
         const int process = select_photon_process(mc, mp, mpa, mr, p.rng);
+        auto put = [&](float amount, float energy) {  // local deposit of an electron of that energy
+            deposit<kPlain>(P, B, p.beamlet(), p.x, p.y, p.z, voxel, amount,
+                            kPlain ? 1.0f : spr_factor(P, energy, mat), dep);
+        };
 
         if (process == 3) {  // coherent
             const float c = sample_coherent_cos_theta(T, mat, p.e, p.rng);
+            p.rng.reserve(1);
             const float phi = kTwoPi * p.rng.uniform();
             rotate_direction(p.ux, p.uy, p.uz, c, phi);
-        } else if (process == 0) {  // Compton
-            if (P.split_n > 1 && p.primary) {
-                // Compton splitting of a source photon (photon.py:190-224): N
-                // copies of weight w/N, each pushed as a non-primary photon.
-                const float split_w = p.w / (float)P.split_n;
-                for (int k = 0; k < P.split_n; ++k) {
-                    const float ratio = sample_compton_energy_ratio(p.e, p.rng);
-                    const float recoil = p.e * (1.0f - ratio);
-                    const float phi = kTwoPi * p.rng.uniform();
-                    if (P.transport_electrons && recoil > ecut) {
-                        float ex = p.ux, ey = p.uy, ez = p.uz;
-                        rotate_direction(ex, ey, ez, compton_electron_cos_theta(p.e, ratio),
-                                         phi + kPi);
-                        const StreamId sid = p.rng.spawn();
-                        queue_push(P, q_el, kElectron, p.beamlet, recoil, split_w, p.x, p.y, p.z,
-                                   ex, ey, ez, sid, n_push);
-                    } else {
-                        deposit(P, B, base, p.x, p.y, p.z, split_w * recoil,
-                                spr_factor(P, recoil, mat), dep);
-                    }
-                    float gx = p.ux, gy = p.uy, gz = p.uz;
-                    rotate_direction(gx, gy, gz, compton_cos_theta(p.e, ratio), phi);
-                    const float es = p.e * ratio;
-                    if (es <= pcut) {
-                        deposit(P, B, base, p.x, p.y, p.z, split_w * es, spr_factor(P, es, mat),
-                                dep);
-                        continue;
-                    }
-                    float cw = split_w;
-                    bool keep = true;
-                    if (es < kRouletteMeV && cw < kRouletteWeightCap) {
-                        const float nw = roulette_weight(cw, kRouletteSurvival, p.rng);
-                        escape(B, (cw - nw) * es);
-                        if (nw == 0.0f) keep = false;
-                        else cw = nw;
-                    }
-                    if (keep) {
-                        const StreamId sid = p.rng.spawn();
-                        queue_push(P, q_out, kPhoton, p.beamlet, es, cw, p.x, p.y, p.z, gx, gy, gz,
-                                   sid, n_push);
-                    }
+            continue;
+        }
+        if (!kPlain && process == 0 && P.split_n > 1 && p.primary()) {
+            // Compton splitting of a source photon (photon.py:190-224): N
+            // copies of weight w/N, each pushed as a non-primary photon.
+            const float split_w = p.w / (float)P.split_n;
+            for (int k = 0; k < P.split_n; ++k) {
+                const float ratio = sample_compton_energy_ratio(p.e, p.rng);
+                const float recoil = p.e * (1.0f - ratio);
+                p.rng.reserve(4);
+                const float phi = kTwoPi * p.rng.uniform();
+                if (P.transport_electrons && recoil > ecut) {
+                    float ex = p.ux, ey = p.uy, ez = p.uz;
+                    rotate_direction(ex, ey, ez, compton_electron_cos_theta(p.e, ratio), phi + kPi);
+                    const StreamId sid = p.rng.spawn();
+                    queue_push(P, q_el, kElectron, p.beamlet(), recoil, split_w, p.x, p.y, p.z, ex, ey, ez, sid,
+                               n_push);
+                } else {
+                    put(split_w * recoil, recoil);
                 }
-                active = false;
-                continue;
+                float gx = p.ux, gy = p.uy, gz = p.uz;
+                rotate_direction(gx, gy, gz, compton_cos_theta(p.e, ratio), phi);
+                const float es = p.e * ratio;
+                if (es <= pcut) {
+                    put(split_w * es, es);
+                    continue;
+                }
+                float cw = split_w;
+                bool keep = true;
+                p.rng.reserve(4);
+                if (es < kRouletteMeV && cw < kRouletteWeightCap) {
+                    const float nw = roulette_weight(cw, kRouletteSurvival, p.rng);
+                    escape(B, (cw - nw) * es);
+                    if (nw == 0.0f) keep = false;
+                    else cw = nw;
+                }
+                if (keep) {
+                    const StreamId sid = p.rng.spawn();
+                    queue_push(P, q_out, kPhoton, p.beamlet(), es, cw, p.x, p.y, p.z, gx, gy, gz, sid, n_push);
+                }
             }
-            const float ratio = sample_compton_energy_ratio(p.e, p.rng);
-            const float recoil = p.e * (1.0f - ratio);
-            const float phi = kTwoPi * p.rng.uniform();
-            if (P.transport_electrons && recoil > ecut) {
-                float ex = p.ux, ey = p.uy, ez = p.uz;
+            active = false;
+            continue;
+        }
+
+        // Compton, photoelectric and pair events each set one electron in motion
+        // (electron energy ee, direction ex, ey, ez): found per process, then
+        // pushed or deposited in one place for all of them.
+        float ratio = 0.0f, phi = 0.0f, kinetic = 0.0f, fraction = 0.0f;
+        float ee, ex = p.ux, ey = p.uy, ez = p.uz;
+        if (process == 0) {
+            ratio = sample_compton_energy_ratio(p.e, p.rng);
+            ee = p.e * (1.0f - ratio);
+        } else if (process == 1) {  // photoelectric: forward, no fluorescence
+            ee = p.e;
+        } else {
+            kinetic = p.e - 2.0f * kElectronMass;
+            ee = kinetic;  // without electron transport the pair's energy stays here
+        }
+        p.rng.reserve(4);
+        if (process == 0) {
+            phi = kTwoPi * p.rng.uniform();
+        } else if (process == 2 && P.transport_electrons) {
+            fraction = p.rng.uniform();
+            ee = fraction * kinetic;
+        }
+        if (P.transport_electrons && ee > ecut) {
+            if (process == 0)
                 rotate_direction(ex, ey, ez, compton_electron_cos_theta(p.e, ratio), phi + kPi);
-                const StreamId sid = p.rng.spawn();
-                queue_push(P, q_el, kElectron, p.beamlet, recoil, p.w, p.x, p.y, p.z, ex, ey, ez,
-                           sid, n_push);
-            } else {
-                deposit(P, B, base, p.x, p.y, p.z, p.w * recoil, spr_factor(P, recoil, mat), dep);
-            }
+            const StreamId sid = p.rng.spawn();
+            queue_push(P, q_el, kElectron, p.beamlet(), ee, p.w, p.x, p.y, p.z, ex, ey, ez, sid, n_push);
+        } else {
+            put(p.w * ee, ee);
+        }
+
+        if (process == 0) {
             rotate_direction(p.ux, p.uy, p.uz, compton_cos_theta(p.e, ratio), phi);
             p.e *= ratio;
             if (p.e <= pcut) {
-                deposit(P, B, base, p.x, p.y, p.z, p.w * p.e, spr_factor(P, p.e, mat), dep);
+                put(p.w * p.e, p.e);
                 active = false;
                 continue;
             }
             if (p.e < kRouletteMeV && p.w < kRouletteWeightCap) {
+                p.rng.reserve(1);
                 const float nw = roulette_weight(p.w, kRouletteSurvival, p.rng);
                 escape(B, (p.w - nw) * p.e);
                 if (nw == 0.0f) {
@@ -870,47 +945,22 @@ __global__ void __launch_bounds__(256, kMinBlocks) photon_kernel(TransportParams
                 }
                 p.w = nw;
             }
-        } else if (process == 1) {  // photoelectric: forward, no fluorescence
-            if (P.transport_electrons && p.e > ecut) {
-                const StreamId sid = p.rng.spawn();
-                queue_push(P, q_el, kElectron, p.beamlet, p.e, p.w, p.x, p.y, p.z, p.ux, p.uy,
-                           p.uz, sid, n_push);
-            } else {
-                deposit(P, B, base, p.x, p.y, p.z, p.w * p.e, spr_factor(P, p.e, mat), dep);
-            }
-            active = false;
-        } else {  // pair production
-            const float kinetic = p.e - 2.0f * kElectronMass;
-            if (P.transport_electrons) {
-                const float fraction = p.rng.uniform();
-                const float share_e = fraction * kinetic;
-                const float share_p = (1.0f - fraction) * kinetic;
-                if (share_e > ecut) {
-                    const StreamId sid = p.rng.spawn();
-                    queue_push(P, q_el, kElectron, p.beamlet, share_e, p.w, p.x, p.y, p.z, p.ux,
-                               p.uy, p.uz, sid, n_push);
-                } else {
-                    deposit(P, B, base, p.x, p.y, p.z, p.w * share_e, spr_factor(P, share_e, mat),
-                            dep);
-                }
-                if (share_p > ecut) {
-                    const StreamId sid = p.rng.spawn();
-                    queue_push(P, q_el, kPositron, p.beamlet, share_p, p.w, p.x, p.y, p.z, p.ux,
-                               p.uy, p.uz, sid, n_push);
-                } else {
-                    deposit(P, B, base, p.x, p.y, p.z, p.w * share_p, spr_factor(P, share_p, mat),
-                            dep);
-                    annihilate_at_rest(P, B, p, base, q_out, spr_factor(P, kElectronMass, mat),
-                                       dep, n_push);
-                }
-            } else {
-                deposit(P, B, base, p.x, p.y, p.z, p.w * kinetic, spr_factor(P, kinetic, mat),
-                        dep);
-                annihilate_at_rest(P, B, p, base, q_out, spr_factor(P, kElectronMass, mat), dep,
-                                   n_push);
-            }
-            active = false;
+            continue;
         }
+        if (process == 2) {  // pair production: the positron
+            const float share_p = (1.0f - fraction) * kinetic;
+            if (P.transport_electrons && share_p > ecut) {
+                p.rng.reserve(3);
+                const StreamId sid = p.rng.spawn();
+                queue_push(P, q_el, kPositron, p.beamlet(), share_p, p.w, p.x, p.y, p.z, p.ux, p.uy, p.uz, sid,
+                           n_push);
+            } else {
+                if (P.transport_electrons) put(p.w * share_p, share_p);
+                annihilate_at_rest<kPlain>(P, B, p, voxel, q_out,
+                                           kPlain ? 1.0f : spr_factor(P, kElectronMass, mat), dep, n_push);
+            }
+        }
+        active = false;
     }
 
     block_sum_add(&B.flights, n_flight);
@@ -932,7 +982,7 @@ __global__ void __launch_bounds__(256, kMinBlocks) photon_kernel(TransportParams
 }
 
 // ---- the primary generator ---------------------------------------------------------
-// The round's admission window [cursor, limit) of the batch block, one thread
+// The round's admission window [cursor, limit) of the wave, one thread
 // per primary (kernels.py:1888-2401): sampled at full warp width, flown
 // through vacuum to the grid, then queued with its stream position — photons
 // into the round's photon input queue behind the secondaries already there,
@@ -958,7 +1008,7 @@ __global__ void __launch_bounds__(256) generate_kernel(TransportParams P) {
         if (kind == kPhoton) {
             if (enter_grid(P, B, p, 0.0f)) queue_suspend(P, q_ph, p, n_push);
         } else {  // charged primary: to the electron queue unchanged (it enters there)
-            queue_push(P, q_el, kind, p.beamlet, p.e, p.w, p.x, p.y, p.z, p.ux, p.uy, p.uz,
+            queue_push(P, q_el, kind, p.beamlet(), p.e, p.w, p.x, p.y, p.z, p.ux, p.uy, p.uz,
                        p.rng.state(), n_push);
         }
     }
@@ -967,16 +1017,21 @@ __global__ void __launch_bounds__(256) generate_kernel(TransportParams P) {
     flush_books(P, B);
 }
 
-__device__ __forceinline__ long long col_base(const TransportParams& P, const Particle& p) {
-    return (long long)p.beamlet * P.col_stride;
-}
-
 // Annihilation energy a positron still carries (2 m c^2), booked with it on escape.
-__device__ __forceinline__ float rest_energy(const Particle& p) {
-    return p.kind == kPositron ? 2.0f * kElectronMass : 0.0f;
+template <class R>
+__device__ __forceinline__ float rest_energy(const ParticleOf<R>& p) {
+    return p.kind() == kPositron ? 2.0f * kElectronMass : 0.0f;
 }
 
 // ---- the electron kernel -------------------------------------------------------------
+// What bounds both transport kernels: instruction issue with half the lanes
+// active, then the latency of the voxel and queue gathers, not HBM.  On the
+// 100-column 128^3 Dij (1.7e8 substeps, 7.8e7 flights) the draws from a ring in
+// shared memory, the plain scoring path and the terminal step folded into the
+// refill took the electron kernel from 17.5 to 12.4 ms and the photon kernel from
+// 13.6 to 12.1 ms.
+constexpr int kElectronThreads = 512;  // the largest block of the electron kernel
+
 // One lane runs one electron or positron to ECUT (Class II condensed history,
 // electron.py:345-481); delta rays go to the next round's electron queue,
 // bremsstrahlung and annihilation photons to the next photon round.
@@ -984,11 +1039,15 @@ __device__ __forceinline__ float rest_energy(const Particle& p) {
 // (scattering power, log eta) rows of every material are staged in the block's
 // shared memory (n_materials * n_points * 24 bytes); the inverse-range row
 // (one read per substep) stays on the L1 path.
-// kMinBlocks: as for the photon kernel (4: 64 registers, a few bytes spilled;
-// 3: 85 registers, none).
-template <bool kSmem, int kMinBlocks = 4>
-__global__ void __launch_bounds__(256, kMinBlocks) electron_kernel(TransportParams P) {
+// kMinBlocks: resident blocks of 256 threads per SM the register allocation
+// targets: 4 (64 registers; launched as two blocks of 512, which stage the
+// tables twice per SM instead of four times) or 3 (85).
+// kPlain: as for the photon kernel.
+template <bool kSmem, int kMinBlocks, bool kPlain>
+__global__ void __launch_bounds__(kMinBlocks == 4 ? kElectronThreads : 256, kMinBlocks == 4 ? 2 : kMinBlocks)
+electron_kernel(TransportParams P) {
     __shared__ BlockBooks B;
+    __shared__ uint32_t ring[kRingWords * kElectronThreads];
     extern __shared__ __align__(16) unsigned char pmc_smem[];
     const float4* tab_ea = P.tab.ea;
     const float2* tab_eb = P.tab.eb;
@@ -1010,10 +1069,12 @@ __global__ void __launch_bounds__(256, kMinBlocks) electron_kernel(TransportPara
     const float pcut = P.pcut, ecut = P.ecut;
 
     unsigned int n_sub = 0, n_push = 0;  // per lane and launch
-    HeldSink dep;
-    // The particle's column offset (col_base) is recomputed at each deposit
-    // instead of being held in two registers for the particle's whole life.
-    Particle p;
+    HeldSink<BinOf<kPlain>> dep;
+    ParticleOf<RingRng<kElectronThreads>> p;
+    p.meta = 0u;
+    p.rng.k0 = P.seed_lo;
+    p.rng.k1 = P.seed_hi;
+    p.rng.ring = ring + threadIdx.x;
     bool active = false, exhausted = false, dry = false;
     int tail = 0;  // substeps of the current particle since its warp found the round dry
 
@@ -1022,11 +1083,30 @@ __global__ void __launch_bounds__(256, kMinBlocks) electron_kernel(TransportPara
             if (__any_sync(0xffffffffu, (*(volatile int*)&S->flags) & (kFlagOverflow | kFlagStepCap)))
                 break;
         }
-        if (!active) dep.release(P);  // the finished particle's last held deposit
+        // A particle that came to rest deposits and its lane takes the next one in
+        // the same turn of the loop, so that no lane sits out a substep in between
+        // (an electron lives 4.5 substeps on average).
+        if (active && p.e <= ecut) {  // terminal: local deposit (electron.py:347-365)
+            if (++p.steps > P.max_steps) {
+                atomicOr(&S->flags, kFlagStepCap);
+                escape(B, p.w * (p.e + rest_energy(p)));
+            } else {
+                const BinOf<kPlain> flat = voxel_of<kPlain>(p.x, p.y, p.z, P.gi);
+                const int voxel = kPlain ? (int)flat : 0;
+                const int tm = kPlain ? 0 : __float_as_int(__ldg(P.vox + flat).y);
+                deposit<kPlain>(P, B, p.beamlet(), p.x, p.y, p.z, voxel, p.w * p.e,
+                                kPlain ? 1.0f : spr_factor(P, p.e, tm), dep);
+                if (p.kind() == kPositron)
+                    annihilate_at_rest<kPlain>(P, B, p, voxel, q_ph,
+                                               kPlain ? 1.0f : spr_factor(P, kElectronMass, tm), dep, n_push);
+            }
+            active = false;
+        }
+        if (!active) dep.release(P, p.beamlet());  // the finished particle's last held deposit
         if (!active && !exhausted) {
             const unsigned int i = fetch_one(&S->head[q_in]);
             if (i < n_in) {
-                load_slot(P, P.q[q_in], i, p);
+                load_slot(P.q[q_in], i, p);
                 active = enter_grid(P, B, p, rest_energy(p));
                 tail = 0;
             } else {
@@ -1035,7 +1115,7 @@ __global__ void __launch_bounds__(256, kMinBlocks) electron_kernel(TransportPara
         }
         if (!__any_sync(0xffffffffu, active || !exhausted)) break;
         if (!dry) dry = __any_sync(0xffffffffu, exhausted);
-        if (!active) continue;
+        if (!active || p.e <= ecut) continue;
         // Park a particle that outlives the round's input by tail_steps substeps
         // (its held deposit is released at the top of the next iteration).
         if (dry && ++tail > P.tail_steps) {
@@ -1050,17 +1130,9 @@ __global__ void __launch_bounds__(256, kMinBlocks) electron_kernel(TransportPara
             active = false;
             continue;
         }
-        if (p.e <= ecut) {  // terminal: local deposit (electron.py:347-365)
-            const int tm = __float_as_int(__ldg(P.vox + flat_index(p.x, p.y, p.z, P.gi)).y);
-            deposit(P, B, col_base(P, p), p.x, p.y, p.z, p.w * p.e, spr_factor(P, p.e, tm), dep);
-            if (p.kind == kPositron)
-                annihilate_at_rest(P, B, p, col_base(P, p), q_ph, spr_factor(P, kElectronMass, tm), dep,
-                                   n_push);
-            active = false;
-            continue;
-        }
         ++n_sub;
-        const float2 vx = __ldg(P.vox + flat_index(p.x, p.y, p.z, P.gi));
+        p.rng.fill_both();  // a substep's five draws: path, brems, hinge point, angle, azimuth
+        const float2 vx = __ldg(P.vox + voxel_of<kPlain>(p.x, p.y, p.z, P.gi));
         const float rho = vx.x;
         const int mat = __float_as_int(vx.y);
         const long long row = (long long)mat * T.n_points;
@@ -1104,7 +1176,7 @@ __global__ void __launch_bounds__(256, kMinBlocks) electron_kernel(TransportPara
         brems_step_parameters(p.e, A.w, rho, s, pcut, emit_p, local_brems);
         const float continuous = de + local_brems;
         const bool emit_brems = p.rng.uniform() < emit_p;
-        const float factor = spr_factor(P, p.e, mat);
+        const float factor = kPlain ? 1.0f : spr_factor(P, p.e, mat);
 
         // --- random hinge: move, deflect, move ---
         const float s1 = p.rng.uniform() * s;
@@ -1113,7 +1185,7 @@ __global__ void __launch_bounds__(256, kMinBlocks) electron_kernel(TransportPara
         if (s > 0.0f) d1 = continuous * (s1 / s);
         const float d2 = continuous - d1;
 
-        deposit_spread(P, B, col_base(P, p), p.x, p.y, p.z, p.ux, p.uy, p.uz, s1, p.w * d1, factor, dep);
+        deposit_spread<kPlain>(P, B, p.beamlet(), p.x, p.y, p.z, p.ux, p.uy, p.uz, s1, p.w * d1, factor, dep);
         p.e -= d1;
         p.x += p.ux * s1;
         p.y += p.uy * s1;
@@ -1138,6 +1210,7 @@ __global__ void __launch_bounds__(256, kMinBlocks) electron_kernel(TransportPara
         rotate_direction(p.ux, p.uy, p.uz, cos_hinge, phi);
 
         if (emit_brems && p.e > pcut) {
+            p.rng.reserve(2);
             float k = sample_brems_energy(p.e, pcut, p.rng);
             k = fminf(k, p.e - d2);
             if (k > pcut) {
@@ -1147,17 +1220,19 @@ __global__ void __launch_bounds__(256, kMinBlocks) electron_kernel(TransportPara
                     escape(B, (p.w - pw) * k);
                 }
                 if (pw > 0.0f) {
+                    p.rng.reserve(3);
                     const StreamId sid = p.rng.spawn();
-                    queue_push(P, q_ph, kPhoton, p.beamlet, k, pw, p.x, p.y, p.z, p.ux, p.uy, p.uz,
+                    queue_push(P, q_ph, kPhoton, p.beamlet(), k, pw, p.x, p.y, p.z, p.ux, p.uy, p.uz,
                                sid, n_push);
                 }
             } else {
-                deposit_or_escape(P, B, col_base(P, p), p.x, p.y, p.z, p.w * k, spr_factor(P, k, mat), dep);
+                deposit_or_escape<kPlain>(P, B, p.beamlet(), p.x, p.y, p.z, p.w * k,
+                                          kPlain ? 1.0f : spr_factor(P, k, mat), dep);
             }
             p.e -= k;
         }
 
-        deposit_spread(P, B, col_base(P, p), p.x, p.y, p.z, p.ux, p.uy, p.uz, s2, p.w * d2, factor, dep);
+        deposit_spread<kPlain>(P, B, p.beamlet(), p.x, p.y, p.z, p.ux, p.uy, p.uz, s2, p.w * d2, factor, dep);
         p.e -= d2;
         p.x += p.ux * s2;
         p.y += p.uy * s2;
@@ -1173,18 +1248,19 @@ __global__ void __launch_bounds__(256, kMinBlocks) electron_kernel(TransportPara
             const float w = sample_moller_delta_energy(p.e, ecut, p.rng);
             float cd, cp;
             moller_direction_cosines(p.e, w, cd, cp);
+            p.rng.reserve(4);
             const float mphi = kTwoPi * p.rng.uniform();
             float dx = p.ux, dy = p.uy, dz = p.uz;
             rotate_direction(dx, dy, dz, cd, mphi);
             const StreamId sid = p.rng.spawn();
-            queue_push(P, q_out, kElectron, p.beamlet, w, p.w, p.x, p.y, p.z, dx, dy, dz, sid,
+            queue_push(P, q_out, kElectron, p.beamlet(), w, p.w, p.x, p.y, p.z, dx, dy, dz, sid,
                        n_push);
             rotate_direction(p.ux, p.uy, p.uz, cp, mphi + kPi);
             p.e -= w;
         }
     }
 
-    dep.release(P);
+    dep.release(P, p.beamlet());
     block_sum_add(&B.substeps, n_sub);
     block_sum_add(&B.deposits, dep.n);
     block_sum_add(&B.pushes, n_push);
