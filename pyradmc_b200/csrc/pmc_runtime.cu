@@ -87,8 +87,9 @@ struct pmc_engine {
     size_t gs_cap = 0;
 
     // transport buffers
-    DevBuf queues;                // P0, P1, E0, E1, q_capacity slots each
-    unsigned int q_capacity = 0;
+    DevBuf queues;                // P0, P1, E0, E1, q_slots slots each
+    unsigned int q_capacity = 0;  // particles a queue may hold
+    unsigned int q_slots = 0;     // slots behind it
     DevBuf edep, s1, s2;          // [columns][col_stride] quanta and float64 sums
     DevBuf dirty, touched;        // sector bitmaps of edep / of the sums (pmc_reduce.cuh)
     bool edep_clean = false;      // every quanta entry is zero (true after a completed run)
@@ -387,13 +388,10 @@ int build_graph(pmc_engine* e, const TransportParams& P, const LaunchShape& L) {
 
 __global__ void init_batch_kernel(Sched* S, int batch, unsigned long long block_end,
                                   unsigned long long budget, long long max_rounds,
-                                  unsigned long long cond) {
+                                  unsigned long long cond, int window_el) {
     S->p_in = 0;
     S->e_in = 0;
-    for (int i = 0; i < 4; ++i) {
-        S->count[i] = 0u;
-        S->head[i] = 0u;
-    }
+    for (int i = 0; i < 4; ++i) retire_queue(S, i);
     S->cursor = 0ull;
     S->block_end = block_end;
     S->budget = budget;
@@ -404,6 +402,7 @@ __global__ void init_batch_kernel(Sched* S, int batch, unsigned long long block_
     S->rounds = 0;
     S->max_rounds = max_rounds;
     S->cond_handle = cond;
+    open_window(S, window_el);
 }
 
 struct SchedHost {
@@ -433,6 +432,7 @@ int check_flags(pmc_engine* e, const Sched& s) {
 struct RunPlan {
     LaunchShape shape;
     unsigned long long budget = 0;
+    unsigned int capacity = 0;  // particles a queue may hold in this call
     int wave = 1;  // batches transported together, each into its own quanta map
     long long max_steps = 0;
     int tail_steps = 0;
@@ -492,12 +492,21 @@ int prepare_transport(pmc_engine* e, const pmc_run_params* p, unsigned long long
     if (cap64 > 0x7fffffffull)
         return fail(e, PMC_ERR_INVALID, "chunk_size * queue_factor exceeds the queue index range");
     const unsigned int cap = (unsigned int)cap64;
-    if (cap > e->q_capacity) {
-        e->q_capacity = 0;  // (a failed call leaves no queue behind)
-        rc = ensure(e, e->queues, 4 * (size_t)cap * sizeof(Slot));
+    // room for the slots that chunked pushes and the primaries' window leave dead
+    // (two chunks and the window's own; a round's dead slots go with its queue)
+    const unsigned long long dead =
+        plan->budget + (unsigned long long)kChunk * (plan->shape.grid_ph + 2ull * plan->shape.grid_el + 2ull);
+    const unsigned long long slots64 = cap64 + dead;
+    if (slots64 > 0xffffffffull)
+        return fail(e, PMC_ERR_INVALID, "chunk_size * queue_factor exceeds the queue index range");
+    if (cap > e->q_capacity || (unsigned int)slots64 > e->q_slots) {
+        e->q_capacity = e->q_slots = 0;  // (a failed call leaves no queue behind)
+        rc = ensure(e, e->queues, 4 * (size_t)slots64 * sizeof(Slot));
         if (rc) return rc;
         e->q_capacity = cap;
+        e->q_slots = (unsigned int)slots64;
     }
+    plan->capacity = std::min(e->q_capacity, e->q_slots - (unsigned int)dead);
     plan->max_steps = p->max_steps > 0 ? p->max_steps : kDefaultMaxSteps;
     plan->tail_steps = p->tail_steps > 0 ? p->tail_steps
                        : p->tail_steps < 0 ? 0x7fffffff : kDefaultTailSteps;
@@ -512,8 +521,9 @@ TransportParams make_params(pmc_engine* e, const pmc_run_params* p, const RunPla
     P.cyl = e->cyl;
     P.vox = e->d_vox;
     P.tab = e->tab;
-    for (int i = 0; i < 4; ++i) P.q[i] = (Slot*)e->queues.p + (size_t)i * e->q_capacity;
-    P.capacity = e->q_capacity;
+    for (int i = 0; i < 4; ++i) P.q[i] = (Slot*)e->queues.p + (size_t)i * e->q_slots;
+    P.capacity = plan.capacity;
+    P.slots = e->q_slots;
     P.sched = e->d_sched;
     P.gen = e->d_gen;
     P.edep = (unsigned long long*)e->edep.p;
@@ -557,7 +567,7 @@ int run_wave(pmc_engine* e, const pmc_run_params* p, const RunPlan& plan, Transp
         }
     }
     init_batch_kernel<<<1, 1, 0, e->stream>>>(e->d_sched, batch, block, plan.budget, kMaxRounds,
-                                              graph ? (unsigned long long)e->cond : 0ull);
+                                              graph ? (unsigned long long)e->cond : 0ull, P.window_el);
     PMC_CUDA(e, cudaGetLastError());
     e->counters.kernel_launches += 1;
     if (graph) {
@@ -1470,6 +1480,7 @@ int pmc_run_forward(pmc_engine* e, const pmc_source_desc* src, const pmc_run_par
     if (rc) return rc;
     PMC_CUDA(e, cudaMemsetAsync(e->d_total_q, 0, sizeof(unsigned long long), e->stream));
     TransportParams P = make_params(e, p, plan);
+    P.window_el = (G.type == 0 || G.type == 1) && G.kind != PMC_PHOTON ? 1 : 0;
     float t_tr = 0.0f, t_red = 0.0f;
     for (int b = 0; b < p->n_batches; b += plan.wave) {
         const int in_wave = std::min(plan.wave, p->n_batches - b);

@@ -34,11 +34,22 @@ constexpr int kFlagOverflow = 1;
 constexpr int kFlagStepCap = 2;
 constexpr int kFlagRoundCap = 4;
 
+// A counter on a cache line of its own: atomics on one line pass one at a time.
+struct alignas(128) Counter32 {
+    unsigned int v;
+};
+
 // Device-resident scheduling state of one drain (a wave of statistical batches).
+// A queue (P0, P1, E0, E1) fills from both ends: whole chunks and the window of
+// fresh primaries from slot 0 up (bottom), single particles from its last slot
+// down (top).  Some bottom slots stay dead (marked; counted in `dead`).
 struct Sched {
+    Counter32 bottom[4];
+    Counter32 top[4];
+    Counter32 head[4];              // fetch heads
+    Counter32 dead[4];
     int p_in, e_in;                 // input photon / electron queue (0/1)
-    unsigned int count[4];          // push counters: P0, P1, E0, E1
-    unsigned int head[4];           // fetch heads
+    unsigned int window_base;       // first slot of the round's fresh primaries
     unsigned long long cursor;      // next primary of the wave
     unsigned long long limit;       // admission limit of the current round
     unsigned long long block_end;   // primaries in the wave
@@ -141,7 +152,9 @@ struct TransportParams {
     const float2* vox;    // (density, material bits) per transport voxel
     Tables tab;
     Slot* q[4];           // P0, P1, E0, E1
-    unsigned int capacity;
+    unsigned int capacity;     // particles a queue may hold
+    unsigned int slots;        // slots behind it: capacity and room for dead ones
+    int window_el;             // fresh primaries enter the electron queue (a charged source)
     Sched* sched;
     const GenDesc* gen;
     unsigned long long* edep;  // [batch of the wave][group][col_stride] int64 quanta
@@ -164,6 +177,7 @@ struct TransportParams {
 struct BlockBooks {
     unsigned long long flights, interactions, substeps, deposits, pushes, primaries;
     long long escaped, unscored, deposited, emitted, violations;
+    unsigned long long dead;  // slots a generator block left dead
 };
 
 __device__ __forceinline__ long long quantize_signed(float amount) {
@@ -330,18 +344,140 @@ __device__ __forceinline__ void deposit_spread(const TransportParams& P, BlockBo
     }
 }
 
-// Warp-aggregated queue push (one atomic per converged group of pushing lanes).
-__device__ __forceinline__ void queue_push(const TransportParams& P, int qi, int kind, int beamlet,
-                                           float e, float w, float x, float y, float z, float ux,
-                                           float uy, float uz, const StreamId& sid,
-                                           unsigned int& n_push) {
+// ---- queue slots ------------------------------------------------------------------
+// One atomic on a queue's counter per pushing group of lanes, and one per refill,
+// held the transport kernels to about one such atomic per nanosecond over the
+// whole GPU (two thirds of the photon kernel's stalls on a 1.2e6-primary round).
+// So a block takes slots kChunk at a time: its word (shared memory) is the chunk's
+// number above kOffBits bits of fill.  A group adds its size; the group that takes
+// a chunk's last slot opens the next one and publishes it, and groups that come
+// while it does so go to the top of the queue instead of waiting.  At most one add
+// per lane can follow the chunk's end before the next chunk is published, so the
+// fill never carries into the chunk number.  The slots a block leaves unused are
+// marked dead.
+constexpr unsigned int kChunk = 128;
+constexpr int kOffBits = 11;
+constexpr unsigned int kOffMask = (1u << kOffBits) - 1u;
+constexpr unsigned int kChunkedSlots = kChunk << (32 - kOffBits);  // slots a chunk number can name
+constexpr uint32_t kDeadMeta = 0xffffffffu;
+static_assert(kChunk + 1024 < kOffMask, "a block's lanes fit above the chunk in the fill field");
+
+__device__ __forceinline__ unsigned int round_to_chunk(unsigned long long n) {
+    return (unsigned int)((n + kChunk - 1) / kChunk * kChunk);
+}
+
+// Chunks pay where a round is long and the slots left unused do not count: at
+// 512 input particles per block and more (a small round takes single slots).
+__device__ __forceinline__ bool chunked_round(const TransportParams& P, unsigned int n_in) {
+    return n_in >= 512u * gridDim.x && P.slots <= kChunkedSlots;
+}
+
+// One thread: the block's first chunk of queue qi.
+__device__ __forceinline__ uint32_t open_chunk(const TransportParams& P, int qi) {
+    return atomicAdd(&P.sched->bottom[qi].v, kChunk) / kChunk << kOffBits;
+}
+
+// A slot of queue qi for every lane that gets here together (word: the block's
+// chunk, or null for single slots); P.slots and up when there is none.
+__device__ __forceinline__ unsigned int claim_slot(const TransportParams& P, int qi, uint32_t* word) {
     cg::coalesced_group g = cg::coalesced_threads();
-    unsigned int base = 0;
-    if (g.thread_rank() == 0) base = atomicAdd(&P.sched->count[qi], (unsigned int)g.size());
-    base = g.shfl(base, 0);
-    const unsigned int idx = base + g.thread_rank();
+    const unsigned int n = (unsigned int)g.size(), r = (unsigned int)g.thread_rank();
+    unsigned int first = 0u, rest = 0u, served = 0u;  // served lanes from `first`, the others from `rest`
+    if (r == 0u) {
+        bool single = true;
+        if (word != nullptr && (*(volatile uint32_t*)word & kOffMask) < kChunk) {
+            const uint32_t w = atomicAdd(word, n);
+            const unsigned int off = w & kOffMask;
+            if (off < kChunk) {
+                first = (w >> kOffBits) * kChunk + off;
+                served = min(n, kChunk - off);
+                single = false;
+                if (off + n >= kChunk) {  // the chunk's last slot: open the next
+                    rest = atomicAdd(&P.sched->bottom[qi].v, kChunk);
+                    atomicExch(word, (rest / kChunk << kOffBits) | (n - served));
+                }
+            }
+        }
+        if (single) {
+            rest = atomicAdd(&P.sched->top[qi].v, n);
+            served |= 0x100u;
+        }
+    }
+    first = g.shfl(first, 0);
+    rest = g.shfl(rest, 0);
+    served = g.shfl(served, 0);
+    if (served & 0x100u) return rest + r < P.slots ? P.slots - 1u - (rest + r) : P.slots;
+    return r < served ? first + r : rest + (r - served);
+}
+
+// Mark what is left of the block's chunk (whole block, after its last push).
+__device__ inline void close_chunk(const TransportParams& P, int qi, uint32_t word) {
+    const unsigned int off = word & kOffMask;
+    if (off >= kChunk) return;
+    if (threadIdx.x == 0) atomicAdd(&P.sched->dead[qi].v, kChunk - off);
+    for (unsigned int k = off + threadIdx.x; k < kChunk; k += blockDim.x) {
+        const unsigned int slot = (word >> kOffBits) * kChunk + k;
+        if (slot < P.slots) P.q[qi][slot].d = make_uint4(kDeadMeta, 0u, 0u, 0u);
+    }
+}
+
+// A round's input: particle i of queue qi, and how a warp takes its share.  The
+// warp claims particles `claim` at a time (one atomic, their slots prefetched into
+// the L2) and hands them to its idle lanes; small rounds are claimed one by one,
+// so that every warp gets some.
+struct Input {
+    int qi;
+    unsigned int n_bottom, n;        // particles from the bottom, in all
+    unsigned int next, left, claim;  // the warp's claimed particles; how many it claims
+
+    __device__ __forceinline__ void open(const TransportParams& P, int queue) {
+        Sched* S = P.sched;
+        qi = queue;
+        const unsigned int b = S->bottom[qi].v, t = S->top[qi].v;
+        n_bottom = min(b, P.slots);
+        n = n_bottom + min(t, P.slots - n_bottom);
+        if ((unsigned long long)b + t > (unsigned long long)P.capacity + S->dead[qi].v) {  // too many live ones
+            atomicOr(&S->flags, kFlagOverflow);
+            n = n_bottom = 0u;
+        }
+        const unsigned int warps = gridDim.x * (blockDim.x / 32u);
+        claim = n / warps >= 128u ? 32u : n / warps >= 16u ? 4u : 1u;
+        next = left = 0u;
+    }
+    __device__ __forceinline__ const Slot* slot(const TransportParams& P, unsigned int i) const {
+        return P.q[qi] + (i < n_bottom ? i : P.slots - 1u - (i - n_bottom));
+    }
+    // The particle number of each lane that wants one (all lanes of the warp call).
+    __device__ __forceinline__ unsigned int take(const TransportParams& P, bool want) {
+        const unsigned int need = __ballot_sync(0xffffffffu, want);
+        const unsigned int lane = threadIdx.x & 31u;
+        const unsigned int cnt = (unsigned int)__popc(need);
+        const unsigned int rank = (unsigned int)__popc(need & ((1u << lane) - 1u));
+        unsigned int i = next + rank;
+        if (cnt > left) {
+            const unsigned int more = max(claim, cnt - left);
+            unsigned int b = 0u;
+            if (lane == 0u) b = atomicAdd(&P.sched->head[qi].v, more);
+            b = __shfl_sync(0xffffffffu, b, 0);
+            if (lane < more && b + lane < n)
+                asm volatile("prefetch.global.L2 [%0];" ::"l"(__cvta_generic_to_global(slot(P, b + lane))));
+            if (rank >= left) i = b + (rank - left);
+            next = b + (cnt - left);
+            left = more - (cnt - left);
+        } else {
+            next += cnt;
+            left -= cnt;
+        }
+        return i;
+    }
+};
+
+__device__ __forceinline__ void queue_push(const TransportParams& P, int qi, uint32_t* word, int kind,
+                                           int beamlet, float e, float w, float x, float y, float z, float ux,
+                                           float uy, float uz, const StreamId& sid, unsigned int& n_push) {
+    const unsigned int idx = claim_slot(P, qi, word);
     ++n_push;
-    if (idx >= P.capacity) {
+    if (idx >= P.slots) {
         atomicOr(&P.sched->flags, kFlagOverflow);
         return;
     }
@@ -350,30 +486,6 @@ __device__ __forceinline__ void queue_push(const TransportParams& P, int qi, int
     s->b = make_float4(z, ux, uy, uz);
     s->c = make_uint4(sid.id_lo, sid.id_hi, sid.tag, sid.ctr);
     s->d = make_uint4(pack_meta(kind, 0, beamlet), 0u, 0u, 0u);
-}
-
-// Park an unfinished particle in queue qi for the next round: its whole state
-// (phase space, kind, primary flag, beamlet, stream position, steps taken)
-// goes into the slot, so the next round continues it exactly where it stopped.
-template <class R>
-struct ParticleOf;
-template <class R>
-__device__ __forceinline__ void queue_suspend(const TransportParams& P, int qi, const ParticleOf<R>& p,
-                                              unsigned int& n_push);
-
-__device__ __forceinline__ unsigned long long fetch_one(unsigned long long* ctr) {
-    cg::coalesced_group g = cg::coalesced_threads();
-    unsigned long long base = 0;
-    if (g.thread_rank() == 0) base = atomicAdd(ctr, (unsigned long long)g.size());
-    base = g.shfl(base, 0);
-    return base + g.thread_rank();
-}
-__device__ __forceinline__ unsigned int fetch_one(unsigned int* ctr) {
-    cg::coalesced_group g = cg::coalesced_threads();
-    unsigned int base = 0;
-    if (g.thread_rank() == 0) base = atomicAdd(ctr, (unsigned int)g.size());
-    base = g.shfl(base, 0);
-    return base + g.thread_rank();
 }
 
 // ---- particle state ----------------------------------------------------------------
@@ -389,9 +501,9 @@ struct ParticleOf {
 };
 using Particle = ParticleOf<Rng>;  // of the generator
 
+// False for a dead slot.
 template <class R>
-__device__ __forceinline__ void load_slot(const Slot* q, unsigned int i, ParticleOf<R>& p) {
-    const Slot* s = q + i;
+__device__ __forceinline__ bool load_slot(const Slot* s, ParticleOf<R>& p) {
     const float4 a = s->a, b = s->b;
     const uint4 c = s->c, d = s->d;
     p.e = a.x; p.w = a.y; p.x = a.z; p.y = a.w;
@@ -399,27 +511,31 @@ __device__ __forceinline__ void load_slot(const Slot* q, unsigned int i, Particl
     p.meta = d.x;
     p.steps = (int)d.y;
     p.rng.load(StreamId{c.x, c.y, c.z, c.w});
+    return d.x != kDeadMeta;
 }
 
+// A particle's whole state (phase space, kind, primary flag, beamlet, stream
+// position, steps taken) in a slot: whoever loads it continues exactly there.
 template <class R>
-__device__ __forceinline__ void queue_suspend(const TransportParams& P, int qi, const ParticleOf<R>& p,
-                                              unsigned int& n_push) {
-    cg::coalesced_group g = cg::coalesced_threads();
-    unsigned int base = 0;
-    if (g.thread_rank() == 0) base = atomicAdd(&P.sched->count[qi], (unsigned int)g.size());
-    base = g.shfl(base, 0);
-    const unsigned int idx = base + g.thread_rank();
-    ++n_push;
-    if (idx >= P.capacity) {
-        atomicOr(&P.sched->flags, kFlagOverflow);
-        return;
-    }
-    Slot* s = P.q[qi] + idx;
+__device__ __forceinline__ void store_slot(Slot* s, const ParticleOf<R>& p) {
     const StreamId sid = p.rng.state();
     s->a = make_float4(p.e, p.w, p.x, p.y);
     s->b = make_float4(p.z, p.ux, p.uy, p.uz);
     s->c = make_uint4(sid.id_lo, sid.id_hi, sid.tag, sid.ctr);
     s->d = make_uint4(p.meta, (uint32_t)p.steps, 0u, 0u);
+}
+
+// Queue an unfinished particle (parked for the next round, or a fresh one).
+template <class R>
+__device__ __forceinline__ void queue_suspend(const TransportParams& P, int qi, const ParticleOf<R>& p,
+                                              unsigned int& n_push) {
+    const unsigned int idx = claim_slot(P, qi, nullptr);
+    ++n_push;
+    if (idx >= P.slots) {
+        atomicOr(&P.sched->flags, kFlagOverflow);
+        return;
+    }
+    store_slot(P.q[qi] + idx, p);
 }
 
 // Copy `n` table entries into the block's shared memory (strided over the block).
@@ -669,11 +785,25 @@ __device__ __forceinline__ void annihilate_at_rest(const TransportParams& P, Blo
     for (int k = 0; k < 2; ++k) {  // two photons back to back
         p.rng.reserve(3);
         const StreamId sid = p.rng.spawn();
-        queue_push(P, q_photon, kPhoton, p.beamlet(), kElectronMass, p.w, p.x, p.y, p.z, ax, ay, az, sid, n_push);
+        queue_push(P, q_photon, nullptr, kPhoton, p.beamlet(), kElectronMass, p.w, p.x, p.y, p.z, ax, ay, az, sid,
+                   n_push);
         ax = -ax;
         ay = -ay;
         az = -az;
     }
+}
+
+__device__ __forceinline__ void retire_queue(Sched* S, int qi) {
+    S->bottom[qi].v = S->top[qi].v = S->head[qi].v = S->dead[qi].v = 0u;
+}
+
+// Set the next admission window's slots aside at the bottom of the queue its
+// primaries enter (nothing else is pushed until they are written).
+__device__ __forceinline__ void open_window(Sched* S, int window_el) {
+    unsigned int* bottom = &S->bottom[window_el ? 2 + S->e_in : S->p_in].v;
+    const unsigned int base = __ldcg(bottom);
+    S->window_base = base;
+    *bottom = base + round_to_chunk(S->limit - S->cursor);
 }
 
 // ---- last-block scheduler steps ------------------------------------------------------
@@ -709,7 +839,7 @@ __device__ inline void flush_books(const TransportParams& P, BlockBooks& B) {
 
 __device__ __forceinline__ void init_books(BlockBooks& B) {
     if (threadIdx.x == 0) {
-        B.flights = B.interactions = B.substeps = B.deposits = B.pushes = B.primaries = 0ull;
+        B.flights = B.interactions = B.substeps = B.deposits = B.pushes = B.primaries = B.dead = 0ull;
         B.escaped = B.unscored = B.deposited = B.emitted = B.violations = 0ll;
     }
     __syncthreads();
@@ -753,7 +883,13 @@ __global__ void __launch_bounds__(kPhotonThreads, kMinBlocks) photon_kernel(Tran
     Sched* S = P.sched;
     const int pin = S->p_in, ein = S->e_in;
     const int q_in = pin, q_out = pin ^ 1, q_el = 2 + ein;
-    const unsigned int n_in = min(S->count[q_in], P.capacity);
+    Input in;
+    in.open(P, q_in);
+    __shared__ uint32_t chunk_el;  // the block's chunk of the electron queue
+    const bool chunked = chunked_round(P, in.n);
+    if (threadIdx.x == 0) chunk_el = chunked ? open_chunk(P, q_el) : 0u;
+    __syncthreads();
+    uint32_t* const word_el = chunked ? &chunk_el : nullptr;
     const Tables& T = P.tab;
     const float pcut = P.pcut, ecut = P.ecut;
 
@@ -763,6 +899,8 @@ __global__ void __launch_bounds__(kPhotonThreads, kMinBlocks) photon_kernel(Tran
     p.rng.k0 = P.seed_lo;
     p.rng.k1 = P.seed_hi;
     p.rng.ring = ring + threadIdx.x;
+    long long escaped = 0;  // most photons end that way: summed per lane, booked once
+    auto leave = [&](float amount) { escaped += quantize_signed(amount); };
     bool active = false, exhausted = false, dry = false;
     int tail = 0;  // steps of the current photon since its warp found the round dry
     float e_tab = -1.0f, maj = 0.0f;
@@ -775,15 +913,17 @@ __global__ void __launch_bounds__(kPhotonThreads, kMinBlocks) photon_kernel(Tran
             if (__any_sync(0xffffffffu, (*(volatile int*)&S->flags) & (kFlagOverflow | kFlagStepCap)))
                 break;
         }
-        if (!active && !exhausted) {  // the round's photons: secondaries, parked, then primaries
-            const unsigned int i = fetch_one(&S->head[q_in]);
-            if (i < n_in) {
-                load_slot(P.q[q_in], i, p);
-                active = enter_grid(P, B, p, 0.0f);
-                e_tab = -1.0f;
-                tail = 0;
-            } else {
-                exhausted = true;
+        const bool want = !active && !exhausted;  // the round's photons: secondaries, primaries, parked
+        if (__any_sync(0xffffffffu, want)) {
+            const unsigned int i = in.take(P, want);
+            if (want) {
+                if (i < in.n) {
+                    active = load_slot(in.slot(P, i), p) && enter_grid(P, B, p, 0.0f);
+                    e_tab = -1.0f;
+                    tail = 0;
+                } else {
+                    exhausted = true;
+                }
             }
         }
         if (!__any_sync(0xffffffffu, active || !exhausted)) break;
@@ -801,7 +941,7 @@ __global__ void __launch_bounds__(kPhotonThreads, kMinBlocks) photon_kernel(Tran
         // ---- one Woodcock flight (photon.py:150-181) ----
         if (++p.steps > P.max_steps) {
             atomicOr(&S->flags, kFlagStepCap);
-            escape(B, p.w * p.e);
+            leave(p.w * p.e);
             active = false;
             continue;
         }
@@ -818,7 +958,7 @@ __global__ void __launch_bounds__(kPhotonThreads, kMinBlocks) photon_kernel(Tran
         p.y += step * p.uy;
         p.z += step * p.uz;
         if (!point_inside(p.x, p.y, p.z, P.gi)) {
-            escape(B, p.w * p.e);
+            leave(p.w * p.e);
             active = false;
             continue;
         }
@@ -835,7 +975,7 @@ __global__ void __launch_bounds__(kPhotonThreads, kMinBlocks) photon_kernel(Tran
         const float mu_real = mc + mp + mpa + mr;
         if (mu_real > maj * (1.0f + 1.0e-9f)) {
             book_add(&B.violations, 1);
-            escape(B, p.w * p.e);
+            leave(p.w * p.e);
             active = false;
             continue;
         }
@@ -867,7 +1007,7 @@ __global__ void __launch_bounds__(kPhotonThreads, kMinBlocks) photon_kernel(Tran
                     float ex = p.ux, ey = p.uy, ez = p.uz;
                     rotate_direction(ex, ey, ez, compton_electron_cos_theta(p.e, ratio), phi + kPi);
                     const StreamId sid = p.rng.spawn();
-                    queue_push(P, q_el, kElectron, p.beamlet(), recoil, split_w, p.x, p.y, p.z, ex, ey, ez, sid,
+                    queue_push(P, q_el, word_el, kElectron, p.beamlet(), recoil, split_w, p.x, p.y, p.z, ex, ey, ez, sid,
                                n_push);
                 } else {
                     put(split_w * recoil, recoil);
@@ -884,13 +1024,13 @@ __global__ void __launch_bounds__(kPhotonThreads, kMinBlocks) photon_kernel(Tran
                 p.rng.reserve(4);
                 if (es < kRouletteMeV && cw < kRouletteWeightCap) {
                     const float nw = roulette_weight(cw, kRouletteSurvival, p.rng);
-                    escape(B, (cw - nw) * es);
+                    leave((cw - nw) * es);
                     if (nw == 0.0f) keep = false;
                     else cw = nw;
                 }
                 if (keep) {
                     const StreamId sid = p.rng.spawn();
-                    queue_push(P, q_out, kPhoton, p.beamlet(), es, cw, p.x, p.y, p.z, gx, gy, gz, sid, n_push);
+                    queue_push(P, q_out, nullptr, kPhoton, p.beamlet(), es, cw, p.x, p.y, p.z, gx, gy, gz, sid, n_push);
                 }
             }
             active = false;
@@ -922,7 +1062,7 @@ __global__ void __launch_bounds__(kPhotonThreads, kMinBlocks) photon_kernel(Tran
             if (process == 0)
                 rotate_direction(ex, ey, ez, compton_electron_cos_theta(p.e, ratio), phi + kPi);
             const StreamId sid = p.rng.spawn();
-            queue_push(P, q_el, kElectron, p.beamlet(), ee, p.w, p.x, p.y, p.z, ex, ey, ez, sid, n_push);
+            queue_push(P, q_el, word_el, kElectron, p.beamlet(), ee, p.w, p.x, p.y, p.z, ex, ey, ez, sid, n_push);
         } else {
             put(p.w * ee, ee);
         }
@@ -938,7 +1078,7 @@ __global__ void __launch_bounds__(kPhotonThreads, kMinBlocks) photon_kernel(Tran
             if (p.e < kRouletteMeV && p.w < kRouletteWeightCap) {
                 p.rng.reserve(1);
                 const float nw = roulette_weight(p.w, kRouletteSurvival, p.rng);
-                escape(B, (p.w - nw) * p.e);
+                leave((p.w - nw) * p.e);
                 if (nw == 0.0f) {
                     active = false;
                     continue;
@@ -952,8 +1092,8 @@ __global__ void __launch_bounds__(kPhotonThreads, kMinBlocks) photon_kernel(Tran
             if (P.transport_electrons && share_p > ecut) {
                 p.rng.reserve(3);
                 const StreamId sid = p.rng.spawn();
-                queue_push(P, q_el, kPositron, p.beamlet(), share_p, p.w, p.x, p.y, p.z, p.ux, p.uy, p.uz, sid,
-                           n_push);
+                queue_push(P, q_el, word_el, kPositron, p.beamlet(), share_p, p.w, p.x, p.y, p.z, p.ux, p.uy,
+                           p.uz, sid, n_push);
             } else {
                 if (P.transport_electrons) put(p.w * share_p, share_p);
                 annihilate_at_rest<kPlain>(P, B, p, voxel, q_out,
@@ -963,6 +1103,9 @@ __global__ void __launch_bounds__(kPhotonThreads, kMinBlocks) photon_kernel(Tran
         active = false;
     }
 
+    __syncthreads();
+    if (chunked) close_chunk(P, q_el, chunk_el);
+    block_sum_add(reinterpret_cast<unsigned long long*>(&B.escaped), (unsigned long long)escaped);
     block_sum_add(&B.flights, n_flight);
     block_sum_add(&B.interactions, n_inter);
     block_sum_add(&B.deposits, dep.n);
@@ -972,8 +1115,7 @@ __global__ void __launch_bounds__(kPhotonThreads, kMinBlocks) photon_kernel(Tran
     // The last block retires the consumed photon queue; the round's admission
     // window has been generated.
     if (last_block_arrives(S) && threadIdx.x == 0) {
-        S->count[q_in] = 0u;
-        S->head[q_in] = 0u;
+        retire_queue(S, q_in);
         S->p_in = q_out;
         S->cursor = S->limit;
         S->blocks_done = 0u;
@@ -984,37 +1126,56 @@ __global__ void __launch_bounds__(kPhotonThreads, kMinBlocks) photon_kernel(Tran
 // ---- the primary generator ---------------------------------------------------------
 // The round's admission window [cursor, limit) of the wave, one thread
 // per primary (kernels.py:1888-2401): sampled at full warp width, flown
-// through vacuum to the grid, then queued with its stream position — photons
-// into the round's photon input queue behind the secondaries already there,
-// charged primaries into its electron queue.  The photon kernel then loads
-// every particle the same way, and no lane of it idles behind another's
-// primary sampling.
+// through vacuum to the grid, then queued with its stream position.  The slots
+// are set aside by the scheduler, primary t in slot window_base + (t - cursor)
+// (no atomics) of the photon queue, behind the secondaries already there, or of
+// the electron queue for a charged source; a primary that is not to be
+// transported there leaves its slot dead, a charged one of a mixed source goes to
+// the electron queue.
 __global__ void __launch_bounds__(256) generate_kernel(TransportParams P) {
     __shared__ BlockBooks B;
     init_books(B);
     Sched* S = P.sched;
     const unsigned long long cursor = S->cursor, limit = S->limit;
     const int q_ph = S->p_in, q_el = 2 + S->e_in;
+    const int q_win = P.window_el ? q_el : q_ph;
+    const unsigned int base = S->window_base;
     const int batch = S->batch;
     const GenDesc& G = *P.gen;
-    unsigned int n_push = 0, n_prim = 0;
+    unsigned int n_push = 0, n_prim = 0, n_dead = 0;
     const unsigned long long stride = (unsigned long long)gridDim.x * blockDim.x;
-    for (unsigned long long t = cursor + (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x;
-         t < limit; t += stride) {
+    const unsigned int window = round_to_chunk(limit - cursor);
+    for (unsigned long long k = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x; k < window; k += stride) {
         Particle p;
-        ++n_prim;
-        const int kind = generate_primary(P, G, batch, t, p, B);
-        if (kind < 0) continue;
-        if (kind == kPhoton) {
-            if (enter_grid(P, B, p, 0.0f)) queue_suspend(P, q_ph, p, n_push);
-        } else {  // charged primary: to the electron queue unchanged (it enters there)
-            queue_push(P, q_el, kind, p.beamlet(), p.e, p.w, p.x, p.y, p.z, p.ux, p.uy, p.uz,
-                       p.rng.state(), n_push);
+        const unsigned int slot = base + (unsigned int)k;
+        bool queued = false;
+        if (cursor + k < limit) {
+            ++n_prim;
+            const int kind = generate_primary(P, G, batch, cursor + k, p, B);
+            if (kind >= 0 && P.window_el) {
+                queued = true;  // (it enters the grid in the electron kernel)
+            } else if (kind == kPhoton) {
+                queued = enter_grid(P, B, p, 0.0f);
+            } else if (kind > 0) {
+                queue_push(P, q_el, nullptr, kind, p.beamlet(), p.e, p.w, p.x, p.y, p.z, p.ux, p.uy, p.uz,
+                           p.rng.state(), n_push);
+            }
+        }
+        n_push += queued ? 1u : 0u;
+        n_dead += queued ? 0u : 1u;
+        if (slot >= P.slots) {
+            atomicOr(&S->flags, kFlagOverflow);
+        } else if (queued) {
+            store_slot(P.q[q_win] + slot, p);
+        } else {
+            P.q[q_win][slot].d = make_uint4(kDeadMeta, 0u, 0u, 0u);
         }
     }
     block_sum_add(&B.pushes, n_push);
     block_sum_add(&B.primaries, n_prim);
+    block_sum_add(&B.dead, n_dead);
     flush_books(P, B);
+    if (threadIdx.x == 0 && B.dead) atomicAdd(&S->dead[q_win].v, (unsigned int)B.dead);
 }
 
 // Annihilation energy a positron still carries (2 m c^2), booked with it on escape.
@@ -1064,7 +1225,17 @@ electron_kernel(TransportParams P) {
     Sched* S = P.sched;
     const int pin = S->p_in, ein = S->e_in;
     const int q_in = 2 + ein, q_out = 2 + (ein ^ 1), q_ph = pin;
-    const unsigned int n_in = min(S->count[q_in], P.capacity);
+    Input in;
+    in.open(P, q_in);
+    __shared__ uint32_t chunks[2];  // the block's chunks of the next electron and photon queues
+    const bool chunked = chunked_round(P, in.n);
+    if (threadIdx.x == 0 && chunked) {
+        chunks[0] = open_chunk(P, q_out);
+        chunks[1] = open_chunk(P, q_ph);
+    }
+    __syncthreads();
+    uint32_t* const word_el = chunked ? chunks : nullptr;
+    uint32_t* const word_ph = chunked ? chunks + 1 : nullptr;
     const Tables& T = P.tab;
     const float pcut = P.pcut, ecut = P.ecut;
 
@@ -1103,14 +1274,16 @@ electron_kernel(TransportParams P) {
             active = false;
         }
         if (!active) dep.release(P, p.beamlet());  // the finished particle's last held deposit
-        if (!active && !exhausted) {
-            const unsigned int i = fetch_one(&S->head[q_in]);
-            if (i < n_in) {
-                load_slot(P.q[q_in], i, p);
-                active = enter_grid(P, B, p, rest_energy(p));
-                tail = 0;
-            } else {
-                exhausted = true;
+        const bool want = !active && !exhausted;
+        if (__any_sync(0xffffffffu, want)) {
+            const unsigned int i = in.take(P, want);
+            if (want) {
+                if (i < in.n) {
+                    active = load_slot(in.slot(P, i), p) && enter_grid(P, B, p, rest_energy(p));
+                    tail = 0;
+                } else {
+                    exhausted = true;
+                }
             }
         }
         if (!__any_sync(0xffffffffu, active || !exhausted)) break;
@@ -1222,7 +1395,7 @@ electron_kernel(TransportParams P) {
                 if (pw > 0.0f) {
                     p.rng.reserve(3);
                     const StreamId sid = p.rng.spawn();
-                    queue_push(P, q_ph, kPhoton, p.beamlet(), k, pw, p.x, p.y, p.z, p.ux, p.uy, p.uz,
+                    queue_push(P, q_ph, word_ph, kPhoton, p.beamlet(), k, pw, p.x, p.y, p.z, p.ux, p.uy, p.uz,
                                sid, n_push);
                 }
             } else {
@@ -1253,7 +1426,7 @@ electron_kernel(TransportParams P) {
             float dx = p.ux, dy = p.uy, dz = p.uz;
             rotate_direction(dx, dy, dz, cd, mphi);
             const StreamId sid = p.rng.spawn();
-            queue_push(P, q_out, kElectron, p.beamlet(), w, p.w, p.x, p.y, p.z, dx, dy, dz, sid,
+            queue_push(P, q_out, word_el, kElectron, p.beamlet(), w, p.w, p.x, p.y, p.z, dx, dy, dz, sid,
                        n_push);
             rotate_direction(p.ux, p.uy, p.uz, cp, mphi + kPi);
             p.e -= w;
@@ -1261,6 +1434,11 @@ electron_kernel(TransportParams P) {
     }
 
     dep.release(P, p.beamlet());
+    __syncthreads();
+    if (chunked) {
+        close_chunk(P, q_out, chunks[0]);
+        close_chunk(P, q_ph, chunks[1]);
+    }
     block_sum_add(&B.substeps, n_sub);
     block_sum_add(&B.deposits, dep.n);
     block_sum_add(&B.pushes, n_push);
@@ -1269,15 +1447,18 @@ electron_kernel(TransportParams P) {
     // The last block retires the consumed electron queue, opens the next
     // admission window and publishes whether any work is left.
     if (last_block_arrives(S) && threadIdx.x == 0) {
-        S->count[q_in] = 0u;
-        S->head[q_in] = 0u;
+        retire_queue(S, q_in);
         S->e_in = ein ^ 1;
         S->rounds += 1;
         S->total_rounds += 1;
         const unsigned long long next_limit = S->cursor + S->budget;
         S->limit = next_limit < S->block_end ? next_limit : S->block_end;
-        const bool work = S->cursor < S->block_end || S->count[S->p_in] > 0u ||
-                          S->count[2 + (ein ^ 1)] > 0u;
+        // particles queued, beside the dead slots
+        auto queued = [S](int qi) {
+            return __ldcg(&S->bottom[qi].v) + __ldcg(&S->top[qi].v) > __ldcg(&S->dead[qi].v);
+        };
+        const bool work = S->cursor < S->block_end || queued(S->p_in) || queued(S->e_in + 2);
+        open_window(S, P.window_el);
         int remaining = work ? 1 : 0;
         if (S->flags & (kFlagOverflow | kFlagStepCap)) remaining = 0;
         if (remaining && S->rounds >= S->max_rounds) {
