@@ -72,6 +72,32 @@ __host__ __device__ inline void philox4x32_10(uint32_t c[4], uint32_t k0, uint32
     }
 }
 
+// The same with the ten rounds' keys at hand: rk[2 i], rk[2 i + 1] = k0 + i W0, k1 + i W1.
+struct PhiloxKeys {
+    uint32_t rk[20];
+};
+inline PhiloxKeys philox_keys(uint32_t k0, uint32_t k1) {
+    PhiloxKeys k;
+    for (uint32_t i = 0; i < 10u; ++i) {
+        k.rk[2 * i] = k0 + i * kPhiloxW0;
+        k.rk[2 * i + 1] = k1 + i * kPhiloxW1;
+    }
+    return k;
+}
+__device__ __forceinline__ void philox4x32_10(uint32_t c[4], const PhiloxKeys& k) {
+#pragma unroll
+    for (int round = 0; round < 10; ++round) {
+        const uint32_t lo0 = kPhiloxM0 * c[0];
+        const uint32_t hi0 = __umulhi(kPhiloxM0, c[0]);
+        const uint32_t lo1 = kPhiloxM1 * c[2];
+        const uint32_t hi1 = __umulhi(kPhiloxM1, c[2]);
+        c[0] = hi1 ^ c[1] ^ k.rk[2 * round];
+        c[1] = lo1;
+        c[2] = hi0 ^ c[3] ^ k.rk[2 * round + 1];
+        c[3] = lo0;
+    }
+}
+
 // Stream identity carried by a queued particle (16 bytes).
 struct StreamId {
     uint32_t id_lo, id_hi, tag, ctr;
@@ -139,9 +165,13 @@ struct Rng {
 // kernel (a lane's words lie kStride apart, so a warp's draws never share a bank).
 constexpr int kRingWords = 8;
 
-template <int kStride>
+// kKeys: the round keys come from the kernel's parameters instead of being added
+// up in every refill (photon kernel 5.6 -> 5.0 ms on the 100-column 128^3 Dij; in
+// the electron kernel, two blocks at once, the added registers cost 1 ms of 9.8).
+template <int kStride, bool kKeys>
 struct RingRng {
-    uint32_t k0, k1;   // run seed
+    uint32_t k0, k1;         // run seed
+    const PhiloxKeys* keys;  // of the run seed (kKeys)
     uint32_t id_lo, id_hi, tag;
     uint32_t ctr;      // uniforms consumed
     uint32_t end;      // words [ctr, end) are in the ring (end a multiple of 4, end - ctr <= 8)
@@ -157,7 +187,8 @@ struct RingRng {
     // Block `block` of the stream into its half of the ring.
     __device__ __forceinline__ void fill(uint32_t block) {
         uint32_t c[4] = {block, id_lo, id_hi, tag};
-        philox4x32_10(c, k0, k1);
+        if constexpr (kKeys) philox4x32_10(c, *keys);
+        else philox4x32_10(c, k0, k1);
         uint32_t* r = ring + (block & 1u) * (4 * kStride);
         r[0] = c[0];
         r[kStride] = c[1];

@@ -131,147 +131,217 @@ __device__ __forceinline__ void column_max(unsigned long long best, unsigned lon
     if ((threadIdx.x & 31) == 0 && best) atomicMax(col_max_bits, best);
 }
 
-// The part of the sector bitmaps one warp walks: `words` consecutive words (1 to
-// 32, dividing a tile's 32) of one column, one per lane.
+// How the fold and finalize walk the sector bitmaps.  A part is `words` consecutive
+// words (1 to 32, dividing a tile's 32) of one column, one per lane of a warp.  The
+// warps of a resident grid claim `claim` parts at a time from a counter, the next
+// part's words on their way while the current one is folded.  Most parts of a Dij
+// are empty and the full ones lie side by side (a beam's core): with a warp
+// launched per tile, the launches of the empty ones and the blocks that held one
+// full tile each took most of the time (16 % of the warps active), and parts dealt
+// out in turn still left some warps half again as long as the others.
 struct FoldShape {
     long long n_vox, stride;  // voxels and entries of a column
-    int words;                // bitmap words per warp
-    int parts_per_col;        // warps per column
-    long long n_parts;        // warps in all
+    int words;                // bitmap words per part
+    int parts_per_col;
+    unsigned int n_parts, claim;
+    unsigned int* next;       // parts claimed so far (zero at launch)
     int n_maps;               // quanta maps of the wave, in batch order
     long long map_entries;    // entries of one map
 };
 
+// The next claim of a warp: its first part (n_parts and up: none left).
+__device__ __forceinline__ unsigned int claim_parts(const FoldShape& f) {
+    unsigned int t = 0u;
+    if ((threadIdx.x & 31) == 0) t = atomicAdd(f.next, f.claim);
+    return __shfl_sync(0xffffffffu, t, 0);
+}
+
+// x / y correctly rounded, from r = 1 / y correctly rounded: two Newton corrections
+// of x r, each with an exact remainder (Markstein, "Computation of elementary
+// functions on the IBM RISC System/6000 processor", IBM J. Res. Dev. 34, 1990: the
+// second one rounds correctly, the first having left a quotient within one unit in
+// the last place).  Finite operands away from the ends of the exponent range, or
+// y = r = 0, which gives 0.
+__device__ __forceinline__ double divide_by(double x, double y, double r) {
+    double q = __dmul_rn(x, r);
+    q = __fma_rn(__fma_rn(-q, y, x), r, q);
+    return __fma_rn(__fma_rn(-q, y, x), r, q);
+}
+
 // Fold a wave's quanta maps, batch by batch, into the running sums and consume
 // them (reset the folded entries): d = q * 1e-9 / (mass * n), s1 += d, s2 += d^2
-// (kernels.py:804-852).  A lane owns one dirty sector: its mass, sums and quanta
-// are read with 16-byte loads and every batch of the wave is added in registers,
-// so the sums cross memory once per wave instead of once per batch.  kFinal: the
-// wave holds every batch of the run, so every touched sector is dirty here and
-// the mean, sigma and column maximum are written at once (finalize_sparse_kernel
-// otherwise).  What bounds it: the latency of the scattered 32-byte sectors.  A
-// warp walks as few bitmap words as leaves the GPU enough warps (fold_words): on
-// a 16^3 map one warp walking the whole map took 88 us a batch, all latency.
+// (kernels.py:804-852).  A lane owns half a dirty sector (two entries, 16-byte
+// loads) and goes through those of the wave's maps whose own bitmap has the sector,
+// in batch order (most sectors are hit in one or two of the batches), the next
+// map's quanta on their way while the current ones are added in registers; the
+// sums cross memory once per wave.  kFinal: the wave holds every batch of the run,
+// so every touched sector is dirty here and the mean, sigma and column maximum are
+// written at once (finalize_sparse_kernel otherwise).  What bounds it: the latency
+// of scattered 32-byte sectors, some 1e7 of them per wave of the 100-column 128^3
+// Dij, then the issue of the float64 arithmetic (one reciprocal per entry instead
+// of a division per entry and batch).
+constexpr int kWaveMaps = 32;  // the most maps of a wave
+
 template <bool kFinal>
-__global__ void __launch_bounds__(kReduceThreads)
+__global__ void __launch_bounds__(kReduceThreads, 4)
 fold_sparse_kernel(unsigned long long* __restrict__ edep, const double* __restrict__ mass,
                    const double* __restrict__ col_nhist, FoldShape f, double* __restrict__ s1,
                    double* __restrict__ s2, unsigned int* __restrict__ dirty,
                    unsigned int* __restrict__ touched, int n_batches,
                    unsigned long long* __restrict__ col_max_bits, unsigned long long* __restrict__ total_q) {
+    __shared__ unsigned int map_word[kReduceThreads / 32][kWaveMaps][32];  // the part's words, map by map
     const int lane = threadIdx.x & 31;
-    const long long t = (long long)blockIdx.x * (kReduceThreads / 32) + (threadIdx.x >> 5);
-    if (t >= f.n_parts) return;  // warp-uniform
-    const long long col = t / f.parts_per_col;
-    const long long word0 = (t - col * f.parts_per_col) * f.words;  // in the column
-    const long long widx = col * (f.stride / kWordEntries) + word0 + lane;
+    unsigned int (*mine)[32] = map_word[threadIdx.x >> 5];
     const long long map_words = f.map_entries / kWordEntries;
-    const bool mine = lane < f.words;
-    unsigned int w = 0u;
-    for (int m = 0; m < f.n_maps; ++m)
-        if (mine) w |= dirty[m * map_words + widx];
-    if (__ballot_sync(0xffffffffu, w != 0u) == 0u) return;
-    const unsigned int tw = mine ? touched[widx] : 0u;
-    const int incl = warp_inclusive_scan(__popc(w));
-    const int total = __shfl_sync(0xffffffffu, incl, 31);
-    const double nh = col_nhist[col];
     const double n = (double)n_batches;
-    unsigned long long local = 0, best = 0;
-    for (int k0 = 0; k0 < total; k0 += 32) {
-        const int k = k0 + lane;
-        int bit;
-        const int j = nth_set_sector(w, incl, k, bit);
-        const unsigned int twj = __shfl_sync(0xffffffffu, tw, j);
-        if (k >= total) continue;
-        const bool first = ((twj >> bit) & 1u) == 0u;
-        const long long v0 = (word0 + j) * kWordEntries + bit * kSectorEntries;
-        const long long at = col * f.stride + v0;
-        SectorD a, b;
-        double m_nh[kSectorEntries];
-#pragma unroll
-        for (int e = 0; e < kSectorEntries; ++e) {
-            const double m = v0 + e < f.n_vox ? mass[v0 + e] : 0.0;
-            m_nh[e] = m > 0.0 ? __dmul_rn(m, nh) : 0.0;
-            a.v[e] = b.v[e] = 0.0;
-        }
-        if (!first) {
-            a.load(s1 + at);
-            b.load(s2 + at);
-        }
+    // a part's words lie at part * words (the columns' words follow one another)
+    auto dirty_word = [&](unsigned int part, unsigned int end) {
+        unsigned int w = 0u;
+        if (part < end && lane < f.words) {
+            const unsigned int* p = dirty + (long long)part * f.words + lane;
 #pragma unroll 4
-        for (int m = 0; m < f.n_maps; ++m) {
-            ulonglong2* q = reinterpret_cast<ulonglong2*>(edep + m * f.map_entries + at);
-            const ulonglong2 lo = q[0], hi = q[1];
-            const unsigned long long qe[kSectorEntries] = {lo.x, lo.y, hi.x, hi.y};
-            if ((lo.x | lo.y | hi.x | hi.y) == 0ull) continue;
-            q[0] = q[1] = make_ulonglong2(0ull, 0ull);
-#pragma unroll
-            for (int e = 0; e < kSectorEntries; ++e) {
-                if (qe[e] == 0ull) continue;
-                double d = 0.0;
-                if (m_nh[e] > 0.0) d = __ddiv_rn(__dmul_rn((double)(long long)qe[e], kQuantum), m_nh[e]);
-                a.v[e] = __dadd_rn(a.v[e], d);
-                b.v[e] = __dadd_rn(b.v[e], __dmul_rn(d, d));
-                local += qe[e];
-            }
+            for (int m = 0; m < f.n_maps; ++m) w |= p[m * map_words];
         }
-        if constexpr (kFinal) {
-#pragma unroll
-            for (int e = 0; e < kSectorEntries; ++e) {
-                finalize_entry(a.v[e], b.v[e], n, n_batches);
-                const unsigned long long bits = (unsigned long long)__double_as_longlong(a.v[e]);
-                best = bits > best ? bits : best;  // mean >= 0: bit order is value order
+        return w;
+    };
+    unsigned long long local = 0;
+    for (unsigned int t = claim_parts(f), end; t < f.n_parts; t = claim_parts(f))
+    for (unsigned int w_next = dirty_word(t, end = min(t + f.claim, f.n_parts)); t < end; ++t) {
+        const unsigned int w = w_next;
+        w_next = dirty_word(t + 1u, end);
+        if (__ballot_sync(0xffffffffu, w != 0u) == 0u) continue;
+        const long long widx = (long long)t * f.words + lane;
+        const long long col = t / f.parts_per_col;
+        const long long word0 = (t - col * f.parts_per_col) * f.words;  // in the column
+        const unsigned int tw = lane < f.words ? touched[widx] : 0u;
+#pragma unroll 4
+        for (int m = 0; m < f.n_maps; ++m) mine[m][lane] = lane < f.words ? dirty[m * map_words + widx] : 0u;
+        __syncwarp();
+        const int incl = warp_inclusive_scan(__popc(w));
+        const int total = __shfl_sync(0xffffffffu, incl, 31);
+        const double nh = col_nhist[col];
+        unsigned long long best = 0;
+        for (int k0 = 0; k0 < total; k0 += 16) {
+            const int k = k0 + (lane >> 1);
+            int bit;
+            const int j = nth_set_sector(w, incl, k, bit);
+            const unsigned int twj = __shfl_sync(0xffffffffu, tw, j);
+            if (k >= total) continue;
+            const long long v = (word0 + j) * kWordEntries + bit * kSectorEntries + 2 * (lane & 1);
+            const long long at = col * f.stride + v;
+            unsigned int maps = 0u;  // the maps that hold this sector
+#pragma unroll 4
+            for (int m = 0; m < f.n_maps; ++m) maps |= ((mine[m][j] >> bit) & 1u) << m;
+            auto quanta = [&](unsigned int left) {
+                return reinterpret_cast<ulonglong2*>(edep + (__ffs((int)left) - 1) * f.map_entries + at);
+            };
+            ulonglong2* q_at = quanta(maps);
+            ulonglong2 q = *q_at;
+            double2 a = make_double2(0.0, 0.0), b = a, y = a;
+            if ((twj >> bit) & 1u) {  // folded before
+                a = *reinterpret_cast<const double2*>(s1 + at);
+                b = *reinterpret_cast<const double2*>(s2 + at);
             }
+            if (v < f.n_vox) y.x = mass[v];
+            if (v + 1 < f.n_vox) y.y = mass[v + 1];
+            y.x = y.x > 0.0 ? __dmul_rn(y.x, nh) : 0.0;
+            y.y = y.y > 0.0 ? __dmul_rn(y.y, nh) : 0.0;
+            const double rx = y.x > 0.0 ? __drcp_rn(y.x) : 0.0, ry = y.y > 0.0 ? __drcp_rn(y.y) : 0.0;
+            for (;;) {
+                maps &= maps - 1u;
+                ulonglong2* const next_at = maps ? quanta(maps) : q_at;
+                ulonglong2 q_next = q;
+                if (maps) q_next = *next_at;
+                if ((q.x | q.y) != 0ull) *q_at = make_ulonglong2(0ull, 0ull);
+                const double dx = divide_by(__dmul_rn((double)(long long)q.x, kQuantum), y.x, rx);
+                const double dy = divide_by(__dmul_rn((double)(long long)q.y, kQuantum), y.y, ry);
+                a.x = __dadd_rn(a.x, dx);
+                a.y = __dadd_rn(a.y, dy);
+                b.x = __dadd_rn(b.x, __dmul_rn(dx, dx));
+                b.y = __dadd_rn(b.y, __dmul_rn(dy, dy));
+                local += q.x + q.y;
+                if (maps == 0u) break;
+                q = q_next;
+                q_at = next_at;
+            }
+            if constexpr (kFinal) {
+                finalize_entry(a.x, b.x, n, n_batches);
+                finalize_entry(a.y, b.y, n, n_batches);
+                const unsigned long long bx = (unsigned long long)__double_as_longlong(a.x);
+                const unsigned long long by = (unsigned long long)__double_as_longlong(a.y);
+                best = max(best, max(bx, by));  // mean >= 0: bit order is value order
+            }
+            *reinterpret_cast<double2*>(s1 + at) = a;
+            *reinterpret_cast<double2*>(s2 + at) = b;
         }
-        a.store(s1 + at);
-        b.store(s2 + at);
+        if (w != 0u) {
+            for (int m = 0; m < f.n_maps; ++m)
+                if (mine[m][lane]) dirty[m * map_words + widx] = 0u;
+            touched[widx] = tw | w;
+        }
+        __syncwarp();
+        if constexpr (kFinal) column_max(best, col_max_bits + col);
     }
-    if (w != 0u) {
-        for (int m = 0; m < f.n_maps; ++m) dirty[m * map_words + widx] = 0u;
-        touched[widx] = tw | w;
-    }
-    if constexpr (kFinal) column_max(best, col_max_bits + col);
     local = warp_sum_u64(local);
     if (lane == 0 && local) atomicAdd(total_q, local);
 }
 
 // Mean and sigma of the touched sectors, in place, with the column maximum of
-// the mean (one atomic per warp).
-__global__ void __launch_bounds__(kReduceThreads)
+// the mean (one atomic per warp and part).
+__global__ void __launch_bounds__(kReduceThreads, 3)
 finalize_sparse_kernel(double* __restrict__ s1, double* __restrict__ s2, FoldShape f, int n_batches,
                        const unsigned int* __restrict__ touched,
                        unsigned long long* __restrict__ col_max_bits) {
     const int lane = threadIdx.x & 31;
-    const long long t = (long long)blockIdx.x * (kReduceThreads / 32) + (threadIdx.x >> 5);
-    if (t >= f.n_parts) return;
-    const long long col = t / f.parts_per_col;
-    const long long word0 = (t - col * f.parts_per_col) * f.words;
-    const unsigned int w =
-        lane < f.words ? touched[col * (f.stride / kWordEntries) + word0 + lane] : 0u;
-    if (__ballot_sync(0xffffffffu, w != 0u) == 0u) return;
-    const int incl = warp_inclusive_scan(__popc(w));
-    const int total = __shfl_sync(0xffffffffu, incl, 31);
     const double n = (double)n_batches;
-    unsigned long long best = 0ull;
-    for (int k0 = 0; k0 < total; k0 += 32) {
-        const int k = k0 + lane;
-        int bit;
-        const int j = nth_set_sector(w, incl, k, bit);
-        if (k >= total) continue;
-        const long long at = col * f.stride + (word0 + j) * kWordEntries + bit * kSectorEntries;
+    auto word = [&](unsigned int part, unsigned int end) {
+        return part < end && lane < f.words ? touched[(long long)part * f.words + lane] : 0u;
+    };
+    for (unsigned int t = claim_parts(f), end; t < f.n_parts; t = claim_parts(f))
+    for (unsigned int w_next = word(t, end = min(t + f.claim, f.n_parts)); t < end; ++t) {
+        const unsigned int w = w_next;
+        w_next = word(t + 1u, end);
+        if (__ballot_sync(0xffffffffu, w != 0u) == 0u) continue;
+        const long long col = t / f.parts_per_col;
+        const long long word0 = (t - col * f.parts_per_col) * f.words;
+        const int incl = warp_inclusive_scan(__popc(w));
+        const int total = __shfl_sync(0xffffffffu, incl, 31);
+        unsigned long long best = 0ull;
+        // the next sector's sums are on their way while this one's are finalized
+        auto sector = [&](int k) {
+            int bit;
+            const int j = nth_set_sector(w, incl, k, bit);
+            return k < total ? col * f.stride + (word0 + j) * kWordEntries + bit * kSectorEntries : -1ll;
+        };
         SectorD a, b;
-        a.load(s1 + at);
-        b.load(s2 + at);
-#pragma unroll
-        for (int e = 0; e < kSectorEntries; ++e) {
-            finalize_entry(a.v[e], b.v[e], n, n_batches);
-            const unsigned long long bits = (unsigned long long)__double_as_longlong(a.v[e]);
-            best = bits > best ? bits : best;
+        long long at = sector(lane);
+        if (at >= 0) {
+            a.load(s1 + at);
+            b.load(s2 + at);
         }
-        a.store(s1 + at);
-        b.store(s2 + at);
+        for (int k0 = 0; k0 < total; k0 += 32) {
+            SectorD a_next, b_next;
+            const long long at_next = sector(k0 + 32 + lane);
+            if (at_next >= 0) {
+                a_next.load(s1 + at_next);
+                b_next.load(s2 + at_next);
+            }
+            if (at >= 0) {
+#pragma unroll
+                for (int e = 0; e < kSectorEntries; ++e) {
+                    finalize_entry(a.v[e], b.v[e], n, n_batches);
+                    const unsigned long long bits = (unsigned long long)__double_as_longlong(a.v[e]);
+                    best = bits > best ? bits : best;
+                }
+                a.store(s1 + at);
+                b.store(s2 + at);
+            }
+            at = at_next;
+            a = a_next;
+            b = b_next;
+        }
+        column_max(best, col_max_bits + col);
     }
-    column_max(best, col_max_bits + col);
 }
 
 // Kept entries of the touched sectors of one (column, tile); one warp each.

@@ -98,6 +98,7 @@ struct pmc_engine {
     Counters* d_counters = nullptr;
     GenDesc* d_gen = nullptr;
     unsigned long long* d_total_q = nullptr;
+    unsigned int* d_fold_next = nullptr;  // parts the fold or finalize has claimed
     unsigned long long* d_colmax = nullptr;
     long long colmax_len = 0;
     DevBuf tile_counts, tile_offsets, col_counts, out_idx, out_dose, out_sigma, col_nhist;
@@ -275,17 +276,17 @@ GridInfo make_grid(int nx, int ny, int nz, const double o[3], const double s[3])
 constexpr int kDefaultTailSteps = 96;  // steps after a round runs dry before a particle is parked
 
 // Kernel variants: tables in shared memory or not, the register budget
-// (resident blocks of 256 per SM: 0 = each kernel's default, else 3 or 4), and
-// plain scoring.
+// (resident blocks of 256 per SM: 0 = each kernel's default — photons 4, electrons
+// 3 — else 3 or 4), and plain scoring.
 template <bool kPlain>
 void* photon_variant(bool smem, int occ) {
-    if (occ == 4) return smem ? (void*)photon_kernel<true, 4, kPlain> : (void*)photon_kernel<false, 4, kPlain>;
+    if (occ != 3) return smem ? (void*)photon_kernel<true, 4, kPlain> : (void*)photon_kernel<false, 4, kPlain>;
     return smem ? (void*)photon_kernel<true, 3, kPlain> : (void*)photon_kernel<false, 3, kPlain>;
 }
 template <bool kPlain>
 void* electron_variant(bool smem, int occ) {
-    if (occ == 3) return smem ? (void*)electron_kernel<true, 3, kPlain> : (void*)electron_kernel<false, 3, kPlain>;
-    return smem ? (void*)electron_kernel<true, 4, kPlain> : (void*)electron_kernel<false, 4, kPlain>;
+    if (occ == 4) return smem ? (void*)electron_kernel<true, 4, kPlain> : (void*)electron_kernel<false, 4, kPlain>;
+    return smem ? (void*)electron_kernel<true, 3, kPlain> : (void*)electron_kernel<false, 3, kPlain>;
 }
 void* photon_fn(const LaunchShape& L) {
     return L.plain ? photon_variant<true>(L.smem, L.occ) : photon_variant<false>(L.smem, L.occ);
@@ -305,9 +306,9 @@ bool plain_scoring(const pmc_engine* e, const pmc_run_params* p) {
 int transport_launch_shape(pmc_engine* e, const pmc_run_params* p, LaunchShape* L) {
     L->occ = (p->blocks_per_sm == 3 || p->blocks_per_sm == 4) ? p->blocks_per_sm : 0;
     L->plain = plain_scoring(e, p);
-    // default: blocks of 256, and 512 for the 64-register electron kernel
+    // default: blocks of 256, and two of 384 per SM for the electron kernel
     L->block_ph = p->block_size > 0 ? p->block_size : kPhotonThreads;
-    L->block_el = p->block_size > 0 ? p->block_size : L->occ == 3 ? 256 : kElectronThreads;
+    L->block_el = p->block_size > 0 ? p->block_size : L->occ == 4 ? 256 : kElectronThreads;
     if (L->block_ph % 32 != 0 || L->block_ph > 256) return fail(e, PMC_ERR_INVALID, "block_size must be a multiple of 32 and <= 256");
     const size_t rows = (size_t)e->tab.n_materials * (size_t)e->tab.n_points;
     L->smem_ph = rows * sizeof(float4) + (size_t)e->tab.n_points * sizeof(float);
@@ -480,7 +481,8 @@ int prepare_transport(pmc_engine* e, const pmc_run_params* p, unsigned long long
         const double map_bytes = sizeof(double) * (double)stride_for(e->si.n_voxels) * std::max(cols, 1);
         const double by_memory = std::floor(kWaveBytes / map_bytes) + 1.0;
         const unsigned long long by_work = std::max(1ull, 64ull * resident / std::max(1ull, block));
-        const int most = (int)std::min((double)std::min<unsigned long long>(by_work, p->n_batches), by_memory);
+        const int most = (int)std::min(
+            (double)std::min(std::min<unsigned long long>(by_work, p->n_batches), (unsigned long long)kWaveMaps), by_memory);
         const int n_waves = (p->n_batches + most - 1) / most;
         plan->wave = (p->n_batches + n_waves - 1) / n_waves;  // waves of about the same size
     }
@@ -532,6 +534,7 @@ TransportParams make_params(pmc_engine* e, const pmc_run_params* p, const RunPla
     P.counters = e->d_counters;
     P.seed_lo = (uint32_t)(p->seed & 0xffffffffull);
     P.seed_hi = (uint32_t)(p->seed >> 32);
+    P.keys = philox_keys(P.seed_lo, P.seed_hi);
     P.pcut = (float)p->pcut;
     P.ecut = (float)p->ecut;
     P.step_fraction = (float)p->step_energy_fraction;
@@ -597,21 +600,32 @@ int reduce_blocks(long long n_warps) {
     return (int)((n_warps + kReduceThreads / 32 - 1) / (kReduceThreads / 32));
 }
 
-// Bitmap words per warp of the fold and finalize: a whole tile's 32 while that
-// still leaves 32 warps per SM, fewer (down to one) on smaller maps, where the
-// longest warp's chain of sectors is the kernel's time.
-FoldShape fold_shape(const pmc_engine* e, long long n_vox, int group, int n_maps) {
-    FoldShape f{};
-    f.n_vox = n_vox;
-    f.stride = e->col_stride;
-    f.n_maps = n_maps;
-    f.map_entries = e->col_stride * group;
-    const long long words = f.map_entries / kWordEntries;
-    f.words = 32;
-    while (f.words > 1 && words / f.words < 32ll * e->sm_count) f.words /= 2;
-    f.parts_per_col = (int)(e->col_stride / kWordEntries / f.words);
-    f.n_parts = (long long)f.parts_per_col * group;
-    return f;
+constexpr int kFoldBlocks = 4;  // blocks of the fold per SM (finalize: 3 resident, the rest follow)
+
+// Bitmap words per part of the fold and finalize: 8 (at most 256 sectors, 16 turns
+// of a warp), fewer (down to one) where that leaves a warp without a part, more
+// where the parts would not fit their 32-bit number; about eight claims per warp.
+int fold_shape(pmc_engine* e, long long n_vox, int group, int n_maps, FoldShape* f) {
+    f->n_vox = n_vox;
+    f->stride = e->col_stride;
+    f->n_maps = n_maps;
+    f->map_entries = e->col_stride * group;
+    const long long words = f->map_entries / kWordEntries;
+    const long long warps = (long long)kFoldBlocks * e->sm_count * (kReduceThreads / 32);
+    f->words = 8;
+    while (f->words > 1 && words / f->words < warps) f->words /= 2;
+    while (f->words < 32 && words / f->words > (1ll << 30)) f->words *= 2;
+    if (words / f->words > (1ll << 31)) return fail(e, PMC_ERR_INVALID, "too many scoring entries in one group");
+    f->parts_per_col = (int)(e->col_stride / kWordEntries / f->words);
+    f->n_parts = (unsigned int)f->parts_per_col * (unsigned int)group;
+    f->claim = std::max(1u, (unsigned int)(f->n_parts / (8 * warps)));
+    f->next = e->d_fold_next;
+    PMC_CUDA(e, cudaMemsetAsync(e->d_fold_next, 0, sizeof(unsigned int), e->stream));
+    return PMC_OK;
+}
+
+int fold_blocks(const pmc_engine* e, const FoldShape& f) {
+    return std::min(kFoldBlocks * e->sm_count, reduce_blocks(f.n_parts));
 }
 
 // Fold the n_maps quanta maps of a wave; `last`: they hold every batch of the
@@ -619,9 +633,11 @@ FoldShape fold_shape(const pmc_engine* e, long long n_vox, int group, int n_maps
 // called; d_colmax cleared by the caller).
 int launch_fold(pmc_engine* e, long long n_vox, int group, const double* d_col_nhist, int n_maps,
                 int n_batches, bool last) {
-    const FoldShape f = fold_shape(e, n_vox, group, n_maps);
+    FoldShape f{};
+    const int rc = fold_shape(e, n_vox, group, n_maps, &f);
+    if (rc) return rc;
     auto kernel = last ? fold_sparse_kernel<true> : fold_sparse_kernel<false>;
-    kernel<<<reduce_blocks(f.n_parts), kReduceThreads, 0, e->stream>>>(
+    kernel<<<fold_blocks(e, f), kReduceThreads, 0, e->stream>>>(
         (unsigned long long*)e->edep.p, e->d_mass, d_col_nhist, f, (double*)e->s1.p, (double*)e->s2.p,
         (unsigned int*)e->dirty.p, (unsigned int*)e->touched.p, n_batches, e->d_colmax, e->d_total_q);
     PMC_CUDA(e, cudaGetLastError());
@@ -644,8 +660,10 @@ int clear_colmax(pmc_engine* e, int group) {
 int launch_finalize(pmc_engine* e, long long n_vox, int group, int n_batches) {
     int rc = clear_colmax(e, group);
     if (rc) return rc;
-    const FoldShape f = fold_shape(e, n_vox, group, 1);
-    finalize_sparse_kernel<<<reduce_blocks(f.n_parts), kReduceThreads, 0, e->stream>>>(
+    FoldShape f{};
+    rc = fold_shape(e, n_vox, group, 1, &f);
+    if (rc) return rc;
+    finalize_sparse_kernel<<<fold_blocks(e, f), kReduceThreads, 0, e->stream>>>(
         (double*)e->s1.p, (double*)e->s2.p, f, n_batches, (const unsigned int*)e->touched.p, e->d_colmax);
     PMC_CUDA(e, cudaGetLastError());
     e->counters.reduce_launches += 1;
@@ -955,6 +973,7 @@ int pmc_create(pmc_engine** out, int device_ordinal) {
     if (st == cudaSuccess) st = cudaMalloc(&e->d_counters, sizeof(Counters));
     if (st == cudaSuccess) st = cudaMalloc(&e->d_gen, sizeof(GenDesc));
     if (st == cudaSuccess) st = cudaMalloc(&e->d_total_q, sizeof(unsigned long long));
+    if (st == cudaSuccess) st = cudaMalloc(&e->d_fold_next, sizeof(unsigned int));
     if (st == cudaSuccess) st = cudaMalloc(&e->d_nnz, sizeof(unsigned long long));
     for (int i = 0; i < 4 && st == cudaSuccess; ++i) st = cudaEventCreate(&e->ev[i]);
     if (st != cudaSuccess) {
@@ -985,7 +1004,7 @@ void pmc_destroy(pmc_engine* e) {
                       &e->stage})
         if (b->p) cudaFree(b->p);
     for (void* p : {(void*)e->d_sched, (void*)e->d_counters, (void*)e->d_gen,
-                    (void*)e->d_total_q, (void*)e->d_colmax, (void*)e->d_nnz})
+                    (void*)e->d_total_q, (void*)e->d_fold_next, (void*)e->d_colmax, (void*)e->d_nnz})
         if (p) cudaFree(p);
     for (cudaEvent_t ev : e->ev)
         if (ev) cudaEventDestroy(ev);

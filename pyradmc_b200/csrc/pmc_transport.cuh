@@ -162,6 +162,7 @@ struct TransportParams {
     long long col_stride;      // entries per column: scoring voxels rounded up to a tile
     Counters* counters;
     uint32_t seed_lo, seed_hi;
+    PhiloxKeys keys;      // of the seed
     float pcut, ecut;
     float step_fraction;
     float deposit_resolution;
@@ -366,26 +367,65 @@ __device__ __forceinline__ unsigned int round_to_chunk(unsigned long long n) {
     return (unsigned int)((n + kChunk - 1) / kChunk * kChunk);
 }
 
-// Chunks pay where a round is long and the slots left unused do not count: at
-// 512 input particles per block and more (a small round takes single slots).
-__device__ __forceinline__ bool chunked_round(const TransportParams& P, unsigned int n_in) {
-    return n_in >= 512u * gridDim.x && P.slots <= kChunkedSlots;
+// One round of a kernel as its blocks see it, in shared memory: the particles of
+// its input queue, and the two queues it pushes to with the block's chunk of each
+// (chunk number above kOffBits bits of fill; kChunk and more: closed, slots are
+// taken singly from the top).
+struct Round {
+    int q_in, q_out[2];
+    unsigned int n_bottom, n;  // particles from the bottom of the input queue, in all
+    unsigned int claim;        // particles a warp claims at a time
+    uint32_t chunk[2];
+    unsigned int pushes;
+};
+
+// One thread of the block.  Chunks (of the queues in `chunk_mask`) pay where a
+// round is long and the slots left unused do not count, at 512 input particles
+// per block and more; small rounds take single slots, and claim few particles at
+// a time, so that every warp gets some.
+__device__ __forceinline__ void open_round(const TransportParams& P, Round& R, int q_in, int q_out0, int q_out1,
+                                           unsigned int chunk_mask) {
+    Sched* S = P.sched;
+    R.q_in = q_in;
+    R.q_out[0] = q_out0;
+    R.q_out[1] = q_out1;
+    const unsigned int b = S->bottom[q_in].v, t = S->top[q_in].v;
+    R.n_bottom = min(b, P.slots);
+    R.n = R.n_bottom + min(t, P.slots - R.n_bottom);
+    if ((unsigned long long)b + t > (unsigned long long)P.capacity + S->dead[q_in].v) {  // too many live ones
+        atomicOr(&S->flags, kFlagOverflow);
+        R.n = R.n_bottom = 0u;
+    }
+    const unsigned int warps = gridDim.x * (blockDim.x / 32u);
+    R.claim = R.n / warps >= 128u ? 32u : R.n / warps >= 16u ? 4u : 1u;
+    const bool chunked = R.n >= 512u * gridDim.x && P.slots <= kChunkedSlots;
+    for (int k = 0; k < 2; ++k)
+        R.chunk[k] = chunked && (chunk_mask >> k & 1u)
+                         ? atomicAdd(&S->bottom[R.q_out[k]].v, kChunk) / kChunk << kOffBits
+                         : kChunk;
+    R.pushes = 0u;
 }
 
-// One thread: the block's first chunk of queue qi.
-__device__ __forceinline__ uint32_t open_chunk(const TransportParams& P, int qi) {
-    return atomicAdd(&P.sched->bottom[qi].v, kChunk) / kChunk << kOffBits;
+// A single slot of queue qi for every lane that gets here together, from the top
+// down; P.slots when there is none.
+__device__ __forceinline__ unsigned int single_slot(const TransportParams& P, int qi) {
+    cg::coalesced_group g = cg::coalesced_threads();
+    unsigned int base = 0u;
+    if (g.thread_rank() == 0) base = atomicAdd(&P.sched->top[qi].v, (unsigned int)g.size());
+    base = g.shfl(base, 0) + (unsigned int)g.thread_rank();
+    return base < P.slots ? P.slots - 1u - base : P.slots;
 }
 
-// A slot of queue qi for every lane that gets here together (word: the block's
-// chunk, or null for single slots); P.slots and up when there is none.
-__device__ __forceinline__ unsigned int claim_slot(const TransportParams& P, int qi, uint32_t* word) {
+// A slot of output queue k for every lane that gets here together; P.slots and up
+// when there is none.
+__device__ __forceinline__ unsigned int claim_slot(const TransportParams& P, Round& R, int k) {
     cg::coalesced_group g = cg::coalesced_threads();
     const unsigned int n = (unsigned int)g.size(), r = (unsigned int)g.thread_rank();
     unsigned int first = 0u, rest = 0u, served = 0u;  // served lanes from `first`, the others from `rest`
     if (r == 0u) {
+        uint32_t* word = &R.chunk[k];
         bool single = true;
-        if (word != nullptr && (*(volatile uint32_t*)word & kOffMask) < kChunk) {
+        if ((*(volatile uint32_t*)word & kOffMask) < kChunk) {
             const uint32_t w = atomicAdd(word, n);
             const unsigned int off = w & kOffMask;
             if (off < kChunk) {
@@ -393,15 +433,16 @@ __device__ __forceinline__ unsigned int claim_slot(const TransportParams& P, int
                 served = min(n, kChunk - off);
                 single = false;
                 if (off + n >= kChunk) {  // the chunk's last slot: open the next
-                    rest = atomicAdd(&P.sched->bottom[qi].v, kChunk);
+                    rest = atomicAdd(&P.sched->bottom[R.q_out[k]].v, kChunk);
                     atomicExch(word, (rest / kChunk << kOffBits) | (n - served));
                 }
             }
         }
         if (single) {
-            rest = atomicAdd(&P.sched->top[qi].v, n);
-            served |= 0x100u;
+            rest = atomicAdd(&P.sched->top[R.q_out[k]].v, n);
+            served = 0x100u;
         }
+        atomicAdd(&R.pushes, n);
     }
     first = g.shfl(first, 0);
     rest = g.shfl(rest, 0);
@@ -410,57 +451,43 @@ __device__ __forceinline__ unsigned int claim_slot(const TransportParams& P, int
     return r < served ? first + r : rest + (r - served);
 }
 
-// Mark what is left of the block's chunk (whole block, after its last push).
-__device__ inline void close_chunk(const TransportParams& P, int qi, uint32_t word) {
-    const unsigned int off = word & kOffMask;
-    if (off >= kChunk) return;
-    if (threadIdx.x == 0) atomicAdd(&P.sched->dead[qi].v, kChunk - off);
-    for (unsigned int k = off + threadIdx.x; k < kChunk; k += blockDim.x) {
-        const unsigned int slot = (word >> kOffBits) * kChunk + k;
-        if (slot < P.slots) P.q[qi][slot].d = make_uint4(kDeadMeta, 0u, 0u, 0u);
+// Mark what is left of the block's chunks (whole block, after its last push).
+__device__ inline void close_round(const TransportParams& P, const Round& R) {
+    for (int k = 0; k < 2; ++k) {
+        const uint32_t word = R.chunk[k];
+        const unsigned int off = word & kOffMask;
+        if (off >= kChunk) continue;
+        if (threadIdx.x == 0) atomicAdd(&P.sched->dead[R.q_out[k]].v, kChunk - off);
+        for (unsigned int i = off + threadIdx.x; i < kChunk; i += blockDim.x) {
+            const unsigned int slot = (word >> kOffBits) * kChunk + i;
+            if (slot < P.slots) P.q[R.q_out[k]][slot].d = make_uint4(kDeadMeta, 0u, 0u, 0u);
+        }
     }
 }
 
-// A round's input: particle i of queue qi, and how a warp takes its share.  The
-// warp claims particles `claim` at a time (one atomic, their slots prefetched into
-// the L2) and hands them to its idle lanes; small rounds are claimed one by one,
-// so that every warp gets some.
-struct Input {
-    int qi;
-    unsigned int n_bottom, n;        // particles from the bottom, in all
-    unsigned int next, left, claim;  // the warp's claimed particles; how many it claims
+__device__ __forceinline__ const Slot* input_slot(const TransportParams& P, const Round& R, unsigned int i) {
+    return P.q[R.q_in] + (i < R.n_bottom ? i : P.slots - 1u - (i - R.n_bottom));
+}
 
-    __device__ __forceinline__ void open(const TransportParams& P, int queue) {
-        Sched* S = P.sched;
-        qi = queue;
-        const unsigned int b = S->bottom[qi].v, t = S->top[qi].v;
-        n_bottom = min(b, P.slots);
-        n = n_bottom + min(t, P.slots - n_bottom);
-        if ((unsigned long long)b + t > (unsigned long long)P.capacity + S->dead[qi].v) {  // too many live ones
-            atomicOr(&S->flags, kFlagOverflow);
-            n = n_bottom = 0u;
-        }
-        const unsigned int warps = gridDim.x * (blockDim.x / 32u);
-        claim = n / warps >= 128u ? 32u : n / warps >= 16u ? 4u : 1u;
-        next = left = 0u;
-    }
-    __device__ __forceinline__ const Slot* slot(const TransportParams& P, unsigned int i) const {
-        return P.q[qi] + (i < n_bottom ? i : P.slots - 1u - (i - n_bottom));
-    }
+// How a warp takes its share of the round's input: particles claimed R.claim at a
+// time (one atomic, their slots prefetched into the L2) and handed to idle lanes.
+struct Claim {
+    unsigned int next = 0u, left = 0u;
     // The particle number of each lane that wants one (all lanes of the warp call).
-    __device__ __forceinline__ unsigned int take(const TransportParams& P, bool want) {
+    __device__ __forceinline__ unsigned int take(const TransportParams& P, const Round& R, bool want) {
         const unsigned int need = __ballot_sync(0xffffffffu, want);
         const unsigned int lane = threadIdx.x & 31u;
         const unsigned int cnt = (unsigned int)__popc(need);
         const unsigned int rank = (unsigned int)__popc(need & ((1u << lane) - 1u));
         unsigned int i = next + rank;
         if (cnt > left) {
-            const unsigned int more = max(claim, cnt - left);
+            const unsigned int more = max(R.claim, cnt - left);
             unsigned int b = 0u;
-            if (lane == 0u) b = atomicAdd(&P.sched->head[qi].v, more);
+            if (lane == 0u) b = atomicAdd(&P.sched->head[R.q_in].v, more);
             b = __shfl_sync(0xffffffffu, b, 0);
-            if (lane < more && b + lane < n)
-                asm volatile("prefetch.global.L2 [%0];" ::"l"(__cvta_generic_to_global(slot(P, b + lane))));
+            if (lane < more && b + lane < R.n)
+                asm volatile("prefetch.global.L2 [%0];" ::"l"(
+                    __cvta_generic_to_global(input_slot(P, R, b + lane))));
             if (rank >= left) i = b + (rank - left);
             next = b + (cnt - left);
             left = more - (cnt - left);
@@ -472,11 +499,9 @@ struct Input {
     }
 };
 
-__device__ __forceinline__ void queue_push(const TransportParams& P, int qi, uint32_t* word, int kind,
-                                           int beamlet, float e, float w, float x, float y, float z, float ux,
-                                           float uy, float uz, const StreamId& sid, unsigned int& n_push) {
-    const unsigned int idx = claim_slot(P, qi, word);
-    ++n_push;
+__device__ __forceinline__ void write_particle(const TransportParams& P, int qi, unsigned int idx, int kind,
+                                               int beamlet, float e, float w, float x, float y, float z,
+                                               float ux, float uy, float uz, const StreamId& sid) {
     if (idx >= P.slots) {
         atomicOr(&P.sched->flags, kFlagOverflow);
         return;
@@ -486,6 +511,13 @@ __device__ __forceinline__ void queue_push(const TransportParams& P, int qi, uin
     s->b = make_float4(z, ux, uy, uz);
     s->c = make_uint4(sid.id_lo, sid.id_hi, sid.tag, sid.ctr);
     s->d = make_uint4(pack_meta(kind, 0, beamlet), 0u, 0u, 0u);
+}
+
+__device__ __forceinline__ void queue_push(const TransportParams& P, Round& R, int k, int kind, int beamlet,
+                                           float e, float w, float x, float y, float z, float ux, float uy,
+                                           float uz, const StreamId& sid) {
+    const unsigned int idx = claim_slot(P, R, k);
+    write_particle(P, R.q_out[k], idx, kind, beamlet, e, w, x, y, z, ux, uy, uz, sid);
 }
 
 // ---- particle state ----------------------------------------------------------------
@@ -525,17 +557,12 @@ __device__ __forceinline__ void store_slot(Slot* s, const ParticleOf<R>& p) {
     s->d = make_uint4(p.meta, (uint32_t)p.steps, 0u, 0u);
 }
 
-// Queue an unfinished particle (parked for the next round, or a fresh one).
+// Park an unfinished particle in output queue k for the next round.
 template <class R>
-__device__ __forceinline__ void queue_suspend(const TransportParams& P, int qi, const ParticleOf<R>& p,
-                                              unsigned int& n_push) {
-    const unsigned int idx = claim_slot(P, qi, nullptr);
-    ++n_push;
-    if (idx >= P.slots) {
-        atomicOr(&P.sched->flags, kFlagOverflow);
-        return;
-    }
-    store_slot(P.q[qi] + idx, p);
+__device__ __forceinline__ void queue_suspend(const TransportParams& P, Round& round, int k, const ParticleOf<R>& p) {
+    const unsigned int idx = claim_slot(P, round, k);
+    if (idx >= P.slots) atomicOr(&P.sched->flags, kFlagOverflow);
+    else store_slot(P.q[round.q_out[k]] + idx, p);
 }
 
 // Copy `n` table entries into the block's shared memory (strided over the block).
@@ -545,25 +572,17 @@ __device__ __forceinline__ void stage(T* dst, const T* src, int n) {
 }
 
 // Vacuum flight to the grid for a particle born outside (photon.py:137-148);
-// returns false (energy escaped) when the flight misses the grid.
+// returns false (its energy escapes) when the flight misses the grid.
 template <class R>
-__device__ __forceinline__ bool enter_grid(const TransportParams& P, BlockBooks& B, ParticleOf<R>& p,
-                                           float latent) {
+__device__ __forceinline__ bool enter_grid(const TransportParams& P, ParticleOf<R>& p) {
     if (point_inside(p.x, p.y, p.z, P.gi)) return true;
     float t = slab_entry_distance(p.x, p.y, p.z, p.ux, p.uy, p.uz, P.gi);
-    if (t >= kInfinityCm) {
-        escape(B, p.w * (p.e + latent));
-        return false;
-    }
+    if (t >= kInfinityCm) return false;
     t += kEntryNudge;
     p.x += t * p.ux;
     p.y += t * p.uy;
     p.z += t * p.uz;
-    if (!point_inside(p.x, p.y, p.z, P.gi)) {
-        escape(B, p.w * (p.e + latent));
-        return false;
-    }
-    return true;
+    return point_inside(p.x, p.y, p.z, P.gi);
 }
 
 // The transmission of a user mask plane along the primary's full line
@@ -624,7 +643,7 @@ __device__ inline float stack_transmission(const GenDesc& G, const Particle& p) 
 // (same uniforms, same order).  Returns the particle kind, or -1 when the
 // source emits nothing for this history (a masked fan's zero transmission).
 __device__ inline int generate_primary(const TransportParams& P, const GenDesc& G, int batch,
-                                       unsigned long long t, Particle& p, BlockBooks& B) {
+                                       unsigned long long t, Particle& p, long long& emitted) {
     // G is the device-resident descriptor, read field by field as needed.
     int local = 0;
     int map = 0;  // the wave's quanta map this primary's batch scores into
@@ -764,16 +783,16 @@ __device__ inline int generate_primary(const TransportParams& P, const GenDesc& 
     }
     if (G.book_emitted) {
         const float latent = kind == kPositron ? 2.0f * kElectronMass : 0.0f;
-        book_add(&B.emitted, quantize_signed(p.w * (p.e + latent)));
+        emitted += quantize_signed(p.w * (p.e + latent));
     }
     return kind;
 }
 
 // ---- annihilation at rest (transport/particles.py:75, kernels.py:675) ------------
+// (output queue 1 is the photon queue of both kernels)
 template <bool kPlain, class R, class Sink>
 __device__ __forceinline__ void annihilate_at_rest(const TransportParams& P, BlockBooks& B, ParticleOf<R>& p,
-                                                   int voxel, int q_photon, float factor, Sink& sink,
-                                                   unsigned int& n_push) {
+                                                   int voxel, Round& round, float factor, Sink& sink) {
     if (P.pcut >= kElectronMass) {
         deposit<kPlain>(P, B, p.beamlet(), p.x, p.y, p.z, voxel, p.w * 2.0f * kElectronMass, factor, sink);
         return;
@@ -785,8 +804,7 @@ __device__ __forceinline__ void annihilate_at_rest(const TransportParams& P, Blo
     for (int k = 0; k < 2; ++k) {  // two photons back to back
         p.rng.reserve(3);
         const StreamId sid = p.rng.spawn();
-        queue_push(P, q_photon, nullptr, kPhoton, p.beamlet(), kElectronMass, p.w, p.x, p.y, p.z, ax, ay, az, sid,
-                   n_push);
+        queue_push(P, round, 1, kPhoton, p.beamlet(), kElectronMass, p.w, p.x, p.y, p.z, ax, ay, az, sid);
         ax = -ax;
         ay = -ay;
         az = -az;
@@ -859,12 +877,13 @@ constexpr int kPhotonThreads = 256;  // the largest block of the photon kernel
 // kSmem: the channel rows of every material and the majorant row are staged in
 // the block's shared memory (dynamic, n_materials * n_points * 16 + n_points * 4
 // bytes) instead of being read through L1.
-// kMinBlocks: resident blocks of 256 per SM the register allocation targets.
+// kMinBlocks: resident blocks of 256 per SM the register allocation targets (3:
+// 72 registers, 4: 64, no spills either way).
 // kPlain: dose to medium on the transport grid itself, whole-substep deposits, no
 // Compton splitting, fewer than 2^31 voxels (plain_scoring): a deposit's bin is the
 // voxel already at hand.
 template <bool kSmem, int kMinBlocks, bool kPlain>
-__global__ void __launch_bounds__(kPhotonThreads, kMinBlocks) photon_kernel(TransportParams P) {
+__global__ void __launch_bounds__(kPhotonThreads, kMinBlocks) photon_kernel(const __grid_constant__ TransportParams P) {
     __shared__ BlockBooks B;
     __shared__ uint32_t ring[kRingWords * kPhotonThreads];
     extern __shared__ __align__(16) unsigned char pmc_smem[];
@@ -879,30 +898,23 @@ __global__ void __launch_bounds__(kPhotonThreads, kMinBlocks) photon_kernel(Tran
         tab_ch = sch;
         tab_maj = smaj;
     }
-    init_books(B);  // its barrier also publishes the staged tables
     Sched* S = P.sched;
-    const int pin = S->p_in, ein = S->e_in;
-    const int q_in = pin, q_out = pin ^ 1, q_el = 2 + ein;
-    Input in;
-    in.open(P, q_in);
-    __shared__ uint32_t chunk_el;  // the block's chunk of the electron queue
-    const bool chunked = chunked_round(P, in.n);
-    if (threadIdx.x == 0) chunk_el = chunked ? open_chunk(P, q_el) : 0u;
-    __syncthreads();
-    uint32_t* const word_el = chunked ? &chunk_el : nullptr;
+    __shared__ Round rd;  // pushes electrons (0) and, rarely, photons (1)
+    if (threadIdx.x == 0) open_round(P, rd, S->p_in, 2 + S->e_in, S->p_in ^ 1, 1u);
+    init_books(B);  // its barrier also publishes the round and the staged tables
     const Tables& T = P.tab;
     const float pcut = P.pcut, ecut = P.ecut;
 
-    unsigned int n_flight = 0, n_inter = 0, n_push = 0;  // per lane and launch
+    Claim input;
+    unsigned int n_flight = 0, n_inter = 0;  // per lane and launch
     DirectSink dep;
-    ParticleOf<RingRng<kPhotonThreads>> p;
-    p.rng.k0 = P.seed_lo;
-    p.rng.k1 = P.seed_hi;
+    ParticleOf<RingRng<kPhotonThreads, true>> p;
+    p.rng.keys = &P.keys;
     p.rng.ring = ring + threadIdx.x;
     long long escaped = 0;  // most photons end that way: summed per lane, booked once
     auto leave = [&](float amount) { escaped += quantize_signed(amount); };
-    bool active = false, exhausted = false, dry = false;
-    int tail = 0;  // steps of the current photon since its warp found the round dry
+    bool active = false, exhausted = false;
+    int tail = -1;  // turns since the warp found the round dry
     float e_tab = -1.0f, maj = 0.0f;
     LogIdx li{0, 0.0f};
     int mat_tab = -1;
@@ -915,25 +927,27 @@ __global__ void __launch_bounds__(kPhotonThreads, kMinBlocks) photon_kernel(Tran
         }
         const bool want = !active && !exhausted;  // the round's photons: secondaries, primaries, parked
         if (__any_sync(0xffffffffu, want)) {
-            const unsigned int i = in.take(P, want);
+            const unsigned int i = input.take(P, rd, want);
             if (want) {
-                if (i < in.n) {
-                    active = load_slot(in.slot(P, i), p) && enter_grid(P, B, p, 0.0f);
+                if (i < rd.n) {
+                    if (load_slot(input_slot(P, rd, i), p)) {
+                        active = enter_grid(P, p);
+                        if (!active) leave(p.w * p.e);
+                    }
                     e_tab = -1.0f;
-                    tail = 0;
                 } else {
                     exhausted = true;
                 }
             }
         }
         if (!__any_sync(0xffffffffu, active || !exhausted)) break;
-        if (!dry) dry = __any_sync(0xffffffffu, exhausted);
-        if (!active) continue;
         // Once the round's input has run dry, a photon that still needs more than
         // tail_steps flights is parked for the next round instead of holding its
         // warp (and its block's barrier) while every other lane idles.
-        if (dry && ++tail > P.tail_steps) {
-            queue_suspend(P, q_out, p, n_push);
+        if (tail >= 0 || __any_sync(0xffffffffu, exhausted)) ++tail;
+        if (!active) continue;
+        if (tail >= P.tail_steps) {
+            queue_suspend(P, rd, 1, p);
             active = false;
             continue;
         }
@@ -1007,8 +1021,7 @@ __global__ void __launch_bounds__(kPhotonThreads, kMinBlocks) photon_kernel(Tran
                     float ex = p.ux, ey = p.uy, ez = p.uz;
                     rotate_direction(ex, ey, ez, compton_electron_cos_theta(p.e, ratio), phi + kPi);
                     const StreamId sid = p.rng.spawn();
-                    queue_push(P, q_el, word_el, kElectron, p.beamlet(), recoil, split_w, p.x, p.y, p.z, ex, ey, ez, sid,
-                               n_push);
+                    queue_push(P, rd, 0, kElectron, p.beamlet(), recoil, split_w, p.x, p.y, p.z, ex, ey, ez, sid);
                 } else {
                     put(split_w * recoil, recoil);
                 }
@@ -1030,7 +1043,7 @@ __global__ void __launch_bounds__(kPhotonThreads, kMinBlocks) photon_kernel(Tran
                 }
                 if (keep) {
                     const StreamId sid = p.rng.spawn();
-                    queue_push(P, q_out, nullptr, kPhoton, p.beamlet(), es, cw, p.x, p.y, p.z, gx, gy, gz, sid, n_push);
+                    queue_push(P, rd, 1, kPhoton, p.beamlet(), es, cw, p.x, p.y, p.z, gx, gy, gz, sid);
                 }
             }
             active = false;
@@ -1062,7 +1075,7 @@ __global__ void __launch_bounds__(kPhotonThreads, kMinBlocks) photon_kernel(Tran
             if (process == 0)
                 rotate_direction(ex, ey, ez, compton_electron_cos_theta(p.e, ratio), phi + kPi);
             const StreamId sid = p.rng.spawn();
-            queue_push(P, q_el, word_el, kElectron, p.beamlet(), ee, p.w, p.x, p.y, p.z, ex, ey, ez, sid, n_push);
+            queue_push(P, rd, 0, kElectron, p.beamlet(), ee, p.w, p.x, p.y, p.z, ex, ey, ez, sid);
         } else {
             put(p.w * ee, ee);
         }
@@ -1092,31 +1105,30 @@ __global__ void __launch_bounds__(kPhotonThreads, kMinBlocks) photon_kernel(Tran
             if (P.transport_electrons && share_p > ecut) {
                 p.rng.reserve(3);
                 const StreamId sid = p.rng.spawn();
-                queue_push(P, q_el, word_el, kPositron, p.beamlet(), share_p, p.w, p.x, p.y, p.z, p.ux, p.uy,
-                           p.uz, sid, n_push);
+                queue_push(P, rd, 0, kPositron, p.beamlet(), share_p, p.w, p.x, p.y, p.z, p.ux, p.uy, p.uz, sid);
             } else {
                 if (P.transport_electrons) put(p.w * share_p, share_p);
-                annihilate_at_rest<kPlain>(P, B, p, voxel, q_out,
-                                           kPlain ? 1.0f : spr_factor(P, kElectronMass, mat), dep, n_push);
+                annihilate_at_rest<kPlain>(P, B, p, voxel, rd,
+                                           kPlain ? 1.0f : spr_factor(P, kElectronMass, mat), dep);
             }
         }
         active = false;
     }
 
     __syncthreads();
-    if (chunked) close_chunk(P, q_el, chunk_el);
+    close_round(P, rd);
+    if (threadIdx.x == 0) B.pushes += rd.pushes;
     block_sum_add(reinterpret_cast<unsigned long long*>(&B.escaped), (unsigned long long)escaped);
     block_sum_add(&B.flights, n_flight);
     block_sum_add(&B.interactions, n_inter);
     block_sum_add(&B.deposits, dep.n);
-    block_sum_add(&B.pushes, n_push);
     flush_books(P, B);
 
     // The last block retires the consumed photon queue; the round's admission
     // window has been generated.
     if (last_block_arrives(S) && threadIdx.x == 0) {
-        retire_queue(S, q_in);
-        S->p_in = q_out;
+        retire_queue(S, rd.q_in);
+        S->p_in = rd.q_out[1];
         S->cursor = S->limit;
         S->blocks_done = 0u;
         __threadfence();
@@ -1132,7 +1144,7 @@ __global__ void __launch_bounds__(kPhotonThreads, kMinBlocks) photon_kernel(Tran
 // the electron queue for a charged source; a primary that is not to be
 // transported there leaves its slot dead, a charged one of a mixed source goes to
 // the electron queue.
-__global__ void __launch_bounds__(256) generate_kernel(TransportParams P) {
+__global__ void __launch_bounds__(256) generate_kernel(const __grid_constant__ TransportParams P) {
     __shared__ BlockBooks B;
     init_books(B);
     Sched* S = P.sched;
@@ -1143,6 +1155,7 @@ __global__ void __launch_bounds__(256) generate_kernel(TransportParams P) {
     const int batch = S->batch;
     const GenDesc& G = *P.gen;
     unsigned int n_push = 0, n_prim = 0, n_dead = 0;
+    long long emitted = 0, escaped = 0;  // per thread, booked once per warp
     const unsigned long long stride = (unsigned long long)gridDim.x * blockDim.x;
     const unsigned int window = round_to_chunk(limit - cursor);
     for (unsigned long long k = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x; k < window; k += stride) {
@@ -1151,14 +1164,16 @@ __global__ void __launch_bounds__(256) generate_kernel(TransportParams P) {
         bool queued = false;
         if (cursor + k < limit) {
             ++n_prim;
-            const int kind = generate_primary(P, G, batch, cursor + k, p, B);
+            const int kind = generate_primary(P, G, batch, cursor + k, p, emitted);
             if (kind >= 0 && P.window_el) {
                 queued = true;  // (it enters the grid in the electron kernel)
             } else if (kind == kPhoton) {
-                queued = enter_grid(P, B, p, 0.0f);
+                queued = enter_grid(P, p);
+                if (!queued) escaped += quantize_signed(p.w * p.e);
             } else if (kind > 0) {
-                queue_push(P, q_el, nullptr, kind, p.beamlet(), p.e, p.w, p.x, p.y, p.z, p.ux, p.uy, p.uz,
-                           p.rng.state(), n_push);
+                write_particle(P, q_el, single_slot(P, q_el), kind, p.beamlet(), p.e, p.w, p.x, p.y, p.z, p.ux,
+                               p.uy, p.uz, p.rng.state());
+                ++n_push;
             }
         }
         n_push += queued ? 1u : 0u;
@@ -1174,6 +1189,8 @@ __global__ void __launch_bounds__(256) generate_kernel(TransportParams P) {
     block_sum_add(&B.pushes, n_push);
     block_sum_add(&B.primaries, n_prim);
     block_sum_add(&B.dead, n_dead);
+    block_sum_add(reinterpret_cast<unsigned long long*>(&B.emitted), (unsigned long long)emitted);
+    block_sum_add(reinterpret_cast<unsigned long long*>(&B.escaped), (unsigned long long)escaped);
     flush_books(P, B);
     if (threadIdx.x == 0 && B.dead) atomicAdd(&S->dead[q_win].v, (unsigned int)B.dead);
 }
@@ -1191,7 +1208,7 @@ __device__ __forceinline__ float rest_energy(const ParticleOf<R>& p) {
 // shared memory, the plain scoring path and the terminal step folded into the
 // refill took the electron kernel from 17.5 to 12.4 ms and the photon kernel from
 // 13.6 to 12.1 ms.
-constexpr int kElectronThreads = 512;  // the largest block of the electron kernel
+constexpr int kElectronThreads = 384;  // the largest block of the electron kernel
 
 // One lane runs one electron or positron to ECUT (Class II condensed history,
 // electron.py:345-481); delta rays go to the next round's electron queue,
@@ -1201,12 +1218,14 @@ constexpr int kElectronThreads = 512;  // the largest block of the electron kern
 // shared memory (n_materials * n_points * 24 bytes); the inverse-range row
 // (one read per substep) stays on the L1 path.
 // kMinBlocks: resident blocks of 256 threads per SM the register allocation
-// targets: 4 (64 registers; launched as two blocks of 512, which stage the
-// tables twice per SM instead of four times) or 3 (85).
+// targets: 3 (85 registers; by default launched as two blocks of 384, which stage
+// the tables twice per SM instead of three times) or 4 (64, with spills: 10.0 ms
+// against 9.8 on the 100-column 128^3 Dij, and the longest electron of a small
+// round takes longer: 0.35 against 0.30 ms on a 16^3 run).
 // kPlain: as for the photon kernel.
 template <bool kSmem, int kMinBlocks, bool kPlain>
-__global__ void __launch_bounds__(kMinBlocks == 4 ? kElectronThreads : 256, kMinBlocks == 4 ? 2 : kMinBlocks)
-electron_kernel(TransportParams P) {
+__global__ void __launch_bounds__(kMinBlocks == 3 ? kElectronThreads : 256, kMinBlocks == 3 ? 2 : kMinBlocks)
+electron_kernel(const __grid_constant__ TransportParams P) {
     __shared__ BlockBooks B;
     __shared__ uint32_t ring[kRingWords * kElectronThreads];
     extern __shared__ __align__(16) unsigned char pmc_smem[];
@@ -1221,33 +1240,23 @@ electron_kernel(TransportParams P) {
         tab_ea = sea;
         tab_eb = seb;
     }
-    init_books(B);  // its barrier also publishes the staged tables
     Sched* S = P.sched;
-    const int pin = S->p_in, ein = S->e_in;
-    const int q_in = 2 + ein, q_out = 2 + (ein ^ 1), q_ph = pin;
-    Input in;
-    in.open(P, q_in);
-    __shared__ uint32_t chunks[2];  // the block's chunks of the next electron and photon queues
-    const bool chunked = chunked_round(P, in.n);
-    if (threadIdx.x == 0 && chunked) {
-        chunks[0] = open_chunk(P, q_out);
-        chunks[1] = open_chunk(P, q_ph);
-    }
-    __syncthreads();
-    uint32_t* const word_el = chunked ? chunks : nullptr;
-    uint32_t* const word_ph = chunked ? chunks + 1 : nullptr;
+    __shared__ Round rd;  // pushes the next round's electrons (0) and photons (1)
+    if (threadIdx.x == 0) open_round(P, rd, 2 + S->e_in, 2 + (S->e_in ^ 1), S->p_in, 3u);
+    init_books(B);  // its barrier also publishes the round and the staged tables
     const Tables& T = P.tab;
     const float pcut = P.pcut, ecut = P.ecut;
 
-    unsigned int n_sub = 0, n_push = 0;  // per lane and launch
+    Claim input;
+    unsigned int n_sub = 0;  // per lane and launch
     HeldSink<BinOf<kPlain>> dep;
-    ParticleOf<RingRng<kElectronThreads>> p;
+    ParticleOf<RingRng<kElectronThreads, false>> p;
     p.meta = 0u;
     p.rng.k0 = P.seed_lo;
     p.rng.k1 = P.seed_hi;
     p.rng.ring = ring + threadIdx.x;
-    bool active = false, exhausted = false, dry = false;
-    int tail = 0;  // substeps of the current particle since its warp found the round dry
+    bool active = false, exhausted = false;
+    int tail = -1;  // turns since the warp found the round dry
 
     for (unsigned int it = 0;; ++it) {
         if ((it & 255u) == 0u) {
@@ -1268,31 +1277,33 @@ electron_kernel(TransportParams P) {
                 deposit<kPlain>(P, B, p.beamlet(), p.x, p.y, p.z, voxel, p.w * p.e,
                                 kPlain ? 1.0f : spr_factor(P, p.e, tm), dep);
                 if (p.kind() == kPositron)
-                    annihilate_at_rest<kPlain>(P, B, p, voxel, q_ph,
-                                               kPlain ? 1.0f : spr_factor(P, kElectronMass, tm), dep, n_push);
+                    annihilate_at_rest<kPlain>(P, B, p, voxel, rd,
+                                               kPlain ? 1.0f : spr_factor(P, kElectronMass, tm), dep);
             }
             active = false;
         }
         if (!active) dep.release(P, p.beamlet());  // the finished particle's last held deposit
         const bool want = !active && !exhausted;
         if (__any_sync(0xffffffffu, want)) {
-            const unsigned int i = in.take(P, want);
+            const unsigned int i = input.take(P, rd, want);
             if (want) {
-                if (i < in.n) {
-                    active = load_slot(in.slot(P, i), p) && enter_grid(P, B, p, rest_energy(p));
-                    tail = 0;
+                if (i < rd.n) {
+                    if (load_slot(input_slot(P, rd, i), p)) {
+                        active = enter_grid(P, p);
+                        if (!active) escape(B, p.w * (p.e + rest_energy(p)));
+                    }
                 } else {
                     exhausted = true;
                 }
             }
         }
         if (!__any_sync(0xffffffffu, active || !exhausted)) break;
-        if (!dry) dry = __any_sync(0xffffffffu, exhausted);
+        if (tail >= 0 || __any_sync(0xffffffffu, exhausted)) ++tail;
         if (!active || p.e <= ecut) continue;
         // Park a particle that outlives the round's input by tail_steps substeps
         // (its held deposit is released at the top of the next iteration).
-        if (dry && ++tail > P.tail_steps) {
-            queue_suspend(P, q_out, p, n_push);
+        if (tail >= P.tail_steps) {
+            queue_suspend(P, rd, 0, p);
             active = false;
             continue;
         }
@@ -1395,8 +1406,7 @@ electron_kernel(TransportParams P) {
                 if (pw > 0.0f) {
                     p.rng.reserve(3);
                     const StreamId sid = p.rng.spawn();
-                    queue_push(P, q_ph, word_ph, kPhoton, p.beamlet(), k, pw, p.x, p.y, p.z, p.ux, p.uy, p.uz,
-                               sid, n_push);
+                    queue_push(P, rd, 1, kPhoton, p.beamlet(), k, pw, p.x, p.y, p.z, p.ux, p.uy, p.uz, sid);
                 }
             } else {
                 deposit_or_escape<kPlain>(P, B, p.beamlet(), p.x, p.y, p.z, p.w * k,
@@ -1426,8 +1436,7 @@ electron_kernel(TransportParams P) {
             float dx = p.ux, dy = p.uy, dz = p.uz;
             rotate_direction(dx, dy, dz, cd, mphi);
             const StreamId sid = p.rng.spawn();
-            queue_push(P, q_out, word_el, kElectron, p.beamlet(), w, p.w, p.x, p.y, p.z, dx, dy, dz, sid,
-                       n_push);
+            queue_push(P, rd, 0, kElectron, p.beamlet(), w, p.w, p.x, p.y, p.z, dx, dy, dz, sid);
             rotate_direction(p.ux, p.uy, p.uz, cp, mphi + kPi);
             p.e -= w;
         }
@@ -1435,20 +1444,17 @@ electron_kernel(TransportParams P) {
 
     dep.release(P, p.beamlet());
     __syncthreads();
-    if (chunked) {
-        close_chunk(P, q_out, chunks[0]);
-        close_chunk(P, q_ph, chunks[1]);
-    }
+    close_round(P, rd);
+    if (threadIdx.x == 0) B.pushes += rd.pushes;
     block_sum_add(&B.substeps, n_sub);
     block_sum_add(&B.deposits, dep.n);
-    block_sum_add(&B.pushes, n_push);
     flush_books(P, B);
 
     // The last block retires the consumed electron queue, opens the next
     // admission window and publishes whether any work is left.
     if (last_block_arrives(S) && threadIdx.x == 0) {
-        retire_queue(S, q_in);
-        S->e_in = ein ^ 1;
+        retire_queue(S, rd.q_in);
+        S->e_in = rd.q_out[0] - 2;
         S->rounds += 1;
         S->total_rounds += 1;
         const unsigned long long next_limit = S->cursor + S->budget;
