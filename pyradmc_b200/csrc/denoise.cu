@@ -838,7 +838,7 @@ bool umma_plan(const ConvShape& s, UmmaConv& u, int& smem, int& ctas_per_sm) {
     u.plane_bytes = (unsigned)npos * 16;
     u.halo_bytes = u.plane_bytes * cpt;
     const int extra = 16;  // mbarrier + tensor-memory address
-    const int all_chunks = 27 * cpt + (s.cin == 8 ? 1 : 0);
+    const int all_chunks = (int)w_chunks_of(cpt);
     const int base = (int)u.halo_bytes + kUSlack + extra;
     const int per_tap = cpt * s.cout * 16 + cpt * 8;  // weights + descriptor table entries
     if (base + all_chunks * (s.cout * 16 + 8) <= kSmemPerBlockMax) {
@@ -949,8 +949,11 @@ bool ws_plan(const ConvShape& s, WsConv& p, int& smem, int& ctas_per_sm) {
     const int cpt = s.cin / 8, N = s.cout;
     p = WsConv{};
     p.s = s;
-    p.tz = s.cin <= 16 && s.cout <= 16 ? 4 : (s.cin <= 48 ? 2 : 1);
+    // taller tiles fold more of an MMA's outputs together; one slice where the
+    // weights are streamed or an MMA is full already
+    p.tz = s.cin <= 32 && s.cout <= 32 ? 4 : (s.cin <= 48 || s.cout <= 32 ? 2 : 1);
     while (p.tz > 1 && 2 * p.tz * N > 512) --p.tz;
+    if (p.tz == 3) p.tz = 2;
     if (2 * p.tz * N > 512) return false;
     p.box_bytes = (unsigned)((p.tz + 2) * kUHY * kUHX * 16);
     p.plane_bytes = (p.box_bytes + 127u) & ~127u;
@@ -963,10 +966,12 @@ bool ws_plan(const ConvShape& s, WsConv& p, int& smem, int& ctas_per_sm) {
         // even groups only (cg = 1 pairs taps, one K step in 28 on a zero chunk,
         // and measured slower than one block per SM with the whole halo)
         if (cpt % cg || (cg % 2 && cg != cpt)) continue;
-        const unsigned chunks = 27u * cg + (cg == 1 ? 1u : 0u);  // per group (cg = 1: zero partner)
+        const unsigned chunks = w_chunks_of(cg);  // per group
         const unsigned stage = round128((unsigned)cg * p.plane_bytes + kUSlack);
-        const int n_st = cg == cpt ? 2 : 3;
-        const long long need = (long long)n_st * stage + (long long)(cpt / cg) * chunks * N * 16 + bars;
+        int n_st = cg == cpt ? 2 : 3;
+        const long long fixed = (long long)(cpt / cg) * chunks * N * 16 + bars;
+        if (n_st * (long long)stage + fixed > kSmemPerBlockMax) n_st = 2;
+        const long long need = (long long)n_st * stage + fixed;
         if (need > kSmemPerBlockMax) continue;
         if (p.cg != 0 && need > pair_smem) continue;  // a smaller group only to reach two blocks per SM
         p.cg = cg;
@@ -984,7 +989,7 @@ bool ws_plan(const ConvShape& s, WsConv& p, int& smem, int& ctas_per_sm) {
         for (int want = 3; want >= 2 && p.cg == 0; --want)
             for (int cg = cpt; cg >= 1; --cg) {
                 if (cpt % cg || (cg > 1 && cg % 2)) continue;
-                const unsigned chunks = 27u * cg + (cg == 1 ? 1u : 0u);
+                const unsigned chunks = w_chunks_of(cg);
                 const unsigned halo = (unsigned)cg * p.plane_bytes + kUSlack;
                 const unsigned stage = round128(halo + chunks * N * 16);
                 const int fixed = bars;

@@ -12,9 +12,9 @@
 // layout of a UMMA shared-memory descriptor (start address, LBO = distance
 // of the second 8-element K half, SBO = 160 B), so every tap is one
 // descriptor offset into the same halo and no im2col copy exists.  Weights
-// sit in shared memory as w[chunk][cout][8] (the B operand, SBO = 128 B,
-// LBO = cout * 16 B).  One thread issues the MMAs (M = 128, N = cout,
-// K = 16 per instruction); tcgen05.commit arrives on an mbarrier that every
+// sit in shared memory as w[chunk][cout][8] (the B operand, SBO = 128 B), in the
+// order of w_place.  One thread issues the MMAs (M = 128, N = up to 3 cout,
+// K = 16 per instruction: umma_issue_taps); tcgen05.commit arrives on an mbarrier that every
 // thread waits on, with a time limit that records a failure instead of
 // hanging.  The epilogue reads the fp32 accumulators from tensor memory
 // (tcgen05.ld, one row per thread), adds the bias, applies ReLU and stores
@@ -39,7 +39,7 @@ struct UmmaConv {
     int passes;
     int tiles_d, tiles_h, tiles_w, n_tiles;
     unsigned halo_bytes, plane_bytes;
-    unsigned w_chunks;  // weight chunks staged per pass (incl. the cin = 8 pad partner)
+    unsigned w_chunks;  // weight chunks staged per pass (incl. the cin = 8 zero partners)
     unsigned k_steps;   // K steps (16-wide) per pass: descriptor table entries
     unsigned tmem_cols;
     int ystride;        // channels per voxel of the output tensor (>= cout: a channel slice)
@@ -135,48 +135,87 @@ __host__ __device__ constexpr uint32_t tap_off16(int t) {
     return (uint32_t)((t / 9) * kUHY * kUHX + ((t / 3) % 3) * kUHX + t % 3);
 }
 
+// Where weight chunk (tap, q) of a group of cg 8-channel chunks stands in shared
+// memory, in chunks of [cout][8]: for each (dy, dx, q) the three dz of a tap side by
+// side, the farthest first, so that the rows of dz = 2, 1, 0 are one B operand of
+// 3 cout rows.
+__host__ __device__ constexpr int w_place(int tap, int q, int cg) {
+    return ((tap % 9) * cg + q) * 3 + 2 - tap / 9;
+}
+// The chunk that stands at place `at`, as tap * cg + q; 27 * cg and up: the zero
+// partner of the last tap (cg = 1).
+__host__ __device__ constexpr int w_chunk_at(int at, int cg) {
+    const int t = at / 3;
+    return t / cg < 9 ? ((2 - at % 3) * 9 + t / cg) * cg + t % cg : 27 * cg;
+}
+// Weight chunks of a group: 27 per 8-channel chunk, and for cg = 1 the three of
+// the zero partner.
+__host__ __device__ constexpr unsigned w_chunks_of(int cg) { return 27u * cg + (cg == 1 ? 3u : 0u); }
+
 // Issues the MMAs of all 27 taps over CG 8-channel chunks for the tz slices of
 // a tile: A from the halo planes at a_addr (plane_bytes apart), B from the
-// weight chunks [tap * CG + q][N][8] at b_addr, slice sl into accumulator
-// columns d0 + sl * N, in the order slice, tap, chunk pair.  Every descriptor is
-// the slice's base descriptor plus an offset fixed at compile time within a
-// group of 9 taps (7 tap pairs for CG = 1), so the issuing thread runs no loads
-// and little arithmetic between MMAs (a thread issuing from a descriptor table
-// in shared memory measured ~50-120 cycles per MMA, well above the tensor
-// cores' ~35 for M = 128, N <= 32).  The tap loop stays a loop of such groups
-// and the slice loop is not unrolled: with the 14 or 27 MMAs of a slice
-// unrolled in full for CG = 1 and 2, this build computed wrong sums (tested
-// against the oracle), while the grouped form is exact for every CG.  With CG = 1 a K step
-// pairs two taps: the second half's LBO is the distance between their rows and
-// the last tap pairs with a zero weight chunk.  accumulate: whether the first
-// K step adds to the accumulator (a later channel group of the same tile).
+// weight chunks at b_addr (w_place), output slice sl in accumulator columns d0 + sl * N.
+//
+// An M = 128 MMA reads its 4 KB of A from shared memory at 128 bytes a cycle
+// whatever its N, which is what bounds N = 16 and 32.  So the loop runs over the
+// halo's slices, and one MMA takes halo slice zz to all the outputs it belongs to:
+// slice zz - 2 as dz = 2, zz - 1 as dz = 1, zz as dz = 0, side by side in the
+// accumulator and in the weights (N = 3 cout, fewer at the tile's ends): (tz + 2) * 9
+// MMAs per K step instead of tz * 27.  Every output still takes its products in the
+// order dz, (dy, dx), chunk pair.  An output's first K step overwrites, the
+// others' of that MMA add: it is split there.
+//
+// Every descriptor is the slice's base descriptor plus an offset fixed at compile
+// time, so the issuing thread runs no loads and little arithmetic between MMAs (a
+// thread issuing from a descriptor table in shared memory measured ~50-120 cycles
+// per MMA).  The slice loop is not unrolled: with the 14 or 27 MMAs of a slice
+// unrolled in full for CG = 1 and 2, an earlier build computed wrong sums (tested
+// against the oracle); nine are exact for every CG.  With CG = 1 a K step pairs two
+// taps of a halo slice: the second half's LBO is the distance between their rows and
+// the last tap pairs with zero weights.  accumulate: whether the first K step adds
+// to the accumulator (a later channel group of the same tile).
 template <int CG>
 __device__ __forceinline__ void umma_issue_taps(uint32_t d0, uint32_t a_addr, uint32_t plane_bytes,
-                                                uint32_t b_addr, int N, int tz, uint32_t idesc,
+                                                uint32_t b_addr, int N, int tz, uint32_t /*idesc*/,
                                                 bool accumulate) {
     constexpr uint64_t slice16 = (uint64_t)(kUHY * kUHX);
     const uint64_t a0 = umma_smem_desc(a_addr, CG == 1 ? 0u : plane_bytes, kUHX * 16);
-    const uint64_t b0 = umma_smem_desc(b_addr, (uint32_t)N * 16, 128);
+    const uint64_t b0 = umma_smem_desc(b_addr, 3u * (uint32_t)N * 16, 128);
     const uint64_t plane16 = plane_bytes >> 4;
+    const uint64_t n3 = 3u * (uint64_t)N;
+    const int fold = min(3, 256 / N);  // outputs of one MMA: N is at most 256
 #pragma unroll 1
-    for (int sl = 0; sl < tz; ++sl) {
-        const uint32_t d = d0 + (uint32_t)(sl * N);
-        const uint64_t as = a0 + slice16 * (uint64_t)sl;
-        if constexpr (CG == 1) {
-#pragma unroll 7
-            for (int tap = 0; tap < 27; tap += 2) {
-                const uint64_t lbo16 = tap + 1 < 27 ? tap_off16(tap + 1) - tap_off16(tap) : 1u;
-                umma_bf16(d, as + tap_off16(tap) + (lbo16 << 16), b0 + (uint64_t)(tap * N), idesc,
-                          (accumulate || tap > 0) ? 1u : 0u);
-            }
-        } else {
-#pragma unroll 9
-            for (int tap = 0; tap < 27; ++tap)
+    for (int zz = 0; zz < tz + 2; ++zz) {
+        const uint64_t as = a0 + slice16 * (uint64_t)zz;
+        const int hi = min(zz, tz - 1);
+#pragma unroll 1
+        for (int lo = max(zz - 2, 0); lo <= hi; lo += fold) {
+            const int cnt = min(fold, hi - lo + 1);
+            const bool fresh = !accumulate && lo + cnt - 1 == zz;  // its last output starts here
+            const uint32_t d = d0 + (uint32_t)(lo * N);
+            const uint64_t bs = b0 + (uint64_t)((2 - zz + lo) * N);
+            const uint32_t id = umma_instr_desc(cnt * N);
+            if (fresh && cnt > 1) umma_bf16(d, as + (CG == 1 ? (uint64_t)1 << 16 : 0u), bs, umma_instr_desc((cnt - 1) * N), 1u);
+            const uint32_t d_first = fresh ? d + (uint32_t)((cnt - 1) * N) : d;
+            const uint64_t b_first = fresh ? bs + (uint64_t)((cnt - 1) * N) : bs;
+            const uint32_t id_first = fresh ? umma_instr_desc(N) : id;
+            if constexpr (CG == 1) {
+                umma_bf16(d_first, as + ((uint64_t)1 << 16), b_first, id_first, fresh ? 0u : 1u);
 #pragma unroll
-                for (int q = 0; q < CG; q += 2)
-                    umma_bf16(d, as + tap_off16(tap) + plane16 * (uint64_t)q,
-                              b0 + (uint64_t)((tap * CG + q) * N), idesc,
-                              (accumulate || tap > 0 || q > 0) ? 1u : 0u);
+                for (int t = 2; t < 9; t += 2) {
+                    const uint64_t lbo16 = t + 1 < 9 ? tap_off16(t + 1) - tap_off16(t) : 1u;
+                    umma_bf16(d, as + tap_off16(t) + (lbo16 << 16), bs + (uint64_t)t * n3, id, 1u);
+                }
+            } else {
+                umma_bf16(d_first, as, b_first, id_first, fresh ? 0u : 1u);
+#pragma unroll
+                for (int t = 0; t < 9; ++t)
+#pragma unroll
+                    for (int q = 0; q < CG; q += 2)
+                        if (t > 0 || q > 0)
+                            umma_bf16(d, as + tap_off16(t) + plane16 * (uint64_t)q,
+                                      bs + (uint64_t)(t * CG + q) * n3, id, 1u);
+            }
         }
     }
 }
@@ -255,14 +294,18 @@ conv3d_umma_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __r
             const int j1 = t1 * cpt;
             const int k_begin = j0 / 2, k_end = (j1 + 1) / 2;
             if (u.passes > 1 || !weights_resident) {
-                const int n_chunks = (int)u.w_chunks < (j1 - j0 + (j1 - j0) % 2) ? (int)u.w_chunks
-                                                                               : (j1 - j0 + (j1 - j0) % 2);
+                // one pass: in the order of umma_issue_taps (the chunks past the 27
+                // taps are zero padding); several: as they come
+                const int n_chunks = u.passes == 1 ? (int)u.w_chunks
+                                     : (int)u.w_chunks < (j1 - j0 + (j1 - j0) % 2) ? (int)u.w_chunks
+                                                                                   : (j1 - j0 + (j1 - j0) % 2);
                 for (int i = tid; i < n_chunks * N; i += blockDim.x) {
                     const int n = i % N, jj = i / N;
+                    const int from = u.passes == 1 ? w_chunk_at(jj, cpt) : j0 + jj;
                     cp_async16(wbuf + ((size_t)jj * N + n) * 16,
-                               wt + (long long)n * s.kpad + (long long)(j0 + jj) * 8, true);
+                               wt + (long long)n * s.kpad + (long long)from * 8, true);
                 }
-                for (int k = k_begin + tid; k < k_end; k += blockDim.x) {
+                for (int k = k_begin + tid; u.passes > 1 && k < k_end; k += blockDim.x) {
                     const int j = 2 * k;
                     const int tap = j / cpt, q = j % cpt;
                     const uint32_t a_addr = halo_s + (uint32_t)q * u.plane_bytes + tap_offset(tap);
@@ -485,7 +528,8 @@ conv3d_umma_pipe_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16
     const int n_chunks = (int)u.w_chunks;
     for (int i = tid; i < n_chunks * N; i += blockDim.x) {
         const int n = i % N, jj = i / N;
-        cp_async16(wbuf + ((size_t)jj * N + n) * 16, wt + (long long)n * s.kpad + (long long)jj * 8, true);
+        cp_async16(wbuf + ((size_t)jj * N + n) * 16,
+                   wt + (long long)n * s.kpad + (long long)w_chunk_at(jj, CPT) * 8, true);
     }
     if ((int)blockIdx.x < u.n_tiles) umma_load_halo<CPT>(x, u, blockIdx.x, halo0, tid);
     cp_async_commit();

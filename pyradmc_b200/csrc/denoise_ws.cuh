@@ -20,7 +20,8 @@
 //     to the producer and each finished tile to the epilogue.
 //   * warps 2-5 drain an accumulator (tcgen05.ld, bias, ReLU, bf16 stores, one
 //     output voxel per thread) and release it.
-// Resident weights are staged once per block as [group][tap][chunk][cout][8].
+// Resident weights are staged once per block as [group][chunks in the order of
+// w_place][cout][8].
 // With one channel group and resident weights the MMAs of a slice are issued
 // in the order of conv3d_umma_kernel, so the two produce identical bits.
 // Every mbarrier wait gives up after kUWaitNs, records the failure in shared
@@ -48,7 +49,7 @@ struct WsConv {
     unsigned box_bytes;      // bytes one halo copy writes
     unsigned halo_part;      // cg planes + zeroed slack: offset of a stage's weights
     unsigned stage_bytes;    // stride between stage buffers
-    unsigned w_chunks;       // weight chunks of one channel group (cg = 1: with a zero partner)
+    unsigned w_chunks;       // weight chunks of one channel group (cg = 1: with the zero partners)
     unsigned tx_bytes;       // bytes the copy engine writes per stage
     unsigned acc_cols;       // tensor-memory columns of one accumulator: tz * cout
     unsigned tmem_cols;      // allocated: two accumulators, a power of two >= 32
@@ -139,7 +140,7 @@ conv3d_ws_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     unsigned char* stage0 = smem;  // stage b at stage0 + b * stage_bytes
     unsigned char* wres = smem + (size_t)S * p.stage_bytes;  // resident weights (streamed: empty)
-    // resident weights: [group][tap][chunk][cout][8], w_chunks per group
+    // resident weights: [group][w_place][cout][8], w_chunks per group
     const size_t group_bytes = (size_t)p.w_chunks * N * 16;
     const size_t wres_bytes = p.streamed ? 0 : (size_t)p.groups * group_bytes;
     uint64_t* bars = reinterpret_cast<uint64_t*>(wres + wres_bytes);  // full[S], empty[S], acc_full[2], acc_free[2]
@@ -164,16 +165,17 @@ conv3d_ws_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant
             if (byte >= (unsigned)cg * p.plane_bytes || byte % p.plane_bytes >= p.box_bytes) st[i] = 0u;
         }
         if (p.streamed && cg == 1)
-            for (int i = tid; i < N * 4; i += blockDim.x) st[(p.halo_part + 27u * N * 16u) / 4 + i] = 0u;
+            for (int i = tid; i < 3 * N * 4; i += blockDim.x) st[(p.halo_part + 27u * N * 16u) / 4 + i] = 0u;
     }
     if (!p.streamed)
         for (int i = tid; i < p.groups * (int)p.w_chunks * N; i += blockDim.x) {
             const int n = i % N, c = i / N;
             const int g = c / (int)p.w_chunks, jj = c % (int)p.w_chunks;
-            const int chunk = (jj / cg) * cpt + g * cg + jj % cg;  // tap * cpt + channel chunk
-            const uint4 v = jj < 27 * cg
+            const int in_group = w_chunk_at(jj, cg);  // tap * cg + q
+            const int chunk = in_group / cg * cpt + g * cg + in_group % cg;
+            const uint4 v = in_group < 27 * cg
                                 ? *reinterpret_cast<const uint4*>(wt + (long long)n * s.kpad + chunk * 8)
-                                : make_uint4(0u, 0u, 0u, 0u);  // the cg = 1 pad partner
+                                : make_uint4(0u, 0u, 0u, 0u);  // the cg = 1 zero partner
             *reinterpret_cast<uint4*>(wres + ((size_t)c * N + n) * 16) = v;
         }
     if (tid == 0) {
@@ -217,7 +219,7 @@ conv3d_ws_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant
                     if (p.streamed)
                         for (int tap = 0; tap < 27; ++tap)
                             for (int q = 0; q < cg; ++q)
-                                tma_load_2d(dst + p.halo_part + (uint32_t)(tap * cg + q) * N * 16, &wmap,
+                                tma_load_2d(dst + p.halo_part + (uint32_t)w_place(tap, q, cg) * N * 16, &wmap,
                                             (tap * cpt + g * cg + q) * 8, 0, full(b));
                     ++st;
                 }
