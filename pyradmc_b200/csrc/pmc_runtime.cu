@@ -1884,8 +1884,8 @@ int pmc_truncate_dense(pmc_engine* e, const double* mean, const double* sigma, i
     if (rc) return rc;
     {
         const int n_tiles = (int)(e->col_stride / kTileVoxels);
-        colmax_kernel<<<dim3(n_tiles, n_cols), kReduceThreads, 0, e->stream>>>(
-            (const double*)e->s1.p, n_vox, e->col_stride, e->d_colmax);
+        colmax_kernel<<<dim3(reduce_blocks(n_tiles), n_cols), kReduceThreads, 0, e->stream>>>(
+            (const double*)e->s1.p, n_vox, e->col_stride, n_tiles, e->d_colmax, nullptr);
         PMC_CUDA(e, cudaGetLastError());
     }
     e->dij_indptr.assign(1, 0);
@@ -1926,7 +1926,7 @@ struct StaticScratch {
     unsigned long long total;
     unsigned long long pad[31];
     unsigned int tile_counts[kStaticMaxTiles];
-    unsigned long long tile_offsets[kStaticMaxTiles];
+    unsigned long long tile_offsets[kStaticMaxTiles];  // first the tiles' maxima, then their offsets
 };
 
 static __device__ __align__(256) StaticScratch g_static_scratch;
@@ -1975,10 +1975,11 @@ int pmc_dij_compact_static(const double* mean, const double* sigma, int32_t n_co
     // The array keeps the previous call's contents: the maxima must restart at 0.
     if (cudaMemsetAsync(scratch->col_max, 0, sizeof(unsigned long long) * n_cols, st) != cudaSuccess)
         return PMC_ERR_CUDA;
-    const dim3 grid((unsigned)n_tiles, (unsigned)n_cols);
-    colmax_kernel<<<grid, kReduceThreads, 0, st>>>(mean, n_vox, n_vox, scratch->col_max);
-    count_kept_kernel<<<grid, kReduceThreads, 0, st>>>(mean, n_vox, (int)n_tiles, truncation,
-                                                        scratch->col_max, scratch->tile_counts);
+    const dim3 grid((unsigned)reduce_blocks(n_tiles), (unsigned)n_cols);
+    unsigned long long* tile_max = scratch->tile_offsets;  // (the offsets are written after the counts)
+    colmax_kernel<<<grid, kReduceThreads, 0, st>>>(mean, n_vox, n_vox, (int)n_tiles, scratch->col_max, tile_max);
+    count_kept_kernel<<<grid, kReduceThreads, 0, st>>>(mean, n_vox, (int)n_tiles, truncation, scratch->col_max,
+                                                        tile_max, scratch->tile_counts);
     scan_tiles_kernel<<<1, 1024, 0, st>>>(scratch->tile_counts, n_tiles * n_cols,
                                           scratch->tile_offsets, n_cols, (int)n_tiles,
                                           scratch->col_counts, &scratch->total);
@@ -1993,8 +1994,8 @@ int pmc_dij_compact_static(const double* mean, const double* sigma, int32_t n_co
     if (total > 0) {
         if (!out_indices || !out_dose || !out_sigma) return PMC_ERR_INVALID;
         compact_kernel<<<grid, kReduceThreads, 0, st>>>(
-            mean, sigma, n_vox, (int)n_tiles, truncation, scratch->col_max, scratch->tile_offsets,
-            (long long*)out_indices, out_dose, out_sigma);
+            mean, sigma, n_vox, (int)n_tiles, truncation, scratch->col_max, scratch->tile_counts,
+            scratch->tile_offsets, (long long*)out_indices, out_dose, out_sigma);
     }
     if (cudaMemcpyAsync(col_counts, scratch->col_counts, sizeof(long long) * n_cols,
                         cudaMemcpyDeviceToDevice, st) != cudaSuccess)
