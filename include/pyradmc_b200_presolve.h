@@ -114,6 +114,22 @@ int pmc_presolve_head(const pmc_head_stack* stack, const pmc_head_mu* mu, const 
                       float* out_pos, float* out_dir, float* out_weight, int64_t* count,
                       double* dropped);
 
+/* The same for a caller that keeps its memory: columns is one host array of eight
+ * columns of n (energy, x, y, z, direction cosines u, v, w, weight; page-locked for a
+ * copy at the link's rate), workspace at least pmc_presolve_workspace bytes of device
+ * memory (256-byte aligned), the out_* arrays are device memory, and all work is
+ * ordered on `stream`, which is synchronized before the return.  The phase space
+ * comes out as it is handed on: directions renormalized, weights scaled by
+ * particles / n (in float64, rounded once).  PMC_ERR_CAPACITY when more than
+ * `capacity` particles are kept (*count says how many; nothing is written). */
+int pmc_presolve_workspace(const pmc_head_stack* stack, const pmc_head_mu* mu, const pmc_head_params* params,
+                           int64_t n, int64_t* bytes);
+int pmc_presolve_head_device(const pmc_head_stack* stack, const pmc_head_mu* mu, const pmc_head_params* params,
+                             int64_t n, const float* columns, void* workspace, int64_t workspace_bytes,
+                             int64_t capacity, int32_t* out_kind, float* out_energy, float* out_pos,
+                             float* out_dir, float* out_weight, int64_t* count, double* dropped,
+                             void* stream);
+
 #ifdef __cplusplus
 }
 #endif

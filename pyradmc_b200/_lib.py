@@ -296,7 +296,7 @@ SIGNATURES: dict[str, tuple[object, list]] = {
     ),
 }
 
-# The head pre-solve (include/pyradmc_b200_presolve.h): host arrays throughout.
+# The head pre-solve (include/pyradmc_b200_presolve.h).
 _dp = C.POINTER(C.c_double)
 
 
@@ -331,6 +331,12 @@ SIGNATURES.update({
     "pmc_presolve_head": (C.c_int, [C.POINTER(HeadStack), C.POINTER(HeadMu), C.POINTER(HeadParams),
                                     C.c_int64, _fp, _fp, _fp, _fp, C.c_int64, _ip, _fp, _fp, _fp, _fp,
                                     _lp, _dp]),
+    "pmc_presolve_workspace": (C.c_int, [C.POINTER(HeadStack), C.POINTER(HeadMu), C.POINTER(HeadParams),
+                                         C.c_int64, _lp]),
+    "pmc_presolve_head_device": (C.c_int, [C.POINTER(HeadStack), C.POINTER(HeadMu), C.POINTER(HeadParams),
+                                           C.c_int64, C.c_void_p, C.c_void_p, C.c_int64, C.c_int64,
+                                           C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p,
+                                           _lp, _dp, C.c_void_p]),
 })
 
 # The denoiser's entry points (include/pyradmc_b200_denoise.h); every pointer is

@@ -15,6 +15,7 @@
 #pragma once
 
 #include "pmc_common.cuh"
+#include "pmc_scan.cuh"
 
 namespace pmc {
 
@@ -507,56 +508,6 @@ count_kept_kernel(const double* __restrict__ mean, long long n_vox, int n_tiles,
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) c += __shfl_xor_sync(0xffffffffu, c, off);
     if (lane == 0) tile_counts[col * n_tiles + tile] = c;
-}
-
-// Exclusive scan of the tile counts in CSC order (column-major, tiles
-// ascending) with per-column totals; one block over pieces of 4096 counts, four per
-// thread, scanned by warp shuffles (two barriers a piece; ten doubling steps over
-// 1024-wide pieces took 117 us for 52 k tiles, 465 us for 205 k).
-__global__ void __launch_bounds__(1024)
-scan_tiles_kernel(const unsigned int* __restrict__ tile_counts, long long n,
-                  unsigned long long* __restrict__ tile_offsets, int n_cols, int n_tiles,
-                  long long* __restrict__ col_counts, unsigned long long* __restrict__ total) {
-    __shared__ unsigned int warp_sum[2][32];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    unsigned long long carry = 0ull;
-    int flip = 0;
-    for (long long base = 0; base < n; base += 4096, flip ^= 1) {
-        const long long i = base + 4 * (long long)threadIdx.x;
-        unsigned int v[4];
-#pragma unroll
-        for (int k = 0; k < 4; ++k) v[k] = i + k < n ? tile_counts[i + k] : 0u;
-        const unsigned int mine = v[0] + v[1] + v[2] + v[3];
-        unsigned int incl = mine;  // a piece holds at most 4096 tiles of 4096 voxels: 2^24
-#pragma unroll
-        for (int off = 1; off < 32; off <<= 1) {
-            const unsigned int y = __shfl_up_sync(0xffffffffu, incl, off);
-            if (lane >= off) incl += y;
-        }
-        if (lane == 31) warp_sum[flip][warp] = incl;
-        __syncthreads();  // (the other half is not written before the next piece's barrier)
-        const unsigned int w = warp_sum[flip][lane];
-        unsigned int w_incl = w;
-#pragma unroll
-        for (int off = 1; off < 32; off <<= 1) {
-            const unsigned int y = __shfl_up_sync(0xffffffffu, w_incl, off);
-            if (lane >= off) w_incl += y;
-        }
-        unsigned long long at = carry + __shfl_sync(0xffffffffu, w_incl - w, warp) + (incl - mine);
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            if (i + k < n) tile_offsets[i + k] = at;
-            at += v[k];
-        }
-        carry += __shfl_sync(0xffffffffu, w_incl, 31);
-    }
-    if (threadIdx.x == 0) *total = carry;
-    __syncthreads();  // the block's offsets are written
-    for (int c = threadIdx.x; c < n_cols; c += blockDim.x) {
-        const unsigned long long from = __ldcg(tile_offsets + (long long)c * n_tiles);
-        const unsigned long long to = c + 1 < n_cols ? __ldcg(tile_offsets + (long long)(c + 1) * n_tiles) : carry;
-        col_counts[c] = (long long)(to - from);
-    }
 }
 
 // Write the kept entries of one (column, tile) in ascending voxel order at the

@@ -38,6 +38,13 @@ struct DevBuf {
     size_t bytes = 0;
 };
 
+// What a call reads back besides its results, laid out alike on the device.
+struct Status {
+    Sched sched;
+    Counters counters;
+    unsigned long long total_q;  // quanta folded
+};
+
 // Launch shape of the primary generator and the two transport kernels.
 struct LaunchShape {
     int grid_ph = 0, grid_el = 0;
@@ -94,10 +101,11 @@ struct pmc_engine {
     DevBuf dirty, touched;        // sector bitmaps of edep / of the sums (pmc_reduce.cuh)
     bool edep_clean = false;      // every quanta entry is zero (true after a completed run)
     long long col_stride = 0;     // entries per column of the maps in the current call
-    Sched* d_sched = nullptr;
-    Counters* d_counters = nullptr;
+    Sched* d_sched = nullptr;        // one block: scheduler, counters and deposited total,
+    Counters* d_counters = nullptr;  // read back together
     GenDesc* d_gen = nullptr;
     unsigned long long* d_total_q = nullptr;
+    Status* status = nullptr;      // page-locked copy of that block
     unsigned int* d_fold_next = nullptr;  // parts the fold or finalize has claimed
     unsigned long long* d_colmax = nullptr;
     long long colmax_len = 0;
@@ -406,14 +414,18 @@ __global__ void init_batch_kernel(Sched* S, int batch, unsigned long long block_
     open_window(S, window_el);
 }
 
-struct SchedHost {
-    Sched s;
-};
+// Queue the copy of the device's status block; valid once the stream is done.
+int fetch_status(pmc_engine* e) {
+    PMC_CUDA(e, cudaMemcpyAsync(e->status, e->d_sched, sizeof(Status), cudaMemcpyDeviceToHost, e->stream));
+    e->d2h_bytes += (unsigned long long)(sizeof(Status));
+    return PMC_OK;
+}
 
 int read_sched(pmc_engine* e, Sched* out) {
-    PMC_CUDA(e, cudaMemcpyAsync(out, e->d_sched, sizeof(Sched), cudaMemcpyDeviceToHost, e->stream));
-        e->d2h_bytes += (unsigned long long)(sizeof(Sched));
+    const int rc = fetch_status(e);
+    if (rc) return rc;
     PMC_CUDA(e, cudaStreamSynchronize(e->stream));
+    *out = e->status->sched;
     return PMC_OK;
 }
 
@@ -789,19 +801,14 @@ int fill_bitmap(pmc_engine* e, DevBuf& b, int group, unsigned int v) {
 
 int reset_counters(pmc_engine* e) {
     std::memset(&e->counters, 0, sizeof e->counters);
-    PMC_CUDA(e, cudaMemsetAsync(e->d_counters, 0, sizeof(Counters), e->stream));
-    PMC_CUDA(e, cudaMemsetAsync(e->d_sched, 0, sizeof(Sched), e->stream));
+    PMC_CUDA(e, cudaMemsetAsync(e->d_sched, 0, sizeof(Status), e->stream));
     return PMC_OK;
 }
 
+// The call's counters and books, from the status block last read.
 int finish_counters(pmc_engine* e, pmc_books* books) {
-    Counters c{};
-    Sched s{};
-    PMC_CUDA(e, cudaMemcpyAsync(&c, e->d_counters, sizeof c, cudaMemcpyDeviceToHost, e->stream));
-        e->d2h_bytes += (unsigned long long)(sizeof c);
-    PMC_CUDA(e, cudaMemcpyAsync(&s, e->d_sched, sizeof s, cudaMemcpyDeviceToHost, e->stream));
-        e->d2h_bytes += (unsigned long long)(sizeof s);
-    PMC_CUDA(e, cudaStreamSynchronize(e->stream));
+    const Counters& c = e->status->counters;
+    const Sched& s = e->status->sched;
     e->counters.rounds = s.total_rounds;
     e->counters.kernel_launches += 3 * s.total_rounds + e->counters.reduce_launches;
     e->counters.photon_flights = (int64_t)c.flights;
@@ -811,6 +818,8 @@ int finish_counters(pmc_engine* e, pmc_books* books) {
     e->counters.queue_pushes = (int64_t)c.pushes;
     e->counters.primaries = (int64_t)c.primaries;
     if (books) {
+        std::memset(books, 0, sizeof *books);
+        books->deposited = (int64_t)e->status->total_q;
         books->escaped = c.escaped;
         books->unscored = c.unscored;
         books->emitted = c.emitted;
@@ -969,10 +978,15 @@ int pmc_create(pmc_engine** out, int device_ordinal) {
     if (st == cudaSuccess) st = cudaStreamCreateWithFlags(&e->own_stream, cudaStreamNonBlocking);
     e->stream = e->own_stream;
     if (st == cudaSuccess) st = cudaDeviceGetAttribute(&e->sm_count, cudaDevAttrMultiProcessorCount, device_ordinal);
-    if (st == cudaSuccess) st = cudaMalloc(&e->d_sched, sizeof(Sched));
-    if (st == cudaSuccess) st = cudaMalloc(&e->d_counters, sizeof(Counters));
+    Status* block = nullptr;
+    if (st == cudaSuccess) st = cudaMalloc(&block, sizeof(Status));
+    if (st == cudaSuccess) {
+        e->d_sched = &block->sched;
+        e->d_counters = &block->counters;
+        e->d_total_q = &block->total_q;
+        st = cudaMallocHost(&e->status, sizeof(Status));
+    }
     if (st == cudaSuccess) st = cudaMalloc(&e->d_gen, sizeof(GenDesc));
-    if (st == cudaSuccess) st = cudaMalloc(&e->d_total_q, sizeof(unsigned long long));
     if (st == cudaSuccess) st = cudaMalloc(&e->d_fold_next, sizeof(unsigned int));
     if (st == cudaSuccess) st = cudaMalloc(&e->d_nnz, sizeof(unsigned long long));
     for (int i = 0; i < 4 && st == cudaSuccess; ++i) st = cudaEventCreate(&e->ev[i]);
@@ -1003,8 +1017,8 @@ void pmc_destroy(pmc_engine* e) {
                       &e->out_dose, &e->out_sigma, &e->col_nhist, &e->dirty, &e->touched,
                       &e->stage})
         if (b->p) cudaFree(b->p);
-    for (void* p : {(void*)e->d_sched, (void*)e->d_counters, (void*)e->d_gen,
-                    (void*)e->d_total_q, (void*)e->d_fold_next, (void*)e->d_colmax, (void*)e->d_nnz})
+    if (e->status) cudaFreeHost(e->status);
+    for (void* p : {(void*)e->d_sched, (void*)e->d_gen, (void*)e->d_fold_next, (void*)e->d_colmax, (void*)e->d_nnz})
         if (p) cudaFree(p);
     for (cudaEvent_t ev : e->ev)
         if (ev) cudaEventDestroy(ev);
@@ -1497,7 +1511,6 @@ int pmc_run_forward(pmc_engine* e, const pmc_source_desc* src, const pmc_run_par
     const bool one_wave = plan.wave >= p->n_batches;
     if (one_wave) rc = clear_colmax(e, 1);
     if (rc) return rc;
-    PMC_CUDA(e, cudaMemsetAsync(e->d_total_q, 0, sizeof(unsigned long long), e->stream));
     TransportParams P = make_params(e, p, plan);
     P.window_el = (G.type == 0 || G.type == 1) && G.kind != PMC_PHOTON ? 1 : 0;
     float t_tr = 0.0f, t_red = 0.0f;
@@ -1510,40 +1523,41 @@ int pmc_run_forward(pmc_engine* e, const pmc_source_desc* src, const pmc_run_par
         rc = launch_fold(e, n_vox, 1, (const double*)e->col_nhist.p, in_wave, p->n_batches, one_wave);
         if (rc) return rc;
         PMC_CUDA(e, cudaEventRecord(e->ev[2], e->stream));
-        PMC_CUDA(e, cudaEventSynchronize(e->ev[2]));
+        if (one_wave) break;  // nothing to wait for before the results
+        Sched s;
+        rc = read_sched(e, &s);
+        if (!rc) rc = check_flags(e, s);
+        if (rc) return rc;
         float a = 0, c = 0;
         cudaEventElapsedTime(&a, e->ev[0], e->ev[1]);
         cudaEventElapsedTime(&c, e->ev[1], e->ev[2]);
         t_tr += a;
         t_red += c;
-        Sched s;
-        rc = read_sched(e, &s);
-        if (rc) return rc;
-        rc = check_flags(e, s);
-        if (rc) return rc;
         for (int k = 0; k < in_wave && e->progress; ++k) e->progress(e->progress_user, per_batch);
     }
-    PMC_CUDA(e, cudaEventRecord(e->ev[0], e->stream));
-    if (!one_wave) rc = launch_finalize(e, n_vox, 1, p->n_batches);
-    if (rc) return rc;
-    PMC_CUDA(e, cudaEventRecord(e->ev[1], e->stream));
+    if (!one_wave) {
+        rc = launch_finalize(e, n_vox, 1, p->n_batches);
+        if (rc) return rc;
+        PMC_CUDA(e, cudaEventRecord(e->ev[3], e->stream));
+    }
     PMC_CUDA(e, cudaMemcpyAsync(dose, e->s1.p, sizeof(double) * n_vox, cudaMemcpyDeviceToHost, e->stream));
-        e->d2h_bytes += (unsigned long long)(sizeof(double) * n_vox);
     PMC_CUDA(e, cudaMemcpyAsync(dose_sigma, e->s2.p, sizeof(double) * n_vox, cudaMemcpyDeviceToHost, e->stream));
-        e->d2h_bytes += (unsigned long long)(sizeof(double) * n_vox);
-    unsigned long long total_q = 0;
-    PMC_CUDA(e, cudaMemcpyAsync(&total_q, e->d_total_q, sizeof total_q, cudaMemcpyDeviceToHost, e->stream));
-        e->d2h_bytes += (unsigned long long)(sizeof total_q);
-    PMC_CUDA(e, cudaStreamSynchronize(e->stream));
+    e->d2h_bytes += 2ull * (unsigned long long)(sizeof(double) * n_vox);
+    Sched s;
+    rc = read_sched(e, &s);
+    if (!rc) rc = check_flags(e, s);
+    if (rc) return rc;
     e->edep_clean = true;  // every batch folded: every quanta entry consumed
     float c = 0;
-    cudaEventElapsedTime(&c, e->ev[0], e->ev[1]);
+    if (one_wave) {
+        cudaEventElapsedTime(&t_tr, e->ev[0], e->ev[1]);
+        cudaEventElapsedTime(&c, e->ev[1], e->ev[2]);
+        for (int k = 0; k < p->n_batches && e->progress; ++k) e->progress(e->progress_user, per_batch);
+    } else {
+        cudaEventElapsedTime(&c, e->ev[2], e->ev[3]);
+    }
     e->counters.transport_ms = t_tr;
     e->counters.reduce_ms = t_red + c;
-    if (books) {
-        std::memset(books, 0, sizeof *books);
-        books->deposited = (int64_t)total_q;
-    }
     return finish_counters(e, books);
 }
 
@@ -1610,7 +1624,6 @@ int pmc_run_dij(pmc_engine* e, const pmc_beamlet_desc* src, const int64_t* count
     }
     rc = reset_counters(e);
     if (rc) return rc;
-    PMC_CUDA(e, cudaMemsetAsync(e->d_total_q, 0, sizeof(unsigned long long), e->stream));
     e->dij_indptr.assign(1, 0);
     e->csc_nnz = 0;
     float t_tr = 0.0f, t_red = 0.0f;
@@ -1705,7 +1718,18 @@ int pmc_run_dij(pmc_engine* e, const pmc_beamlet_desc* src, const int64_t* count
             if (rc) return rc;
             PMC_CUDA(e, cudaEventRecord(bev[2], e->stream));
         }
-        PMC_CUDA(e, cudaEventSynchronize(e->batch_ev[3 * (size_t)n_waves - 1]));
+        // finalize + count + scan, then (after the entry total is known) compact;
+        // device time only, the host read of the total in between excluded.  The
+        // status comes with the total, in the same wait.
+        unsigned long long g_nnz = 0;
+        std::vector<long long> g_counts;
+        PMC_CUDA(e, cudaEventRecord(e->ev[0], e->stream));
+        if (!one_wave) rc = launch_finalize(e, n_vox, gs, p->n_batches);
+        if (rc) return rc;
+        PMC_CUDA(e, cudaEventRecord(e->ev[1], e->stream));
+        rc = fetch_status(e);
+        if (!rc) rc = truncate_count(e, n_vox, gs, p->truncation, &g_nnz, &g_counts);
+        if (rc) return rc;
         for (int v = 0; v < n_waves; ++v) {
             const cudaEvent_t* bev = e->batch_ev.data() + 3 * v;
             float a = 0, c = 0;
@@ -1714,22 +1738,9 @@ int pmc_run_dij(pmc_engine* e, const pmc_beamlet_desc* src, const int64_t* count
             t_tr += a;
             t_red += c;
         }
-        Sched s;
-        rc = read_sched(e, &s);
-        if (rc) return rc;
-        rc = check_flags(e, s);
+        rc = check_flags(e, e->status->sched);
         if (rc) return rc;
         e->edep_clean = true;  // every batch of the group folded: every quanta entry consumed
-        // finalize + count + scan, then (after the entry total is known) compact;
-        // device time only, the host read of the total in between excluded.
-        unsigned long long g_nnz = 0;
-        std::vector<long long> g_counts;
-        PMC_CUDA(e, cudaEventRecord(e->ev[0], e->stream));
-        if (!one_wave) rc = launch_finalize(e, n_vox, gs, p->n_batches);
-        if (rc) return rc;
-        PMC_CUDA(e, cudaEventRecord(e->ev[1], e->stream));
-        rc = truncate_count(e, n_vox, gs, p->truncation, &g_nnz, &g_counts);
-        if (rc) return rc;
         // room for this group's entries; after the first of several groups,
         // for all of them at its density plus a quarter (a few large grows
         // instead of one per group: each grow is an allocation and a copy)
@@ -1760,17 +1771,9 @@ int pmc_run_dij(pmc_engine* e, const pmc_beamlet_desc* src, const int64_t* count
         }
     }
     free_run_allocs(e);
-    unsigned long long total_q = 0;
-    PMC_CUDA(e, cudaMemcpyAsync(&total_q, e->d_total_q, sizeof total_q, cudaMemcpyDeviceToHost, e->stream));
-        e->d2h_bytes += (unsigned long long)(sizeof total_q);
-    PMC_CUDA(e, cudaStreamSynchronize(e->stream));
     e->counters.transport_ms = t_tr;
     e->counters.reduce_ms = t_red;
     *nnz_out = (int64_t)e->csc_nnz;
-    if (books) {
-        std::memset(books, 0, sizeof *books);
-        books->deposited = (int64_t)total_q;
-    }
     return finish_counters(e, books);
 }
 

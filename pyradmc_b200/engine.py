@@ -961,8 +961,8 @@ class B200Engine:
         n_vox = (int(np.prod(scoring.shape)) if scoring is not None
                  else int(np.prod(self.grid.shape)))
         shape = tuple(scoring.shape) if scoring is not None else tuple(self.grid.shape)
-        dose = np.zeros(n_vox, dtype=np.float64)
-        sigma = np.zeros(n_vox, dtype=np.float64)
+        dose = _pinned_array(n_vox, np.float64)  # (written whole by the call)
+        sigma = _pinned_array(n_vox, np.float64)
         books = _lib.Books()
         tick = _lib.PROGRESS_FN(lambda _u, n: emitter.tick(int(n)))
         native = self._native()

@@ -231,32 +231,9 @@ def presolve_head_device(source, *, cross_sections=None, n_histories: int, seed:
     if np.asarray(mu_tables.log_total).shape[0] < len(pairs):
         raise ValueError(f"the mu tables have {np.asarray(mu_tables.log_total).shape[0]} rows, need {len(pairs)}")
 
-    f32 = lambda a: np.ascontiguousarray(a, dtype=np.float32)  # noqa: E731
     n = int(n_histories)
-    energy = f32(columns["energy"])
-    pos = f32(np.stack([columns["x"], columns["y"], columns["z"]], axis=1))
-    dirs = f32(np.stack([columns["ux"], columns["uy"], columns["uz"]], axis=1))
-    weight = f32(columns["weight"])
     fc = 1 if resolved == "first_compton" else 0
     capacity = n * (1 + fc * (1 + 2 * (air is not None)))
-    if return_device_source:  # the compaction writes straight into these device tensors
-        dev = torch.device(device)
-        t_kind = torch.empty(capacity, dtype=torch.int32, device=dev)
-        t_e = torch.empty(capacity, dtype=torch.float32, device=dev)
-        t_p = torch.empty((capacity, 3), dtype=torch.float32, device=dev)
-        t_d = torch.empty((capacity, 3), dtype=torch.float32, device=dev)
-        t_w = torch.empty(capacity, dtype=torch.float32, device=dev)
-        as_ptr = lambda t, ct: C.cast(C.c_void_p(t.data_ptr()), C.POINTER(ct))  # noqa: E731
-        outs = (as_ptr(t_kind, C.c_int32), as_ptr(t_e, C.c_float), as_ptr(t_p, C.c_float),
-                as_ptr(t_d, C.c_float), as_ptr(t_w, C.c_float))
-    else:
-        out_kind = np.empty(capacity, dtype=np.int32)
-        out_e = np.empty(capacity, dtype=np.float32)
-        out_p = np.empty((capacity, 3), dtype=np.float32)
-        out_d = np.empty((capacity, 3), dtype=np.float32)
-        out_w = np.empty(capacity, dtype=np.float32)
-        outs = (_lib.ptr(out_kind, C.c_int32), _lib.ptr(out_e, C.c_float), _lib.ptr(out_p, C.c_float),
-                _lib.ptr(out_d, C.c_float), _lib.ptr(out_w, C.c_float))
     cs = compiled.to_c()
     mu, keep = mu_tables.to_c()
     params = _lib.HeadParams(first_compton=fc, has_air=int(air is not None), air_row=air_row,
@@ -267,28 +244,30 @@ def presolve_head_device(source, *, cross_sections=None, n_histories: int, seed:
                              outputs_on_device=int(bool(return_device_source)))
     count, dropped = C.c_int64(), C.c_double()
     lib = _lib.load()
+    if return_device_source:
+        dps = _presolve_on_device(lib, cs, mu, params, columns, n, capacity, torch.device(device), count, dropped,
+                                  float(source.max_energy))
+        del keep
+        return (dps, float(dropped.value)) if return_dropped else dps
+    f32 = lambda a: np.ascontiguousarray(a, dtype=np.float32)  # noqa: E731
+    energy = f32(columns["energy"])
+    pos = f32(np.stack([columns["x"], columns["y"], columns["z"]], axis=1))
+    dirs = f32(np.stack([columns["ux"], columns["uy"], columns["uz"]], axis=1))
+    weight = f32(columns["weight"])
+    out_kind = np.empty(capacity, dtype=np.int32)
+    out_e = np.empty(capacity, dtype=np.float32)
+    out_p = np.empty((capacity, 3), dtype=np.float32)
+    out_d = np.empty((capacity, 3), dtype=np.float32)
+    out_w = np.empty(capacity, dtype=np.float32)
     with torch.cuda.device(torch.device(device)):
         code = lib.pmc_presolve_head(C.byref(cs), C.byref(mu), C.byref(params), n,
                                      _lib.ptr(energy, C.c_float), _lib.ptr(pos, C.c_float),
                                      _lib.ptr(dirs, C.c_float), _lib.ptr(weight, C.c_float), capacity,
-                                     *outs, C.byref(count), C.byref(dropped))
+                                     _lib.ptr(out_kind, C.c_int32), _lib.ptr(out_e, C.c_float),
+                                     _lib.ptr(out_p, C.c_float), _lib.ptr(out_d, C.c_float),
+                                     _lib.ptr(out_w, C.c_float), C.byref(count), C.byref(dropped))
     del keep
-    if code != _lib.PMC_OK:
-        raise RuntimeError(f"pmc_presolve_head failed ({code})")
-    k = int(count.value)
-    if k == 0:
-        raise ValueError("the pre-solve kept no particles; check the geometry and cutoffs")
-    if return_device_source:
-        # the host path's arithmetic on the device: directions renormalized
-        # and weights scaled per original primary (head.py:296-314) in
-        # float64, then rounded to float32 as the engine's upload rounds them,
-        # so both hand-offs carry the same records bit for bit
-        d64 = t_d[:k].double()
-        n2 = (d64[:, 0] * d64[:, 0] + d64[:, 1] * d64[:, 1]) + d64[:, 2] * d64[:, 2]
-        dps = DevicePhaseSpace(t_kind[:k].clone(), t_e[:k].clone(), t_p[:k].clone(),
-                               (d64 / torch.sqrt(n2).unsqueeze(1)).float(),
-                               (t_w[:k].double() * (k / n)).float(), float(source.max_energy))
-        return (dps, float(dropped.value)) if return_dropped else dps
+    k = _kept(code, count)
     d = out_d[:k].astype(np.float64)
     d /= np.linalg.norm(d, axis=1, keepdims=True)  # float32 round-off
     ps = InMemoryPhaseSpaceSource(
@@ -298,6 +277,49 @@ def presolve_head_device(source, *, cross_sections=None, n_histories: int, seed:
         # normalized per original primary (head.py:296-314)
         weight=out_w[:k].astype(np.float64) * (k / n))
     return (ps, float(dropped.value)) if return_dropped else ps
+
+
+def _kept(code: int, count) -> int:
+    if code != _lib.PMC_OK:
+        raise RuntimeError(f"pmc_presolve_head failed ({code})")
+    if count.value == 0:
+        raise ValueError("the pre-solve kept no particles; check the geometry and cutoffs")
+    return int(count.value)
+
+
+def _presolve_on_device(lib, cs, mu, params, columns, n: int, capacity: int, device, count, dropped,
+                        max_energy: float) -> DevicePhaseSpace:
+    """The pre-solve with its population left in device tensors: the primaries'
+    columns rounded to float32 into page-locked memory (torch's threaded copy) and
+    sent in one transfer, all device memory from torch's allocator, everything on
+    the current stream.  The compaction renormalizes and scales as
+    ``_Population.build`` does, in float64 rounded once to float32 as the engine's
+    upload rounds it, so both hand-offs carry the same records bit for bit."""
+    import torch
+
+    with torch.cuda.device(device):
+        host = torch.empty((8, n), dtype=torch.float32, pin_memory=True)
+        for i, key in enumerate(("energy", "x", "y", "z", "ux", "uy", "uz", "weight")):
+            a = np.asarray(columns[key]).reshape(-1)
+            if a.size < n:
+                raise ValueError(f"the source sampled {a.size} values of {key!r} for {n} primaries")
+            if a.dtype not in (np.float64, np.float32) or not a.flags.writeable:
+                a = a.astype(np.float32)
+            host[i].copy_(torch.from_numpy(a[:n]))
+        empty = lambda *shape, dtype=torch.float32: torch.empty(shape, dtype=dtype, device=device)  # noqa: E731
+        kind, energy, weight = empty(capacity, dtype=torch.int32), empty(capacity), empty(capacity)
+        pos, dirs = empty(capacity, 3), empty(capacity, 3)
+        size = C.c_int64()
+        code = lib.pmc_presolve_workspace(C.byref(cs), C.byref(mu), C.byref(params), n, C.byref(size))
+        if code == _lib.PMC_OK:
+            ws = empty(size.value, dtype=torch.uint8)
+            code = lib.pmc_presolve_head_device(
+                C.byref(cs), C.byref(mu), C.byref(params), n, host.data_ptr(), ws.data_ptr(), size.value, capacity,
+                kind.data_ptr(), energy.data_ptr(), pos.data_ptr(), dirs.data_ptr(), weight.data_ptr(),
+                C.byref(count), C.byref(dropped), torch.cuda.current_stream(device).cuda_stream)
+    k = _kept(code, count)
+    cut = (lambda t: t[:k]) if 2 * k >= capacity else (lambda t: t[:k].clone())  # not half empty
+    return DevicePhaseSpace(cut(kind), cut(energy), cut(pos), cut(dirs), cut(weight), max_energy)
 
 
 def stack_path_lengths(stack, points, directions, from_origin: bool = False) -> np.ndarray:

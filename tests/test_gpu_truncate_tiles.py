@@ -32,8 +32,8 @@ def test_truncation_equals_numpy(gpu, n_vox, truncation, odd):
     keep = []
     for col in mean:
         positive = col[col > 0.0]  # NaN compares false
-        threshold = truncation * (positive.max() if positive.size else 0.0)
         with np.errstate(invalid="ignore"):
+            threshold = truncation * (positive.max() if positive.size else 0.0)
             keep.append(np.flatnonzero((col >= threshold) & (col > 0.0)))
     indptr, idx, dose, sig = denoise_dij.compact(torch.from_numpy(mean).to(gpu), torch.from_numpy(sigma).to(gpu),
                                                  truncation)
