@@ -943,17 +943,12 @@ int dispatch_umma_pipe(const __nv_bfloat16* x, const __nv_bfloat16* w, const flo
 // 1.22 ms whole at one).  Otherwise the
 // weights are streamed with the stages, in channel groups as large as three
 // stages allow (two where three never fit).
-bool ws_plan(const ConvShape& s, WsConv& p, int& smem, int& ctas_per_sm) {
-    if (s.cout % 16 || s.cout < 16 || s.cout > 256) return false;
-    if (!(s.cin == 8 || s.cin % 16 == 0)) return false;
+// at_cg: the channel group to keep, 0 to choose it.
+bool ws_plan_at(const ConvShape& s, int tz, int at_cg, WsConv& p, int& smem, int& ctas_per_sm) {
     const int cpt = s.cin / 8, N = s.cout;
     p = WsConv{};
     p.s = s;
-    // taller tiles fold more of an MMA's outputs together; one slice where the
-    // weights are streamed or an MMA is full already
-    p.tz = s.cin <= 32 && s.cout <= 32 ? 4 : (s.cin <= 48 || s.cout <= 32 ? 2 : 1);
-    while (p.tz > 1 && 2 * p.tz * N > 512) --p.tz;
-    if (p.tz == 3) p.tz = 2;
+    p.tz = tz;
     if (2 * p.tz * N > 512) return false;
     p.box_bytes = (unsigned)((p.tz + 2) * kUHY * kUHX * 16);
     p.plane_bytes = (p.box_bytes + 127u) & ~127u;
@@ -965,7 +960,7 @@ bool ws_plan(const ConvShape& s, WsConv& p, int& smem, int& ctas_per_sm) {
     for (int cg = cpt; cg >= 1; --cg) {
         // even groups only (cg = 1 pairs taps, one K step in 28 on a zero chunk,
         // and measured slower than one block per SM with the whole halo)
-        if (cpt % cg || (cg % 2 && cg != cpt)) continue;
+        if (cpt % cg || (cg % 2 && cg != cpt) || (at_cg && cg != at_cg)) continue;
         const unsigned chunks = w_chunks_of(cg);  // per group
         const unsigned stage = round128((unsigned)cg * p.plane_bytes + kUSlack);
         int n_st = cg == cpt ? 2 : 3;
@@ -986,9 +981,10 @@ bool ws_plan(const ConvShape& s, WsConv& p, int& smem, int& ctas_per_sm) {
         if (need <= pair_smem) break;
     }
     if (p.cg == 0) {  // streamed weights: the largest channel group with 3 stages, else 2
-        for (int want = 3; want >= 2 && p.cg == 0; --want)
-            for (int cg = cpt; cg >= 1; --cg) {
-                if (cpt % cg || (cg > 1 && cg % 2)) continue;
+        // (cg = 1 pairs taps, ten for nine: last)
+        for (int want = 3, least = 2; least >= 1 && p.cg == 0; want == 3 ? --want : (want = 3, --least))
+            for (int cg = cpt; cg >= least; --cg) {
+                if (cpt % cg || (cg > 1 && cg % 2) || (at_cg && cg != at_cg)) continue;
                 const unsigned chunks = w_chunks_of(cg);
                 const unsigned halo = (unsigned)cg * p.plane_bytes + kUSlack;
                 const unsigned stage = round128(halo + chunks * N * 16);
@@ -1032,6 +1028,34 @@ bool ws_plan(const ConvShape& s, WsConv& p, int& smem, int& ctas_per_sm) {
         if (smem > kSmemPerBlockMax) smem = kSmemPerBlockMax;
     }
     ctas_per_sm = per_sm;
+    return true;
+}
+
+// The plan at the tile depth that suits the shape: deep tiles fold more of an MMA's
+// outputs together and read fewer halo slices, and where the weights are streamed
+// they serve more voxels (192 -> 64: 0.87 MB from the L2 per output slice at tz = 1,
+// 0.27 at 4); shallow ones where deep ones would leave SMs without a tile.  The
+// channel groups, which set the order of an output's sum, are the deepest plan's, so
+// that a window's values do not depend on how many windows share the launch.
+bool ws_plan(const ConvShape& s, WsConv& p, int& smem, int& ctas_per_sm) {
+    if (s.cout % 16 || s.cout < 16 || s.cout > 256) return false;
+    if (!(s.cin == 8 || s.cin % 16 == 0)) return false;
+    constexpr int kSms = 148;
+    int tz = s.cin <= 32 && s.cout <= 32 ? 4 : (s.cin <= 48 || s.cout <= 32 ? 2 : 1);
+    while (tz > 1 && !ws_plan_at(s, tz, 0, p, smem, ctas_per_sm)) tz /= 2;
+    if (!ws_plan_at(s, tz, 0, p, smem, ctas_per_sm)) return false;
+    if (p.streamed)  // the depth of the streamed layers
+        for (tz = s.cout <= 64 ? 4 : s.cout <= 128 ? 2 : 1; !ws_plan_at(s, tz, 0, p, smem, ctas_per_sm); tz /= 2)
+            if (tz == 1) return false;
+    const WsConv deep = p;
+    for (; tz > 1 && p.n_tiles < kSms; tz /= 2) {
+        WsConv q{};
+        int q_smem = 0, q_per_sm = 0;
+        if (!ws_plan_at(s, tz / 2, deep.cg, q, q_smem, q_per_sm) || q.streamed != deep.streamed) break;
+        p = q;
+        smem = q_smem;
+        ctas_per_sm = q_per_sm;
+    }
     return true;
 }
 
