@@ -1031,6 +1031,46 @@ bool ws_plan_at(const ConvShape& s, int tz, int at_cg, WsConv& p, int& smem, int
     return true;
 }
 
+constexpr int kPlanSms = 148;
+
+// Turn a tile plan into one of runs along d (conv3d_zs_kernel) where its terms hold:
+// the same channel groups, stages of two halo slices, up to four stages where they fit
+// (two blocks an SM with several groups keep the tiles' count).  Tiles -> runs, 100
+// windows of 64 x 64 x 72 voxels: 48 -> 16 2.45 -> 1.43 ms, 16 -> 16 0.67 -> 0.58; of
+// 32 x 32 x 36: 96 -> 32 1.27 -> 0.59, 32 -> 32 0.29 -> 0.21, 16 -> 32 0.16 -> 0.13.
+bool zs_plan(WsConv& p, int& smem, int& ctas_per_sm) {
+    const ConvShape& s = p.s;
+    const int N = s.cout;
+    if (p.streamed || p.cg < 2 || 3 * N > 256) return false;
+    WsConv q = p;
+    q.tz = kRunSlices;
+    q.box_bytes = (unsigned)(q.tz * kUHY * kUHX * 16);
+    q.plane_bytes = (q.box_bytes + 127u) & ~127u;
+    q.halo_part = (unsigned)q.cg * q.plane_bytes;
+    q.stage_bytes = (q.halo_part + 127u) & ~127u;
+    q.tx_bytes = (unsigned)q.cg * q.box_bytes;
+    const int weights = q.groups * (int)q.w_chunks * N * 16;
+    const int most = kSmemPerSM / ctas_per_sm - kSmemReserved < kSmemPerBlockMax
+                         ? kSmemPerSM / ctas_per_sm - kSmemReserved : kSmemPerBlockMax;
+    q.ring = 512 / ctas_per_sm / N / q.tz;
+    if (q.ring < 3) return false;
+    const int bars = 8 * (2 * kWsMaxStages + 2 * q.ring) + 16 + 2 * N * 4;  // and bias, head weights
+    if (q.groups == 1 || ctas_per_sm == 1)
+        for (q.stages = kWsMaxStages; q.stages > p.stages; --q.stages)
+            if (q.stages * (int)q.stage_bytes + weights + bars <= most) break;
+    const int need = q.stages * (int)q.stage_bytes + weights + bars;
+    if (need > most) return false;
+    // all of the block's share, so that no further block takes tensor memory
+    smem = need > kSmemPerSM / (ctas_per_sm + 1) - kSmemReserved ? need : kSmemPerSM / (ctas_per_sm + 1);
+    q.tmem_cols = 512u / (unsigned)ctas_per_sm;
+    q.line = (s.d + kRunSlices - 1) / kRunSlices * kRunSlices;
+    const long long slices = (long long)s.n * q.tiles_h * q.tiles_w * q.line;
+    if (slices > (1LL << 30)) return false;
+    q.n_tiles = (int)slices;
+    p = q;
+    return true;
+}
+
 // The plan at the tile depth that suits the shape: deep tiles fold more of an MMA's
 // outputs together and read fewer halo slices, and where the weights are streamed
 // they serve more voxels (192 -> 64: 0.87 MB from the L2 per output slice at tz = 1,
@@ -1040,7 +1080,6 @@ bool ws_plan_at(const ConvShape& s, int tz, int at_cg, WsConv& p, int& smem, int
 bool ws_plan(const ConvShape& s, WsConv& p, int& smem, int& ctas_per_sm) {
     if (s.cout % 16 || s.cout < 16 || s.cout > 256) return false;
     if (!(s.cin == 8 || s.cin % 16 == 0)) return false;
-    constexpr int kSms = 148;
     int tz = s.cin <= 32 && s.cout <= 32 ? 4 : (s.cin <= 48 || s.cout <= 32 ? 2 : 1);
     while (tz > 1 && !ws_plan_at(s, tz, 0, p, smem, ctas_per_sm)) tz /= 2;
     if (!ws_plan_at(s, tz, 0, p, smem, ctas_per_sm)) return false;
@@ -1048,7 +1087,8 @@ bool ws_plan(const ConvShape& s, WsConv& p, int& smem, int& ctas_per_sm) {
         for (tz = s.cout <= 64 ? 4 : s.cout <= 128 ? 2 : 1; !ws_plan_at(s, tz, 0, p, smem, ctas_per_sm); tz /= 2)
             if (tz == 1) return false;
     const WsConv deep = p;
-    for (; tz > 1 && p.n_tiles < kSms; tz /= 2) {
+    if (zs_plan(p, smem, ctas_per_sm)) return true;
+    for (; tz > 1 && p.n_tiles < kPlanSms; tz /= 2) {
         WsConv q{};
         int q_smem = 0, q_per_sm = 0;
         if (!ws_plan_at(s, tz / 2, deep.cg, q, q_smem, q_per_sm) || q.streamed != deep.streamed) break;
@@ -1083,8 +1123,8 @@ EncodeTiledFn encode_tiled() {
 // cout).  False when the driver refuses them (the caller then takes another
 // kernel).
 // The halo map alone: the NDHWC bf16 activation x of shape s, box 8 channels
-// x 10 x 18 x (tz + 2) x 1, zero fill outside.
-bool halo_tensor_map(const __nv_bfloat16* x, const ConvShape& s, int tz, CUtensorMap& xm) {
+// x 10 x 18 x `slices` x 1, zero fill outside.
+bool halo_tensor_map(const __nv_bfloat16* x, const ConvShape& s, int slices, CUtensorMap& xm) {
     const EncodeTiledFn enc = encode_tiled();
     if (!enc || reinterpret_cast<uintptr_t>(x) % 16) return false;
     const cuuint64_t e = sizeof(__nv_bfloat16);
@@ -1092,7 +1132,7 @@ bool halo_tensor_map(const __nv_bfloat16* x, const ConvShape& s, int tz, CUtenso
                                 (cuuint64_t)s.n};
     const cuuint64_t xstride[4] = {xdim[0] * e, xdim[0] * xdim[1] * e, xdim[0] * xdim[1] * xdim[2] * e,
                                    xdim[0] * xdim[1] * xdim[2] * xdim[3] * e};
-    const cuuint32_t xbox[5] = {8, (cuuint32_t)kUHX, (cuuint32_t)kUHY, (cuuint32_t)(tz + 2), 1};
+    const cuuint32_t xbox[5] = {8, (cuuint32_t)kUHX, (cuuint32_t)kUHY, (cuuint32_t)slices, 1};
     const cuuint32_t ones[5] = {1, 1, 1, 1, 1};
     return enc(&xm, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, const_cast<__nv_bfloat16*>(x), xdim, xstride, xbox,
                ones, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
@@ -1107,7 +1147,7 @@ bool ws_tensor_maps(const __nv_bfloat16* x, const __nv_bfloat16* w, const WsConv
     const ConvShape& s = p.s;
     const cuuint64_t e = sizeof(__nv_bfloat16);
     const cuuint32_t ones[5] = {1, 1, 1, 1, 1};
-    if (!halo_tensor_map(x, s, p.tz, xm)) return false;
+    if (!halo_tensor_map(x, s, p.line ? p.tz : p.tz + 2, xm)) return false;
     const cuuint64_t wdim[2] = {(cuuint64_t)s.kpad, (cuuint64_t)s.cout};
     const cuuint64_t wstride[1] = {(cuuint64_t)s.kpad * e};
     const cuuint32_t wbox[2] = {8, (cuuint32_t)s.cout};
@@ -1118,16 +1158,31 @@ bool ws_tensor_maps(const __nv_bfloat16* x, const __nv_bfloat16* w, const WsConv
 
 template <int CG>
 int launch_ws(const CUtensorMap& xm, const CUtensorMap& wm, const __nv_bfloat16* w, const float* bias,
-              __nv_bfloat16* y, const WsConv& p, int smem, int per_sm, int relu, cudaStream_t st,
+              __nv_bfloat16* y, WsConv& p, int smem, int per_sm, int relu, cudaStream_t st,
               const WsHead& head) {
     int dev = 0, sms = 0;
     if (cudaGetDevice(&dev) != cudaSuccess ||
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-        cudaFuncSetAttribute(conv3d_ws_kernel<CG>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) !=
-            cudaSuccess)
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
         return -2;
-    const int grid = p.n_tiles < sms * per_sm ? p.n_tiles : sms * per_sm;
-    conv3d_ws_kernel<CG><<<grid, kWsThreads, smem, st>>>(xm, wm, w, bias, y, p, relu, head);
+    const int blocks = sms * per_sm;
+    if constexpr (CG > 1) {
+        if (p.line) {
+            // whole stages, so that an output's place in its stage, and with it the order
+            // of its sum over several channel groups, does not depend on the windows
+            p.share = ((p.n_tiles + blocks - 1) / blocks + kRunSlices - 1) / kRunSlices * kRunSlices;
+            if (cudaFuncSetAttribute(conv3d_zs_kernel<CG>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) !=
+                cudaSuccess)
+                return -2;
+            conv3d_zs_kernel<CG><<<(p.n_tiles + p.share - 1) / p.share, kWsThreads, smem, st>>>(xm, w, bias, y, p,
+                                                                                               relu, head);
+            return launched();
+        }
+    }
+    if (cudaFuncSetAttribute(conv3d_ws_kernel<CG>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) !=
+        cudaSuccess)
+        return -2;
+    conv3d_ws_kernel<CG><<<p.n_tiles < blocks ? p.n_tiles : blocks, kWsThreads, smem, st>>>(xm, wm, w, bias, y, p,
+                                                                                            relu, head);
     return launched();
 }
 
@@ -1214,7 +1269,7 @@ int try_wgrad_umma(const __nv_bfloat16* x, const __nv_bfloat16* g, float* dw, fl
     WgConv p;
     int smem = 0;
     CUtensorMap xm;
-    if (!wg_plan(s, p, smem) || !halo_tensor_map(x, s, p.tz, xm)) return -1;
+    if (!wg_plan(s, p, smem) || !halo_tensor_map(x, s, p.tz + 2, xm)) return -1;
     if (reinterpret_cast<uintptr_t>(g) % 16 || reinterpret_cast<uintptr_t>(dw) % 16) return -1;
     int dev = 0, sms = 0;
     if (cudaGetDevice(&dev) != cudaSuccess ||

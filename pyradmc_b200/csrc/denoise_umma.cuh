@@ -58,19 +58,41 @@ __device__ __forceinline__ uint32_t umma_instr_desc(int n) {
     return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | (8u << 24);
 }
 
-__device__ __forceinline__ void umma_bf16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc,
-                                          uint32_t idesc, uint32_t accumulate) {
+// The index of the calling warp, uniform to the compiler too.
+__device__ __forceinline__ int warp_index() { return __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0); }
+
+// 1 in the one lane of the (whole) calling warp that issues MMAs and commits.
+__device__ __forceinline__ uint32_t elect_lane() {
+    uint32_t lead;
     asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(tmem_d),
-        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate));
+        "{\n\t.reg .pred P;\n\t"
+        "elect.sync _|P, 0xffffffff;\n\t"
+        "selp.b32 %0, 1, 0, P;\n\t}\n"
+        : "=r"(lead));
+    return lead;
 }
 
-__device__ __forceinline__ void umma_commit(uint32_t mbar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                     mbar)
-                 : "memory");
+// D (+)= A B, issued by the lane with lead = 1.  The whole warp runs the issuing loops
+// and only this instruction is predicated: descriptors are operands of the warp, and
+// under a branch taken by one lane each had to be carried over from a lane's
+// registers first (measured 54 -> 18 ns an MMA at N = 96).
+__device__ __forceinline__ void umma_bf16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc,
+                                          uint32_t idesc, uint32_t accumulate, uint32_t lead) {
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t"
+        "setp.ne.b32 q, %5, 0;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(tmem_d),
+        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(lead));
+}
+
+__device__ __forceinline__ void umma_commit(uint32_t mbar, uint32_t lead) {
+    asm volatile(
+        "{\n\t.reg .pred q;\n\t"
+        "setp.ne.b32 q, %1, 0;\n\t"
+        "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}\n" ::"r"(mbar),
+        "r"(lead)
+        : "memory");
 }
 
 __device__ __forceinline__ void mbar_init(uint32_t mbar, uint32_t count) {
@@ -83,22 +105,28 @@ __device__ __forceinline__ unsigned long long global_ns() {
     return t;
 }
 
+// Whether the phase `parity` has completed.  The waits below read the timer only after
+// a first try: reading it takes longer than the rest of a wait that has nothing to wait for.
+__device__ __forceinline__ bool mbar_try(uint32_t mbar, uint32_t parity) {
+    uint32_t done;
+    asm volatile(
+        "{\n\t.reg .pred P1;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 P1, [%1], %2;\n\t"
+        "selp.b32 %0, 1, 0, P1;\n\t}\n"
+        : "=r"(done)
+        : "r"(mbar), "r"(parity)
+        : "memory");
+    return done != 0;
+}
+
 // Poll the mbarrier phase until it completes or kUWaitNs have passed (then
 // false); each poll may suspend the thread for a short while.
 __device__ __forceinline__ bool mbar_wait(uint32_t mbar, uint32_t phase) {
+    if (mbar_try(mbar, phase)) return true;
     const unsigned long long start = global_ns();
-    for (;;) {
-        uint32_t done;
-        asm volatile(
-            "{\n\t.reg .pred P1;\n\t"
-            "mbarrier.try_wait.parity.shared::cta.b64 P1, [%1], %2;\n\t"
-            "selp.b32 %0, 1, 0, P1;\n\t}\n"
-            : "=r"(done)
-            : "r"(mbar), "r"(phase)
-            : "memory");
-        if (done) return true;
+    while (!mbar_try(mbar, phase))
         if (global_ns() - start > kUWaitNs) return false;
-    }
+    return true;
 }
 
 __device__ __forceinline__ void tc_fence_before() {
@@ -152,6 +180,45 @@ __host__ __device__ constexpr int w_chunk_at(int at, int cg) {
 // the zero partner.
 __host__ __device__ constexpr unsigned w_chunks_of(int cg) { return 27u * cg + (cg == 1 ? 3u : 0u); }
 
+// Issues the MMAs of one halo slice for `cnt` neighbouring output slices: A from the
+// slice's rows at descriptor `as`, B from the weight rows of those outputs' dz at
+// descriptor `bs`, accumulators from column d on, cout = N columns each.  fresh: the
+// last of the outputs starts here (its first K step overwrites, the others' adds:
+// the MMA is split there).
+//
+// Every descriptor is the slice's base descriptor plus an offset fixed at compile
+// time, so the issuing thread runs no loads and little arithmetic between MMAs (a
+// thread issuing from a descriptor table in shared memory measured ~50-120 cycles
+// per MMA).  With CG = 1 a K step pairs two taps of the halo slice: the second
+// half's LBO is the distance between their rows and the last tap pairs with zero
+// weights.
+template <int CG>
+__device__ __forceinline__ void umma_issue_slice(uint32_t d, uint64_t as, uint64_t bs, uint64_t plane16, int N,
+                                                 int cnt, bool fresh, uint32_t lead) {
+    const uint64_t n3 = 3u * (uint64_t)N;
+    const uint32_t id = umma_instr_desc(cnt * N);
+    const uint64_t a_first = CG == 1 ? as + ((uint64_t)1 << 16) : as;
+    const uint32_t old = fresh ? (uint32_t)((cnt - 1) * N) : 0u;  // columns of the outputs already begun
+    if (fresh && cnt > 1) umma_bf16(d, a_first, bs, umma_instr_desc((int)old), 1u, lead);
+    umma_bf16(d + old, a_first, bs + old, fresh ? umma_instr_desc(N) : id, fresh ? 0u : 1u,
+              lead);
+    if constexpr (CG == 1) {
+#pragma unroll
+        for (int t = 2; t < 9; t += 2) {
+            const uint64_t lbo16 = t + 1 < 9 ? tap_off16(t + 1) - tap_off16(t) : 1u;
+            umma_bf16(d, as + tap_off16(t) + (lbo16 << 16), bs + (uint64_t)t * n3, id, 1u, lead);
+        }
+    } else {
+#pragma unroll
+        for (int t = 0; t < 9; ++t)
+#pragma unroll
+            for (int q = 0; q < CG; q += 2)
+                if (t > 0 || q > 0)
+                    umma_bf16(d, as + tap_off16(t) + plane16 * (uint64_t)q, bs + (uint64_t)(t * CG + q) * n3, id, 1u,
+                              lead);
+    }
+}
+
 // Issues the MMAs of all 27 taps over CG 8-channel chunks for the tz slices of
 // a tile: A from the halo planes at a_addr (plane_bytes apart), B from the
 // weight chunks at b_addr (w_place), output slice sl in accumulator columns d0 + sl * N.
@@ -162,60 +229,29 @@ __host__ __device__ constexpr unsigned w_chunks_of(int cg) { return 27u * cg + (
 // slice zz - 2 as dz = 2, zz - 1 as dz = 1, zz as dz = 0, side by side in the
 // accumulator and in the weights (N = 3 cout, fewer at the tile's ends): (tz + 2) * 9
 // MMAs per K step instead of tz * 27.  Every output still takes its products in the
-// order dz, (dy, dx), chunk pair.  An output's first K step overwrites, the
-// others' of that MMA add: it is split there.
+// order dz, (dy, dx), chunk pair.
 //
-// Every descriptor is the slice's base descriptor plus an offset fixed at compile
-// time, so the issuing thread runs no loads and little arithmetic between MMAs (a
-// thread issuing from a descriptor table in shared memory measured ~50-120 cycles
-// per MMA).  The slice loop is not unrolled: with the 14 or 27 MMAs of a slice
-// unrolled in full for CG = 1 and 2, an earlier build computed wrong sums (tested
-// against the oracle); nine are exact for every CG.  With CG = 1 a K step pairs two
-// taps of a halo slice: the second half's LBO is the distance between their rows and
-// the last tap pairs with zero weights.  accumulate: whether the first K step adds
-// to the accumulator (a later channel group of the same tile).
+// The slice loop is not unrolled: with the 14 or 27 MMAs of a slice unrolled in full
+// for CG = 1 and 2, an earlier build computed wrong sums (tested against the
+// oracle); nine are exact for every CG.  accumulate: whether the first K step adds to
+// the accumulator (a later channel group of the same tile).
 template <int CG>
 __device__ __forceinline__ void umma_issue_taps(uint32_t d0, uint32_t a_addr, uint32_t plane_bytes,
-                                                uint32_t b_addr, int N, int tz, uint32_t /*idesc*/,
-                                                bool accumulate) {
+                                                uint32_t b_addr, int N, int tz, bool accumulate,
+                                                uint32_t lead) {
     constexpr uint64_t slice16 = (uint64_t)(kUHY * kUHX);
     const uint64_t a0 = umma_smem_desc(a_addr, CG == 1 ? 0u : plane_bytes, kUHX * 16);
     const uint64_t b0 = umma_smem_desc(b_addr, 3u * (uint32_t)N * 16, 128);
-    const uint64_t plane16 = plane_bytes >> 4;
-    const uint64_t n3 = 3u * (uint64_t)N;
     const int fold = min(3, 256 / N);  // outputs of one MMA: N is at most 256
 #pragma unroll 1
     for (int zz = 0; zz < tz + 2; ++zz) {
-        const uint64_t as = a0 + slice16 * (uint64_t)zz;
         const int hi = min(zz, tz - 1);
 #pragma unroll 1
         for (int lo = max(zz - 2, 0); lo <= hi; lo += fold) {
             const int cnt = min(fold, hi - lo + 1);
-            const bool fresh = !accumulate && lo + cnt - 1 == zz;  // its last output starts here
-            const uint32_t d = d0 + (uint32_t)(lo * N);
-            const uint64_t bs = b0 + (uint64_t)((2 - zz + lo) * N);
-            const uint32_t id = umma_instr_desc(cnt * N);
-            if (fresh && cnt > 1) umma_bf16(d, as + (CG == 1 ? (uint64_t)1 << 16 : 0u), bs, umma_instr_desc((cnt - 1) * N), 1u);
-            const uint32_t d_first = fresh ? d + (uint32_t)((cnt - 1) * N) : d;
-            const uint64_t b_first = fresh ? bs + (uint64_t)((cnt - 1) * N) : bs;
-            const uint32_t id_first = fresh ? umma_instr_desc(N) : id;
-            if constexpr (CG == 1) {
-                umma_bf16(d_first, as + ((uint64_t)1 << 16), b_first, id_first, fresh ? 0u : 1u);
-#pragma unroll
-                for (int t = 2; t < 9; t += 2) {
-                    const uint64_t lbo16 = t + 1 < 9 ? tap_off16(t + 1) - tap_off16(t) : 1u;
-                    umma_bf16(d, as + tap_off16(t) + (lbo16 << 16), bs + (uint64_t)t * n3, id, 1u);
-                }
-            } else {
-                umma_bf16(d_first, as, b_first, id_first, fresh ? 0u : 1u);
-#pragma unroll
-                for (int t = 0; t < 9; ++t)
-#pragma unroll
-                    for (int q = 0; q < CG; q += 2)
-                        if (t > 0 || q > 0)
-                            umma_bf16(d, as + tap_off16(t) + plane16 * (uint64_t)q,
-                                      bs + (uint64_t)(t * CG + q) * n3, id, 1u);
-            }
+            umma_issue_slice<CG>(d0 + (uint32_t)(lo * N), a0 + slice16 * (uint64_t)zz,
+                                 b0 + (uint64_t)((2 - zz + lo) * N), plane_bytes >> 4, N, cnt,
+                                 !accumulate && lo + cnt - 1 == zz, lead);
         }
     }
 }
@@ -230,7 +266,7 @@ conv3d_umma_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __r
     const ConvShape& s = u.s;
     const int N = s.cout;
     constexpr int cpt = CPT;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = warp_index(), lane = tid & 31;
     unsigned char* halo = smem;
     unsigned char* wbuf = smem + u.halo_bytes + kUSlack;
     // per-pass descriptor table: A (slice 0) and B descriptor of every K step
@@ -321,10 +357,11 @@ conv3d_umma_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __r
             cp_async_wait<0>();
             fence_async_smem();
             __syncthreads();
-            if (tid == 0 && u.passes == 1) {
+            if (warp == 0 && u.passes == 1) {
+                const uint32_t lead = elect_lane();
                 tc_fence_after();
-                umma_issue_taps<CPT>(tmem, halo_s, u.plane_bytes, w_s, N, u.tz, idesc, false);
-                umma_commit(mbar);
+                umma_issue_taps<CPT>(tmem, halo_s, u.plane_bytes, w_s, N, u.tz, false, lead);
+                umma_commit(mbar, lead);
             } else if (tid == 0) {
                 tc_fence_after();
                 const int n_k = k_end - k_begin;
@@ -334,9 +371,9 @@ conv3d_umma_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __r
                     const uint32_t d_tmem = tmem + (uint32_t)(sl * N);
                     for (int k = 0; k < n_k; ++k)
                         umma_bf16(d_tmem, dtab[2 * k] + slice_inc * (uint64_t)sl, dtab[2 * k + 1],
-                                  idesc, (pass > 0 || k > 0) ? 1u : 0u);
+                                  idesc, (pass > 0 || k > 0) ? 1u : 0u, 1u);
                 }
-                umma_commit(mbar);
+                umma_commit(mbar, 1u);
             }
             const int ok = mbar_wait(mbar, phase) ? 1 : 0;
             phase ^= 1u;
@@ -497,7 +534,7 @@ conv3d_umma_pipe_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16
     extern __shared__ __align__(1024) unsigned char smem[];
     const ConvShape& s = u.s;
     const int N = s.cout;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = warp_index(), lane = tid & 31;
     const unsigned buf_stride = u.halo_bytes + kUSlack;  // halo + its zeroed slack
     unsigned char* halo0 = smem;
     unsigned char* wbuf = smem + 2 * buf_stride;
@@ -521,7 +558,6 @@ conv3d_umma_pipe_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
-    const uint32_t idesc = umma_instr_desc(N);
     const uint32_t acc_cols = (uint32_t)(u.tz * N);
 
     // resident weights and the descriptor table (A relative to buffer 0)
@@ -543,11 +579,12 @@ conv3d_umma_pipe_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16
         fence_async_smem();
         tc_fence_before();
         __syncthreads();
-        if (tid == 0) {
+        if (warp == 0) {
+            const uint32_t lead = elect_lane();
             tc_fence_after();
             umma_issue_taps<CPT>(tmem + (uint32_t)b * acc_cols, halo_s + (uint32_t)b * buf_stride,
-                                 u.plane_bytes, w_s, N, u.tz, idesc, false);
-            umma_commit(mbar);
+                                 u.plane_bytes, w_s, N, u.tz, false, lead);
+            umma_commit(mbar, lead);
         }
         // the next tile's halo into the other buffer (its last reader, the MMAs
         // of the previous tile, completed before the previous wait returned)

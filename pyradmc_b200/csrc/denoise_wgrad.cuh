@@ -202,13 +202,13 @@ conv3d_wgrad_umma_kernel(const __grid_constant__ CUtensorMap xmap,
 #pragma unroll
                         for (int r = 0; r < kUTY / 2; ++r)  // K = 16 voxels: output rows 2r, 2r + 1
                             umma_bf16(d, as + (uint64_t)(2 * r) * a_row, bs + (uint64_t)(2 * r * kUHX), idesc,
-                                      r == 0 ? acc0 : 1u);
+                                      r == 0 ? acc0 : 1u, 1u);
                     }
                 }
-                umma_commit(empty(b));
+                umma_commit(empty(b), 1u);
                 last = st;
             }
-            if (st == n_stages && n_stages > 0) umma_commit(acc_full);
+            if (st == n_stages && n_stages > 0) umma_commit(acc_full, 1u);
             if (last >= 0) mbar_wait(empty(last % S), (uint32_t)((last / S) & 1));
         }
     } else {

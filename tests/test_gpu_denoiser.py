@@ -367,6 +367,41 @@ def test_tensor_memory_convolution_matches_oracle(gpu, shape):
         np.testing.assert_array_equal(outs[4], outs[2])
 
 
+# runs along d: several per block (windows x tiles above two blocks an SM), odd and
+# short depths, one and several channel groups, an accumulator ring of 4 and of 8
+@pytest.mark.parametrize("shape", [(40, 7, 40, 20, 16, 16), (34, 1, 40, 24, 16, 32), (34, 9, 40, 24, 32, 32),
+                                   (20, 13, 33, 17, 32, 64), (24, 11, 40, 24, 48, 16), (20, 6, 40, 24, 96, 32)])
+def test_convolution_along_runs_does_not_depend_on_the_other_windows(gpu, shape):
+    """The warp-specialized kernel over many windows at once against the mma.sync
+    kernel (fp32 sums of the same products: a bf16 rounding step apart) and, bit for
+    bit, against itself over one window alone, whose runs are cut differently."""
+    import torch
+
+    n, d, h, w, cin, cout = shape
+    rng = np.random.default_rng(300 + sum(shape))
+    x = bf16(rng.normal(size=(n, d, h, w, cin)))
+    wt, kpad = _weights(rng, cin, cout)
+    bias = rng.normal(size=cout).astype(np.float32)
+    lib = _lib.load()
+    dx, dw, db = _dev(x, torch.bfloat16), _dev(wt, torch.bfloat16), _dev(bias, torch.float32)
+
+    def conv(part, impl):
+        y = torch.full((*part.shape[:4], cout), float("nan"), dtype=torch.bfloat16, device=gpu)
+        previous = lib.pmd_conv3d_impl(impl)
+        try:
+            assert lib.pmd_conv3d(part.data_ptr(), dw.data_ptr(), db.data_ptr(), y.data_ptr(),
+                                  *part.shape[:4], cin, cout, kpad, 0, None) == 0
+        finally:
+            lib.pmd_conv3d_impl(previous)
+        return y.float().cpu().numpy()
+
+    got, plain = conv(dx, 4), conv(dx, 1)
+    assert lib.pmd_conv3d_failures() == 0
+    np.testing.assert_allclose(got, plain, rtol=2 * BF16_REL, atol=1e-5 * np.abs(plain).max())
+    for k in (0, n // 2, n - 1):
+        np.testing.assert_array_equal(conv(dx[k:k + 1].contiguous(), 4)[0], got[k])
+
+
 def test_tensor_memory_path_rejects_what_it_does_not_cover(gpu):
     lib = _lib.load()
     previous = lib.pmd_conv3d_impl(2)
