@@ -1206,6 +1206,64 @@ int try_ws(const __nv_bfloat16* x, const __nv_bfloat16* w, const float* bias, __
 }
 
 // ---- weight gradient on the tensor cores ---------------------------------------------
+// The plan of conv3d_wgrad_fold_kernel (cout 16 and 32): the tile depth and halo channel
+// group of the least time to the last tile, in waves of tiles x MMAs of a tile x the
+// cycles of one (its operands' reads from shared memory: 2 KB per 64 rows of M and N / 4
+// cycles).  Ties go to the shallower tile.
+bool wg_fold_plan(const ConvShape& s, WgConv& p, int& smem) {
+    if (s.cout != 16 && s.cout != 32) return false;
+    if (s.cin != 8 && (s.cin % 16 || s.cin > 256)) return false;
+    const int cpt = s.cin / 8;
+    p = WgConv{};
+    p.s = s;
+    p.dz_fold = 1;
+    p.dx_fold = s.cin == 8 ? 1 : 0;
+    p.n_units = p.dx_fold ? 3 : 9;
+    p.cols_per_unit = p.dx_fold ? 32u : (unsigned)s.cin;
+    const int fit = 512 / (int)p.cols_per_unit;
+    p.unit_groups = (p.n_units + fit - 1) / fit;
+    p.units = (p.n_units + p.unit_groups - 1) / p.unit_groups;
+    p.tmem_cols = 32;
+    while (p.tmem_cols < (unsigned)p.units * p.cols_per_unit) p.tmem_cols *= 2;
+    p.stages = 2;
+    p.tiles_h = (s.h + kUTY - 1) / kUTY;
+    p.tiles_w = (s.w + kUTX - 1) / kUTX;
+    const long long columns = (long long)s.n * p.tiles_h * p.tiles_w;
+    long long best = 0;
+    for (int tz = 1; tz <= 16 && tz <= s.d; ++tz)
+        for (int ncg = cpt; ncg >= 1; --ncg) {
+            if (cpt % ncg || (ncg % 2 && cpt != 1)) continue;
+            const unsigned box = (unsigned)((tz + 2) * kUHY * kUHX * 16);
+            const unsigned plane = (box + 127u) / 128u * 128u;
+            const unsigned stage = ((unsigned)ncg * plane + 1023u) / 1024u * 1024u;
+            const unsigned dyb = (unsigned)(p.stages * (tz + 2) + 3) * (unsigned)(s.cout / 8) * 2048u;
+            const long long need = (long long)p.stages * stage + dyb + 1024;
+            if (need > kSmemPerBlockMax) continue;
+            const int n_mma = p.dx_fold ? 32 : 8 * ncg, tiles_d = (s.d + tz - 1) / tz;
+            const int per_group = kPlanSms / p.unit_groups;
+            const long long waves = (columns * tiles_d + per_group - 1) / per_group;
+            const long long cost = waves * (cpt / ncg) * (tz + 2) * (s.cout + n_mma / 4);
+            if (columns * tiles_d > (1LL << 30) || (best && cost >= best)) continue;
+            best = cost;
+            p.tz = tz;
+            p.tiles_d = tiles_d;
+            p.n_tiles = (int)(columns * tiles_d);
+            p.ncg = ncg;
+            p.chunk_groups = cpt / ncg;
+            p.n_mma = n_mma;
+            p.b_sbo = p.dx_fold ? 16u : plane;
+            p.plane_bytes = plane;
+            p.box_bytes = box;
+            p.halo_bytes = (unsigned)ncg * plane;
+            p.stage_bytes = stage;
+            p.dy_bytes = dyb;
+            p.tx_bytes = (unsigned)ncg * box;
+            // one block per SM: its accumulators may take all 512 tensor-memory columns
+            smem = (int)need < kSmemPerSM / 2 + 1024 ? kSmemPerSM / 2 + 1024 : (int)need;
+        }
+    return best > 0;
+}
+
 // The plan of conv3d_wgrad_umma_kernel: the largest tile depth (2, else 1) and
 // halo channel group (all chunks, else fewer, an even count) for which two or
 // three stages fit shared memory; groups of accumulator units (taps, or with
@@ -1269,20 +1327,22 @@ int try_wgrad_umma(const __nv_bfloat16* x, const __nv_bfloat16* g, float* dw, fl
     WgConv p;
     int smem = 0;
     CUtensorMap xm;
-    if (!wg_plan(s, p, smem) || !halo_tensor_map(x, s, p.tz + 2, xm)) return -1;
+    if (!(wg_fold_plan(s, p, smem) || wg_plan(s, p, smem)) || !halo_tensor_map(x, s, p.tz + 2, xm)) return -1;
     if (reinterpret_cast<uintptr_t>(g) % 16 || reinterpret_cast<uintptr_t>(dw) % 16) return -1;
     int dev = 0, sms = 0;
     if (cudaGetDevice(&dev) != cudaSuccess ||
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-        cudaFuncSetAttribute(conv3d_wgrad_umma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) !=
-            cudaSuccess) {
+        cudaFuncSetAttribute(p.dz_fold ? conv3d_wgrad_fold_kernel : conv3d_wgrad_umma_kernel,
+                             cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) {
         code = -2;
         return 1;
     }
     int per_group = sms / p.unit_groups;
     if (per_group > p.n_tiles) per_group = p.n_tiles;
     if (per_group < 1) per_group = 1;
-    conv3d_wgrad_umma_kernel<<<per_group * p.unit_groups, kWgThreads, smem, st>>>(xm, g, dw, db, p);
+    const int grid = per_group * p.unit_groups;
+    if (p.dz_fold) conv3d_wgrad_fold_kernel<<<grid, kWgThreads, smem, st>>>(xm, g, dw, db, p);
+    else conv3d_wgrad_umma_kernel<<<grid, kWgThreads, smem, st>>>(xm, g, dw, db, p);
     code = launched();
     return 1;
 }
@@ -1395,7 +1455,7 @@ int pmd_conv3d_wgrad_plan(int n, int d, int h, int wd, int cin, int cout, int* i
     ConvShape s{n, d, h, wd, cin, cout, (27 * cin + 63) / 64 * 64};
     WgConv p;
     int smem = 0;
-    if (!wg_plan(s, p, smem)) return -1;
+    if (!wg_fold_plan(s, p, smem) && !wg_plan(s, p, smem)) return -1;
     const int v[8] = {p.tz, p.ncg, p.chunk_groups, p.units, p.unit_groups, p.stages, (int)p.stage_bytes,
                       (int)p.tmem_cols};
     for (int i = 0; i < 8; ++i) info[i] = v[i];

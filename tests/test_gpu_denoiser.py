@@ -134,6 +134,15 @@ def test_conv3d_weight_gradient_matches_oracle(gpu, shape):
         assert (gw[:, 27 * cin:] == 0).all()
 
 
+# cout 16 and 32, where one product covers the three d taps: one slice, one more and one
+# less than the tiles are deep, several tiles per block, several channel and tap groups
+@pytest.mark.parametrize("shape", [(1, 1, 16, 8, 16, 16), (3, 19, 17, 9, 16, 16), (1, 13, 20, 10, 8, 16),
+                                   (2, 9, 33, 8, 96, 32), (5, 40, 16, 24, 48, 16), (1, 7, 16, 8, 256, 32),
+                                   (9, 5, 72, 40, 32, 32)])
+def test_weight_gradient_folded_over_d_matches_oracle(gpu, shape):
+    test_conv3d_weight_gradient_matches_oracle(gpu, shape)
+
+
 @pytest.mark.parametrize("shape", [(1, 8, 8, 8, 16, 16), (2, 6, 5, 7, 48, 16), (1, 4, 6, 4, 96, 32),
                                    (1, 4, 4, 4, 192, 64), (1, 2, 4, 4, 64, 128),
                                    (1, 4, 4, 4, 128, 64), (1, 4, 4, 4, 32, 16)])
