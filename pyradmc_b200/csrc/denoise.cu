@@ -965,7 +965,7 @@ bool ws_plan_at(const ConvShape& s, int tz, int at_cg, WsConv& p, int& smem, int
         const unsigned stage = round128((unsigned)cg * p.plane_bytes + kUSlack);
         int n_st = cg == cpt ? 2 : 3;
         const long long fixed = (long long)(cpt / cg) * chunks * N * 16 + bars;
-        if (n_st * (long long)stage + fixed > kSmemPerBlockMax) n_st = 2;
+        if (at_cg && n_st * (long long)stage + fixed > kSmemPerBlockMax) n_st = 2;
         const long long need = (long long)n_st * stage + fixed;
         if (need > kSmemPerBlockMax) continue;
         if (p.cg != 0 && need > pair_smem) continue;  // a smaller group only to reach two blocks per SM
@@ -981,9 +981,8 @@ bool ws_plan_at(const ConvShape& s, int tz, int at_cg, WsConv& p, int& smem, int
         if (need <= pair_smem) break;
     }
     if (p.cg == 0) {  // streamed weights: the largest channel group with 3 stages, else 2
-        // (cg = 1 pairs taps, ten for nine: last)
-        for (int want = 3, least = 2; least >= 1 && p.cg == 0; want == 3 ? --want : (want = 3, --least))
-            for (int cg = cpt; cg >= least; --cg) {
+        for (int want = 3; want >= 2 && p.cg == 0; --want)
+            for (int cg = cpt; cg >= 1; --cg) {
                 if (cpt % cg || (cg > 1 && cg % 2) || (at_cg && cg != at_cg)) continue;
                 const unsigned chunks = w_chunks_of(cg);
                 const unsigned halo = (unsigned)cg * p.plane_bytes + kUSlack;
@@ -1037,7 +1036,7 @@ constexpr int kPlanSms = 148;
 // the same channel groups, stages of two halo slices, up to four stages where they fit
 // (two blocks an SM with several groups keep the tiles' count).  Tiles -> runs, 100
 // windows of 64 x 64 x 72 voxels: 48 -> 16 2.45 -> 1.43 ms, 16 -> 16 0.67 -> 0.58; of
-// 32 x 32 x 36: 96 -> 32 1.27 -> 0.59, 32 -> 32 0.29 -> 0.21, 16 -> 32 0.16 -> 0.13.
+// 32 x 32 x 36: 96 -> 32 1.27 -> 0.92, 32 -> 32 0.29 -> 0.21, 16 -> 32 0.16 -> 0.14.
 bool zs_plan(WsConv& p, int& smem, int& ctas_per_sm) {
     const ConvShape& s = p.s;
     const int N = s.cout;
@@ -1052,8 +1051,9 @@ bool zs_plan(WsConv& p, int& smem, int& ctas_per_sm) {
     const int weights = q.groups * (int)q.w_chunks * N * 16;
     const int most = kSmemPerSM / ctas_per_sm - kSmemReserved < kSmemPerBlockMax
                          ? kSmemPerSM / ctas_per_sm - kSmemReserved : kSmemPerBlockMax;
-    q.ring = 512 / ctas_per_sm / N / q.tz;
-    if (q.ring < 3) return false;
+    q.ring = 1;
+    while (2 * q.ring <= 512 / ctas_per_sm / N / q.tz) q.ring *= 2;
+    if (q.ring < 4) return false;
     const int bars = 8 * (2 * kWsMaxStages + 2 * q.ring) + 16 + 2 * N * 4;  // and bias, head weights
     if (q.groups == 1 || ctas_per_sm == 1)
         for (q.stages = kWsMaxStages; q.stages > p.stages; --q.stages)
@@ -1064,6 +1064,11 @@ bool zs_plan(WsConv& p, int& smem, int& ctas_per_sm) {
     smem = need > kSmemPerSM / (ctas_per_sm + 1) - kSmemReserved ? need : kSmemPerSM / (ctas_per_sm + 1);
     q.tmem_cols = 512u / (unsigned)ctas_per_sm;
     q.line = (s.d + kRunSlices - 1) / kRunSlices * kRunSlices;
+    // a group lags two batches behind the one before, and one more is being stored; else
+    // runs of ring batches, the first of which has no output, the tile's in equal parts
+    const int most_run = kRunSlices * (q.ring - 1), runs = (q.line + most_run - 1) / most_run;
+    q.run = q.ring >= 2 * q.groups + 1 ? q.line
+                                       : ((q.line + runs - 1) / runs + kRunSlices - 1) / kRunSlices * kRunSlices;
     const long long slices = (long long)s.n * q.tiles_h * q.tiles_w * q.line;
     if (slices > (1LL << 30)) return false;
     q.n_tiles = (int)slices;
@@ -1080,12 +1085,22 @@ bool zs_plan(WsConv& p, int& smem, int& ctas_per_sm) {
 bool ws_plan(const ConvShape& s, WsConv& p, int& smem, int& ctas_per_sm) {
     if (s.cout % 16 || s.cout < 16 || s.cout > 256) return false;
     if (!(s.cin == 8 || s.cin % 16 == 0)) return false;
-    int tz = s.cin <= 32 && s.cout <= 32 ? 4 : (s.cin <= 48 || s.cout <= 32 ? 2 : 1);
-    while (tz > 1 && !ws_plan_at(s, tz, 0, p, smem, ctas_per_sm)) tz /= 2;
+    // the channel groups, and with them the order of a sum, are those of shallow tiles
+    int tz = s.cin <= 16 && s.cout <= 16 ? 4 : (s.cin <= 48 ? 2 : 1);
+    while (tz > 1 && 2 * tz * s.cout > 512) --tz;
     if (!ws_plan_at(s, tz, 0, p, smem, ctas_per_sm)) return false;
-    if (p.streamed)  // the depth of the streamed layers
-        for (tz = s.cout <= 64 ? 4 : s.cout <= 128 ? 2 : 1; !ws_plan_at(s, tz, 0, p, smem, ctas_per_sm); tz /= 2)
-            if (tz == 1) return false;
+    // the depth at which they run
+    int deep_tz = p.streamed ? (s.cout <= 64 ? 4 : s.cout <= 128 ? 2 : 1)
+                             : s.cin <= 32 && s.cout <= 32 ? 4 : (s.cin <= 48 || s.cout <= 32 ? 2 : 1);
+    for (; deep_tz > tz; deep_tz /= 2) {
+        WsConv q{};
+        int q_smem = 0, q_per_sm = 0;
+        if (!ws_plan_at(s, deep_tz, p.cg, q, q_smem, q_per_sm) || q.streamed != p.streamed) continue;
+        p = q;
+        smem = q_smem;
+        ctas_per_sm = q_per_sm;
+        tz = deep_tz;
+    }
     const WsConv deep = p;
     if (zs_plan(p, smem, ctas_per_sm)) return true;
     for (; tz > 1 && p.n_tiles < kPlanSms; tz /= 2) {
@@ -1167,9 +1182,7 @@ int launch_ws(const CUtensorMap& xm, const CUtensorMap& wm, const __nv_bfloat16*
     const int blocks = sms * per_sm;
     if constexpr (CG > 1) {
         if (p.line) {
-            // whole stages, so that an output's place in its stage, and with it the order
-            // of its sum over several channel groups, does not depend on the windows
-            p.share = ((p.n_tiles + blocks - 1) / blocks + kRunSlices - 1) / kRunSlices * kRunSlices;
+            p.share = ((p.n_tiles + blocks - 1) / blocks + kRunSlices - 1) / kRunSlices * kRunSlices;  // whole batches
             if (cudaFuncSetAttribute(conv3d_zs_kernel<CG>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) !=
                 cudaSuccess)
                 return -2;

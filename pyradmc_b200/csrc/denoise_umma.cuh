@@ -166,19 +166,17 @@ __host__ __device__ constexpr uint32_t tap_off16(int t) {
 // Where weight chunk (tap, q) of a group of cg 8-channel chunks stands in shared
 // memory, in chunks of [cout][8]: for each (dy, dx, q) the three dz of a tap side by
 // side, the farthest first, so that the rows of dz = 2, 1, 0 are one B operand of
-// 3 cout rows.
+// 3 cout rows; for cg = 1, whose K steps pair taps, in the taps' order.
 __host__ __device__ constexpr int w_place(int tap, int q, int cg) {
-    return ((tap % 9) * cg + q) * 3 + 2 - tap / 9;
+    return cg == 1 ? tap : ((tap % 9) * cg + q) * 3 + 2 - tap / 9;
 }
-// The chunk that stands at place `at`, as tap * cg + q; 27 * cg and up: the zero
-// partner of the last tap (cg = 1).
+// The chunk that stands at place `at`, as tap * cg + q; 27 (cg = 1): the zero partner of
+// the last tap.
 __host__ __device__ constexpr int w_chunk_at(int at, int cg) {
-    const int t = at / 3;
-    return t / cg < 9 ? ((2 - at % 3) * 9 + t / cg) * cg + t % cg : 27 * cg;
+    return cg == 1 ? at : ((2 - at % 3) * 9 + at / 3 / cg) * cg + at / 3 % cg;
 }
-// Weight chunks of a group: 27 per 8-channel chunk, and for cg = 1 the three of
-// the zero partner.
-__host__ __device__ constexpr unsigned w_chunks_of(int cg) { return 27u * cg + (cg == 1 ? 3u : 0u); }
+// Weight chunks of a group: 27 per 8-channel chunk, and for cg = 1 the zero partner.
+__host__ __device__ constexpr unsigned w_chunks_of(int cg) { return 27u * cg + (cg == 1 ? 1u : 0u); }
 
 // Issues the MMAs of one halo slice for `cnt` neighbouring output slices: A from the
 // slice's rows at descriptor `as`, B from the weight rows of those outputs' dz at
@@ -189,34 +187,23 @@ __host__ __device__ constexpr unsigned w_chunks_of(int cg) { return 27u * cg + (
 // Every descriptor is the slice's base descriptor plus an offset fixed at compile
 // time, so the issuing thread runs no loads and little arithmetic between MMAs (a
 // thread issuing from a descriptor table in shared memory measured ~50-120 cycles
-// per MMA).  With CG = 1 a K step pairs two taps of the halo slice: the second
-// half's LBO is the distance between their rows and the last tap pairs with zero
-// weights.
+// per MMA).
 template <int CG>
 __device__ __forceinline__ void umma_issue_slice(uint32_t d, uint64_t as, uint64_t bs, uint64_t plane16, int N,
                                                  int cnt, bool fresh, uint32_t lead) {
     const uint64_t n3 = 3u * (uint64_t)N;
     const uint32_t id = umma_instr_desc(cnt * N);
-    const uint64_t a_first = CG == 1 ? as + ((uint64_t)1 << 16) : as;
     const uint32_t old = fresh ? (uint32_t)((cnt - 1) * N) : 0u;  // columns of the outputs already begun
-    if (fresh && cnt > 1) umma_bf16(d, a_first, bs, umma_instr_desc((int)old), 1u, lead);
-    umma_bf16(d + old, a_first, bs + old, fresh ? umma_instr_desc(N) : id, fresh ? 0u : 1u,
+    if (fresh && cnt > 1) umma_bf16(d, as, bs, umma_instr_desc((int)old), 1u, lead);
+    umma_bf16(d + old, as, bs + old, fresh ? umma_instr_desc(N) : id, fresh ? 0u : 1u,
               lead);
-    if constexpr (CG == 1) {
 #pragma unroll
-        for (int t = 2; t < 9; t += 2) {
-            const uint64_t lbo16 = t + 1 < 9 ? tap_off16(t + 1) - tap_off16(t) : 1u;
-            umma_bf16(d, as + tap_off16(t) + (lbo16 << 16), bs + (uint64_t)t * n3, id, 1u, lead);
-        }
-    } else {
+    for (int t = 0; t < 9; ++t)
 #pragma unroll
-        for (int t = 0; t < 9; ++t)
-#pragma unroll
-            for (int q = 0; q < CG; q += 2)
-                if (t > 0 || q > 0)
-                    umma_bf16(d, as + tap_off16(t) + plane16 * (uint64_t)q, bs + (uint64_t)(t * CG + q) * n3, id, 1u,
-                              lead);
-    }
+        for (int q = 0; q < CG; q += 2)
+            if (t > 0 || q > 0)
+                umma_bf16(d, as + tap_off16(t) + plane16 * (uint64_t)q, bs + (uint64_t)(t * CG + q) * n3, id, 1u,
+                          lead);
 }
 
 // Issues the MMAs of all 27 taps over CG 8-channel chunks for the tz slices of
@@ -231,6 +218,11 @@ __device__ __forceinline__ void umma_issue_slice(uint32_t d, uint64_t as, uint64
 // MMAs per K step instead of tz * 27.  Every output still takes its products in the
 // order dz, (dy, dx), chunk pair.
 //
+// With CG = 1 a K step pairs two taps: the second half's LBO is the distance between
+// their rows, and the last tap pairs with zero weights.  Those pairs run across dz, so
+// each output slice has its 14 MMAs to itself (pairs within a slice would be 15, and
+// another order of the sum).
+//
 // The slice loop is not unrolled: with the 14 or 27 MMAs of a slice unrolled in full
 // for CG = 1 and 2, an earlier build computed wrong sums (tested against the
 // oracle); nine are exact for every CG.  accumulate: whether the first K step adds to
@@ -241,6 +233,27 @@ __device__ __forceinline__ void umma_issue_taps(uint32_t d0, uint32_t a_addr, ui
                                                 uint32_t lead) {
     constexpr uint64_t slice16 = (uint64_t)(kUHY * kUHX);
     const uint64_t a0 = umma_smem_desc(a_addr, CG == 1 ? 0u : plane_bytes, kUHX * 16);
+    if constexpr (CG == 1) {
+        const uint64_t b1 = umma_smem_desc(b_addr, (uint32_t)N * 16, 128);
+        const uint32_t id = umma_instr_desc(N);
+#pragma unroll 1
+        for (int sl = 0; sl < tz; ++sl) {
+            const uint64_t as = a0 + slice16 * (uint64_t)sl;
+            // two loops of seven, so that every offset is fixed at compile time
+#pragma unroll
+            for (int tap = 0; tap < 14; tap += 2)
+                umma_bf16(d0 + (uint32_t)(sl * N),
+                          as + tap_off16(tap) + ((uint64_t)(tap_off16(tap + 1) - tap_off16(tap)) << 16),
+                          b1 + (uint64_t)(tap * N), id, (accumulate || tap > 0) ? 1u : 0u, lead);
+#pragma unroll
+            for (int tap = 14; tap < 27; tap += 2)
+                umma_bf16(d0 + (uint32_t)(sl * N),
+                          as + tap_off16(tap) +
+                              ((uint64_t)(tap < 26 ? tap_off16(tap + 1) - tap_off16(tap) : 1u) << 16),
+                          b1 + (uint64_t)(tap * N), id, 1u, lead);
+        }
+        return;
+    }
     const uint64_t b0 = umma_smem_desc(b_addr, 3u * (uint32_t)N * 16, 128);
     const int fold = min(3, 256 / N);  // outputs of one MMA: N is at most 256
 #pragma unroll 1

@@ -58,7 +58,8 @@ struct WsConv {
     // one (h, w) tile after another
     int line;                // slices of a tile, d rounded up to even; 0: tiles
     int share;               // slices of a block, even
-    int ring;                // accumulator batches (of kRunSlices) in tensor memory
+    int run;                 // most slices of a run, even; line unless the groups take whole runs
+    int ring;                // a power of two: accumulator batches (of kRunSlices) in tensor memory
 };
 
 // An optional 1x1x1 head fused into the epilogue: out[m] = b + base[m] +
@@ -244,7 +245,7 @@ conv3d_ws_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant
             if (byte >= (unsigned)cg * p.plane_bytes || byte % p.plane_bytes >= p.box_bytes) st[i] = 0u;
         }
         if (p.streamed && cg == 1)
-            for (int i = tid; i < 3 * N * 4; i += blockDim.x) st[(p.halo_part + 27u * N * 16u) / 4 + i] = 0u;
+            for (int i = tid; i < N * 4; i += blockDim.x) st[(p.halo_part + 27u * N * 16u) / 4 + i] = 0u;
     }
     if (!p.streamed) ws_stage_weights<CG>(wres, wt, p, tid);
     if (tid == 0) {
@@ -368,7 +369,11 @@ conv3d_ws_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant
 // twice, and the copy engine, which moves these 16-byte rows, was as busy as the
 // tensor cores), and halo slice i always adds to outputs i - 2, i - 1 and i of the run:
 // N = 3 cout for all but the run's first and last slices.  Chunk c, halo slices
-// [c T, c T + T), completes the batch of outputs [c T - 2, c T + T - 2).  The
+// [c T, c T + T), completes the batch of outputs [c T - 2, c T + T - 2).  Channel group
+// g follows two chunks behind group g - 1: an output has all its slices of one group
+// before the first of the next, the order of the tiles.  Where the ring cannot hold so
+// many batches (96 -> 32 has six groups) a group takes the whole run before the next
+// one starts, and a run is as long as the ring.  The
 // accumulators of `ring` batches lie one after another in tensor memory, used in
 // turn across runs; an MMA that reaches past the last one is split there.  A block takes
 // an equal share of all slices, whatever tile they lie in.  With its operands uniform
@@ -431,7 +436,7 @@ conv3d_zs_kernel(const __grid_constant__ CUtensorMap xmap, const __nv_bfloat16* 
     auto run_at = [&](int at, int& nb, int& z0, int& len, int& y0, int& x0) {
         int t = at / p.line;
         z0 = at % p.line;
-        const int next = min(at1, at - z0 + p.line);
+        const int next = min(min(at1, at - z0 + p.line), at + p.run);
         len = min(next - at, s.d - z0);
         x0 = t % p.tiles_w * kUTX;
         t /= p.tiles_w;
@@ -440,6 +445,8 @@ conv3d_zs_kernel(const __grid_constant__ CUtensorMap xmap, const __nv_bfloat16* 
         return next;
     };
     auto chunks_of = [&](int len) { return (len + 2 + T - 1) / T; };
+    // chunks by which a channel group follows the one before
+    auto lag_of = [&](int n_chunks) { return p.run < p.line ? n_chunks : 2; };
 
     if (warp == 0) {
         // ---- producer ----
@@ -450,8 +457,11 @@ conv3d_zs_kernel(const __grid_constant__ CUtensorMap xmap, const __nv_bfloat16* 
             for (int at = at0; at < at1 && !stop;) {
                 int nb, z0, len, y0, x0;
                 at = run_at(at, nb, z0, len, y0, x0);
-                for (int c = 0; c < chunks_of(len) && !stop; ++c)
+                const int n_chunks = chunks_of(len), lag = lag_of(n_chunks);
+                for (int step = 0; step < n_chunks + lag * (p.groups - 1) && !stop; ++step)
                     for (int g = 0; g < p.groups; ++g) {
+                        const int c = step - lag * g;
+                        if (c < 0 || c >= n_chunks) continue;
                         if (!ws_wait(empty(b), free_phase, failed)) {
                             stop = true;
                             break;
@@ -479,18 +489,18 @@ conv3d_zs_kernel(const __grid_constant__ CUtensorMap xmap, const __nv_bfloat16* 
         const int R = RB * T;
         int b = 0, last = -1;                // the next stage's buffer; the last one committed
         uint32_t phase = 0u, last_phase = 0u;
-        int batch = 0;                       // ring place of the batch that this chunk completes
+        int batch = 0;                       // batches of the runs before
         int next = 0;                        // and of the next one to acquire
         uint32_t next_phase = 1u;            // the first round through the ring waits for nothing
         bool stop = false;
         for (int at = at0; at < at1 && !stop;) {
             int nb, z0, len, y0, x0;
             at = run_at(at, nb, z0, len, y0, x0);
-            const int n_chunks = chunks_of(len);
+            const int n_chunks = chunks_of(len), lag = lag_of(n_chunks);
             int owned = 0;  // batches of this run free to write
-            for (int c = 0; c < n_chunks && !stop; ++c) {
-                // the batch this chunk completes and the one it begins
-                for (; owned < min(c + 2, n_chunks) && !stop; ++owned) {
+            for (int step = 0; step < n_chunks + lag * (p.groups - 1) && !stop; ++step) {
+                // the batch that group 0 goes on with and the one it begins
+                for (; owned < min(step + 2, n_chunks) && !stop; ++owned) {
                     stop = !ws_wait_warp(acc_free(next), next_phase, failed);
                     if (++next == RB) {
                         next = 0;
@@ -500,13 +510,15 @@ conv3d_zs_kernel(const __grid_constant__ CUtensorMap xmap, const __nv_bfloat16* 
                 if (stop) break;
                 tc_fence_after();
                 for (int g = 0; g < p.groups; ++g) {
+                    const int c = step - lag * g;
+                    if (c < 0 || c >= n_chunks) continue;
                     if (!ws_wait_warp(full(b), phase, failed)) {
                         stop = true;
                         break;
                     }
                     tc_fence_after();
-                    const uint64_t a0 =
-                        umma_smem_desc(st_s + (uint32_t)b * p.stage_bytes, p.plane_bytes, kUHX * 16);
+                    const int place = (batch + c) & (RB - 1);  // of batch c
+                    const uint64_t a0 = umma_smem_desc(st_s + (uint32_t)b * p.stage_bytes, p.plane_bytes, kUHX * 16);
                     const uint64_t b0 =
                         umma_smem_desc(w_s + (uint32_t)((size_t)g * group_bytes), 3u * (uint32_t)N * 16, 128);
 #pragma unroll 1
@@ -515,7 +527,7 @@ conv3d_zs_kernel(const __grid_constant__ CUtensorMap xmap, const __nv_bfloat16* 
                         const int hi = min(i, len - 1);
 #pragma unroll 1
                         for (int lo = max(i - 2, 0); lo <= hi;) {
-                            int slot = batch * T + lo + 2 - c * T;  // output lo's ring slot
+                            int slot = place * T + lo + 2 - c * T;  // output lo's ring slot
                             if (slot >= R) slot -= R;
                             const int cnt = min(hi - lo + 1, R - slot);
                             umma_issue_slice<CG>(tmem + (uint32_t)(slot * N), a0 + slice16 * (uint64_t)k,
@@ -531,10 +543,10 @@ conv3d_zs_kernel(const __grid_constant__ CUtensorMap xmap, const __nv_bfloat16* 
                         b = 0;
                         phase ^= 1u;
                     }
+                    if (g == p.groups - 1) umma_commit(acc_full(place), lead);
                 }
-                if (!stop) umma_commit(acc_full(batch), lead);
-                if (++batch == RB) batch = 0;
             }
+            batch += n_chunks;
         }
         // MMAs still in flight finish before the tensor memory is freed
         if (last >= 0) mbar_wait(empty(last), last_phase);
