@@ -48,6 +48,13 @@ int pmd_conv3d_head(const void* x, const void* w, const float* bias, const float
                     const float* head_b, const float* base, float* out, int n, int d, int h,
                     int w_, int cin, int cout, int kpad, int relu, void* stream);
 
+/* pmd_conv3d over the channels of two tensors one after the other, up [n][d][h][w][c_up]
+ * and skip [n][d][h][w][c_skip], which need not be copied into one: the same values
+ * as pmd_upcat then pmd_conv3d.  -1 (nothing launched) where the
+ * warp-specialized kernel does not cover the shape or another kernel is selected. */
+int pmd_conv3d_skip(const void* up, const void* skip, const void* w, const float* bias, void* y, int n, int d,
+                    int h, int w_, int c_up, int c_skip, int cout, int kpad, int relu, void* stream);
+
 /* Selects the convolution kernels of pmd_conv3d: 0 (default) the warp-specialized
  * kernel below wherever it applies except cin = 8, then the single-buffered
  * tensor-memory kernel (tcgen05.mma, accumulators in TMEM; cout a multiple of 16 up to 192,
@@ -117,6 +124,9 @@ int pmd_avgpool_grad(const void* gy, void* gx, int n, int d, int h, int w, int c
  * d, h, w even; fewer than 2^31 elements. */
 int pmd_upcat(const void* up, const void* skip, void* out, int n, int d, int h, int w, int c_up,
               int c_skip, void* stream);
+/* The upsampled part of pmd_upcat alone: out [n][d][h][w][c] (d, h, w even) from up
+ * [n][d / 2][h / 2][w / 2][c]. */
+int pmd_upsample(const void* up, void* out, int n, int d, int h, int w, int c, void* stream);
 int pmd_upcat_grad(const void* gout, void* gup, void* gskip, int n, int d, int h, int w, int c_up,
                    int c_skip, int accumulate, void* stream);
 

@@ -360,6 +360,8 @@ SIGNATURES.update({
     "pmd_avgpool": (_i, [_v, _v, _i, _i, _i, _i, _i, _v]),
     "pmd_avgpool_grad": (_i, [_v, _v, _i, _i, _i, _i, _i, _i, _v]),
     "pmd_upcat": (_i, [_v, _v, _v, _i, _i, _i, _i, _i, _i, _v]),
+    "pmd_conv3d_skip": (_i, [_v, _v, _v, _v, _v, _i, _i, _i, _i, _i, _i, _i, _i, _i, _v]),
+    "pmd_upsample": (_i, [_v, _v, _i, _i, _i, _i, _i, _v]),
     "pmd_upcat_grad": (_i, [_v, _v, _v, _i, _i, _i, _i, _i, _i, _i, _v]),
     "pmd_head": (_i, [_v, _v, _v, _v, _v, _l, _i, _v]),
     "pmd_head_grad": (_i, [_v, _v, _v, _v, _v, _v, _l, _i, _v]),

@@ -435,6 +435,27 @@ __global__ void upcat_kernel(const uint4* up, const uint4* skip, uint4* out, int
     }
 }
 
+// Nearest 2x upsampling alone: a thread reads one vector and writes its 8 children, bound by
+// those writes (a thread per child, with its own chain of divisions, took 1.5 times the
+// time of its bytes).
+__global__ void upsample_kernel(const uint4* up, uint4* out, int n, int d, int h, int w, int c8) {
+    const int d2 = d / 2, h2 = h / 2, w2 = w / 2;
+    const int total = n * d2 * h2 * w2 * c8;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
+        const uint4 v = __ldg(up + i);
+        int t = i;
+        const int cc = t % c8; t /= c8;
+        const int xx = t % w2; t /= w2;
+        const int yy = t % h2; t /= h2;
+        const int zz = t % d2;
+        const int nn = t / d2;
+        uint4* o = out + (size_t)(((nn * d + 2 * zz) * h + 2 * yy) * w + 2 * xx) * c8 + cc;
+#pragma unroll
+        for (int k = 0; k < 8; ++k)
+            o[(size_t)(((k >> 2) * h + ((k >> 1) & 1)) * w + (k & 1)) * c8] = v;
+    }
+}
+
 // Gradient of upcat: the up part sums its 8 children; the skip part is copied
 // (added onto an existing skip gradient when `accumulate`).
 __global__ void upcat_grad_kernel(const uint4* gout, uint4* gup, uint4* gskip, int n, int d, int h,
@@ -1154,15 +1175,21 @@ bool halo_tensor_map(const __nv_bfloat16* x, const ConvShape& s, int slices, CUt
                CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-bool ws_tensor_maps(const __nv_bfloat16* x, const __nv_bfloat16* w, const WsConv& p, CUtensorMap& xm,
-                    CUtensorMap& wm) {
+bool ws_tensor_maps(const __nv_bfloat16* x, const __nv_bfloat16* skip, const __nv_bfloat16* w, const WsConv& p,
+                    CUtensorMap& xm, CUtensorMap& sm, CUtensorMap& wm) {
     const EncodeTiledFn enc = encode_tiled();
     if (!enc) return false;
     if (reinterpret_cast<uintptr_t>(x) % 16 || reinterpret_cast<uintptr_t>(w) % 16) return false;
     const ConvShape& s = p.s;
     const cuuint64_t e = sizeof(__nv_bfloat16);
     const cuuint32_t ones[5] = {1, 1, 1, 1, 1};
-    if (!halo_tensor_map(x, s, p.line ? p.tz : p.tz + 2, xm)) return false;
+    const int slices = p.line ? p.tz : p.tz + 2;
+    ConvShape first = s, second = s;
+    first.cin = p.split * 8;
+    second.cin = s.cin - first.cin;
+    if (!halo_tensor_map(x, first, slices, xm)) return false;
+    if (second.cin == 0) sm = xm;
+    else if (!halo_tensor_map(skip, second, slices, sm)) return false;
     const cuuint64_t wdim[2] = {(cuuint64_t)s.kpad, (cuuint64_t)s.cout};
     const cuuint64_t wstride[1] = {(cuuint64_t)s.kpad * e};
     const cuuint32_t wbox[2] = {8, (cuuint32_t)s.cout};
@@ -1172,7 +1199,7 @@ bool ws_tensor_maps(const __nv_bfloat16* x, const __nv_bfloat16* w, const WsConv
 }
 
 template <int CG>
-int launch_ws(const CUtensorMap& xm, const CUtensorMap& wm, const __nv_bfloat16* w, const float* bias,
+int launch_ws(const CUtensorMap& xm, const CUtensorMap& sm, const CUtensorMap& wm, const __nv_bfloat16* w, const float* bias,
               __nv_bfloat16* y, WsConv& p, int smem, int per_sm, int relu, cudaStream_t st,
               const WsHead& head) {
     int dev = 0, sms = 0;
@@ -1186,7 +1213,7 @@ int launch_ws(const CUtensorMap& xm, const CUtensorMap& wm, const __nv_bfloat16*
             if (cudaFuncSetAttribute(conv3d_zs_kernel<CG>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) !=
                 cudaSuccess)
                 return -2;
-            conv3d_zs_kernel<CG><<<(p.n_tiles + p.share - 1) / p.share, kWsThreads, smem, st>>>(xm, w, bias, y, p,
+            conv3d_zs_kernel<CG><<<(p.n_tiles + p.share - 1) / p.share, kWsThreads, smem, st>>>(xm, sm, w, bias, y, p,
                                                                                                relu, head);
             return launched();
         }
@@ -1194,7 +1221,7 @@ int launch_ws(const CUtensorMap& xm, const CUtensorMap& wm, const __nv_bfloat16*
     if (cudaFuncSetAttribute(conv3d_ws_kernel<CG>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) !=
         cudaSuccess)
         return -2;
-    conv3d_ws_kernel<CG><<<p.n_tiles < blocks ? p.n_tiles : blocks, kWsThreads, smem, st>>>(xm, wm, w, bias, y, p,
+    conv3d_ws_kernel<CG><<<p.n_tiles < blocks ? p.n_tiles : blocks, kWsThreads, smem, st>>>(xm, sm, wm, w, bias, y, p,
                                                                                             relu, head);
     return launched();
 }
@@ -1202,18 +1229,21 @@ int launch_ws(const CUtensorMap& xm, const CUtensorMap& wm, const __nv_bfloat16*
 // 1 launched (code: 0, or -2 from launched()), -1 when the plan or the tensor
 // maps do not cover the call.
 int try_ws(const __nv_bfloat16* x, const __nv_bfloat16* w, const float* bias, __nv_bfloat16* y,
-           const ConvShape& s, int relu, cudaStream_t st, int& code, const WsHead& head = WsHead{}) {
+           const ConvShape& s, int relu, cudaStream_t st, int& code, const WsHead& head = WsHead{},
+           const __nv_bfloat16* skip = nullptr, int c_skip = 0) {
     WsConv p{};
     int smem = 0, per_sm = 0;
-    CUtensorMap xm, wm;
-    if (!ws_plan(s, p, smem, per_sm) || !ws_tensor_maps(x, w, p, xm, wm)) return -1;
+    CUtensorMap xm, sm, wm;
+    if (!ws_plan(s, p, smem, per_sm)) return -1;
+    p.split = (s.cin - c_skip) / 8;
+    if (!ws_tensor_maps(x, skip, w, p, xm, sm, wm)) return -1;
     switch (p.cg) {
-        case 1: code = launch_ws<1>(xm, wm, w, bias, y, p, smem, per_sm, relu, st, head); return 1;
-        case 2: code = launch_ws<2>(xm, wm, w, bias, y, p, smem, per_sm, relu, st, head); return 1;
-        case 4: code = launch_ws<4>(xm, wm, w, bias, y, p, smem, per_sm, relu, st, head); return 1;
-        case 6: code = launch_ws<6>(xm, wm, w, bias, y, p, smem, per_sm, relu, st, head); return 1;
-        case 8: code = launch_ws<8>(xm, wm, w, bias, y, p, smem, per_sm, relu, st, head); return 1;
-        case 12: code = launch_ws<12>(xm, wm, w, bias, y, p, smem, per_sm, relu, st, head); return 1;
+        case 1: code = launch_ws<1>(xm, sm, wm, w, bias, y, p, smem, per_sm, relu, st, head); return 1;
+        case 2: code = launch_ws<2>(xm, sm, wm, w, bias, y, p, smem, per_sm, relu, st, head); return 1;
+        case 4: code = launch_ws<4>(xm, sm, wm, w, bias, y, p, smem, per_sm, relu, st, head); return 1;
+        case 6: code = launch_ws<6>(xm, sm, wm, w, bias, y, p, smem, per_sm, relu, st, head); return 1;
+        case 8: code = launch_ws<8>(xm, sm, wm, w, bias, y, p, smem, per_sm, relu, st, head); return 1;
+        case 12: code = launch_ws<12>(xm, sm, wm, w, bias, y, p, smem, per_sm, relu, st, head); return 1;
         default: return -1;
     }
 }
@@ -1463,6 +1493,19 @@ int pmd_conv3d_head(const void* x, const void* w, const float* bias, const float
     return -1;
 }
 
+int pmd_conv3d_skip(const void* up, const void* skip, const void* w, const float* bias, void* y, int n, int d, int h,
+                    int wd, int c_up, int c_skip, int cout, int kpad, int relu, void* stream) {
+    if (c_up < 8 || c_skip < 8 || c_up % 8 || c_skip % 8 || c_up > 4096 || c_skip > 4096) return -1;
+    ConvShape s{n, d, h, wd, c_up + c_skip, cout, kpad};
+    if (n < 1 || d < 1 || h < 1 || wd < 1 || kpad % 64 || kpad < 27 * s.cin) return -1;
+    if (g_conv_impl != 0 && g_conv_impl != 4) return -1;
+    int code = 0;
+    if (try_ws((const __nv_bfloat16*)up, (const __nv_bfloat16*)w, bias, (__nv_bfloat16*)y, s, relu,
+               (cudaStream_t)stream, code, WsHead{}, (const __nv_bfloat16*)skip, c_skip) == 1)
+        return code;
+    return -1;
+}
+
 int pmd_conv3d_wgrad_plan(int n, int d, int h, int wd, int cin, int cout, int* info) {
     if (!info || n < 1 || d < 1 || h < 1 || wd < 1 || cin < 8 || cin % 8) return -1;
     ConvShape s{n, d, h, wd, cin, cout, (27 * cin + 63) / 64 * 64};
@@ -1588,6 +1631,15 @@ int pmd_upcat(const void* up, const void* skip, void* out, int n, int d, int h, 
     upcat_kernel<<<grid_for((long long)n * d * h * w * (c_up + c_skip) / 8), 256, 0,
                    (cudaStream_t)stream>>>((const uint4*)up, (const uint4*)skip, (uint4*)out, n, d,
                                            h, w, c_up / 8, c_skip / 8);
+    return launched();
+}
+
+int pmd_upsample(const void* up, void* out, int n, int d, int h, int w, int c, void* stream) {
+    if (n < 1 || d < 2 || h < 2 || w < 2 || d % 2 || h % 2 || w % 2 || c < 8 || c % 8 ||
+        !fits32((long long)n * d * h * w * c))
+        return -1;
+    upsample_kernel<<<grid_for((long long)n * d * h * w * c / 64), 256, 0, (cudaStream_t)stream>>>(
+        (const uint4*)up, (uint4*)out, n, d, h, w, c / 8);
     return launched();
 }
 

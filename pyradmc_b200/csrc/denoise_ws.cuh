@@ -54,6 +54,7 @@ struct WsConv {
     unsigned acc_cols;       // tensor-memory columns of one accumulator: tz * cout
     unsigned tmem_cols;      // allocated: two accumulators, a power of two >= 32
     int ystride;             // channels per voxel of the output tensor
+    int split;               // 8-channel chunks of the first input tensor (cin / 8 where it is the only one)
     // conv3d_zs_kernel: output slices instead of tiles (n_tiles counts them), those of
     // one (h, w) tile after another
     int line;                // slices of a tile, d rounded up to even; 0: tiles
@@ -128,6 +129,16 @@ __device__ __forceinline__ void ws_tile_origin(const WsConv& p, int tile, int& n
     z0 = tzi * p.tz;
     y0 = ty * kUTY;
     x0 = tx * kUTX;
+}
+
+// Plane q of a stage: 8-channel chunk `chunk` of the input, whose chunks from p.split on
+// are another tensor's (a skip connection that was not copied behind the upsampled one).
+__device__ __forceinline__ void ws_load_plane(const WsConv& p, uint32_t dst, const CUtensorMap* x,
+                                              const CUtensorMap* skip, int chunk, int q, int cx, int cy, int cz, int cn,
+                                              uint32_t mbar) {
+    const bool second = chunk >= p.split;
+    tma_load_5d(dst + (uint32_t)q * p.plane_bytes, second ? skip : x, (second ? chunk - p.split : chunk) * 8, cx, cy,
+                cz, cn, mbar);
 }
 
 // The weights of every group into shared memory, [group][w_place][cout][8].  Eight
@@ -209,7 +220,8 @@ __device__ __forceinline__ void ws_store_slice(const WsConv& p, uint32_t acc, bo
 // CG = cg, the 8-channel chunks of a stage.
 template <int CG>
 __global__ void __launch_bounds__(kWsThreads, 1)
-conv3d_ws_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap wmap,
+conv3d_ws_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap skip_map,
+                 const __grid_constant__ CUtensorMap wmap,
                  const __nv_bfloat16* __restrict__ wt, const float* __restrict__ bias,
                  __nv_bfloat16* __restrict__ y, WsConv p, int relu, WsHead head) {
     extern __shared__ __align__(1024) unsigned char smem[];
@@ -284,8 +296,7 @@ conv3d_ws_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant
                     mbar_arrive_expect_tx(full(b), p.tx_bytes);
                     const uint32_t dst = st_s + (uint32_t)b * p.stage_bytes;
                     for (int q = 0; q < cg; ++q)
-                        tma_load_5d(dst + (uint32_t)q * p.plane_bytes, &xmap, (g * cg + q) * 8, x0 - 1,
-                                    y0 - 1, z0 - 1, nb, full(b));
+                        ws_load_plane(p, dst, &xmap, &skip_map, g * cg + q, q, x0 - 1, y0 - 1, z0 - 1, nb, full(b));
                     if (p.streamed)
                         for (int tap = 0; tap < 27; ++tap)
                             for (int q = 0; q < cg; ++q)
@@ -385,7 +396,8 @@ constexpr int kRunSlices = 2;  // halo slices of a stage, output slices of a bat
 
 template <int CG>
 __global__ void __launch_bounds__(kWsThreads, 1)
-conv3d_zs_kernel(const __grid_constant__ CUtensorMap xmap, const __nv_bfloat16* __restrict__ wt,
+conv3d_zs_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap skip_map,
+                 const __nv_bfloat16* __restrict__ wt,
                  const float* __restrict__ bias, __nv_bfloat16* __restrict__ y, WsConv p, int relu, WsHead head) {
     extern __shared__ __align__(1024) unsigned char smem[];
     const ConvShape& s = p.s;
@@ -469,8 +481,8 @@ conv3d_zs_kernel(const __grid_constant__ CUtensorMap xmap, const __nv_bfloat16* 
                         mbar_arrive_expect_tx(full(b), p.tx_bytes);
                         const uint32_t dst = st_s + (uint32_t)b * p.stage_bytes;
                         for (int q = 0; q < CG; ++q)
-                            tma_load_5d(dst + (uint32_t)q * p.plane_bytes, &xmap, (g * CG + q) * 8, x0 - 1, y0 - 1,
-                                        z0 - 1 + c * T, nb, full(b));
+                            ws_load_plane(p, dst, &xmap, &skip_map, g * CG + q, q, x0 - 1, y0 - 1, z0 - 1 + c * T, nb,
+                                          full(b));
                         ++st;
                         if (++b == S) {
                             b = 0;

@@ -284,6 +284,24 @@ class UNet3D:
                                   c_skip, self._stream()), "upcat")
         self.launches += 1
 
+    def _upcat_conv(self, up, skip, cat, layer: ConvLayer, y, dims, c_up, c_skip, keep: bool) -> None:
+        """The convolution over (upsampled up, skip).  The concatenation is stored in cat
+        only where it is kept for a backward pass or the kernel that reads the two
+        tensors as they are does not cover the shape."""
+        n, d, h, w = dims
+        if not keep and self.lib.pmd_upsample(up.data_ptr(), cat.data_ptr(), n, d, h, w, c_up,
+                                              self._stream()) == 0:
+            code = self.lib.pmd_conv3d_skip(cat.data_ptr(), skip.data_ptr(), self._ptr16(layer.w_off),
+                                            self._ptr32(self.p32, layer.b_off), y.data_ptr(), n, d, h, w,
+                                            c_up, c_skip, layer.cout, layer.kpad, 1, self._stream())
+            self.launches += 1
+            if code != -1:
+                _check(code, f"conv {layer.name}")
+                self.launches += 1
+                return
+        self._upcat(up, skip, cat, dims, c_up, c_skip)
+        self._conv(cat, layer, y, dims)
+
     def _upcat_grad(self, gout, gup, gskip, dims, c_up, c_skip) -> None:
         _check(self.lib.pmd_upcat_grad(gout.data_ptr(), gup.data_ptr(), gskip.data_ptr(), *dims,
                                        c_up, c_skip, 0, self._stream()), "upcat grad")
@@ -339,14 +357,11 @@ class UNet3D:
         self._pool(a["e2"], a["p2"], d2, c2)
         self._conv(a["p2"], L["mid_a"], a["ma"], d3)
         self._conv(a["ma"], L["mid_b"], a["mb"], d3)
-        self._upcat(a["mb"], a["e2"], a["u2"], d2, c3, c2)
-        self._conv(a["u2"], L["dec2a"], a["d2a"], d2)
+        self._upcat_conv(a["mb"], a["e2"], a["u2"], L["dec2a"], a["d2a"], d2, c3, c2, keep_features)
         self._conv(a["d2a"], L["dec2b"], a["d2"], d2)
-        self._upcat(a["d2"], a["e1"], a["u1"], d1, c2, c1)
-        self._conv(a["u1"], L["dec1a"], a["d1a"], d1)
+        self._upcat_conv(a["d2"], a["e1"], a["u1"], L["dec1a"], a["d1a"], d1, c2, c1, keep_features)
         self._conv(a["d1a"], L["dec1b"], a["d1"], d1)
-        self._upcat(a["d1"], a["e0"], a["u0"], d0, c1, c0)
-        self._conv(a["u0"], L["dec0a"], a["d0a"], d0)
+        self._upcat_conv(a["d1"], a["e0"], a["u0"], L["dec0a"], a["d0a"], d0, c1, c0, keep_features)
         if not keep_features and self.fuse_head and self._conv_head(a["d0a"], L["dec0b"], ws, d0):
             return
         self._conv(a["d0a"], L["dec0b"], a["d0"], d0)

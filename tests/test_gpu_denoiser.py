@@ -411,6 +411,37 @@ def test_convolution_along_runs_does_not_depend_on_the_other_windows(gpu, shape)
         np.testing.assert_array_equal(conv(dx[k:k + 1].contiguous(), 4)[0], got[k])
 
 
+@pytest.mark.parametrize("shape", [(2, 4, 18, 10, 32, 16, 16), (1, 6, 16, 8, 64, 32, 32), (3, 2, 6, 4, 128, 64, 64),
+                                   (1, 8, 20, 12, 8, 24, 32), (2, 4, 8, 8, 48, 16, 128)])
+def test_convolution_over_two_tensors_equals_that_over_their_concatenation(gpu, shape):
+    """pmd_upsample + pmd_conv3d_skip against pmd_upcat + pmd_conv3d: the same products
+    in the same order, bit for bit."""
+    import torch
+
+    n, d, h, w, c_up, c_skip, cout = shape
+    cin = c_up + c_skip
+    rng = np.random.default_rng(500 + sum(shape))
+    wt, kpad = _weights(rng, cin, cout)
+    lib = _lib.load()
+    up = _dev(bf16(rng.normal(size=(n, d // 2, h // 2, w // 2, c_up))), torch.bfloat16)
+    skip = _dev(bf16(rng.normal(size=(n, d, h, w, c_skip))), torch.bfloat16)
+    dw, db = _dev(wt, torch.bfloat16), _dev(rng.normal(size=cout).astype(np.float32), torch.float32)
+    cat = torch.empty((n, d, h, w, cin), dtype=torch.bfloat16, device=gpu)
+    full = torch.empty((n, d, h, w, c_up), dtype=torch.bfloat16, device=gpu)
+    want, got = (torch.full((n, d, h, w, cout), float("nan"), dtype=torch.bfloat16, device=gpu) for _ in range(2))
+    assert lib.pmd_upcat(up.data_ptr(), skip.data_ptr(), cat.data_ptr(), n, d, h, w, c_up, c_skip, None) == 0
+    assert lib.pmd_conv3d(cat.data_ptr(), dw.data_ptr(), db.data_ptr(), want.data_ptr(), n, d, h, w, cin, cout,
+                          kpad, 1, None) == 0
+    assert lib.pmd_upsample(up.data_ptr(), full.data_ptr(), n, d, h, w, c_up, None) == 0
+    assert lib.pmd_conv3d_skip(full.data_ptr(), skip.data_ptr(), dw.data_ptr(), db.data_ptr(), got.data_ptr(),
+                               n, d, h, w, c_up, c_skip, cout, kpad, 1, None) == 0
+    torch.cuda.synchronize()
+    assert lib.pmd_conv3d_failures() == 0
+    np.testing.assert_array_equal(full.cpu().view(torch.int16).numpy(),
+                                  cat[..., :c_up].contiguous().cpu().view(torch.int16).numpy())
+    np.testing.assert_array_equal(got.cpu().view(torch.int16).numpy(), want.cpu().view(torch.int16).numpy())
+
+
 def test_tensor_memory_path_rejects_what_it_does_not_cover(gpu):
     lib = _lib.load()
     previous = lib.pmd_conv3d_impl(2)
