@@ -1030,6 +1030,7 @@ bool ws_plan_at(const ConvShape& s, int tz, int at_cg, WsConv& p, int& smem, int
     while (cols < 2 * p.acc_cols) cols <<= 1;
     p.tmem_cols = cols;
     p.ystride = N;
+    p.parts = 1;
     p.tiles_d = (s.d + p.tz - 1) / p.tz;
     p.tiles_h = (s.h + kUTY - 1) / kUTY;
     p.tiles_w = (s.w + kUTX - 1) / kUTX;
@@ -1103,7 +1104,7 @@ bool zs_plan(WsConv& p, int& smem, int& ctas_per_sm) {
 // 0.27 at 4); shallow ones where deep ones would leave SMs without a tile.  The
 // channel groups, which set the order of an output's sum, are the deepest plan's, so
 // that a window's values do not depend on how many windows share the launch.
-bool ws_plan(const ConvShape& s, WsConv& p, int& smem, int& ctas_per_sm) {
+bool ws_plan(const ConvShape& s, WsConv& p, int& smem, int& ctas_per_sm, bool whole = false) {
     if (s.cout % 16 || s.cout < 16 || s.cout > 256) return false;
     if (!(s.cin == 8 || s.cin % 16 == 0)) return false;
     // the channel groups, and with them the order of a sum, are those of shallow tiles
@@ -1123,6 +1124,37 @@ bool ws_plan(const ConvShape& s, WsConv& p, int& smem, int& ctas_per_sm) {
         tz = deep_tz;
     }
     const WsConv deep = p;
+    if (p.streamed) {
+        // Streamed weights and the halo are both copied 16 bytes a row, and the copies
+        // bound these layers: of the depths and output-channel parts, the least rows to
+        // the last tile, those of the halo (from five dimensions) counted twice.  One
+        // window: a tile of 128 -> 128 copies 55,000 rows of weights and there are 16
+        // tiles, 43 us; in eight parts 26.  Four windows, 192 -> 64: 48 us (60 with the
+        // halo's rows counted once).  whole: no parts (the fused head sums over all
+        // channels).
+        long long best = 0;
+        for (int t = deep.tz; t >= 1; t /= 2)
+            for (int parts = 1; parts <= (whole ? 1 : s.cout / 16); parts *= 2) {
+                ConvShape part = s;
+                part.cout = s.cout / parts;
+                if (s.cout % parts || part.cout % 16) continue;
+                WsConv q{};
+                int q_smem = 0, q_per_sm = 0;
+                if (!ws_plan_at(part, t, deep.cg, q, q_smem, q_per_sm) || !q.streamed) continue;
+                const long long tiles = (long long)q.n_tiles * parts, blocks = (long long)kPlanSms * q_per_sm;
+                const long long rows = (27 * part.cout + 2 * (t + 2) * kUHY * kUHX) * (long long)(s.cin / 8);
+                const long long cost = (tiles + blocks - 1) / blocks * rows * q_per_sm;
+                if (tiles > (1LL << 30) || (best && cost >= best)) continue;
+                best = cost;
+                q.n_tiles = (int)tiles;
+                q.parts = parts;
+                q.ystride = s.cout;
+                p = q;
+                smem = q_smem;
+                ctas_per_sm = q_per_sm;
+            }
+        return true;
+    }
     if (zs_plan(p, smem, ctas_per_sm)) return true;
     for (; tz > 1 && p.n_tiles < kPlanSms; tz /= 2) {
         WsConv q{};
@@ -1190,7 +1222,7 @@ bool ws_tensor_maps(const __nv_bfloat16* x, const __nv_bfloat16* skip, const __n
     if (!halo_tensor_map(x, first, slices, xm)) return false;
     if (second.cin == 0) sm = xm;
     else if (!halo_tensor_map(skip, second, slices, sm)) return false;
-    const cuuint64_t wdim[2] = {(cuuint64_t)s.kpad, (cuuint64_t)s.cout};
+    const cuuint64_t wdim[2] = {(cuuint64_t)s.kpad, (cuuint64_t)(s.cout * p.parts)};
     const cuuint64_t wstride[1] = {(cuuint64_t)s.kpad * e};
     const cuuint32_t wbox[2] = {8, (cuuint32_t)s.cout};
     return enc(&wm, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<__nv_bfloat16*>(w), wdim, wstride, wbox,
@@ -1234,7 +1266,7 @@ int try_ws(const __nv_bfloat16* x, const __nv_bfloat16* w, const float* bias, __
     WsConv p{};
     int smem = 0, per_sm = 0;
     CUtensorMap xm, sm, wm;
-    if (!ws_plan(s, p, smem, per_sm)) return -1;
+    if (!ws_plan(s, p, smem, per_sm, head.w != nullptr)) return -1;
     p.split = (s.cin - c_skip) / 8;
     if (!ws_tensor_maps(x, skip, w, p, xm, sm, wm)) return -1;
     switch (p.cg) {

@@ -13,7 +13,7 @@
 // of the second 8-element K half, SBO = 160 B), so every tap is one
 // descriptor offset into the same halo and no im2col copy exists.  Weights
 // sit in shared memory as w[chunk][cout][8] (the B operand, SBO = 128 B), in the
-// order of w_place.  One thread issues the MMAs (M = 128, N = up to 3 cout,
+// order of w_place.  One warp issues the MMAs (M = 128, N = up to 3 cout,
 // K = 16 per instruction: umma_issue_taps); tcgen05.commit arrives on an mbarrier that every
 // thread waits on, with a time limit that records a failure instead of
 // hanging.  The epilogue reads the fp32 accumulators from tensor memory

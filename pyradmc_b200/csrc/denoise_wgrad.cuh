@@ -29,7 +29,7 @@
 //     (zeros outside the volume), publish it to the tensor cores
 //     (fence.proxy.async) and, in the CTAs of tap group 0, sum the bias
 //     gradient from it;
-//   * warp 1 (one lane): issues M = 128, N = 8 * chunks, K = 16 MMAs with
+//   * warp 1: issues M = 64 or 128, N = 8 * chunks, K = 16 MMAs with
 //     both operands MN-major, commits each stage back to its producers and,
 //     after its last tile, the accumulators to the epilogue.  With cin = 8 the
 //     halo operand's 8-channel groups are instead taken 16 bytes apart, i.e.
@@ -39,7 +39,7 @@
 //     and add them into dW.
 // Every mbarrier wait is bounded (kUWaitNs), records a failure in shared
 // memory and in g_umma_failures, and ends every role's loop; the producer and
-// the MMA thread wait (bounded) for their copies and MMAs in flight before the
+// the MMA warp wait (bounded) for their copies and MMAs in flight before the
 // tensor memory is freed.  No multicast anywhere.
 #pragma once
 
@@ -319,6 +319,9 @@ conv3d_wgrad_umma_kernel(const __grid_constant__ CUtensorMap xmap,
 // between co chunks, so that the chunks of three slices follow one another, LBO 128
 // between rows of 8 voxels), the slices of the stages in one array with two
 // slices of zeros between them: the neighbours of a tile's first and last slices.
+// Bound by the MMAs' operands in shared memory.  Before and after at 4 windows of 64^3:
+// 16 -> 16 0.47 -> 0.11 ms, 48 -> 16 0.57 -> 0.24, 8 -> 16 0.27 -> 0.14, 96 -> 32 at half
+// size 0.23 -> 0.11.  cout = 64 and 128 stay above: their three slices do not fit M.
 // Roles, waits and failure handling as above.
 __global__ void __launch_bounds__(kWgThreads, 1)
 conv3d_wgrad_fold_kernel(const __grid_constant__ CUtensorMap xmap, const __nv_bfloat16* __restrict__ g,

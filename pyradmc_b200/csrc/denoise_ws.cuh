@@ -15,18 +15,19 @@
 //     the whole launch, one TMA copy per 8-channel weight chunk (box 8 x cout of
 //     the [cout][kpad] matrix) joins the stage.  The innermost coordinate of
 //     every copy is a multiple of 8 bf16 = 16 bytes.
-//   * warp 1 (one lane) issues the tcgen05.mma of each stage into one of two
+//   * warp 1 issues the tcgen05.mma of each stage into one of two
 //     accumulators in tensor memory, commits each stage to release its buffer
 //     to the producer and each finished tile to the epilogue.
 //   * warps 2-5 drain an accumulator (tcgen05.ld, bias, ReLU, bf16 stores, one
 //     output voxel per thread) and release it.
-// Resident weights are staged once per block as [group][chunks in the order of
+// With streamed weights the output channels may be split into parts, each a tile of its
+// own (ws_plan).  Resident weights are staged once per block as [group][chunks in the order of
 // w_place][cout][8].
 // With one channel group and resident weights the MMAs of a slice are issued
 // in the order of conv3d_umma_kernel, so the two produce identical bits.
 // Every mbarrier wait gives up after kUWaitNs, records the failure in shared
 // memory and in g_umma_failures, and every role then leaves its loop; the
-// producer waits (bounded) for its copies in flight and the MMA thread for its
+// producer waits (bounded) for its copies in flight and the MMA warp for its
 // MMAs before the tensor memory is freed.  No multicast anywhere.
 #pragma once
 
@@ -54,6 +55,7 @@ struct WsConv {
     unsigned acc_cols;       // tensor-memory columns of one accumulator: tz * cout
     unsigned tmem_cols;      // allocated: two accumulators, a power of two >= 32
     int ystride;             // channels per voxel of the output tensor
+    int parts;               // streamed weights: output-channel parts, each a tile of its own with s.cout = N channels
     int split;               // 8-channel chunks of the first input tensor (cin / 8 where it is the only one)
     // conv3d_zs_kernel: output slices instead of tiles (n_tiles counts them), those of
     // one (h, w) tile after another
@@ -286,7 +288,7 @@ conv3d_ws_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant
             bool stop = false;
             for (int tile = blockIdx.x; tile < p.n_tiles && !stop; tile += gridDim.x) {
                 int nb, z0, y0, x0;
-                ws_tile_origin(p, tile, nb, z0, y0, x0);
+                ws_tile_origin(p, tile / p.parts, nb, z0, y0, x0);
                 for (int g = 0; g < p.groups; ++g) {
                     const int b = st % S, use = st / S;
                     if (use >= 1 && !ws_wait(empty(b), (uint32_t)((use - 1) & 1), failed)) {
@@ -301,7 +303,7 @@ conv3d_ws_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant
                         for (int tap = 0; tap < 27; ++tap)
                             for (int q = 0; q < cg; ++q)
                                 tma_load_2d(dst + p.halo_part + (uint32_t)w_place(tap, q, cg) * N * 16, &wmap,
-                                            (tap * cpt + g * cg + q) * 8, 0, full(b));
+                                            (tap * cpt + g * cg + q) * 8, tile % p.parts * N, full(b));
                     ++st;
                 }
             }
@@ -347,15 +349,16 @@ conv3d_ws_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant
             if (!ok) break;
             tc_fence_after();
             int nb, z0, y0, x0;
-            ws_tile_origin(p, tile, nb, z0, y0, x0);
-            const int yg = y0 + r / kUTX, xg = x0 + r % kUTX;
+            ws_tile_origin(p, tile / p.parts, nb, z0, y0, x0);
+            const int yg = y0 + r / kUTX, xg = x0 + r % kUTX, n0 = tile % p.parts * N;  // the part's first channel
             for (int sl = 0; sl < p.tz; ++sl) {
                 const int z = z0 + sl;
                 const bool in = z < s.d && yg < s.h && xg < s.w;
                 const long long m =
                     (((long long)nb * s.d + (in ? z : 0)) * s.h + (in ? yg : 0)) * s.w + (in ? xg : 0);
-                ws_store_slice(p, tmem + (uint32_t)a * p.acc_cols + (uint32_t)(sl * N), in, m, quarter, bias, y, relu,
-                               head, head.w, in && head.w && head.base ? head.base[m] : 0.0f);
+                ws_store_slice(p, tmem + (uint32_t)a * p.acc_cols + (uint32_t)(sl * N), in, m, quarter,
+                               bias ? bias + n0 : nullptr, y + n0, relu, head, head.w,
+                               in && head.w && head.base ? head.base[m] : 0.0f);
             }
             tc_fence_before();
             mbar_arrive(acc_free(a));

@@ -5,13 +5,14 @@
 // transport/photon.py:100-282 and transport/electron.py:207-482 statement for
 // statement.  The structure is B200-first rather than a translation:
 //   * persistent grids (a multiple of the SM count) with per-lane refill: a
-//     lane whose particle ends takes the next one at once, from the input
-//     queue first and then from the batch's primary cursor, so no lane idles
-//     behind the longest particle of its warp;
+//     lane whose particle ends takes the next one of the input queue at once, so
+//     no lane idles behind the longest particle of its warp;
 //   * primaries are generated at full warp width and queued (generate_kernel);
 //   * queue rotation, the primary admission window and the "work left" flag
 //     are advanced on the device by the last block of each kernel, so a whole
-//     batch drains without one host round trip (and inside one CUDA graph);
+//     wave of batches drains without one host round trip (and inside one CUDA graph);
+//   * no counter that other blocks use is touched per particle: input is claimed
+//     32 particles at a time and output slots are taken in chunks;
 //   * energy books and event counters accumulate in shared memory and reach
 //     global memory once per block.
 #pragma once
