@@ -450,13 +450,13 @@ def denoiser_leg(args, engine, source, counts, stream, device, plain_s_per_dij):
         "windows_tried": {str(k): list(v) for k, v in windows.items()},
         "stage_ms": stages,
         "unet_forward_flops_per_dij": forward_flops_per_voxel() * unet_vox,
-        "roofline": {"bound": "tensor", "kernel": "conv3d_ws_kernel (decoder level 0, 48->16)",
+        "roofline": {"bound": "tensor", "kernel": "conv3d_zs_kernel (decoder level 0, 48->16)",
                      "achieved": conv_tflops, "peak": bf16_peak, "unit": "TFLOP/s",
                      "frac": conv_tflops / bf16_peak,
                      "peak_source": "measured" if "bf16_tflops" in peaks else "fallback",
-                     "shape_cap": "M 128 x N 16 x K 16 MMAs read 4.5 KB of shared memory per "
-                                  "65,536 FLOP: ~0.25 of the bf16 peak at most",
-                     "source": "profiles/conv3d_ws_dec0a_ncu.md"},
+                     "shape_cap": "M 128 x N 48 x K 16 MMAs read 5.5 KB of shared memory per "
+                                  "196,608 FLOP, beside the copies' 16-byte rows",
+                     "source": "profiles/conv3d_zs_wgrad_fold_ncu.md"},
     }
 
 
@@ -1060,9 +1060,9 @@ def b200_arm(args, world, rank, local):
             "issue_bound": {
                 "what": "transport is bounded by instruction issue and load latency, not HBM: "
                         "fraction of cycles each SM sub-partition issued, ncu on a main round "
-                        "of this workload",
-                "photon_kernel": 0.343, "electron_kernel": 0.540,
-                "simd_lanes_active": {"photon_kernel": 7.9 / 32, "electron_kernel": 16.3 / 32},
+                        "of a Dij on this phantom",
+                "photon_kernel": 0.607, "electron_kernel": 0.571,
+                "simd_lanes_active": {"photon_kernel": 10.6 / 32, "electron_kernel": 20.4 / 32},
                 "source": "profiles/transport_main_round_dij100_ncu.md"},
             "algorithmic_bytes": algorithmic_bytes(c),
             "transport_ms": c["transport_ms"],

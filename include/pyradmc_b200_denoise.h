@@ -63,8 +63,8 @@ int pmd_conv3d_skip(const void* up, const void* skip, const void* w, const float
  * tensor-memory kernel only; 3 its pipelined variant only (two halo buffers
  * and two accumulators, one CTA per SM; measured slower than the default on
  * this network's layers, kept for larger tiles); 4 the warp-specialized kernel only (a TMA producer
- * warp, one MMA-issuing thread and four epilogue warps over a ring of stage
- * buffers; cout a multiple of 16 up to 256, cin 8 or any multiple of 16, weights
+ * warp, an MMA-issuing warp and four epilogue warps over a ring of stage
+ * buffers, over runs along d where the weights are resident and 3 cout <= 256, else over tiles; cout a multiple of 16 up to 256, cin 8 or any multiple of 16, weights
  * resident or streamed with the stages).  Other shapes return -1.  impl < 0 only queries.  Returns the
  * previous setting.  Process-wide. */
 int pmd_conv3d_impl(int impl);
@@ -74,7 +74,7 @@ int pmd_conv3d_impl(int impl);
  * warp-specialized, 3 pipelined, 2 single-buffered tensor-memory, 1 mma.sync,
  * -1 none; for the warp-specialized kernel info[1..7] = 8-channel chunks per
  * stage, stages per tile, stage buffers, weights streamed (1) or resident (0),
- * output slices per tile, blocks per SM, shared memory bytes per block (the
+ * output slices per tile (runs: halo slices per stage), blocks per SM, shared memory bytes per block (the
  * single-buffered kernel fills info[5..7]).  Returns 0, or -1 for a NULL info or
  * an invalid shape. */
 int pmd_conv3d_plan(int n, int d, int h, int w_, int cin, int cout, int* info);
