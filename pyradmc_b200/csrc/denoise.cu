@@ -1071,20 +1071,20 @@ bool zs_plan(WsConv& p, int& smem, int& ctas_per_sm) {
     q.stage_bytes = (q.halo_part + 127u) & ~127u;
     q.tx_bytes = (unsigned)q.cg * q.box_bytes;
     const int weights = q.groups * (int)q.w_chunks * N * 16;
-    const int most = kSmemPerSM / ctas_per_sm - kSmemReserved < kSmemPerBlockMax
-                         ? kSmemPerSM / ctas_per_sm - kSmemReserved : kSmemPerBlockMax;
+    int per_sm = ctas_per_sm;
+    if (512 / per_sm / N / q.tz < 4) per_sm = 1;  // 16 -> 48: 4 batches take one block's 384 columns
+    const int most = kSmemPerSM / per_sm - kSmemReserved < kSmemPerBlockMax
+                         ? kSmemPerSM / per_sm - kSmemReserved : kSmemPerBlockMax;
     q.ring = 1;
-    while (2 * q.ring <= 512 / ctas_per_sm / N / q.tz) q.ring *= 2;
+    while (2 * q.ring <= 512 / per_sm / N / q.tz) q.ring *= 2;
     if (q.ring < 4) return false;
     const int bars = 8 * (2 * kWsMaxStages + 2 * q.ring) + 16 + 2 * N * 4;  // and bias, head weights
-    if (q.groups == 1 || ctas_per_sm == 1)
+    if (q.groups == 1 || per_sm == 1)
         for (q.stages = kWsMaxStages; q.stages > p.stages; --q.stages)
             if (q.stages * (int)q.stage_bytes + weights + bars <= most) break;
     const int need = q.stages * (int)q.stage_bytes + weights + bars;
     if (need > most) return false;
-    // all of the block's share, so that no further block takes tensor memory
-    smem = need > kSmemPerSM / (ctas_per_sm + 1) - kSmemReserved ? need : kSmemPerSM / (ctas_per_sm + 1);
-    q.tmem_cols = 512u / (unsigned)ctas_per_sm;
+    q.tmem_cols = 512u / (unsigned)per_sm;
     q.line = (s.d + kRunSlices - 1) / kRunSlices * kRunSlices;
     // a group lags two batches behind the one before, and one more is being stored; else
     // runs of ring batches, the first of which has no output, the tile's in equal parts
@@ -1094,7 +1094,10 @@ bool zs_plan(WsConv& p, int& smem, int& ctas_per_sm) {
     const long long slices = (long long)s.n * q.tiles_h * q.tiles_w * q.line;
     if (slices > (1LL << 30)) return false;
     q.n_tiles = (int)slices;
+    // all of the block's share, so that no further block takes tensor memory
+    smem = need > kSmemPerSM / (per_sm + 1) - kSmemReserved ? need : kSmemPerSM / (per_sm + 1);
     p = q;
+    ctas_per_sm = per_sm;
     return true;
 }
 

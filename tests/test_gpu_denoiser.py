@@ -379,7 +379,7 @@ def test_tensor_memory_convolution_matches_oracle(gpu, shape):
 # runs along d: several per block (windows x tiles above two blocks an SM), odd and
 # short depths, one and several channel groups, an accumulator ring of 4 and of 8
 @pytest.mark.parametrize("shape", [(40, 7, 40, 20, 16, 16), (34, 1, 40, 24, 16, 32), (34, 9, 40, 24, 32, 32),
-                                   (20, 13, 33, 17, 32, 64), (24, 11, 40, 24, 48, 16), (20, 6, 40, 24, 96, 32),
+                                   (20, 13, 33, 17, 32, 64), (24, 11, 40, 24, 48, 16), (20, 6, 40, 24, 96, 32), (24, 11, 40, 24, 16, 48),
                                    # streamed weights: one window in output-channel parts
                                    (24, 8, 8, 9, 128, 128), (12, 16, 16, 18, 192, 64), (9, 5, 17, 10, 64, 192)])
 def test_convolution_along_runs_does_not_depend_on_the_other_windows(gpu, shape):
