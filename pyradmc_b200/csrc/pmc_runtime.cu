@@ -499,7 +499,13 @@ int prepare_transport(pmc_engine* e, const pmc_run_params* p, unsigned long long
         plan->wave = (p->n_batches + n_waves - 1) / n_waves;  // waves of about the same size
     }
     // admission never needs more than a wave's primaries per round
-    plan->budget = p->chunk_size > 0 ? (unsigned long long)p->chunk_size : 16ull * resident;
+    // and, unless the caller chose it, no more than a quarter above one batch's (or 8 per
+    // thread): the queues take 4 KB a primary, and a new engine's first call waits for
+    // their allocation (40 columns of 2.2e5 histories, 8 batches: 10 GB for a wave's
+    // window, 55 ms and more; 5.5 GB for this one)
+    plan->budget = p->chunk_size > 0
+                       ? (unsigned long long)p->chunk_size
+                       : std::min(16ull * resident, std::max(block + block / 4, 8ull * resident));
     plan->budget = std::max(1ull, std::min(plan->budget, block * (unsigned long long)plan->wave));
     const int qf = p->queue_factor > 0 ? p->queue_factor : 16;
     const unsigned long long cap64 = plan->budget * (unsigned long long)qf;
