@@ -319,6 +319,9 @@ conv3d_wgrad_umma_kernel(const __grid_constant__ CUtensorMap xmap,
 // between co chunks, so that the chunks of three slices follow one another, LBO 128
 // between rows of 8 voxels), the slices of the stages in one array with two
 // slices of zeros between them: the neighbours of a tile's first and last slices.
+// A full tile's last halo slice would take a third one for the group that is
+// discarded; it takes the next buffer's first slice, once that is loaded (a third
+// slice of zeros would not fit beside 96 -> 32's deepest tiles).
 // Bound by the MMAs' operands in shared memory.  Before and after at 4 windows of 64^3:
 // 16 -> 16 0.47 -> 0.11 ms, 48 -> 16 0.57 -> 0.24, 8 -> 16 0.27 -> 0.14, 96 -> 32 at half
 // size 0.23 -> 0.11.  cout = 64 and 128 stay above: their three slices do not fit M.
@@ -424,8 +427,15 @@ conv3d_wgrad_fold_kernel(const __grid_constant__ CUtensorMap xmap, const __nv_bf
                     umma_smem_desc(dy_s + (uint32_t)(b * (p.tz + 2)) * slice_bytes, 128u, 2048u);
                 const uint64_t b0 =
                     umma_smem_desc(st_s + (uint32_t)b * p.stage_bytes, kUHX * 16u, p.b_sbo);
+                const bool more = h + 1 < p.chunk_groups || tile + ctas_per_group < p.n_tiles;
 #pragma unroll 1
                 for (int zx = 0; zx < slices; ++zx) {
+                    // the discarded group of a full tile's last slice is the next buffer's
+                    // first: its loaders are waited for (they wait for no MMA of this stage)
+                    if (zx == p.tz + 1 && b + 1 < S && more) {
+                        if (!ws_wait_warp(dfull(b + 1), phase, failed)) stop = true;  // (this stage is still committed)
+                        tc_fence_after();
+                    }
                     const uint64_t as = a0 + (uint64_t)(zx * (int)(slice_bytes >> 4));  // output slice zx - 2
                     const uint64_t bz = b0 + (uint64_t)(zx * kUHY * kUHX);
                     const uint32_t acc0 = tile == cta_in_group && zx == 0 ? 0u : 1u;

@@ -143,6 +143,17 @@ def test_weight_gradient_folded_over_d_matches_oracle(gpu, shape):
     test_conv3d_weight_gradient_matches_oracle(gpu, shape)
 
 
+# blocks of several full tiles, one after another through both buffers: the next tile's
+# output gradient is loaded beside the MMAs that read past the end of this one's
+@pytest.mark.parametrize("shape", [(4, 24, 64, 64, 16, 16), (3, 12, 32, 40, 96, 32)])
+def test_weight_gradient_over_several_tiles_a_block_matches_oracle(gpu, shape):
+    n, d, h, w = shape[:4]
+    tz, _, chunk_groups, _, unit_groups = _wgrad_plan(_lib.load(), shape)[:5]
+    tiles = n * (d // tz) * -(-h // 16) * -(-w // 8)
+    assert d % tz == 0 and tiles * chunk_groups >= 2 * (148 // unit_groups)
+    test_conv3d_weight_gradient_matches_oracle(gpu, shape)
+
+
 @pytest.mark.parametrize("shape", [(1, 8, 8, 8, 16, 16), (2, 6, 5, 7, 48, 16), (1, 4, 6, 4, 96, 32),
                                    (1, 4, 4, 4, 192, 64), (1, 2, 4, 4, 64, 128),
                                    (1, 4, 4, 4, 128, 64), (1, 4, 4, 4, 32, 16)])
