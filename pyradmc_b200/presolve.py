@@ -318,8 +318,12 @@ def _presolve_on_device(lib, cs, mu, params, columns, n: int, capacity: int, dev
                 kind.data_ptr(), energy.data_ptr(), pos.data_ptr(), dirs.data_ptr(), weight.data_ptr(),
                 C.byref(count), C.byref(dropped), torch.cuda.current_stream(device).cuda_stream)
     k = _kept(code, count)
-    cut = (lambda t: t[:k]) if 2 * k >= capacity else (lambda t: t[:k].clone())  # not half empty
-    return DevicePhaseSpace(cut(kind), cut(energy), cut(pos), cut(dirs), cut(weight), max_energy)
+    records = [t[:k] for t in (kind, energy, pos, dirs, weight)]
+    if 2 * k < capacity:  # half empty: keep copies, finished (as the records are) when the call returns
+        with torch.cuda.device(device):
+            records = [t.clone() for t in records]
+            torch.cuda.current_stream(device).synchronize()
+    return DevicePhaseSpace(*records, max_energy)
 
 
 def stack_path_lengths(stack, points, directions, from_origin: bool = False) -> np.ndarray:

@@ -154,3 +154,26 @@ def test_device_phase_space_is_transported_in_place_with_the_same_dose(gpu):
     np.testing.assert_array_equal(a.dose, b.dose)
     np.testing.assert_array_equal(a.dose_sigma, b.dose_sigma)
     assert a.energy_emitted == b.energy_emitted
+
+
+def test_device_phase_space_is_finished_when_the_call_returns(gpu, monkeypatch):
+    """Also where few of the slots are kept and the records are copied together:
+    other streams (the engine's) may read them at once."""
+    import torch
+
+    g = golden()
+    clone = torch.Tensor.clone
+
+    def late(self, **kw):  # some 20 ms of other work on the same stream before each copy
+        torch.cuda._sleep(40_000_000)
+        return clone(self, **kw)
+
+    kw = dict(air=True, pcut=3.0, ecut=3.0, return_device_source=True)  # few secondaries survive
+    want = _run(g, gpu, "first_compton", **kw)
+    assert 2 * len(want) < 4 * case.N
+    want = want.columns()
+    monkeypatch.setattr(torch.Tensor, "clone", late)
+    got = _run(g, gpu, "first_compton", **kw)
+    assert torch.cuda.current_stream(gpu).query()
+    for name, column in got.columns().items():
+        np.testing.assert_array_equal(column, want[name])
