@@ -900,6 +900,8 @@ class B200Engine:
             kind = (source.particle_type - 1).to(torch.int32).contiguous()  # IAEA code -> PMC_* kind
             cols = [t.contiguous() for t in (source.energy, source.pos, source.dir, source.weight)]
             keep += [kind, *cols]
+            # made on torch's current stream, read on the engine's own, which waits for no other
+            torch.cuda.current_stream(dev).synchronize()
             dptr = lambda t, ct: C.cast(C.c_void_p(t.data_ptr()), C.POINTER(ct))  # noqa: E731
             src.type = _lib.PMC_SRC_PHASESPACE_DEVICE
             src.n_records = int(kind.shape[0])

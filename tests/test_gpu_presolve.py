@@ -177,3 +177,25 @@ def test_device_phase_space_is_finished_when_the_call_returns(gpu, monkeypatch):
     assert torch.cuda.current_stream(gpu).query()
     for name, column in got.columns().items():
         np.testing.assert_array_equal(column, want[name])
+
+
+def test_engine_waits_for_the_stream_that_makes_the_device_phase_space(gpu):
+    """Its records (and the kinds converted for the call) may still be queued on
+    torch's current stream when the run starts."""
+    import torch
+
+    from pyradmc_b200 import B200Engine
+    from pyradmc_b200.model import AnalyticWaterTables, VoxelGrid
+
+    g = golden()
+    dev = _run(g, gpu, "first_compton", air=True, return_device_source=True)
+    grid = VoxelGrid.uniform_water((16, 16, 16), (1.0, 1.0, 1.0), origin=(0.0, 0.0, -4.5))
+    engine = B200Engine(grid, AnalyticWaterTables(geometry_densities=grid.max_density_by_material()), device=gpu)
+    want = engine.run(dev, n_histories=40_000, n_batches=4, seed=case.SEED)
+    with torch.cuda.stream(torch.cuda.Stream(gpu)):
+        torch.cuda._sleep(100_000_000)  # some 50 ms of other work first
+        late = PS.DevicePhaseSpace(*(t.clone() for t in (dev.particle_type, dev.energy, dev.pos, dev.dir, dev.weight)),
+                                   dev.max_energy)
+        got = engine.run(late, n_histories=40_000, n_batches=4, seed=case.SEED)
+    np.testing.assert_array_equal(got.dose, want.dose)
+    assert got.energy_emitted == want.energy_emitted
