@@ -130,6 +130,8 @@ struct pmc_engine {
     std::vector<cudaEvent_t> batch_ev;  // three per wave of a group, read once per group
     unsigned long long h2d_bytes = 0;  // cumulative over the engine's life
     unsigned long long d2h_bytes = 0;
+    bool shared = false;           // the call's batches share waves
+    long long reported = 0;        // histories of the call reported as progress
     pmc_progress_fn progress = nullptr;
     void* progress_user = nullptr;
 };
@@ -507,8 +509,13 @@ int prepare_transport(pmc_engine* e, const pmc_run_params* p, unsigned long long
                        ? (unsigned long long)p->chunk_size
                        : std::min(16ull * resident, std::max(block + block / 4, 8ull * resident));
     plan->budget = std::max(1ull, std::min(plan->budget, block * (unsigned long long)plan->wave));
+    e->shared = plan->wave > 1;
     const int qf = p->queue_factor > 0 ? p->queue_factor : 16;
     const unsigned long long cap64 = plan->budget * (unsigned long long)qf;
+    if (cap64 > 0x7fffffffull && e->shared) {  // the queues of a wave's window cannot be numbered
+        *plan = RunPlan{};
+        return prepare_transport(e, p, block, cols, false, plan);
+    }
     if (cap64 > 0x7fffffffull)
         return fail(e, PMC_ERR_INVALID, "chunk_size * queue_factor exceeds the queue index range");
     const unsigned int cap = (unsigned int)cap64;
@@ -770,16 +777,33 @@ int ensure_maps(pmc_engine* e, int group, long long n_vox, int wave = 1) {
     return rc;
 }
 
-// As ensure_maps for the planned wave, one batch at a time where the device has
-// no room for the wave's maps.
-int ensure_wave_maps(pmc_engine* e, int group, long long n_vox, RunPlan* plan) {
-    int rc = ensure_maps(e, group, n_vox, plan->wave);
-    if (rc == PMC_ERR_OOM && plan->wave > 1) {
-        cudaGetLastError();
-        plan->wave = 1;
-        rc = ensure_maps(e, group, n_vox);
+// Run a transport call with its batches in waves; where the device has no room for
+// the wave's maps and queues (or for a call's beside those an earlier one left), or
+// the wave's window overflows queues that the caller sized, give that memory back and
+// run it batch by batch: what fits then is not refused because of the wave.
+template <typename Call>
+int with_waves(pmc_engine* e, Call call) {
+    e->shared = false;
+    e->reported = 0;
+    int rc = call(true);
+    if (rc != PMC_ERR_OOM && !(rc == PMC_ERR_QUEUE_OVERFLOW && e->shared)) return rc;
+    PMC_CUDA(e, cudaStreamSynchronize(e->stream));
+    for (DevBuf* b : {&e->queues, &e->edep, &e->s1, &e->s2, &e->dirty, &e->touched}) {
+        if (b->p) cudaFree(b->p);
+        *b = DevBuf{};
     }
+    e->q_capacity = e->q_slots = 0;
+    e->edep_clean = false;
+    cudaGetLastError();  // a refused allocation is no error of the launches that follow
+    rc = call(false);
+    if (rc == PMC_ERR_OOM) cudaGetLastError();
     return rc;
+}
+
+// `done` histories of the call are complete (a repeated part is reported once).
+void report(pmc_engine* e, long long done) {
+    if (e->progress && done > e->reported) e->progress(e->progress_user, done - e->reported);
+    e->reported = std::max(e->reported, done);
 }
 
 // Start scoring `group` columns: quanta all zero (cleared in bulk only after a
@@ -1376,18 +1400,16 @@ static int fill_gen_mask(pmc_engine* e, GenDesc& G, const MaskFields& f) {
     return upload_f32(e, m, &G.mask);
 }
 
-int pmc_run_forward(pmc_engine* e, const pmc_source_desc* src, const pmc_run_params* p,
-                    double* dose, double* dose_sigma, pmc_books* books) {
-    if (!e || !src || !p || !dose || !dose_sigma) return PMC_ERR_INVALID;
-    PMC_CUDA(e, cudaSetDevice(e->device));
+static int run_forward(pmc_engine* e, const pmc_source_desc* src, const pmc_run_params* p, bool waves,
+                       double* dose, double* dose_sigma, pmc_books* books) {
     if (p->n_histories < 1) return fail(e, PMC_ERR_INVALID, "need at least one history, got %lld", (long long)p->n_histories);
     if (p->n_batches < 1 || p->n_histories % p->n_batches != 0)
         return fail(e, PMC_ERR_INVALID, "n_histories=%lld not divisible by n_batches=%d", (long long)p->n_histories, p->n_batches);
     RunPlan plan;
-    int rc = prepare_transport(e, p, (unsigned long long)(p->n_histories / p->n_batches), 1, true, &plan);
+    int rc = prepare_transport(e, p, (unsigned long long)(p->n_histories / p->n_batches), 1, waves, &plan);
     if (rc) return rc;
     const long long n_vox = e->si.n_voxels;
-    rc = ensure_wave_maps(e, 1, n_vox, &plan);
+    rc = ensure_maps(e, 1, n_vox, plan.wave);
     if (rc) return rc;
     rc = ensure(e, e->col_nhist, sizeof(double));
     if (rc) return rc;
@@ -1539,7 +1561,7 @@ int pmc_run_forward(pmc_engine* e, const pmc_source_desc* src, const pmc_run_par
         cudaEventElapsedTime(&c, e->ev[1], e->ev[2]);
         t_tr += a;
         t_red += c;
-        for (int k = 0; k < in_wave && e->progress; ++k) e->progress(e->progress_user, per_batch);
+        for (int k = 1; k <= in_wave; ++k) report(e, per_batch * (b + k));
     }
     if (!one_wave) {
         rc = launch_finalize(e, n_vox, 1, p->n_batches);
@@ -1558,7 +1580,7 @@ int pmc_run_forward(pmc_engine* e, const pmc_source_desc* src, const pmc_run_par
     if (one_wave) {
         cudaEventElapsedTime(&t_tr, e->ev[0], e->ev[1]);
         cudaEventElapsedTime(&c, e->ev[1], e->ev[2]);
-        for (int k = 0; k < p->n_batches && e->progress; ++k) e->progress(e->progress_user, per_batch);
+        for (int k = 1; k <= p->n_batches; ++k) report(e, per_batch * k);
     } else {
         cudaEventElapsedTime(&c, e->ev[2], e->ev[3]);
     }
@@ -1567,10 +1589,15 @@ int pmc_run_forward(pmc_engine* e, const pmc_source_desc* src, const pmc_run_par
     return finish_counters(e, books);
 }
 
-int pmc_run_dij(pmc_engine* e, const pmc_beamlet_desc* src, const int64_t* counts,
-                const pmc_run_params* p, int64_t* nnz_out, pmc_books* books) {
-    if (!e || !src || !counts || !p || !nnz_out) return PMC_ERR_INVALID;
+int pmc_run_forward(pmc_engine* e, const pmc_source_desc* src, const pmc_run_params* p,
+                    double* dose, double* dose_sigma, pmc_books* books) {
+    if (!e || !src || !p || !dose || !dose_sigma) return PMC_ERR_INVALID;
     PMC_CUDA(e, cudaSetDevice(e->device));
+    return with_waves(e, [&](bool waves) { return run_forward(e, src, p, waves, dose, dose_sigma, books); });
+}
+
+static int run_dij(pmc_engine* e, const pmc_beamlet_desc* src, const int64_t* counts, const pmc_run_params* p,
+                   bool waves, int64_t* nnz_out, pmc_books* books) {
     const int n_beam = src->n_beamlets;
     if (n_beam < 1) return fail(e, PMC_ERR_INVALID, "need at least one beamlet");
     if (p->n_batches < 1) return fail(e, PMC_ERR_INVALID, "need at least one batch");
@@ -1586,7 +1613,7 @@ int pmc_run_dij(pmc_engine* e, const pmc_beamlet_desc* src, const int64_t* count
     const int all_cols = std::min(n_beam, 4096);
     const int most_cols = p->beamlet_group_size > 0 ? std::min(n_beam, p->beamlet_group_size) : all_cols;
     // (host-sampled primaries are uploaded batch by batch: no waves)
-    int rc = prepare_transport(e, p, all_block, most_cols, src->type != PMC_BEAMLET_UPLOAD, &plan);
+    int rc = prepare_transport(e, p, all_block, most_cols, waves && src->type != PMC_BEAMLET_UPLOAD, &plan);
     if (rc) return rc;
     const long long n_vox = e->si.n_voxels;
     int group = p->beamlet_group_size > 0 ? p->beamlet_group_size : 0;
@@ -1610,7 +1637,7 @@ int pmc_run_dij(pmc_engine* e, const pmc_beamlet_desc* src, const int64_t* count
         group = std::min(group, std::min(n_beam, 4096));
     }
     group = std::min(group, n_beam);
-    rc = ensure_wave_maps(e, group, n_vox, &plan);
+    rc = ensure_maps(e, group, n_vox, plan.wave);
     if (!rc) rc = ensure(e, e->col_nhist, sizeof(double) * group);
     if (rc) return rc;
     // Every in-kernel beamlet source becomes per-beamlet records; the upload
@@ -1770,17 +1797,22 @@ int pmc_run_dij(pmc_engine* e, const pmc_beamlet_desc* src, const int64_t* count
         cudaEventElapsedTime(&c0, e->ev[0], e->ev[1]);  // finalize (count+scan ride in the
         cudaEventElapsedTime(&c1, e->ev[2], e->ev[3]);  // synchronizing read; tiny kernels)
         t_red += c0 + c1;
-        if (e->progress) {
-            long long done = 0;
-            for (int k = 0; k < gs; ++k) done += counts[g0 + k];
-            e->progress(e->progress_user, done);
-        }
+        long long done = 0;
+        for (int k = 0; k < g0 + gs; ++k) done += counts[k];
+        report(e, done);
     }
     free_run_allocs(e);
     e->counters.transport_ms = t_tr;
     e->counters.reduce_ms = t_red;
     *nnz_out = (int64_t)e->csc_nnz;
     return finish_counters(e, books);
+}
+
+int pmc_run_dij(pmc_engine* e, const pmc_beamlet_desc* src, const int64_t* counts,
+                const pmc_run_params* p, int64_t* nnz_out, pmc_books* books) {
+    if (!e || !src || !counts || !p || !nnz_out) return PMC_ERR_INVALID;
+    PMC_CUDA(e, cudaSetDevice(e->device));
+    return with_waves(e, [&](bool waves) { return run_dij(e, src, counts, p, waves, nnz_out, books); });
 }
 
 int pmc_dij_fetch(pmc_engine* e, int64_t* indptr, int64_t* indices, double* dose, double* sigma) {
