@@ -287,6 +287,22 @@ def _kept(code: int, count) -> int:
     return int(count.value)
 
 
+def _column(values, n: int, key: str):
+    """The first n values of a source's column as a tensor on the host: read where they
+    are if torch can (any forward stride), else a copy rounded to float32."""
+    import torch
+
+    a = np.asarray(values).reshape(-1)
+    if a.size < n:
+        raise ValueError(f"the source sampled {a.size} values of {key!r} for {n} primaries")
+    a = a[:n]
+    step = a.strides[0]
+    if (a.dtype not in (np.float64, np.float32) or not (a.flags.writeable and a.flags.aligned)
+            or step < 0 or step % a.itemsize):
+        a = np.array(a, dtype=np.float32)
+    return torch.from_numpy(a)
+
+
 def _presolve_on_device(lib, cs, mu, params, columns, n: int, capacity: int, device, count, dropped,
                         max_energy: float) -> DevicePhaseSpace:
     """The pre-solve with its population left in device tensors: the primaries'
@@ -300,12 +316,7 @@ def _presolve_on_device(lib, cs, mu, params, columns, n: int, capacity: int, dev
     with torch.cuda.device(device):
         host = torch.empty((8, n), dtype=torch.float32, pin_memory=True)
         for i, key in enumerate(("energy", "x", "y", "z", "ux", "uy", "uz", "weight")):
-            a = np.asarray(columns[key]).reshape(-1)
-            if a.size < n:
-                raise ValueError(f"the source sampled {a.size} values of {key!r} for {n} primaries")
-            if a.dtype not in (np.float64, np.float32) or not a.flags.writeable:
-                a = a.astype(np.float32)
-            host[i].copy_(torch.from_numpy(a[:n]))
+            host[i].copy_(_column(columns[key], n, key))
         empty = lambda *shape, dtype=torch.float32: torch.empty(shape, dtype=dtype, device=device)  # noqa: E731
         kind, energy, weight = empty(capacity, dtype=torch.int32), empty(capacity), empty(capacity)
         pos, dirs = empty(capacity, 3), empty(capacity, 3)

@@ -87,3 +87,38 @@ def test_descriptors_from_pyradmc_objects_equal_the_fixture():
     np.testing.assert_allclose(mu.log_energy, g["mu_log_energy"], rtol=0, atol=1e-12)
     np.testing.assert_allclose(mu.log_total, g["mu_log_total"], rtol=0, atol=1e-12)
     np.testing.assert_allclose(mu.log_compton, g["mu_log_compton"], rtol=0, atol=1e-12)
+
+
+def _forms():
+    """One column's float64 values in every form a source may hold them in."""
+    v = np.random.default_rng(5).normal(size=7)
+    packed = np.zeros(7, dtype=[("flag", "u1"), ("x", "<f8")])
+    packed["x"] = v
+    unaligned = np.frombuffer(b"\0" + v.tobytes(), dtype=np.uint8)[1:].copy()
+    shifted = np.empty(8 * 7 + 1, dtype=np.uint8)[1:]
+    shifted[:] = unaligned
+    frozen = v.copy()
+    frozen.flags.writeable = False
+    return v, {
+        "plain": v, "reversed": v[::-1].copy()[::-1], "strided": np.repeat(v, 3)[::3],
+        "column of a matrix": np.column_stack([v, v + 1])[:, 0], "packed record": packed["x"],
+        "unaligned": shifted.view(np.float64), "big endian": v.astype(">f8"), "read only": frozen, "list": list(v),
+        "matrix": v.reshape(7, 1), "long double": v.astype(np.longdouble), "longer": np.append(v, 9.0)}
+
+
+@pytest.mark.parametrize("form", sorted(_forms()[1]))
+def test_columns_of_every_form_are_rounded_alike(form):
+    """What numpy's contiguous float32 copy takes, the device hand-off takes too."""
+    import torch
+
+    v, forms = _forms()
+    got = torch.empty(7, dtype=torch.float32)
+    got.copy_(PS._column(forms[form], 7, "x"))
+    np.testing.assert_array_equal(got.numpy(), v.astype(np.float32))
+
+
+def test_other_column_types_and_a_short_column():
+    for a in (np.arange(5), np.arange(5, dtype=np.float32)[::-1], np.broadcast_to(np.float32(2.5), 5)):
+        np.testing.assert_array_equal(PS._column(a, 5, "weight").numpy(), a.astype(np.float32))
+    with pytest.raises(ValueError, match="sampled 4 values of 'x' for 5"):
+        PS._column(np.zeros(4), 5, "x")
