@@ -161,12 +161,23 @@ __device__ __forceinline__ unsigned int claim_parts(const FoldShape& f) {
 // of x r, each with an exact remainder (Markstein, "Computation of elementary
 // functions on the IBM RISC System/6000 processor", IBM J. Res. Dev. 34, 1990: the
 // second one rounds correctly, the first having left a quotient within one unit in
-// the last place).  Finite operands away from the ends of the exponent range, or
-// y = r = 0, which gives 0.
+// the last place).  For y = r = 0 it gives 0; else y must be a usual divisor: with
+// dividends of 0 or 1e-9 to 1e10 no step then overflows or loses bits.
+__device__ __forceinline__ bool usual_divisor(double y) { return y >= 0x1p-900 && y <= 0x1p900; }
 __device__ __forceinline__ double divide_by(double x, double y, double r) {
     double q = __dmul_rn(x, r);
     q = __fma_rn(__fma_rn(-q, y, x), r, q);
     return __fma_rn(__fma_rn(-q, y, x), r, q);
+}
+
+// *odd = 1 where some mass times a count of histories (1 to 2^100) is no usual divisor
+// (no mass at all is none that the fold divides by).
+__global__ void odd_masses_kernel(const double* __restrict__ mass, long long n, unsigned int* odd) {
+    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n;
+         i += (long long)gridDim.x * blockDim.x) {
+        const double m = mass[i];
+        if (m > 0.0 && !(usual_divisor(m) && usual_divisor(m * 0x1p100))) *odd = 1u;
+    }
 }
 
 // Fold a wave's quanta maps, batch by batch, into the running sums and consume
@@ -181,9 +192,11 @@ __device__ __forceinline__ double divide_by(double x, double y, double r) {
 // of scattered 32-byte sectors, some 1e7 of them per wave of the 100-column 128^3
 // Dij, then the issue of the float64 arithmetic (one reciprocal per entry instead
 // of a division per entry and batch).
+// kDivide: masses that no tissue has (infinite, say) are divided by as they are; in
+// one kernel with the reciprocal the division's registers spill (2.17 -> 2.35 ms).
 constexpr int kWaveMaps = 32;  // the most maps of a wave
 
-template <bool kFinal>
+template <bool kFinal, bool kDivide>
 __global__ void __launch_bounds__(kReduceThreads, 4)
 fold_sparse_kernel(unsigned long long* __restrict__ edep, const double* __restrict__ mass,
                    const double* __restrict__ col_nhist, FoldShape f, double* __restrict__ s1,
@@ -245,17 +258,24 @@ fold_sparse_kernel(unsigned long long* __restrict__ edep, const double* __restri
             }
             if (v < f.n_vox) y.x = mass[v];
             if (v + 1 < f.n_vox) y.y = mass[v + 1];
-            y.x = y.x > 0.0 ? __dmul_rn(y.x, nh) : 0.0;
-            y.y = y.y > 0.0 ? __dmul_rn(y.y, nh) : 0.0;
-            const double rx = y.x > 0.0 ? __drcp_rn(y.x) : 0.0, ry = y.y > 0.0 ? __drcp_rn(y.y) : 0.0;
+            const bool some_x = y.x > 0.0, some_y = y.y > 0.0;  // no mass: no dose
+            y.x = some_x ? __dmul_rn(y.x, nh) : 0.0;
+            y.y = some_y ? __dmul_rn(y.y, nh) : 0.0;
+            const double rx = !kDivide && y.x > 0.0 ? __drcp_rn(y.x) : 0.0;
+            const double ry = !kDivide && y.y > 0.0 ? __drcp_rn(y.y) : 0.0;
+            auto dose = [](unsigned long long quanta, bool some, double by, double r) {
+                const double energy = __dmul_rn((double)(long long)quanta, kQuantum);
+                if constexpr (kDivide) return some && quanta != 0ull ? __ddiv_rn(energy, by) : 0.0;
+                else return divide_by(energy, by, r);
+            };
             for (;;) {
                 maps &= maps - 1u;
                 ulonglong2* const next_at = maps ? quanta(maps) : q_at;
                 ulonglong2 q_next = q;
                 if (maps) q_next = *next_at;
                 if ((q.x | q.y) != 0ull) *q_at = make_ulonglong2(0ull, 0ull);
-                const double dx = divide_by(__dmul_rn((double)(long long)q.x, kQuantum), y.x, rx);
-                const double dy = divide_by(__dmul_rn((double)(long long)q.y, kQuantum), y.y, ry);
+                const double dx = dose(q.x, some_x, y.x, rx);
+                const double dy = dose(q.y, some_y, y.y, ry);
                 a.x = __dadd_rn(a.x, dx);
                 a.y = __dadd_rn(a.y, dy);
                 b.x = __dadd_rn(b.x, __dmul_rn(dx, dx));

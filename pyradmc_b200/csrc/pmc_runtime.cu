@@ -82,6 +82,7 @@ struct pmc_engine {
     float* d_cyl_r2 = nullptr;
     bool custom_scoring = false;
     double* d_mass = nullptr;
+    bool odd_masses = false;      // some mass x histories is no usual divisor (pmc_reduce.cuh)
     size_t mass_cap = 0;
     long long mass_len = 0;
 
@@ -453,6 +454,19 @@ struct RunPlan {
     int tail_steps = 0;
 };
 
+// Which fold the masses in e->d_mass take; waits for the stream.
+int find_odd_masses(pmc_engine* e, long long n) {
+    unsigned int odd = 0;
+    PMC_CUDA(e, cudaMemsetAsync(e->d_fold_next, 0, sizeof odd, e->stream));
+    odd_masses_kernel<<<grid_blocks(n), 256, 0, e->stream>>>(e->d_mass, n, e->d_fold_next);
+    PMC_CUDA(e, cudaGetLastError());
+    PMC_CUDA(e, cudaMemcpyAsync(&odd, e->d_fold_next, sizeof odd, cudaMemcpyDeviceToHost, e->stream));
+    e->d2h_bytes += sizeof odd;
+    PMC_CUDA(e, cudaStreamSynchronize(e->stream));
+    e->odd_masses = odd != 0;
+    return PMC_OK;
+}
+
 long long stride_for(long long n_vox) {
     return (n_vox + kTileVoxels - 1) / kTileVoxels * kTileVoxels;
 }
@@ -661,7 +675,8 @@ int launch_fold(pmc_engine* e, long long n_vox, int group, const double* d_col_n
     FoldShape f{};
     const int rc = fold_shape(e, n_vox, group, n_maps, &f);
     if (rc) return rc;
-    auto kernel = last ? fold_sparse_kernel<true> : fold_sparse_kernel<false>;
+    auto kernel = e->odd_masses ? (last ? fold_sparse_kernel<true, true> : fold_sparse_kernel<false, true>)
+                                : (last ? fold_sparse_kernel<true, false> : fold_sparse_kernel<false, false>);
     kernel<<<fold_blocks(e, f), kReduceThreads, 0, e->stream>>>(
         (unsigned long long*)e->edep.p, e->d_mass, d_col_nhist, f, (double*)e->s1.p, (double*)e->s2.p,
         (unsigned int*)e->dirty.p, (unsigned int*)e->touched.p, n_batches, e->d_colmax, e->d_total_q);
@@ -1093,6 +1108,8 @@ int pmc_upload_grid(pmc_engine* e, int32_t nx, int32_t ny, int32_t nz, const dou
                                                                default_mass ? e->d_mass : nullptr);
     PMC_CUDA(e, cudaGetLastError());
     PMC_CUDA(e, cudaStreamSynchronize(e->stream));
+    if (default_mass) rc = find_odd_masses(e, n);
+    if (rc) return rc;
     e->gi = make_grid(nx, ny, nz, origin, spacing);
     e->has_grid = true;
     e->max_material = max_mat;
@@ -1120,7 +1137,7 @@ int pmc_set_scoring(pmc_engine* e, const pmc_scoring_desc* s) {
         PMC_CUDA(e, cudaGetLastError());
         PMC_CUDA(e, cudaStreamSynchronize(e->stream));
         e->mass_len = n;
-        return PMC_OK;
+        return find_odd_masses(e, n);
     }
     if (!s->voxel_mass) return fail(e, PMC_ERR_INVALID, "invalid scoring grid");
     long long n = 0;
@@ -1168,11 +1185,11 @@ int pmc_set_scoring(pmc_engine* e, const pmc_scoring_desc* s) {
     }
     int rc_mass = ensure_ptr(e, e->d_mass, e->mass_cap, sizeof(double) * (size_t)n);
     if (rc_mass) return rc_mass;
-    PMC_CUDA(e, cudaMemcpy(e->d_mass, s->voxel_mass, sizeof(double) * n, cudaMemcpyHostToDevice));
+    PMC_CUDA(e, cudaMemcpyAsync(e->d_mass, s->voxel_mass, sizeof(double) * n, cudaMemcpyHostToDevice, e->stream));
     e->h2d_bytes += (unsigned long long)(sizeof(double) * n);
     e->mass_len = n;
     e->custom_scoring = true;
-    return PMC_OK;
+    return find_odd_masses(e, n);
 }
 
 int pmc_upload_tables(pmc_engine* e, const pmc_tables_desc* t) {
@@ -1876,12 +1893,17 @@ int pmc_reduce_dense(pmc_engine* e, const int64_t* quanta, int32_t n_batches, in
     double* saved_mass = e->d_mass;
     double* mass = nullptr;
     PMC_CUDA(e, cudaMalloc(&mass, sizeof(double) * n_vox));
-    PMC_CUDA(e, cudaMemcpy(mass, voxel_mass, sizeof(double) * n_vox, cudaMemcpyHostToDevice));
+    PMC_CUDA(e, cudaMemcpyAsync(mass, voxel_mass, sizeof(double) * n_vox, cudaMemcpyHostToDevice, e->stream));
     e->h2d_bytes += (unsigned long long)(sizeof(double) * n_vox);
-    PMC_CUDA(e, cudaMemcpy(e->col_nhist.p, histories_per_batch, sizeof(double) * n_cols, cudaMemcpyHostToDevice));
+    PMC_CUDA(e, cudaMemcpyAsync(e->col_nhist.p, histories_per_batch, sizeof(double) * n_cols, cudaMemcpyHostToDevice,
+                                e->stream));
     e->h2d_bytes += (unsigned long long)(sizeof(double) * n_cols);
     e->d_mass = mass;
-    rc = begin_maps(e, n_cols);
+    const bool saved_odd = e->odd_masses;
+    rc = find_odd_masses(e, n_vox);
+    e->odd_masses = e->odd_masses || !std::all_of(histories_per_batch, histories_per_batch + n_cols,
+                                                  [](double n) { return n >= 1.0 && n <= 0x1p100; });
+    if (!rc) rc = begin_maps(e, n_cols);
     PMC_CUDA(e, cudaMemsetAsync(e->d_total_q, 0, sizeof(unsigned long long), e->stream));
     const size_t row = sizeof(int64_t) * (size_t)n_vox, pitch = sizeof(int64_t) * (size_t)e->col_stride;
     for (int b = 0; b < n_batches && !rc; ++b) {
@@ -1900,6 +1922,7 @@ int pmc_reduce_dense(pmc_engine* e, const int64_t* quanta, int32_t n_batches, in
         if (cudaStreamSynchronize(e->stream) == cudaSuccess) e->edep_clean = true;
     }
     e->d_mass = saved_mass;
+    e->odd_masses = saved_odd;
     cudaFree(mass);
     if (total_quanta) *total_quanta = (int64_t)tq;
     if (rc) return rc;
