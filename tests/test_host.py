@@ -4,9 +4,11 @@ with the reference's exception types and messages (engine.py:512-550,
 
 from __future__ import annotations
 
+import numpy as np
 import pytest
 
 import pyradmc_b200 as P
+from pyradmc_b200.engine import _Block, _ResultArrays
 
 
 @pytest.fixture
@@ -80,3 +82,51 @@ def test_spectrum_mirror_matches_the_packed_reference_cdf():
         assert np.array_equal(spec.cdf, z["cdf"])
     assert spec.max_energy == pytest.approx(5.76)
     assert 1.4 < spec.mean_energy < 1.8
+
+
+class _PlainBlock(_Block):
+    """Stands for a page-locked block where there is no GPU."""
+
+    @staticmethod
+    def _allocate(n):
+        import torch
+
+        return torch.empty(n, dtype=torch.float64)
+
+
+class _RefusedBlock(_Block):
+    @staticmethod
+    def _allocate(n):
+        raise RuntimeError("no page-locked memory")
+
+
+def _is_block(a):
+    while isinstance(a, np.ndarray) and a.base is not None:
+        a = a.base
+    return isinstance(a, _PlainBlock)
+
+
+def test_results_that_are_kept_lock_a_bounded_amount_of_host_memory():
+    n = 1 << 16  # 1 MB a result
+    arrays = _ResultArrays(4 << 20, _PlainBlock)
+    kept = [tuple(a.reshape(256, 256) for a in arrays.pair(n)) for _ in range(6)]  # as a result holds them
+    assert [_is_block(a) and _is_block(b) for a, b in kept] == [True] * 4 + [False] * 2
+    kept[0][0][:] = 1.0
+    assert kept[0][0].sum() == n and kept[1][0].flags.writeable
+    kept[1] = kept[1][0]  # a sigma dropped: its half is free, a whole result is not
+    assert not _is_block(arrays.pair(n)[0])
+    kept[1] = None
+    assert _is_block(arrays.pair(n)[0])
+    kept.clear()
+    assert all(_is_block(arrays.pair(n)[0]) for _ in range(9))  # dropped at once: always a block
+    big = arrays.pair(8 * n)  # above the limit: one at a time
+    assert _is_block(big[0]) and not _is_block(arrays.pair(8 * n)[0]) and not _is_block(arrays.pair(n)[0])
+    del big
+    assert not _is_block(arrays.pair(100)[0])  # small ones are plain
+
+
+def test_results_without_page_locked_memory_are_plain():
+    arrays = _ResultArrays(4 << 20, _RefusedBlock)
+    kept = [arrays.pair(1 << 16) for _ in range(3)]
+    assert all(a.shape == b.shape == (1 << 16,) for a, b in kept)
+    assert arrays._alive == 0
