@@ -367,10 +367,15 @@ int pmc_get_counters(const pmc_engine* engine, pmc_counters* counters);
  * engine's private stream. */
 int pmc_set_stream(pmc_engine* engine, void* stream);
 
-/* Progress: fn(user, histories) is called from the calling thread after each
+/* Progress: fn(user, histories) is called from the calling thread for each
  * completed batch of pmc_run_forward and each completed beamlet group of
- * pmc_run_dij, with the histories that completed (progress.py:71 tick).  A
- * NULL fn disables it. */
+ * pmc_run_dij, with the histories that completed (progress.py:71 tick).
+ * Batches that are transported together complete together: their calls follow
+ * one another, after the results where they are all of the run's.  Together
+ * are at most 64 primaries per resident thread (1e7 on this GPU, some tens of
+ * milliseconds); larger batches are each reported when they are done.  (A
+ * rate is the histories over the time since the call began, not between two
+ * calls.)  A NULL fn disables it. */
 typedef void (*pmc_progress_fn)(void* user, int64_t histories);
 int pmc_set_progress(pmc_engine* engine, pmc_progress_fn fn, void* user);
 

@@ -40,3 +40,19 @@ def test_waves_give_the_same_run(gpu, shape, n_batches):
     dij = P.B200Engine(grid, xs, device=gpu).run_dij(P.BeamletGridSource(6.0, -1.0, (0.0, x), (0.0, y), 1, 1),
                                                      500 * n_batches, n_batches, 3, truncation=0.0)
     assert np.array_equal(dij.column_dense(0), run.dose) and np.array_equal(dij.sigma_dense(0), run.dose_sigma)
+
+
+def test_progress_of_batches_that_complete_together_and_one_by_one(gpu):
+    """One call a batch either way; batches above a wave's 64 primaries per resident
+    thread are reported as each is done, not at the end."""
+    grid = P.VoxelGrid.uniform_water((8, 8, 8), (0.5, 0.5, 0.5))
+    engine = P.B200Engine(grid, P.AnalyticWaterTables(geometry_densities=grid.max_density_by_material()), device=gpu)
+    src = P.ParallelBeamSource(6.0, -1.0, (0.0, 4.0), (0.0, 4.0))
+    events = []
+    engine.run(src, 700, 7, 3, progress=events.append)
+    assert [e.histories_done for e in events] == [100 * k for k in range(1, 8)]
+    events.clear()
+    engine.run(src, 48_000_000, 4, 3, progress=events.append)
+    assert [e.histories_done for e in events] == [12_000_000 * k for k in range(1, 5)]
+    elapsed = [e.elapsed_s for e in events]
+    assert elapsed[0] < 0.7 * elapsed[-1] and elapsed[1] < 0.9 * elapsed[-1]
