@@ -905,8 +905,8 @@ bool umma_plan(const ConvShape& s, UmmaConv& u, int& smem, int& ctas_per_sm) {
 bool umma_pipe_plan(const ConvShape& s, UmmaConv& u, int& smem, int& ctas_per_sm) {
     int base_smem = 0, base_per_sm = 0;
     if (!umma_plan(s, u, base_smem, base_per_sm) || u.passes != 1) return false;
-    const int extra = 16;
-    smem = 2 * ((int)u.halo_bytes + kUSlack) + (int)u.w_chunks * s.cout * 16 + (int)u.k_steps * 16 + extra;
+    const int extra = 16;  // mbarrier + tensor-memory address
+    smem = 2 * ((int)u.halo_bytes + kUSlack) + (int)u.w_chunks * s.cout * 16 + extra;
     if (smem > kSmemPerBlockMax || 2 * u.tz * s.cout > 512) return false;
     unsigned cols = 32;
     while (cols < (unsigned)(2 * u.tz * s.cout)) cols <<= 1;
@@ -1272,13 +1272,11 @@ int try_ws(const __nv_bfloat16* x, const __nv_bfloat16* w, const float* bias, __
     if (!ws_plan(s, p, smem, per_sm, head.w != nullptr)) return -1;
     p.split = (s.cin - c_skip) / 8;
     if (!ws_tensor_maps(x, skip, w, p, xm, sm, wm)) return -1;
-    switch (p.cg) {
+    switch (p.cg) {  // no plan takes other groups: two blocks per SM, or three stages, come first
         case 1: code = launch_ws<1>(xm, sm, wm, w, bias, y, p, smem, per_sm, relu, st, head); return 1;
         case 2: code = launch_ws<2>(xm, sm, wm, w, bias, y, p, smem, per_sm, relu, st, head); return 1;
         case 4: code = launch_ws<4>(xm, sm, wm, w, bias, y, p, smem, per_sm, relu, st, head); return 1;
         case 6: code = launch_ws<6>(xm, sm, wm, w, bias, y, p, smem, per_sm, relu, st, head); return 1;
-        case 8: code = launch_ws<8>(xm, sm, wm, w, bias, y, p, smem, per_sm, relu, st, head); return 1;
-        case 12: code = launch_ws<12>(xm, sm, wm, w, bias, y, p, smem, per_sm, relu, st, head); return 1;
         default: return -1;
     }
 }

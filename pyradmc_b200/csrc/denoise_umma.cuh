@@ -223,10 +223,12 @@ __device__ __forceinline__ void umma_issue_slice(uint32_t d, uint64_t as, uint64
 // each output slice has its 14 MMAs to itself (pairs within a slice would be 15, and
 // another order of the sum).
 //
-// The slice loop is not unrolled: with the 14 or 27 MMAs of a slice unrolled in full
-// for CG = 1 and 2, an earlier build computed wrong sums (tested against the
-// oracle); nine are exact for every CG.  accumulate: whether the first K step adds to
-// the accumulator (a later channel group of the same tile).
+// The slice loop is not unrolled: an earlier form of this loop, one lane issuing under a
+// branch, computed wrong sums (against the oracle) where the 14 or 27 MMAs of a slice
+// were unrolled in full for CG = 1 and 2.  The cause was not found.  A slice here is 7 + 7
+// MMAs in a row for CG = 1 and 9 CG / 2 for the others (9, 18, 27, 36, 54), issued by the
+// whole warp; every CG is compared with the oracle.  accumulate: whether the first K step
+// adds to the accumulator (a later channel group of the same tile).
 template <int CG>
 __device__ __forceinline__ void umma_issue_taps(uint32_t d0, uint32_t a_addr, uint32_t plane_bytes,
                                                 uint32_t b_addr, int N, int tz, bool accumulate,
@@ -551,8 +553,7 @@ conv3d_umma_pipe_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16
     const unsigned buf_stride = u.halo_bytes + kUSlack;  // halo + its zeroed slack
     unsigned char* halo0 = smem;
     unsigned char* wbuf = smem + 2 * buf_stride;
-    uint64_t* dtab = reinterpret_cast<uint64_t*>(wbuf + (size_t)u.w_chunks * N * 16);
-    uint64_t* mbar_p = dtab + 2 * u.k_steps;
+    uint64_t* mbar_p = reinterpret_cast<uint64_t*>(wbuf + (size_t)u.w_chunks * N * 16);
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(mbar_p + 1);
     const uint32_t halo_s = smem_u32(halo0), w_s = smem_u32(wbuf), mbar = smem_u32(mbar_p);
 
@@ -573,7 +574,7 @@ conv3d_umma_pipe_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16
     const uint32_t tmem = *tmem_slot;
     const uint32_t acc_cols = (uint32_t)(u.tz * N);
 
-    // resident weights and the descriptor table (A relative to buffer 0)
+    // resident weights
     const int n_chunks = (int)u.w_chunks;
     for (int i = tid; i < n_chunks * N; i += blockDim.x) {
         const int n = i % N, jj = i / N;
@@ -587,7 +588,7 @@ conv3d_umma_pipe_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16
     int failed = 0, i = 0, prev = -1;
     for (int tile = blockIdx.x; tile < u.n_tiles; tile += gridDim.x, ++i) {
         const int b = i & 1;
-        // this tile's halo (and, first time, the weights and table) has landed
+        // this tile's halo (and, first time, the weights) has landed
         cp_async_wait<0>();
         fence_async_smem();
         tc_fence_before();

@@ -387,6 +387,14 @@ def test_tensor_memory_convolution_matches_oracle(gpu, shape):
         np.testing.assert_array_equal(outs[4], outs[2])
 
 
+# the channel groups whose MMAs no shape above issues in one pass: 36 and 54 of them in
+# a row for each halo slice (8 and 12 chunks; 7 + 7, 9, 18 and 27 are among UMMA_SHAPES)
+@pytest.mark.parametrize("shape", [(2, 5, 17, 9, 64, 16), (1, 3, 33, 10, 96, 16)])
+def test_tensor_memory_convolution_of_the_widest_groups_matches_oracle(gpu, shape):
+    assert _umma_single_pass(*shape[4:])
+    test_tensor_memory_convolution_matches_oracle(gpu, shape)
+
+
 # runs along d: several per block (windows x tiles above two blocks an SM), odd and
 # short depths, one and several channel groups, an accumulator ring of 4 and of 8
 @pytest.mark.parametrize("shape", [(40, 7, 40, 20, 16, 16), (34, 1, 40, 24, 16, 32), (34, 9, 40, 24, 32, 32),
