@@ -1061,8 +1061,8 @@ def b200_arm(args, world, rank, local):
                 "what": "transport is bounded by instruction issue and load latency, not HBM: "
                         "fraction of cycles each SM sub-partition issued, ncu on a main round "
                         "of a Dij on this phantom",
-                "photon_kernel": 0.607, "electron_kernel": 0.571,
-                "simd_lanes_active": {"photon_kernel": 10.6 / 32, "electron_kernel": 20.4 / 32},
+                "photon_kernel": 0.600, "electron_kernel": 0.570,
+                "simd_lanes_active": {"photon_kernel": 11.6 / 32, "electron_kernel": 20.4 / 32},
                 "source": "profiles/transport_main_round_dij100_ncu.md"},
             "algorithmic_bytes": algorithmic_bytes(c),
             "transport_ms": c["transport_ms"],
@@ -1075,8 +1075,50 @@ def b200_arm(args, world, rank, local):
         "clocks": clock,
         "cpu_baseline": base,
     }
-    print(json.dumps(line), flush=True)
+    report(line)
     return 0
+
+
+def short_line(full: dict) -> dict:
+    """The record that is printed.  Of 25 KB, which a reader that keeps the output's last
+    16 cannot parse, it leaves out the denoiser's ladder and its regions' error tables (a
+    region keeps its own error and bias), the plan's ladder but for the errors, and the
+    parity records but for the smallest p; nested floats have seven digits."""
+    line = dict(full)
+    if line["denoiser"]:
+        d = line["denoiser"] = {k: v for k, v in line["denoiser"].items()
+                                if k not in ("ladder", "plain_at_benchmark_counts", "windows_tried")}
+        d["regions"] = {
+            name: {**{k: v for k, v in r.items() if k not in ("denoised", "plain_same_histories", "candidates")},
+                   **{k: r["denoised"][name][k] for k in ("sigma_eq", "bias_integral")}}
+            for name, r in d.get("regions", {}).items()}
+    if line["plan"] and line["plan"].get("denoiser"):
+        line["plan"] = dict(line["plan"])
+        d = line["plan"]["denoiser"] = dict(line["plan"]["denoiser"])
+        d["ladder"] = [[r["fraction_of_plain"], r["denoised"]["0.5"]["sigma_eq"]] for r in d.get("ladder", [])]
+    if line["parity"] and line["parity"].get("records"):
+        line["parity"] = {**{k: v for k, v in line["parity"].items() if k != "records"},
+                          "min_p": min(r["p"] for r in line["parity"]["records"])}
+
+    def digits(v):
+        if isinstance(v, dict):
+            return {k: digits(x) for k, x in v.items()}
+        if isinstance(v, (list, tuple)):
+            return [digits(x) for x in v]
+        return float(f"{v:.7g}") if isinstance(v, float) else v
+
+    return {k: v if isinstance(v, float) else digits(v) for k, v in line.items()}
+
+
+def report(full: dict) -> None:
+    """Print the line; the whole record goes to $PMC_BENCH_REPORT (.parity/bench.json)."""
+    path = Path(os.environ.get("PMC_BENCH_REPORT", ROOT / ".parity" / "bench.json"))
+    try:
+        path.parent.mkdir(parents=True, exist_ok=True)
+        path.write_text(json.dumps(full))
+    except OSError as e:
+        print(f"no full record: {e}", file=sys.stderr)
+    print(json.dumps(short_line(full)), flush=True)
 
 
 def main() -> int:
