@@ -199,3 +199,41 @@ def test_engine_waits_for_the_stream_that_makes_the_device_phase_space(gpu):
         got = engine.run(late, n_histories=40_000, n_batches=4, seed=case.SEED)
     np.testing.assert_array_equal(got.dose, want.dose)
     assert got.energy_emitted == want.energy_emitted
+
+
+def test_c_entry_with_outputs_on_the_device_equals_that_with_host_outputs(gpu):
+    """pmc_presolve_head(outputs_on_device): host records in, device arrays out."""
+    import ctypes as C
+
+    import torch
+
+    from pyradmc_b200 import _lib
+
+    g, n, lib = golden(), 5_000, _lib.load()
+    stack = compiled(g, "s1")
+    cs, (mu, keep) = stack.to_c(), _mu(g).to_c()
+    c = case.FanSource().sample_batch(case.SEED, 0, n)
+    f32 = lambda *k: np.ascontiguousarray(np.column_stack([c[i] for i in k]), dtype=np.float32)  # noqa: E731
+    ins = [f32("energy"), f32("x", "y", "z"), f32("ux", "uy", "uz"), f32("weight")]
+
+    def call(on_device):
+        params = _lib.HeadParams(first_compton=1, has_air=0, air_row=0, air_z_start=0.0, air_z_end=0.0,
+                                 exit_z=case.EXIT_Z, pcut=0.05, ecut=0.2, weight_floor=1e-3, seed=case.SEED,
+                                 outputs_on_device=on_device)
+        outs = [torch.zeros(2 * n, dtype=torch.int32)] + [torch.zeros(2 * n * w) for w in (1, 3, 3, 1)]
+        outs = [t.to(gpu) if on_device else t for t in outs]
+        if on_device:
+            torch.cuda.synchronize(gpu)
+        ptr = lambda t: C.cast(C.c_void_p(t.data_ptr()),  # noqa: E731
+                               C.POINTER(C.c_int32 if t.dtype == torch.int32 else C.c_float))
+        count, dropped = C.c_int64(), C.c_double()
+        assert lib.pmc_presolve_head(C.byref(cs), C.byref(mu), C.byref(params), n,
+                                     *(_lib.ptr(a, C.c_float) for a in ins), 2 * n, *map(ptr, outs),
+                                     C.byref(count), C.byref(dropped)) == 0
+        return count.value, dropped.value, [t.cpu().numpy() for t in outs]
+
+    host, dev = call(0), call(1)
+    del keep
+    assert host[:2] == dev[:2] and n < host[0] < 2 * n
+    for a, b in zip(host[2], dev[2]):
+        np.testing.assert_array_equal(a, b)
