@@ -273,7 +273,9 @@ typedef struct pmc_run_params {
                                before it is parked for the next round; 0: default,
                                < 0: never park */
     int32_t smem_tables;    /* 1: stage the photon and electron table rows in shared
-                               memory, -1: read them through L1, 0: auto */
+                               memory (through L1 where they leave no room for the
+                               blocks' random numbers, 12 KB), -1: read them through
+                               L1, 0: auto */
 } pmc_run_params;
 
 /* Exact integer energy books of a call, in quanta of 1e-9 MeV

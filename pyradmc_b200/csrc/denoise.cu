@@ -1052,7 +1052,7 @@ bool ws_plan_at(const ConvShape& s, int tz, int at_cg, WsConv& p, int& smem, int
     return true;
 }
 
-constexpr int kPlanSms = 148;
+constexpr int kPlanSms = 148;  // of a B200; the plans are also made where there is no GPU
 
 // Turn a tile plan into one of runs along d (conv3d_zs_kernel) where its terms hold:
 // the same channel groups, stages of two halo slices, up to four stages where they fit

@@ -322,8 +322,10 @@ conv3d_wgrad_umma_kernel(const __grid_constant__ CUtensorMap xmap,
 // A full tile's last halo slice would take a third one for the group that is
 // discarded; it takes the next buffer's first slice, once that is loaded (a third
 // slice of zeros would not fit beside 96 -> 32's deepest tiles).
-// Bound by the MMAs' operands in shared memory.  Before and after at 4 windows of 64^3:
-// 16 -> 16 0.47 -> 0.11 ms, 48 -> 16 0.57 -> 0.24, 8 -> 16 0.27 -> 0.14, 96 -> 32 at half
+// Bound by the MMAs' operands in shared memory, and where the layer is small by the bias
+// gradient's atomics (every block adds to the same sums: 8 -> 16 0.145 ms on random values,
+// 0.041 on zeros).  Before and after in a training step of 4 windows of 64^3: 16 -> 16
+// 0.47 -> 0.12 and 0.17 ms, 48 -> 16 0.57 -> 0.25, 8 -> 16 0.27 -> 0.14, 96 -> 32 at half
 // size 0.23 -> 0.11.  cout = 64 and 128 stay above: their three slices do not fit M.
 // Roles, waits and failure handling as above.
 __global__ void __launch_bounds__(kWgThreads, 1)

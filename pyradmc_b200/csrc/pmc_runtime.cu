@@ -484,12 +484,11 @@ constexpr double kWaveBytes = 8.0 * 1024 * 1024 * 1024;
 // particles it holds.  Batches are independent until they are folded, so a wave
 // of them shares the rounds, each scoring into a quanta map of its own, and the
 // fold adds the maps in batch order: the same numbers with the rounds of one
-// batch.  A wave holds up to four admission windows (16 primaries per resident
-// thread each); past that the last rounds no longer show.  Measured, ten batches:
-// a 16^3 run of 80,000 histories 6.25 -> 1.01 ms, a 64^3 field of 1e6 10.8 ->
-// 3.2 ms, a 35-column Dij of 1.4e6 9.5 -> 4.2 ms, the 100-column 128^3 Dij of
-// 1.9e7 (two waves) 39.4 -> 35.6 ms; admission windows of 8 and 4 primaries per
-// thread are slower there (37.6 and 41.8 ms).
+// batch.  A wave holds up to 64 primaries per resident thread; past that the last
+// rounds no longer show.  Measured when the window was 16 per thread, ten batches, before
+// and with waves: a 16^3 run of 80,000 histories 6.25 -> 1.01 ms, a 64^3 field of 1e6
+// 10.8 -> 3.2 ms, a 35-column Dij of 1.4e6 9.5 -> 4.2 ms, the 100-column 128^3 Dij of
+// 1.9e7 (two waves) 39.4 -> 35.6 ms.
 int prepare_transport(pmc_engine* e, const pmc_run_params* p, unsigned long long block, int cols, bool waves,
                       RunPlan* plan) {
     if (!e->has_grid) return fail(e, PMC_ERR_STATE, "no transport grid uploaded");
@@ -514,11 +513,11 @@ int prepare_transport(pmc_engine* e, const pmc_run_params* p, unsigned long long
         const int n_waves = (p->n_batches + most - 1) / most;
         plan->wave = (p->n_batches + n_waves - 1) / n_waves;  // waves of about the same size
     }
-    // admission never needs more than a wave's primaries per round
-    // and, unless the caller chose it, no more than a quarter above one batch's (or 8 per
-    // thread): the queues take 4 KB a primary, and a new engine's first call waits for
-    // their allocation (40 columns of 2.2e5 histories, 8 batches: 10 GB for a wave's
-    // window, 55 ms and more; 5.5 GB for this one)
+    // Admission: 16 primaries per thread, which the 100-column Dij's batches of 1.9e6 come near
+    // (8 and 4 per thread: 37.6 and 41.8 against 35.6 ms there, in the same runs as above),
+    // but never more than the wave's, and no more than a quarter above one batch's or 8 per
+    // thread where that is more: a primary takes 4 KB of queues, which a new engine's first
+    // call has to allocate (40 columns of 2.2e5 histories, 8 batches: 5.5 GB for 10)
     plan->budget = p->chunk_size > 0
                        ? (unsigned long long)p->chunk_size
                        : std::min(16ull * resident, std::max(block + block / 4, 8ull * resident));

@@ -1204,11 +1204,12 @@ __device__ __forceinline__ float rest_energy(const ParticleOf<R>& p) {
 
 // ---- the electron kernel -------------------------------------------------------------
 // What bounds both transport kernels: instruction issue with half the lanes
-// active, then the latency of the voxel and queue gathers, not HBM.  On the
-// 100-column 128^3 Dij (1.7e8 substeps, 7.8e7 flights) the draws from a ring in
-// shared memory, the plain scoring path and the terminal step folded into the
-// refill took the electron kernel from 17.5 to 12.4 ms and the photon kernel from
-// 13.6 to 12.1 ms.
+// active, then the latency of the voxel and queue gathers, not HBM.  On a
+// 100-column 128^3 Dij (1.9e7 histories, 1.7e8 substeps, 7.8e7 flights), electron and
+// photon kernel: 17.5 and 13.6 ms with a Philox block per lane in registers, one
+// scoring path and single queue slots; 12.4 and 12.1 with the ring in shared memory, the
+// plain scoring path and the terminal step folded into the refill; 10.5 and 5.3 with
+// chunked slots and claims; 9.7 and 4.9 with blocks of 384 and the round keys at hand.
 constexpr int kElectronThreads = 384;  // the largest block of the electron kernel
 
 // One lane runs one electron or positron to ECUT (Class II condensed history,

@@ -606,8 +606,9 @@ class B200Engine:
         the library default; a negative value never parks).  Bit-inert.
     smem_tables
         Stage the photon and electron table rows in each block's shared memory
-        (True), read them through L1 (False) or let the library decide (None).
-        Bit-inert: the same values either way.
+        (True; through L1 all the same where they leave no room there), read them
+        through L1 (False) or let the library decide (None).  Bit-inert: the
+        same values either way.
     """
 
     grid: object
